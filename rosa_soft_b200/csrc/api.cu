@@ -5,6 +5,7 @@
 #include <cstdlib>
 #include <limits>
 
+#include "chain_match.cuh"
 #include "common.cuh"
 
 namespace rosa {
@@ -32,7 +33,7 @@ size_t partial_budget_bytes() {
 
 struct FwdLayout {
   PlanLayout plan;
-  size_t best_off, qt_off, kt_off, masks_off;
+  size_t best_off, qt_off, kt_off, start_off, prev_off, low_off, masks_off;
   int64_t mask_words;
   size_t bytes;
 };
@@ -44,29 +45,34 @@ int64_t fwd_items_upper(int64_t N, int64_t S, int64_t uniform_len, bool dense) {
   return N / kFwdBand + S;
 }
 
+// The sizing function knows neither D nor the lengths: both matchers get the most they may need.
+// The bitmaps of the bit-parallel matcher (rows that the chained matcher gave up, H * 2^8 rows of
+// ceil(N / 32) + 1 words) are built after the chains have been walked and take their place.
 FwdLayout fwd_layout(int64_t N, int H, int64_t S, bool transposed_symbols) {
   FwdLayout l;
   l.plan = plan_layout(0, S);
+  const size_t word_rows = (size_t)N * H * sizeof(uint32_t);
   size_t off = l.plan.bytes;
   l.best_off = off;
   off = align_up(off + (size_t)N * H * sizeof(unsigned long long));
   l.qt_off = l.kt_off = 0;
   if (transposed_symbols) {
     l.qt_off = off;
-    off = align_up(off + (size_t)N * H * sizeof(int32_t));
+    off = align_up(off + word_rows);
     l.kt_off = off;
-    off = align_up(off + (size_t)N * H * sizeof(int32_t));
-    // bitmaps over the symbols hashed to 8 bits (prefilter of the wide-symbol matcher)
-    l.mask_words = (N + 31) / 32 + 1;
-    l.masks_off = off;
-    off = align_up(off + ((size_t)H << kMaskSymbolBits) * (size_t)l.mask_words * sizeof(uint32_t));
-  } else {
-    // occurrence bitmaps of the bit-parallel matcher, sized for the widest symbol it serves
-    // (the sizing function does not know D): H * 2^8 rows of ceil(N / 32) + 1 words
-    l.mask_words = (N + 31) / 32 + 1;
-    l.masks_off = off;
-    off = align_up(off + ((size_t)H << kMaskSymbolBits) * (size_t)l.mask_words * sizeof(uint32_t));
+    off = align_up(off + word_rows);
   }
+  l.mask_words = (N + 31) / 32 + 1;
+  l.masks_off = off;
+  l.start_off = off;
+  off = align_up(off + word_rows);
+  l.prev_off = off;
+  off = align_up(off + word_rows);
+  l.low_off = off;
+  off = align_up(off + word_rows);
+  if (!transposed_symbols)
+    off = std::max(off, align_up(l.masks_off + ((size_t)H << kMaskSymbolBits) *
+                                                   (size_t)l.mask_words * sizeof(uint32_t)));
   l.bytes = off;
   return l;
 }
@@ -203,6 +209,12 @@ ROSA_B200_API size_t rosa_b200_hard_forward_workspace_bytes(int64_t N, int H, in
 }
 
 namespace {
+void set_chain_scratch(FwdArgs& a, char* ws, const FwdLayout& l) {
+  a.chain_start = reinterpret_cast<uint32_t*>(ws + l.start_off);
+  a.chain_prev = reinterpret_cast<uint32_t*>(ws + l.prev_off);
+  a.chain_low = reinterpret_cast<uint32_t*>(ws + l.low_off);
+}
+
 // Shared driver of the two forward entry points.  `query` / `key` null: the packed symbols are
 // inputs (already produced by the caller, e.g. by the epilogue of its projection GEMM) and the
 // packing kernel is skipped.  `output_i8` non-null: the routed signs go out as int8.
@@ -238,23 +250,30 @@ int run_hard_forward(const void* query, const void* key, const void* value, int 
   a.best = reinterpret_cast<unsigned long long*>(ws + l.best_off);
   a.sym_seq_stride = dense ? (int64_t)H * uniform_len : 0;
   a.sym_head_stride = dense ? uniform_len : N;
-  // symbols of up to 8 bits index the bitmaps directly; wider ones go through the hashed
-  // prefilter (same 2^8 rows per head)
-  if (D <= kMaskSymbolBits)
-    a.match_masks = reinterpret_cast<uint32_t*>(ws + l.masks_off);
-  else
-    a.hash_masks = reinterpret_cast<uint32_t*>(ws + l.masks_off);
+  set_chain_scratch(a, ws, l);
+  a.match_masks = reinterpret_cast<uint32_t*>(ws + l.masks_off);
   a.mask_words = l.mask_words;
+  const int64_t max_len = dense ? uniform_len : N;
 
-  launch_build_plan(a.plan, st);
-  ROSA_CUDA_OK(cudaGetLastError());
-  ROSA_CUDA_OK(cudaMemsetAsync(a.best, 0, (size_t)N * H * sizeof(unsigned long long), st));
+  if (!dense) {   // a dense batch needs no tables: its sequences and items are arithmetic
+    launch_build_plan(a.plan, st);
+    ROSA_CUDA_OK(cudaGetLastError());
+  }
   if (query != nullptr)
     if (int rc = launch_pack_symbols(query, key, dtype, N, H, D, dense, uniform_len, packed_query,
                                      packed_key, st))
       return rc;
-  if (int rc = launch_hard_match(a, (int)items, st)) return rc;
-  return launch_gather_output(a, st);
+  if (int rc = launch_chain_index(a, max_len, st)) return rc;
+  const bool bits = D <= kMaskSymbolBits;
+  if (int rc = launch_chain_forward(a, bits ? kChainGaveUp : 0ull, st)) return rc;
+  // Rows on chains that are too long.  A chain cannot be longer than the sequence.
+  if (max_len <= kChainLimit) return 0;
+  const int32_t* flag = a.plan.status + 2;
+  if (bits) return launch_match_bits(a, flag, st);
+  // wide symbols: the run-length matcher merges the same winners into the rows that are resolved
+  // and the missing ones into the rest; then all results are written again
+  if (int rc = launch_run_length_match(a, (int)items, flag, st)) return rc;
+  return launch_gather_output(a, flag, st);
 }
 }  // namespace
 
@@ -346,18 +365,24 @@ ROSA_B200_API int rosa_b200_hard_inference(const uint32_t* query_symbols, const 
   a.best = reinterpret_cast<unsigned long long*>(ws + l.best_off);
   a.sym_seq_stride = dense ? uniform_len : 0;  // [H, N] with sequence s starting at s * T
   a.sym_head_stride = N;
-  a.hash_masks = reinterpret_cast<uint32_t*>(ws + l.masks_off);
-  a.mask_words = l.mask_words;
+  set_chain_scratch(a, ws, l);
+  const int64_t max_len = dense ? uniform_len : N;
 
-  launch_build_plan(a.plan, st);
-  ROSA_CUDA_OK(cudaGetLastError());
-  ROSA_CUDA_OK(cudaMemsetAsync(a.best, 0, (size_t)N * H * sizeof(unsigned long long), st));
+  if (!dense) {
+    launch_build_plan(a.plan, st);
+    ROSA_CUDA_OK(cudaGetLastError());
+  }
   if (int rc = launch_transpose_symbols(query_symbols, key_symbols, N, H, a.packed_q, a.packed_k,
                                         st))
     return rc;
-  if (int rc = launch_hard_match(a, (int)fwd_items_upper(N, num_seq, uniform_len, dense), st))
+  if (int rc = launch_chain_index(a, max_len, st)) return rc;
+  if (int rc = launch_chain_inference(a, payload, out, matched_end, st)) return rc;
+  if (max_len <= kChainLimit) return 0;
+  const int32_t* flag = a.plan.status + 2;
+  if (int rc = launch_run_length_match(a, (int)fwd_items_upper(N, num_seq, uniform_len, dense), flag,
+                                       st))
     return rc;
-  return launch_inference_finish(a.plan, a.best, payload, N, H, Hp, Dp, out, matched_end, st);
+  return launch_inference_finish(a.plan, a.best, payload, N, H, Hp, Dp, out, matched_end, flag, st);
 }
 
 ROSA_B200_API size_t rosa_b200_stream_workspace_bytes(int64_t chunk_tokens, int num_heads) {

@@ -109,29 +109,49 @@ __device__ __forceinline__ float load_as_float(const void* p, int64_t idx, int d
 }
 
 // Sequence containing `token`: returns its ordinal, or -1 when the plan is invalid or the
-// token lies outside every sequence.  Dense plans divide; packed plans bisect cu_seqlens.
+// token lies outside every sequence.  Dense batches need no plan tables: the ordinal is a division
+// and nothing is read.  Packed plans bisect the sequence starts.
 __device__ __forceinline__ int find_segment(const Plan& plan, int64_t token, int* start,
                                             int* len) {
-  if (plan.status[0] != 0) return -1;
-  int s;
   if (plan.cu_seqlens == nullptr) {
-    s = (int)(token / plan.uniform_len);
-  } else {
-    int lo = 0, hi = plan.S;  // largest s with seg_start[s] <= token and non-empty
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (plan.seg_start[mid] <= token) lo = mid; else hi = mid;
-    }
-    s = lo;
+    const int s = (int)((uint32_t)token / (uint32_t)plan.uniform_len);   // N * H fits in int32
+    *start = s * plan.uniform_len;
+    *len = plan.uniform_len;
+    return token < plan.N ? s : -1;
   }
-  *start = plan.seg_start[s];
-  *len = plan.seg_len[s];
+  if (plan.status[0] != 0) return -1;
+  int lo = 0, hi = plan.S;  // largest s with seg_start[s] <= token and non-empty
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (plan.seg_start[mid] <= token) lo = mid; else hi = mid;
+  }
+  *start = plan.seg_start[lo];
+  *len = plan.seg_len[lo];
   if (token < *start || token >= (int64_t)*start + *len) return -1;
-  return s;
+  return lo;
+}
+
+// First token and length of sequence `s`.
+__device__ __forceinline__ void segment_bounds(const Plan& plan, int s, int* start, int* len) {
+  const bool dense = plan.cu_seqlens == nullptr;
+  *start = dense ? s * plan.uniform_len : plan.seg_start[s];
+  *len = dense ? plan.uniform_len : plan.seg_len[s];
+}
+
+// Work items of every sequence of a dense batch.
+__host__ __device__ __forceinline__ int dense_items(const Plan& plan) {
+  return plan.uniform_len >= 2 ? (plan.uniform_len - 2 + plan.item_diagonals) / plan.item_diagonals : 0;
 }
 
 // Work item -> (sequence, item index inside the sequence); false when the slot is unused.
 __device__ __forceinline__ bool find_item(const Plan& plan, int slot, int* seq, int* local) {
+  if (plan.cu_seqlens == nullptr) {   // dense: the same number of items in every sequence
+    const int per = dense_items(plan);
+    if (per <= 0 || slot >= per * plan.S) return false;
+    *seq = slot / per;
+    *local = slot - *seq * per;
+    return true;
+  }
   const int total = plan.item_prefix[plan.S];
   if (slot >= total) return false;
   int lo = 0, hi = plan.S;  // largest s with item_prefix[s] <= slot
@@ -275,26 +295,36 @@ struct FwdArgs {
   int32_t* route_token;           // optional
   unsigned long long* best;       // [N*H] (match length << 32 | local route)
   int64_t sym_seq_stride, sym_head_stride;  // packed symbol addressing
+  // Scratch of the chained matcher, addressed like the packed symbols: latest candidate of every
+  // query position, predecessor of every key position, result of the shorter context lengths.
+  // chain_start null selects the run-length matcher alone (no workspace).
+  uint32_t *chain_start, *chain_prev, *chain_low;
   // Per-symbol occurrence bitmaps of the key symbols, [H][2^D][mask_words] over the packed
-  // token axis (bit g of row (h, s) set iff key symbol of token g, head h is s); null selects
-  // the run-length matcher.
+  // token axis (bit g of row (h, s) set iff key symbol of token g, head h is s), for the rows
+  // that the chained matcher gives up (D <= 8); they take the place of its scratch.
   uint32_t* match_masks;
   int64_t mask_words;
-  // Bitmaps over symbols hashed to 8 bits, [H][256][mask_words]: prefilter of the matcher for
-  // wide symbols (batched inference); null when not provided.
-  uint32_t* hash_masks;
 };
 
 int launch_pack_symbols(const void* q, const void* k, int dtype, int64_t N, int H, int D,
                         int dense, int64_t uniform_len, int32_t* packed_q, int32_t* packed_k,
                         cudaStream_t stream);
-int launch_hard_match(const FwdArgs& a, int items_upper, cudaStream_t stream);
-int launch_gather_output(const FwdArgs& a, cudaStream_t stream);
+// chained matcher (chain_match.cu): index, then match and results; a row that gives up raises
+// status[2] and leaves `gave_up_key` as its winner
+int launch_chain_index(const FwdArgs& a, int64_t max_len, cudaStream_t stream);
+int launch_chain_forward(const FwdArgs& a, unsigned long long gave_up_key, cudaStream_t stream);
+int launch_chain_inference(const FwdArgs& a, const float* payload, float* out, int64_t* matched_end,
+                           cudaStream_t stream);
+// matchers of the rows that gave up: they do nothing while *run_flag is zero
+int launch_match_bits(const FwdArgs& a, const int32_t* run_flag, cudaStream_t stream);
+int launch_run_length_match(const FwdArgs& a, int items_upper, const int32_t* run_flag,
+                            cudaStream_t stream);
+int launch_gather_output(const FwdArgs& a, const int32_t* run_flag, cudaStream_t stream);
 int launch_route_inspect(const unsigned long long* best, int64_t count, int32_t* route,
                          int32_t* length, cudaStream_t stream);
 int launch_inference_finish(const Plan& plan, const unsigned long long* best, const float* payload,
                             int64_t N, int H, int Hp, int Dp, float* out, int64_t* matched_end,
-                            cudaStream_t stream);
+                            const int32_t* run_flag, cudaStream_t stream);
 int launch_transpose_symbols(const uint32_t* q, const uint32_t* k, int64_t N, int H, int32_t* qt,
                              int32_t* kt, cudaStream_t stream);
 

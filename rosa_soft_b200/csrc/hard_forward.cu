@@ -4,14 +4,18 @@
 // merge_hard_route and hard_forward_kernel of the reference
 // (rosa_soft/csrc/cuda/rosa_soft_kernels.cu:202-241, 311-531).
 //
-// Matching uses the exact diagonal run-length recurrence
+// Rows are resolved by the chained matcher (chain_match.cu).  Here: packing, and the matchers whose
+// cost does not depend on the data, for the rows that it gives up and for the entry point without a
+// workspace.  Symbols of up to 8 bits: bitmaps of every symbol's occurrences (bit_match.cuh).  Any
+// width: the exact diagonal run-length recurrence
 //     len(i, a) = (q_i == k_{a-1}) ? min(len(i-1, a-1) + 1, W) : 0
-// instead of re-walking every suffix: one thread owns several diagonals, a warp sits
-// on one query row at a time, the per-row winner is reduced with redux.sync and merged
-// across bands with one 64-bit integer atomicMax (order independent, hence exact and
-// deterministic).
+// where one thread owns several diagonals, a warp sits on one query row at a time, the per-row
+// winner is reduced with redux.sync and merged across bands with one 64-bit integer atomicMax
+// (order independent, hence exact and deterministic).
 #include "common.cuh"
 #include "bit_match.cuh"
+#include "chain_match.cuh"
+#include "row_emit.cuh"
 
 namespace rosa {
 
@@ -110,8 +114,8 @@ __global__ void __launch_bounds__(kFwdWarps * 32)
   int seq, local;
   if (!find_item(plan, blockIdx.x, &seq, &local)) return;
   const int h = blockIdx.y;
-  const int start = plan.seg_start[seq];
-  const int len = plan.seg_len[seq];
+  int start, len;
+  segment_bounds(plan, seq, &start, &len);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int delta0 = 1 + local * kFwdBand + warp * (32 * kFwdPerLane);
   if (delta0 > len - 1) return;
@@ -204,8 +208,8 @@ __global__ void __launch_bounds__(kMatchThreads)
   int seq, local;
   if (!find_item(plan, slot, &seq, &local)) return;
   const int h = blockIdx.x - slot * H;
-  const int start = plan.seg_start[seq];
-  const int len = plan.seg_len[seq];
+  int start, len;
+  segment_bounds(plan, seq, &start, &len);
   const int tid = threadIdx.x, lane = tid & 31;
   const int dmin = 1 + local * kFwdBand, dmax = dmin + kFwdBand - 1;
   const bool dense = plan.cu_seqlens == nullptr;
@@ -248,167 +252,72 @@ __global__ void __launch_bounds__(kMatchThreads)
 // ------------------------------------------------- bit-parallel matcher (D <= 8)
 // The matcher itself is bit_match_row (bit_match.cuh).  Here: the occurrence bitmaps of the
 // key symbols over the packed token axis, [H][2^D][mask_words], and the kernel that gives one
-// warp to every (token, head) and writes the row winner without atomics.
+// warp to every row that the chained matcher gave up.
 
-// Occurrence bitmaps: one warp per 32 consecutive tokens of one head; the lanes that share a
-// symbol are found with match.any and the lowest of them stores the word.
+// Occurrence bitmaps: one warp per 32 consecutive tokens of one head writes the word column of
+// all symbols; the lanes that share a symbol are found with match.any and the lowest of them
+// stores the word.
 __global__ void build_match_masks_kernel(Plan plan, const int32_t* __restrict__ ksym, int64_t N,
                                          int H, int D, int64_t sym_seq_stride,
                                          int64_t sym_head_stride, uint32_t* __restrict__ masks,
-                                         int64_t mask_words) {
+                                         int64_t mask_words, const int32_t* __restrict__ run_flag) {
+  if (*run_flag == 0) return;
   const int lane = threadIdx.x & 31;
-  const int64_t warp_id = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t words = (N + 31) >> 5;
-  if (warp_id >= words * H) return;
-  const int h = (int)(warp_id / words);
-  const int64_t word = warp_id - (int64_t)h * words;
-  const int64_t g = word * 32 + lane;
-  // lanes past the end get distinct out-of-range symbols so that they match nobody
-  unsigned sym = 0x80000000u | (unsigned)lane;
-  if (g < N) {
-    int start = 0, len = 0;
-    const int seq = find_segment(plan, g, &start, &len);
-    if (seq >= 0) {
-      const bool dense = plan.cu_seqlens == nullptr;
-      const int64_t idx = (int64_t)seq * sym_seq_stride + (int64_t)h * sym_head_stride +
-                          (dense ? g - start : g);
-      sym = (unsigned)ksym[idx];
+  const int64_t words = (N + 31) >> 5, warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t warp_id = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; warp_id < words * H;
+       warp_id += warps) {
+    const int h = (int)(warp_id / words);
+    const int64_t word = warp_id - (int64_t)h * words;
+    const int64_t g = word * 32 + lane;
+    // lanes past the end get distinct out-of-range symbols so that they match nobody
+    unsigned sym = 0x80000000u | (unsigned)lane;
+    if (g < N) {
+      int start = 0, len = 0;
+      const int seq = find_segment(plan, g, &start, &len);
+      if (seq >= 0) {
+        const bool dense = plan.cu_seqlens == nullptr;
+        const int64_t idx = (int64_t)seq * sym_seq_stride + (int64_t)h * sym_head_stride +
+                            (dense ? g - start : g);
+        sym = (unsigned)ksym[idx];
+      }
     }
+    uint32_t* __restrict__ column = masks + ((int64_t)h << D) * mask_words + word;
+    for (int e = lane; e < 1 << D; e += 32) column[e * mask_words] = 0u;
+    const unsigned peers = __match_any_sync(0xffffffffu, sym);
+    __syncwarp();
+    if (sym < (1u << D) && lane == __ffs(peers) - 1) column[(int64_t)sym * mask_words] = peers;
   }
-  const unsigned peers = __match_any_sync(0xffffffffu, sym);
-  if (sym < (1u << D) && lane == __ffs(peers) - 1)
-    masks[(((int64_t)h << D) + sym) * mask_words + word] = peers;
 }
 
 constexpr int kBitsWarps = 8;
 
+template <typename Emit>
 __global__ void __launch_bounds__(kBitsWarps * 32)
     hard_match_bits_kernel(Plan plan, const int32_t* __restrict__ qsym,
                            const uint32_t* __restrict__ masks, int64_t N, int H, int D, int W,
                            int64_t mask_words, int64_t sym_seq_stride, int64_t sym_head_stride,
-                           unsigned long long* __restrict__ best) {
-  const int lane = threadIdx.x & 31;
-  const int64_t row = (int64_t)blockIdx.x * kBitsWarps + (threadIdx.x >> 5);
-  if (row >= N * H) return;
-  // head-major order: neighbouring warps work on neighbouring rows of one head's bitmaps
-  const int h = (int)(row / N);
-  const int64_t g = row - (int64_t)h * N;
-  unsigned long long* out = best + g * H + h;
-  int start = 0, len = 0;
-  const int seq = find_segment(plan, g, &start, &len);
-  const int i = (int)(g - start);
-  if (seq < 0 || i == 0) {
-    if (lane == 0) *out = 0ull;
-    return;
-  }
-  const bool dense = plan.cu_seqlens == nullptr;
-  const int32_t* __restrict__ q = qsym + (int64_t)seq * sym_seq_stride +
-                                  (int64_t)h * sym_head_stride + (dense ? 0 : start);
+                           const unsigned long long* __restrict__ best,
+                           const int32_t* __restrict__ run_flag, Emit emit) {
   __shared__ BitCandidate queues[kBitsWarps][kBitQueue];
-  const unsigned long long key = bit_match_row(q, masks + ((int64_t)h << D) * mask_words, mask_words,
-                                               start, i, W, lane, queues[threadIdx.x >> 5]);
-  if (lane == 0) *out = key;
-}
-
-// --------------------------------------- hashed prefilter for wide symbols (D > 8)
-// Symbols of up to 32 bits are hashed to 8 bits and the key stream is indexed by the same
-// occurrence bitmaps as above.  The level-1 word of a row then holds every true candidate plus
-// about 1/256 of the other positions; each set bit is verified against the real symbols and
-// extended backwards exactly.  Rows with more than kHashTrueLimit genuine candidates (periodic or
-// constant streams) would cost O(candidates x horizon): they raise a flag instead, and the
-// run-length matcher, whose cost does not depend on the data, then redoes the launch (its
-// atomicMax merges the same exact winners, so rows already resolved keep their value).
-constexpr int kHashTrueLimit = 48;
-
-__device__ __forceinline__ unsigned hash8(unsigned sym) { return (sym * 0x9E3779B1u) >> 24; }
-
-__global__ void build_hash_masks_kernel(Plan plan, const int32_t* __restrict__ ksym, int64_t N,
-                                        int H, int64_t sym_seq_stride, int64_t sym_head_stride,
-                                        uint32_t* __restrict__ masks, int64_t mask_words) {
+  if (*run_flag == 0) return;
   const int lane = threadIdx.x & 31;
-  const int64_t warp_id = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t words = (N + 31) >> 5;
-  if (warp_id >= words * H) return;
-  const int h = (int)(warp_id / words);
-  const int64_t word = warp_id - (int64_t)h * words;
-  const int64_t g = word * 32 + lane;
-  unsigned sym = 0x80000000u | (unsigned)lane;   // lanes past the end match nobody
-  if (g < N) {
+  // head-major order: neighbouring warps work on neighbouring rows of one head's bitmaps
+  for (int64_t row = (int64_t)blockIdx.x * kBitsWarps + (threadIdx.x >> 5); row < N * H;
+       row += (int64_t)gridDim.x * kBitsWarps) {
+    const int h = (int)(row / N);
+    const int64_t g = row - (int64_t)h * N;
+    if (best[g * H + h] != kChainGaveUp) continue;
     int start = 0, len = 0;
     const int seq = find_segment(plan, g, &start, &len);
-    if (seq >= 0) {
-      const bool dense = plan.cu_seqlens == nullptr;
-      sym = hash8((unsigned)ksym[(int64_t)seq * sym_seq_stride + (int64_t)h * sym_head_stride +
-                                 (dense ? g - start : g)]);
-    }
-  }
-  const unsigned peers = __match_any_sync(0xffffffffu, sym);
-  if (sym < 256u && lane == __ffs(peers) - 1)
-    masks[(((int64_t)h << 8) + sym) * mask_words + word] = peers;
-}
-
-__global__ void __launch_bounds__(kBitsWarps * 32)
-    hard_match_hashed_kernel(Plan plan, const int32_t* __restrict__ qsym,
-                             const int32_t* __restrict__ ksym, const uint32_t* __restrict__ masks,
-                             int64_t N, int H, int W, int64_t mask_words, int64_t sym_seq_stride,
-                             int64_t sym_head_stride, unsigned long long* __restrict__ best,
-                             int32_t* __restrict__ overflow_flag) {
-  const int lane = threadIdx.x & 31;
-  const int64_t row = (int64_t)blockIdx.x * kBitsWarps + (threadIdx.x >> 5);
-  if (row >= N * H) return;
-  const int h = (int)(row / N);
-  const int64_t g_row = row - (int64_t)h * N;
-  unsigned long long* out = best + g_row * H + h;
-  int start = 0, len = 0;
-  const int seq = find_segment(plan, g_row, &start, &len);
-  const int i = (int)(g_row - start);
-  if (seq < 0 || i == 0) {
-    if (lane == 0) *out = 0ull;
-    return;
-  }
-  const bool dense = plan.cu_seqlens == nullptr;
-  const int64_t base = (int64_t)seq * sym_seq_stride + (int64_t)h * sym_head_stride +
-                       (dense ? 0 : start);
-  const int32_t* __restrict__ q = qsym + base;       // q[p], k[p]: position p of this sequence
-  const int32_t* __restrict__ k = ksym + base;
-  const int q_i = q[i];
-  const uint32_t* __restrict__ e = masks + (((int64_t)h << 8) + hash8((unsigned)q_i)) * mask_words;
-  const int g_lo = start, g_hi = start + i - 1;
-  const int w_lo = g_lo >> 5, w_hi = g_hi >> 5;
-  int best_len = 0, best_route = 0, genuine = 0;
-  bool stop = false;                                  // uniform: set from votes only
-  for (int wb = w_hi; wb >= w_lo && !stop; wb -= 32) {    // newest positions first
-    const int w = wb - lane;
-    uint32_t bits = w >= w_lo ? e[w] : 0u;
-    if (w == w_hi) bits &= 0xffffffffu >> (31 - (g_hi & 31));
-    if (w == w_lo) bits &= 0xffffffffu << (g_lo & 31);
-    // every lane walks the set bits of its own word, newest first (no warp primitive inside)
-    while (bits != 0u) {
-      const int bit = 31 - __clz(bits);
-      bits &= ~(1u << bit);
-      const int j = 32 * w + bit - start;             // key position inside the sequence
-      if (k[j] != q_i) continue;                      // hash collision
-      if (++genuine > kHashTrueLimit) break;          // bounded work per lane and row
-      int length = 1;
-      const int cap = min(W, j + 1);                  // a match cannot start before the sequence
-      while (length < cap && k[j - length] == q[i - length]) ++length;
-      if (length > best_len || (length == best_len && j + 1 > best_route)) {
-        best_len = length;
-        best_route = j + 1;
-      }
-    }
-    const bool over = __any_sync(0xffffffffu, genuine > kHashTrueLimit);
-    // newer positions were examined first: nothing older can beat a match at the horizon
-    stop = over || __reduce_max_sync(0xffffffffu, best_len) >= W;
-    if (over) best_len = 0;
-  }
-  const bool over = __any_sync(0xffffffffu, genuine > kHashTrueLimit);
-  const int row_len = over ? 0 : __reduce_max_sync(0xffffffffu, best_len);
-  const int row_route =
-      over ? 0 : __reduce_max_sync(0xffffffffu, best_len == row_len ? best_route : 0);
-  if (lane == 0) {
-    *out = row_len > 0 ? ((unsigned long long)(unsigned)row_len << 32) | (unsigned)row_route : 0ull;
-    if (over) atomicExch(overflow_flag, 1);
+    const int i = (int)(g - start);                  // a row that gave up has earlier positions
+    const bool dense = plan.cu_seqlens == nullptr;
+    const int32_t* __restrict__ q = qsym + (int64_t)seq * sym_seq_stride +
+                                    (int64_t)h * sym_head_stride + (dense ? 0 : start);
+    const unsigned long long key =
+        bit_match_row(q, masks + ((int64_t)h << D) * mask_words, mask_words, start, i, W, lane,
+                      queues[threadIdx.x >> 5]);
+    if (lane == 0) emit(g, h, H, start, (int)(key >> 32), (int)(key & 0xffffffffull));
+    __syncwarp();
   }
 }
 
@@ -421,7 +330,9 @@ template <typename T, typename OutT>
 __global__ void gather_output_kernel(Plan plan, const unsigned long long* __restrict__ best,
                                      const T* __restrict__ v, int64_t N, int H, int Hv, int Dv,
                                      int chunk, int vec, OutT* __restrict__ out,
-                                     int32_t* __restrict__ route_token) {
+                                     int32_t* __restrict__ route_token,
+                                     const int32_t* __restrict__ run_flag) {
+  if (run_flag != nullptr && *run_flag == 0) return;
   const int chunks = (Dv + chunk - 1) / chunk;
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= N * H * chunks) return;
@@ -464,7 +375,9 @@ __global__ void gather_output_kernel(Plan plan, const unsigned long long* __rest
 __global__ void inference_finish_kernel(Plan plan, const unsigned long long* __restrict__ best,
                                         const float* __restrict__ payload, int64_t N, int H,
                                         int Hp, int Dp, float* __restrict__ out,
-                                        int64_t* __restrict__ matched_end) {
+                                        int64_t* __restrict__ matched_end,
+                                        const int32_t* __restrict__ run_flag) {
+  if (*run_flag == 0) return;
   const int64_t th = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (th >= N * H) return;
   const int64_t token = th / H;
@@ -537,57 +450,27 @@ int launch_transpose_symbols(const uint32_t* q, const uint32_t* k, int64_t N, in
   return 0;
 }
 
-int launch_hard_match(const FwdArgs& a, int items_upper, cudaStream_t stream) {
-  if (a.match_masks != nullptr) {
-    if (a.N == 0) return 0;
-    {
-      ProfileScope prof("build_match_masks", stream);
-      ROSA_CUDA_OK(cudaMemsetAsync(a.match_masks, 0,
-                                   ((size_t)a.H << a.D) * (size_t)a.mask_words * sizeof(uint32_t),
-                                   stream));
-      const int64_t warps = ((a.N + 31) >> 5) * a.H;
-      build_match_masks_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, stream>>>(
-          a.plan, a.packed_k, a.N, a.H, a.D, a.sym_seq_stride, a.sym_head_stride, a.match_masks,
-          a.mask_words);
-      ROSA_CUDA_OK(cudaGetLastError());
-    }
-    ProfileScope prof("hard_match", stream);
-    const int64_t rows = a.N * a.H;
-    hard_match_bits_kernel<<<(unsigned)((rows + kBitsWarps - 1) / kBitsWarps), kBitsWarps * 32, 0,
-                             stream>>>(a.plan, a.packed_q, a.match_masks, a.N, a.H, a.D, a.W,
-                                       a.mask_words, a.sym_seq_stride, a.sym_head_stride, a.best);
+int launch_match_bits(const FwdArgs& a, const int32_t* run_flag, cudaStream_t stream) {
+  ProfileScope prof("hard_match_bits", stream);
+  // one grid that fills the GPU: it is launched whether or not a row gave up
+  const unsigned grid = 148 * 8;
+  build_match_masks_kernel<<<grid, 256, 0, stream>>>(a.plan, a.packed_k, a.N, a.H, a.D,
+                                                     a.sym_seq_stride, a.sym_head_stride,
+                                                     a.match_masks, a.mask_words, run_flag);
+  ROSA_CUDA_OK(cudaGetLastError());
+  return with_sign_emit(a, [&](auto emit) -> int {
+    hard_match_bits_kernel<<<grid, kBitsWarps * 32, 0, stream>>>(
+        a.plan, a.packed_q, a.match_masks, a.N, a.H, a.D, a.W, a.mask_words, a.sym_seq_stride,
+        a.sym_head_stride, a.best, run_flag, emit);
     ROSA_CUDA_OK(cudaGetLastError());
     return 0;
-  }
+  });
+}
+
+int launch_run_length_match(const FwdArgs& a, int items_upper, const int32_t* run_flag,
+                            cudaStream_t stream) {
   if (items_upper <= 0) return 0;
-  const int32_t* run_flag = nullptr;
-  if (a.hash_masks != nullptr && a.N > 0) {
-    // wide symbols: hashed prefilter first; the run-length matcher below then only runs when
-    // some row had too many genuine candidates (flag in the plan's status words)
-    int32_t* flag = a.plan.status + 2;
-    {
-      ProfileScope prof("build_match_masks", stream);
-      ROSA_CUDA_OK(cudaMemsetAsync(a.hash_masks, 0,
-                                   ((size_t)a.H << 8) * (size_t)a.mask_words * sizeof(uint32_t),
-                                   stream));
-      const int64_t warps = ((a.N + 31) >> 5) * a.H;
-      build_hash_masks_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, stream>>>(
-          a.plan, a.packed_k, a.N, a.H, a.sym_seq_stride, a.sym_head_stride, a.hash_masks,
-          a.mask_words);
-      ROSA_CUDA_OK(cudaGetLastError());
-    }
-    {
-      ProfileScope prof("hard_match_hashed", stream);
-      const int64_t rows = a.N * a.H;
-      hard_match_hashed_kernel<<<(unsigned)((rows + kBitsWarps - 1) / kBitsWarps), kBitsWarps * 32,
-                                 0, stream>>>(a.plan, a.packed_q, a.packed_k, a.hash_masks, a.N, a.H,
-                                              a.W, a.mask_words, a.sym_seq_stride,
-                                              a.sym_head_stride, a.best, flag);
-      ROSA_CUDA_OK(cudaGetLastError());
-    }
-    run_flag = flag;
-  }
-  ProfileScope prof("hard_match", stream);
+  ProfileScope prof("hard_match_runs", stream);
   const int64_t max_len = a.plan.cu_seqlens == nullptr ? a.plan.uniform_len : a.N;
   if (a.W < 2048 && max_len < (1 << 21)) {
     // 32-bit candidate keys: run length in the top 11 bits, route in the low 21
@@ -607,7 +490,7 @@ int launch_hard_match(const FwdArgs& a, int items_upper, cudaStream_t stream) {
 
 namespace {
 template <typename T, typename OutT>
-int launch_gather_t(const FwdArgs& a, OutT* out, cudaStream_t stream) {
+int launch_gather_t(const FwdArgs& a, OutT* out, const int32_t* run_flag, cudaStream_t stream) {
   // vector path: a thread writes 16 bytes of output, i.e. 16 / sizeof(OutT) components, and
   // reads as many value components in 16-byte words
   constexpr int kOutPer = 16 / (int)sizeof(OutT);
@@ -619,32 +502,33 @@ int launch_gather_t(const FwdArgs& a, OutT* out, cudaStream_t stream) {
   const int threads = 256;
   const int64_t blocks = (a.N * a.H * chunks + threads - 1) / threads;
   gather_output_kernel<T, OutT><<<(unsigned)blocks, threads, 0, stream>>>(
-      a.plan, a.best, (const T*)a.v, a.N, a.H, a.Hv, a.Dv, chunk, vec ? 1 : 0, out, a.route_token);
+      a.plan, a.best, (const T*)a.v, a.N, a.H, a.Hv, a.Dv, chunk, vec ? 1 : 0, out, a.route_token,
+      run_flag);
   ROSA_CUDA_OK(cudaGetLastError());
   return 0;
 }
 }  // namespace
 
-int launch_gather_output(const FwdArgs& a, cudaStream_t stream) {
+int launch_gather_output(const FwdArgs& a, const int32_t* run_flag, cudaStream_t stream) {
   ProfileScope prof("gather_output", stream);
   if (a.out_i8 != nullptr) {
-    if (a.dtype == ROSA_B200_F32) return launch_gather_t<float, int8_t>(a, a.out_i8, stream);
-    if (a.dtype == ROSA_B200_F16) return launch_gather_t<__half, int8_t>(a, a.out_i8, stream);
-    return launch_gather_t<__nv_bfloat16, int8_t>(a, a.out_i8, stream);
+    if (a.dtype == ROSA_B200_F32) return launch_gather_t<float, int8_t>(a, a.out_i8, run_flag, stream);
+    if (a.dtype == ROSA_B200_F16) return launch_gather_t<__half, int8_t>(a, a.out_i8, run_flag, stream);
+    return launch_gather_t<__nv_bfloat16, int8_t>(a, a.out_i8, run_flag, stream);
   }
-  if (a.dtype == ROSA_B200_F32) return launch_gather_t<float, float>(a, (float*)a.out, stream);
-  if (a.dtype == ROSA_B200_F16) return launch_gather_t<__half, __half>(a, (__half*)a.out, stream);
-  return launch_gather_t<__nv_bfloat16, __nv_bfloat16>(a, (__nv_bfloat16*)a.out, stream);
+  if (a.dtype == ROSA_B200_F32) return launch_gather_t<float, float>(a, (float*)a.out, run_flag, stream);
+  if (a.dtype == ROSA_B200_F16) return launch_gather_t<__half, __half>(a, (__half*)a.out, run_flag, stream);
+  return launch_gather_t<__nv_bfloat16, __nv_bfloat16>(a, (__nv_bfloat16*)a.out, run_flag, stream);
 }
 
 int launch_inference_finish(const Plan& plan, const unsigned long long* best, const float* payload,
                             int64_t N, int H, int Hp, int Dp, float* out, int64_t* matched_end,
-                            cudaStream_t stream) {
+                            const int32_t* run_flag, cudaStream_t stream) {
   ProfileScope prof("inference_finish", stream);
   const int threads = 256;
   const int64_t blocks = (N * H + threads - 1) / threads;
   inference_finish_kernel<<<(unsigned)blocks, threads, 0, stream>>>(plan, best, payload, N, H, Hp,
-                                                                   Dp, out, matched_end);
+                                                                   Dp, out, matched_end, run_flag);
   ROSA_CUDA_OK(cudaGetLastError());
   return 0;
 }
