@@ -40,11 +40,6 @@ struct FwdLayout {
 
 constexpr int kMaskSymbolBits = 8;   // widest symbol served by the bit-parallel matcher
 
-int64_t fwd_items_upper(int64_t N, int64_t S, int64_t uniform_len, bool dense) {
-  if (dense) return S * (uniform_len >= 2 ? (uniform_len - 1 + kFwdBand - 1) / kFwdBand : 0);
-  return N / kFwdBand + S;
-}
-
 // The sizing function knows neither D nor the lengths: both matchers get the most they may need.
 // The bitmaps of the bit-parallel matcher (rows that the chained matcher gave up, H * 2^8 rows of
 // ceil(N / 32) + 1 words) are built after the chains have been walked and take their place.
@@ -209,7 +204,8 @@ ROSA_B200_API size_t rosa_b200_hard_forward_workspace_bytes(int64_t N, int H, in
 }
 
 namespace {
-void set_chain_scratch(FwdArgs& a, char* ws, const FwdLayout& l) {
+void set_chain_scratch(FwdArgs& a, char* ws, const FwdLayout& l, int64_t max_len) {
+  a.context = chain_context(a.D, a.W, max_len);
   a.chain_start = reinterpret_cast<uint32_t*>(ws + l.start_off);
   a.chain_prev = reinterpret_cast<uint32_t*>(ws + l.prev_off);
   a.chain_low = reinterpret_cast<uint32_t*>(ws + l.low_off);
@@ -233,9 +229,8 @@ int run_hard_forward(const void* query, const void* key, const void* value, int 
   const FwdLayout l = fwd_layout(N, H, num_seq, false);
   ROSA_REQUIRE(workspace_bytes >= l.bytes, "workspace too small: need %zu bytes, got %zu", l.bytes,
                workspace_bytes);
-  const int64_t items = fwd_items_upper(N, num_seq, uniform_len, dense);
-  ROSA_REQUIRE(items * (int64_t)H <= std::numeric_limits<int32_t>::max(),
-               "too many work items: items * heads exceeds the CUDA grid limit");
+  ROSA_REQUIRE(num_seq * (int64_t)H <= std::numeric_limits<int32_t>::max(),
+               "num_seq * heads exceeds the CUDA grid limit");
   cudaStream_t st = as_stream(stream);
   char* ws = static_cast<char*>(workspace);
 
@@ -250,10 +245,10 @@ int run_hard_forward(const void* query, const void* key, const void* value, int 
   a.best = reinterpret_cast<unsigned long long*>(ws + l.best_off);
   a.sym_seq_stride = dense ? (int64_t)H * uniform_len : 0;
   a.sym_head_stride = dense ? uniform_len : N;
-  set_chain_scratch(a, ws, l);
+  const int64_t max_len = dense ? uniform_len : N;
+  set_chain_scratch(a, ws, l, max_len);
   a.match_masks = reinterpret_cast<uint32_t*>(ws + l.masks_off);
   a.mask_words = l.mask_words;
-  const int64_t max_len = dense ? uniform_len : N;
 
   if (!dense) {   // a dense batch needs no tables: its sequences and items are arithmetic
     launch_build_plan(a.plan, st);
@@ -265,15 +260,11 @@ int run_hard_forward(const void* query, const void* key, const void* value, int 
       return rc;
   if (int rc = launch_chain_index(a, max_len, st)) return rc;
   const bool bits = D <= kMaskSymbolBits;
-  if (int rc = launch_chain_forward(a, bits ? kChainGaveUp : 0ull, st)) return rc;
-  // Rows on chains that are too long.  A chain cannot be longer than the sequence.
-  if (max_len <= kChainLimit) return 0;
-  const int32_t* flag = a.plan.status + 2;
-  if (bits) return launch_match_bits(a, flag, st);
-  // wide symbols: the run-length matcher merges the same winners into the rows that are resolved
-  // and the missing ones into the rest; then all results are written again
-  if (int rc = launch_run_length_match(a, (int)items, flag, st)) return rc;
-  return launch_gather_output(a, flag, st);
+  const int limit = bits ? kChainLimitBits : kChainLimitScan;
+  if (int rc = launch_chain_forward(a, limit, st)) return rc;
+  if (max_len <= limit) return 0;              // no chain is longer than its sequence
+  return bits ? launch_match_bits(a, a.plan.status + 2, st)
+              : launch_scan_forward(a, a.plan.status + 2, st);
 }
 }  // namespace
 
@@ -351,6 +342,8 @@ ROSA_B200_API int rosa_b200_hard_inference(const uint32_t* query_symbols, const 
   const FwdLayout l = fwd_layout(N, H, num_seq, true);
   ROSA_REQUIRE(workspace_bytes >= l.bytes, "workspace too small: need %zu bytes, got %zu", l.bytes,
                workspace_bytes);
+  ROSA_REQUIRE(num_seq * (int64_t)H <= std::numeric_limits<int32_t>::max(),
+               "num_seq * heads exceeds the CUDA grid limit");
   cudaStream_t st = as_stream(stream);
   char* ws = static_cast<char*>(workspace);
 
@@ -365,8 +358,8 @@ ROSA_B200_API int rosa_b200_hard_inference(const uint32_t* query_symbols, const 
   a.best = reinterpret_cast<unsigned long long*>(ws + l.best_off);
   a.sym_seq_stride = dense ? uniform_len : 0;  // [H, N] with sequence s starting at s * T
   a.sym_head_stride = N;
-  set_chain_scratch(a, ws, l);
   const int64_t max_len = dense ? uniform_len : N;
+  set_chain_scratch(a, ws, l, max_len);
 
   if (!dense) {
     launch_build_plan(a.plan, st);
@@ -376,13 +369,9 @@ ROSA_B200_API int rosa_b200_hard_inference(const uint32_t* query_symbols, const 
                                         st))
     return rc;
   if (int rc = launch_chain_index(a, max_len, st)) return rc;
-  if (int rc = launch_chain_inference(a, payload, out, matched_end, st)) return rc;
-  if (max_len <= kChainLimit) return 0;
-  const int32_t* flag = a.plan.status + 2;
-  if (int rc = launch_run_length_match(a, (int)fwd_items_upper(N, num_seq, uniform_len, dense), flag,
-                                       st))
-    return rc;
-  return launch_inference_finish(a.plan, a.best, payload, N, H, Hp, Dp, out, matched_end, flag, st);
+  if (int rc = launch_chain_inference(a, payload, out, matched_end, kChainLimitScan, st)) return rc;
+  if (max_len <= kChainLimitScan) return 0;
+  return launch_scan_inference(a, payload, out, matched_end, a.plan.status + 2, st);
 }
 
 ROSA_B200_API size_t rosa_b200_stream_workspace_bytes(int64_t chunk_tokens, int num_heads) {

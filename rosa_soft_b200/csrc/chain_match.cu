@@ -10,19 +10,24 @@ namespace rosa {
 namespace {
 
 // One CTA per (sequence, head), one warp per context length.  A warp takes 16 positions at a
-// time: lanes 0..15 hold the key contexts that end there, lanes 16..31 the query contexts.  One
-// match.any finds the lanes of equal bucket; a lane's predecessor is the nearest lower key lane
-// of its bucket, or, without one, the table entry that earlier steps left.  Only the newest key
-// lane of a bucket writes the table, after all lanes have read it, so the links are those of a
-// strictly sequential pass.  What bounds it is the latency of a step (a table read, the vote and
-// a table write, about 150 cycles) times len / 16; the context words of the next four steps are
-// requested before the current ones are processed, which keeps global latency out of that chain.
+// time: lanes 0..15 hold the key contexts that end there, lanes 16..31 the query contexts.  A table
+// entry is the last step in which a key context fell into the bucket and the mask of its lanes in
+// that step, so one read gives both the latest earlier position and the equal lanes of the step
+// itself.  A step reads the old entry, stores its own and reads back; key lanes whose bit was
+// overwritten by another lane of the same bucket then add it.  The links are those of a strictly
+// sequential pass.  What bounds it is the latency of that chain of three shared-memory accesses
+// times len / 16 (finding the equal lanes with match.any instead took 330-380 ns a step); the
+// symbols of the next eight steps are requested before the current ones are processed, which keeps
+// global latency out of it.  The results of a step are selected, not branched on: 128 ns a step
+// against 315 with branches (4096 tokens, 128 streams: 81 us before).
+template <typename Entry, bool kMerge>
 __global__ void chain_index_kernel(Plan plan, const int32_t* __restrict__ qsym,
                                    const int32_t* __restrict__ ksym, int64_t sym_seq_stride,
                                    int64_t sym_head_stride, int H, int bits, int context,
                                    int hash_bits, uint32_t* __restrict__ start,
                                    uint32_t* __restrict__ prev, uint32_t* __restrict__ low) {
-  extern __shared__ uint32_t tables[];
+  extern __shared__ unsigned long long table_words[];
+  Entry* tables = reinterpret_cast<Entry*>(table_words);
   if (plan.cu_seqlens == nullptr && blockIdx.x == 0 && threadIdx.x < 4) plan.status[threadIdx.x] = 0;
   const int seq = blockIdx.x / H, h = blockIdx.x - seq * H;
   int64_t base = (int64_t)seq * sym_seq_stride + (int64_t)h * sym_head_stride;
@@ -35,69 +40,82 @@ __global__ void chain_index_kernel(Plan plan, const int32_t* __restrict__ qsym,
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int L = context - warp;                    // warp 0: the chained length
   const int entries = (1 << hash_bits) + chain_low_entries(bits, context);
-  for (int e = threadIdx.x; e < entries; e += blockDim.x) tables[e] = 0u;
+  for (int e = threadIdx.x; e < entries; e += blockDim.x) tables[e] = 0;
   __syncthreads();
-  uint32_t* __restrict__ table = warp == 0 ? tables : tables + (1 << hash_bits) + chain_low_entries(bits, L);
+  Entry* table = warp == 0 ? tables : tables + (1 << hash_bits) + chain_low_entries(bits, L);
   const bool is_query = lane >= kChainStep;
   const int l = lane & (kChainStep - 1);
   const int32_t* __restrict__ sym = (is_query ? qsym : ksym) + base;
   const int context_bits = bits * L;
   const uint32_t context_mask = context_bits >= 32 ? 0xffffffffu : (1u << context_bits) - 1u;
   const int first_valid = is_query ? L : L - 1;    // a query at i needs a key context at j < i
-  // bucket of the context that ends at p from its newest two symbols; lanes without one get a
-  // value of their own that matches nobody
+  // bucket of the context that ends at p from its newest two symbols; ~0 where there is none
   auto bucket_of = [&](int p, int newest, int second) -> uint32_t {
-    if (p < first_valid || p >= len) return 0x80000000u | (unsigned)lane;
     uint32_t w = (uint32_t)newest;
     if (L > 1) w |= (uint32_t)second << bits;
-    for (int u = 2; u < L; ++u) w |= (uint32_t)__ldg(sym + p - u) << (bits * u);
+    if (kMerge)
+      for (int u = 2; u < L; ++u)
+        if (p >= first_valid && p < len) w |= (uint32_t)__ldg(sym + p - u) << (bits * u);
     w &= context_mask;
-    return warp == 0 ? chain_bucket(w, context_bits, hash_bits) : w;
+    if (warp == 0) w = chain_bucket(w, context_bits, hash_bits);
+    return p >= first_valid && p < len ? w : 0xffffffffu;
   };
   auto newest_at = [&](int p) { return p < len ? __ldg(sym + p) : 0; };
   auto second_at = [&](int p) { return L > 1 && p >= 1 && p < len ? __ldg(sym + p - 1) : 0; };
-  constexpr int kAhead = 4;
-  uint32_t bucket[kAhead];
+  // where this lane's links go: the chained length writes both kinds, a shorter one the queries'
+  uint32_t* dst = (warp > 0 ? low : is_query ? start : prev) + base;
+  const bool writes = warp == 0 || is_query;
+  const uint32_t tag = warp == 0 ? 0u : (uint32_t)L << 28;
+  uint32_t bucket[kChainAhead];
 #pragma unroll
-  for (int s = 0; s < kAhead; ++s) {
+  for (int s = 0; s < kChainAhead; ++s) {
     const int p = s * kChainStep + l;
     bucket[s] = bucket_of(p, newest_at(p), second_at(p));
   }
-  for (int p0 = 0; p0 < len; p0 += kAhead * kChainStep) {
-    int a[kAhead], b[kAhead];
+  const unsigned own_bit = 1u << l;
+  for (int p0 = 0; p0 < len; p0 += kChainAhead * kChainStep) {
+    int a[kChainAhead], b[kChainAhead];
 #pragma unroll
-    for (int s = 0; s < kAhead; ++s) {
-      const int p = p0 + (kAhead + s) * kChainStep + l;
+    for (int s = 0; s < kChainAhead; ++s) {
+      const int p = p0 + (kChainAhead + s) * kChainStep + l;
       a[s] = newest_at(p);
       b[s] = second_at(p);
     }
 #pragma unroll
-    for (int s = 0; s < kAhead; ++s) {
+    for (int s = 0; s < kChainAhead; ++s) {
       const int p = p0 + s * kChainStep + l;
-      const uint32_t own = bucket[s];
-      const bool valid = (int)own >= 0;
-      const unsigned keys = __match_any_sync(0xffffffffu, own) & 0xffffu;
-      const unsigned below = keys & ((1u << l) - 1u);
-      uint32_t link = 0u;                          // position + 1 of the predecessor
-      if (below != 0u) link = (uint32_t)(p - l + 32 - __clz(below));
-      else if (valid) link = table[own];
+      const bool valid = bucket[s] != 0xffffffffu;
+      const bool is_key = valid && !is_query;
+      Entry* slot = table + (valid ? bucket[s] : 0u);
+      const Entry step = (Entry)(p0 / kChainStep + s + 1) << 16;
+      const Entry old = *slot;
       __syncwarp();
-      if (!is_query && valid && (keys >> l) == 1u) table[own] = (uint32_t)p + 1u;
+      if (is_key) *slot = step | own_bit;
       __syncwarp();
-      if (p < len) {
-        if (warp == 0) {
-          (is_query ? start : prev)[base + p] = link;
-        } else if (is_query) {
-          // one shorter length: its warp owns the array; several: the longest that occurs wins
-          const uint32_t key = link != 0u ? ((uint32_t)L << 28) | link : 0u;
-          if (context == 2) low[base + p] = key;
-          else if (key != 0u) atomicMax(low + base + p, key);
+      Entry now = *slot;
+      if (__any_sync(0xffffffffu, is_key && ((unsigned)now & own_bit) == 0u)) {
+        if (is_key && ((unsigned)now & own_bit) == 0u) atomicOr(slot, (Entry)own_bit);
+        __syncwarp();
+        now = *slot;
+      }
+      // the newest key lane below this one, else the newest of the bucket's last step
+      const unsigned below = (now >> 16) == (step >> 16) ? (unsigned)now & (own_bit - 1u) : 0u;
+      const Entry from = below != 0u ? step | below : old;
+      // position + 1 of the predecessor: bit b of step n (from 1) is position 16 (n - 1) + b
+      uint32_t link = (uint32_t)(from >> 16) * kChainStep + 16u - (uint32_t)__clz((unsigned)from & 0xffffu);
+      link = from != 0 && valid ? link | tag : 0u;
+      if (writes && p < len) {
+        // one shorter length: its warp owns the array; several: the longest that occurs wins
+        if (kMerge && warp > 0) {
+          if (link != 0u) atomicMax(dst + p, link);
+        } else {
+          dst[p] = link;
         }
       }
     }
 #pragma unroll
-    for (int s = 0; s < kAhead; ++s)
-      bucket[s] = bucket_of(p0 + (kAhead + s) * kChainStep + l, a[s], b[s]);
+    for (int s = 0; s < kChainAhead; ++s)
+      bucket[s] = bucket_of(p0 + (kChainAhead + s) * kChainStep + l, a[s], b[s]);
   }
 }
 
@@ -114,7 +132,7 @@ __global__ void __launch_bounds__(kChainRows * kChainHeads)
                        int64_t sym_seq_stride, int64_t sym_head_stride, int64_t N, int H, int W,
                        int context, const uint32_t* __restrict__ start_link,
                        const uint32_t* __restrict__ prev, const uint32_t* __restrict__ low,
-                       int head_blocks, unsigned long long gave_up_key, int32_t* flag, Emit emit) {
+                       int head_blocks, int limit, int32_t* flag, Emit emit) {
   __shared__ uint2 s_win[kChainRows][kChainHeads + 1];   // (length, route)
   __shared__ int s_start[kChainRows];
   const int heads = blockDim.x / kChainRows;             // heads of this CTA
@@ -126,25 +144,24 @@ __global__ void __launch_bounds__(kChainRows * kChainHeads)
   const int64_t g = g0 + lane;
   int start = 0, len = 0, best_len = 0, best_route = 0;
   int seq = -1;
-  bool gave_up = false;
-  if (g < N) seq = find_segment(plan, g, &start, &len);
-  if (seq >= 0 && h < H) {
-    const int i = (int)(g - start);
-    const int64_t base = (int64_t)seq * sym_seq_stride + (int64_t)h * sym_head_stride +
-                         (plan.cu_seqlens == nullptr ? 0 : start);
-    const uint32_t first = start_link[base + i];
-    const uint32_t shorter = context > 1 ? low[base + i] : 0u;
-    chain_walk<int32_t>(qsym + base, ksym + base, prev + base, first, i, W, best_len, best_route,
-                        gave_up);
-    if (best_len < context && !gave_up) {
-      best_len = (int)(shorter >> 28);
-      best_route = (int)(shorter & 0x0fffffffu);
-    }
+  if (g < N && h < H) seq = find_segment(plan, g, &start, &len);
+  const int i = (int)(g - start);
+  int64_t base = 0;
+  uint32_t first = 0u, shorter = 0u;
+  if (seq >= 0) {
+    base = (int64_t)seq * sym_seq_stride + (int64_t)h * sym_head_stride +
+           (plan.cu_seqlens == nullptr ? 0 : start);
+    first = start_link[base + i];
+    if (context > 1) shorter = low[base + i];
   }
-  if (gave_up) {
-    best_len = (int)(gave_up_key >> 32);
-    best_route = (int)(gave_up_key & 0xffffffffull);
+  if (chain_walk<int32_t>(qsym + base, ksym + base, prev + base, first, seq, i, W, limit, lane,
+                          best_len, best_route)) {
+    best_len = (int)(kChainGaveUp >> 32);          // resolved by a matcher of whole warps
+    best_route = 0;
     *flag = 1;
+  } else if (best_len < context) {
+    best_len = (int)(shorter >> 28);
+    best_route = (int)(shorter & 0x0fffffffu);
   }
   s_win[lane][warp] = make_uint2((unsigned)best_len, (unsigned)best_route);
   if (warp == 0) s_start[lane] = start;
@@ -156,15 +173,70 @@ __global__ void __launch_bounds__(kChainRows * kChainHeads)
   }
 }
 
+// A warp resolves a row that gave up by a look at every earlier position, newest first, 32 at a
+// time: lanes whose position agrees with the row here and at the distance of the best length so far
+// extend it.  Cost per row: len / 32 coalesced reads, whatever the chains look like.
+constexpr int kScanWarps = 8;
+
 template <typename Emit>
-int launch_chain_match_t(const FwdArgs& a, unsigned long long gave_up_key, Emit emit,
-                         cudaStream_t stream) {
+__global__ void __launch_bounds__(kScanWarps * 32)
+    scan_match_kernel(Plan plan, const int32_t* __restrict__ qsym, const int32_t* __restrict__ ksym,
+                      int64_t sym_seq_stride, int64_t sym_head_stride, int64_t N, int H, int W,
+                      const int32_t* __restrict__ run_flag, Emit emit) {
+  if (*run_flag == 0) return;
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = (int64_t)gridDim.x * kScanWarps, count = N * H;
+  for (int64_t th0 = ((int64_t)blockIdx.x * kScanWarps + (threadIdx.x >> 5)) * 32; th0 < count;
+       th0 += warps * 32) {
+    const bool mine = th0 + lane < count && emit.pending(th0 + lane);
+    for (unsigned rows = __ballot_sync(0xffffffffu, mine); rows != 0u; rows &= rows - 1u) {
+      const int64_t th = th0 + __ffs(rows) - 1;
+      const int64_t g = th / H;
+      const int h = (int)(th - g * H);
+      int start = 0, len = 0;
+      const int seq = find_segment(plan, g, &start, &len);
+      const int i = (int)(g - start);
+      const int64_t base = (int64_t)seq * sym_seq_stride + (int64_t)h * sym_head_stride +
+                           (plan.cu_seqlens == nullptr ? 0 : start);
+      const int32_t* __restrict__ q = qsym + base;
+      const int32_t* __restrict__ k = ksym + base;
+      const int q_i = q[i];
+      int best_len = 0, best_route = 0;              // the same in every lane
+      for (int top = i - 1; top >= 0 && best_len < min(W, top + 1); top -= 32) {
+        const int j = top - lane;
+        int length = 0;
+        if (j >= best_len && k[j] == q_i && k[j - best_len] == q[i - best_len])
+          length = chain_extend<int32_t>(q, k, i, j, 1, min(W, j + 1));
+        const int longest = __reduce_max_sync(0xffffffffu, length);
+        if (longest > best_len) {
+          best_len = longest;
+          best_route = __reduce_max_sync(0xffffffffu, length == longest ? j + 1 : 0);
+        }
+      }
+      if (lane == 0) emit(g, h, H, start, best_len, best_route);
+    }
+  }
+}
+
+template <typename Emit>
+int launch_scan_match_t(const FwdArgs& a, const int32_t* run_flag, Emit emit, cudaStream_t stream) {
+  ProfileScope prof("hard_match_scan", stream);
+  // a grid that fills the GPU: it is launched whether or not a row gave up
+  scan_match_kernel<Emit><<<148 * 8, kScanWarps * 32, 0, stream>>>(
+      a.plan, a.packed_q, a.packed_k, a.sym_seq_stride, a.sym_head_stride, a.N, a.H, a.W,
+      run_flag, emit);
+  ROSA_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
+template <typename Emit>
+int launch_chain_match_t(const FwdArgs& a, int limit, Emit emit, cudaStream_t stream) {
   const int heads = a.H < kChainHeads ? a.H : kChainHeads;
   const int head_blocks = (a.H + heads - 1) / heads;
   const int64_t tiles = (a.N + kChainRows - 1) / kChainRows;
   chain_match_kernel<Emit><<<(unsigned)(tiles * head_blocks), kChainRows * heads, 0, stream>>>(
       a.plan, a.packed_q, a.packed_k, a.sym_seq_stride, a.sym_head_stride, a.N, a.H, a.W,
-      chain_context(a.D, a.W), a.chain_start, a.chain_prev, a.chain_low, head_blocks, gave_up_key,
+      a.context, a.chain_start, a.chain_prev, a.chain_low, head_blocks, limit,
       a.plan.status + 2, emit);
   ROSA_CUDA_OK(cudaGetLastError());
   return 0;
@@ -174,32 +246,45 @@ int launch_chain_match_t(const FwdArgs& a, unsigned long long gave_up_key, Emit 
 
 int launch_chain_index(const FwdArgs& a, int64_t max_len, cudaStream_t stream) {
   ProfileScope prof("chain_index", stream);
-  const int context = chain_context(a.D, a.W);
-  const int hash_bits = chain_hash_bits(a.D, context, max_len);
-  if (context > 2)   // several shorter lengths merge their results into zeroed words
+  const int hash_bits = chain_hash_bits(a.D, a.context, max_len);
+  if (a.context > 2)   // several shorter lengths merge their results into zeroed words
     ROSA_CUDA_OK(cudaMemsetAsync(a.chain_low, 0, (size_t)a.N * a.H * sizeof(uint32_t), stream));
-  const size_t smem = ((size_t)(1 << hash_bits) + chain_low_entries(a.D, context)) * sizeof(uint32_t);
-  chain_index_kernel<<<(unsigned)(a.plan.S * a.H), 32 * context, smem, stream>>>(
-      a.plan, a.packed_q, a.packed_k, a.sym_seq_stride, a.sym_head_stride, a.H, a.D, context,
+  const size_t entries = (size_t)(1 << hash_bits) + chain_low_entries(a.D, a.context);
+  const unsigned grid = (unsigned)(a.plan.S * a.H);
+  const bool merge = a.context > 2, wide = max_len > 65535 * kChainStep;   // step beyond 16 bits
+  const size_t bytes = entries * (wide ? sizeof(unsigned long long) : sizeof(uint32_t));
+  auto kernel = wide ? (merge ? chain_index_kernel<unsigned long long, true>
+                              : chain_index_kernel<unsigned long long, false>)
+                     : (merge ? chain_index_kernel<uint32_t, true> : chain_index_kernel<uint32_t, false>);
+  if (bytes > 48 * 1024)
+    ROSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  kernel<<<grid, 32 * a.context, bytes, stream>>>(
+      a.plan, a.packed_q, a.packed_k, a.sym_seq_stride, a.sym_head_stride, a.H, a.D, a.context,
       hash_bits, a.chain_start, a.chain_prev, a.chain_low);
   ROSA_CUDA_OK(cudaGetLastError());
   return 0;
 }
 
-int launch_chain_forward(const FwdArgs& a, unsigned long long gave_up_key, cudaStream_t stream) {
+int launch_chain_forward(const FwdArgs& a, int limit, cudaStream_t stream) {
   ProfileScope prof("hard_match", stream);
   return with_sign_emit(a, [&](auto emit) {
-    return launch_chain_match_t(a, gave_up_key, emit, stream);
+    return launch_chain_match_t(a, limit, emit, stream);
   });
 }
 
 int launch_chain_inference(const FwdArgs& a, const float* payload, float* out, int64_t* matched_end,
-                           cudaStream_t stream) {
+                           int limit, cudaStream_t stream) {
   ProfileScope prof("hard_match", stream);
-  const auto aligned = [](const void* p) { return ((uintptr_t)p & 15u) == 0; };
-  PayloadEmit emit{payload, out, matched_end, a.best, a.Hv, a.Dv,
-                   a.Dv % 4 == 0 && aligned(payload) && aligned(out)};
-  return launch_chain_match_t(a, 0ull, emit, stream);
+  return launch_chain_match_t(a, limit, make_payload_emit(a, payload, out, matched_end), stream);
+}
+
+int launch_scan_forward(const FwdArgs& a, const int32_t* run_flag, cudaStream_t stream) {
+  return with_sign_emit(a, [&](auto emit) { return launch_scan_match_t(a, run_flag, emit, stream); });
+}
+
+int launch_scan_inference(const FwdArgs& a, const float* payload, float* out, int64_t* matched_end,
+                          const int32_t* run_flag, cudaStream_t stream) {
+  return launch_scan_match_t(a, run_flag, make_payload_emit(a, payload, out, matched_end), stream);
 }
 
 }  // namespace rosa

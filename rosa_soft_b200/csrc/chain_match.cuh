@@ -21,14 +21,18 @@ namespace rosa {
 
 constexpr int kChainHashBits = 13;    // buckets of the chained contexts: at most 2^13
 constexpr int kChainStep = 16;        // positions a warp indexes at a time
-// A row gives up after this many chain members (streams of very few distinct symbols) and is
-// resolved by the matcher whose cost does not depend on the data.
-constexpr int kChainLimit = 256;
+constexpr int kChainAhead = 8;        // steps between the request of a symbol and its use
+// A row gives up after this many chain members (streams of few distinct symbols, or of passages
+// repeated very often) and is resolved by a whole warp.  Symbols of up to 8 bits have the
+// bit-parallel matcher for that, which is soon the cheaper way; wide ones a scan of all positions.
+constexpr int kChainLimitBits = 64;
+constexpr int kChainLimitScan = 256;
 // Winner that such a row leaves behind (a match length no real row has).
 constexpr unsigned long long kChainGaveUp = 0xffffffffull << 32;
 
-__host__ __device__ inline int chain_context(int bits, int64_t W) {
-  const int c = bits >= 12 ? 1 : (12 + bits - 1) / bits;
+// (The results of the shorter lengths carry a position in 28 bits.)
+inline int chain_context(int bits, int64_t W, int64_t max_len) {
+  const int c = bits >= 12 || max_len >= ((int64_t)1 << 28) ? 1 : (12 + bits - 1) / bits;
   return (int64_t)c < W ? c : (int)W;
 }
 
@@ -51,40 +55,75 @@ __host__ __device__ inline int chain_low_entries(int bits, int L) {
   return n;
 }
 
-// Walks the chain of one row.  `first` is the latest candidate + 1 (0: none), prev[j] the next
-// older candidate + 1.  Candidates come newest first, so only a strictly longer match replaces
-// the best one, and a candidate is worth extending only if it also agrees at the distance of the
-// best length so far.  Returns the length and the route (position + 1) of the latest among the
-// longest; `gave_up` is set when the chain was longer than kChainLimit.
+// Number of equal symbols ending at k[j] and q[i], at most `cap`, of which `length` are known.
+// Four at a time: the loads of a group do not wait for one another.
 template <typename Sym>
-__device__ __forceinline__ void chain_walk(const Sym* __restrict__ q, const Sym* __restrict__ k,
-                                           const uint32_t* __restrict__ prev, uint32_t first, int i,
-                                           int W, int& best_len, int& best_route, bool& gave_up) {
+__device__ __forceinline__ int chain_extend(const Sym* __restrict__ q, const Sym* __restrict__ k, int i,
+                                            int j, int length, int cap) {
+  while (length + 4 <= cap) {
+    const Sym* kp = k + (j - length);
+    const Sym* qp = q + (i - length);
+    const bool e0 = kp[0] == qp[0], e1 = kp[-1] == qp[-1], e2 = kp[-2] == qp[-2],
+               e3 = kp[-3] == qp[-3];
+    if (!(e0 && e1 && e2 && e3)) return length + (!e0 ? 0 : !e1 ? 1 : !e2 ? 2 : 3);
+    length += 4;
+  }
+  while (length < cap && k[j - length] == q[i - length]) ++length;
+  return length;
+}
+
+// Resolves the rows of a warp: 32 consecutive positions of one head, lane by lane (`row` is the
+// sequence of the lane's position, negative for none; q, k and prev start at it).  `first` is the
+// latest candidate + 1 (0: none), prev[j] the next older candidate + 1.
+//
+// Newest candidates first: neighbouring rows inside a repeated passage have neighbouring newest
+// candidates, i.e. they lie on one diagonal, where the match grows by one symbol per row.  Only the
+// first lane of such a run extends its candidate symbol by symbol, the others count from it.  Then
+// every lane walks the rest of its chain: candidates come newest first, so only a strictly longer
+// match replaces the best one, and a candidate is worth extending only if it also agrees at the
+// distance of the best length so far.  Returns the length and the route (position + 1) of the latest
+// among the longest; the result is true when the chain was longer than `limit`.  All lanes call.
+template <typename Sym>
+__device__ __forceinline__ bool chain_walk(const Sym* __restrict__ q, const Sym* __restrict__ k,
+                                           const uint32_t* __restrict__ prev, uint32_t first, int row,
+                                           int i, int W, int limit, int lane, int& best_len,
+                                           int& best_route) {
   best_len = 0;
   best_route = 0;
-  gave_up = false;
+  int j = (int)first - 1;
+  bool equal = false;
+  if (first != 0u) {
+    first = prev[j];
+    equal = k[j] == q[i];
+  }
+  const int diagonal = equal ? i - j : 0;          // positive for a match
+  const int up_diagonal = __shfl_up_sync(0xffffffffu, diagonal, 1);
+  const int up_row = __shfl_up_sync(0xffffffffu, row, 1);
+  const bool leads = lane == 0 || up_diagonal != diagonal || up_row != row;
+  if (equal && leads) best_len = chain_extend<Sym>(q, k, i, j, 1, min(W, j + 1));
+  const unsigned leaders = __ballot_sync(0xffffffffu, leads) & (0xffffffffu >> (31 - lane));
+  const int leader = 31 - __clz(leaders);          // lane 0 leads
+  const int counted = __shfl_sync(0xffffffffu, best_len, leader) + lane - leader;
+  if (equal) {
+    best_len = min(W, counted);
+    best_route = j + 1;
+  }
   int steps = 0;
-  Sym q_next = first != 0u ? q[i] : (Sym)0;        // the symbol at the distance of the best length
-  while (first != 0u) {
-    const int j = (int)first - 1;
+  while (first != 0u && best_len < W) {
+    j = (int)first - 1;
     const int cap = min(W, j + 1);                 // a match cannot start before the sequence
     if (cap <= best_len) break;                    // nor can that of any older candidate
     first = prev[j];
-    if (k[j - best_len] == q_next) {
-      int length = 0;
-      while (length < cap && k[j - length] == q[i - length]) ++length;
+    if (k[j - best_len] == q[i - best_len]) {      // best_len < cap <= j + 1 <= i
+      const int length = chain_extend<Sym>(q, k, i, j, 0, cap);
       if (length > best_len) {
         best_len = length;
         best_route = j + 1;
-        if (length >= W) break;
-        q_next = q[i - length];   // length < W, and length <= j < i: inside the sequence
       }
     }
-    if (++steps == kChainLimit && first != 0u) {
-      gave_up = true;
-      break;
-    }
+    if (++steps == limit) return first != 0u;
   }
+  return false;
 }
 
 }  // namespace rosa

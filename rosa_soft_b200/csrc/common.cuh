@@ -299,6 +299,7 @@ struct FwdArgs {
   // query position, predecessor of every key position, result of the shorter context lengths.
   // chain_start null selects the run-length matcher alone (no workspace).
   uint32_t *chain_start, *chain_prev, *chain_low;
+  int context;                    // chained context length
   // Per-symbol occurrence bitmaps of the key symbols, [H][2^D][mask_words] over the packed
   // token axis (bit g of row (h, s) set iff key symbol of token g, head h is s), for the rows
   // that the chained matcher gives up (D <= 8); they take the place of its scratch.
@@ -309,22 +310,22 @@ struct FwdArgs {
 int launch_pack_symbols(const void* q, const void* k, int dtype, int64_t N, int H, int D,
                         int dense, int64_t uniform_len, int32_t* packed_q, int32_t* packed_k,
                         cudaStream_t stream);
-// chained matcher (chain_match.cu): index, then match and results; a row that gives up raises
-// status[2] and leaves `gave_up_key` as its winner
+// chained matcher (chain_match.cu): index, then match and results; a row whose chain is longer than
+// `limit` raises status[2] and stays pending
 int launch_chain_index(const FwdArgs& a, int64_t max_len, cudaStream_t stream);
-int launch_chain_forward(const FwdArgs& a, unsigned long long gave_up_key, cudaStream_t stream);
+int launch_chain_forward(const FwdArgs& a, int limit, cudaStream_t stream);
 int launch_chain_inference(const FwdArgs& a, const float* payload, float* out, int64_t* matched_end,
-                           cudaStream_t stream);
-// matchers of the rows that gave up: they do nothing while *run_flag is zero
+                           int limit, cudaStream_t stream);
+// matchers of the pending rows: they do nothing while *run_flag is zero
 int launch_match_bits(const FwdArgs& a, const int32_t* run_flag, cudaStream_t stream);
-int launch_run_length_match(const FwdArgs& a, int items_upper, const int32_t* run_flag,
-                            cudaStream_t stream);
-int launch_gather_output(const FwdArgs& a, const int32_t* run_flag, cudaStream_t stream);
+int launch_scan_forward(const FwdArgs& a, const int32_t* run_flag, cudaStream_t stream);
+int launch_scan_inference(const FwdArgs& a, const float* payload, float* out, int64_t* matched_end,
+                          const int32_t* run_flag, cudaStream_t stream);
+// all rows of a call without a workspace
+int launch_run_length_match(const FwdArgs& a, int items_upper, cudaStream_t stream);
+int launch_gather_output(const FwdArgs& a, cudaStream_t stream);
 int launch_route_inspect(const unsigned long long* best, int64_t count, int32_t* route,
                          int32_t* length, cudaStream_t stream);
-int launch_inference_finish(const Plan& plan, const unsigned long long* best, const float* payload,
-                            int64_t N, int H, int Hp, int Dp, float* out, int64_t* matched_end,
-                            const int32_t* run_flag, cudaStream_t stream);
 int launch_transpose_symbols(const uint32_t* q, const uint32_t* k, int64_t N, int H, int32_t* qt,
                              int32_t* kt, cudaStream_t stream);
 

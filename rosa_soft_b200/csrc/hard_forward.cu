@@ -109,8 +109,7 @@ __global__ void __launch_bounds__(kFwdWarps * 32)
     hard_match_kernel(Plan plan, const int32_t* __restrict__ qsym,
                       const int32_t* __restrict__ ksym, int64_t sym_seq_stride,
                       int64_t sym_head_stride, int H, int W,
-                      unsigned long long* __restrict__ best, const int32_t* __restrict__ run_flag) {
-  if (run_flag != nullptr && *run_flag == 0) return;   // only needed when the prefilter gave up
+                      unsigned long long* __restrict__ best) {
   int seq, local;
   if (!find_item(plan, blockIdx.x, &seq, &local)) return;
   const int h = blockIdx.y;
@@ -198,9 +197,7 @@ __global__ void __launch_bounds__(kMatchThreads)
     hard_match_fast_kernel(Plan plan, const int32_t* __restrict__ qsym,
                            const int32_t* __restrict__ ksym, int64_t sym_seq_stride,
                            int64_t sym_head_stride, int H, int W,
-                           unsigned long long* __restrict__ best,
-                           const int32_t* __restrict__ run_flag) {
-  if (run_flag != nullptr && *run_flag == 0) return;   // only needed when the prefilter gave up
+                           unsigned long long* __restrict__ best) {
   __shared__ int s_k[kMatchWin];
   __shared__ int s_q[kMatchRows];
   __shared__ unsigned s_best[kMatchRows];
@@ -296,7 +293,6 @@ __global__ void __launch_bounds__(kBitsWarps * 32)
     hard_match_bits_kernel(Plan plan, const int32_t* __restrict__ qsym,
                            const uint32_t* __restrict__ masks, int64_t N, int H, int D, int W,
                            int64_t mask_words, int64_t sym_seq_stride, int64_t sym_head_stride,
-                           const unsigned long long* __restrict__ best,
                            const int32_t* __restrict__ run_flag, Emit emit) {
   __shared__ BitCandidate queues[kBitsWarps][kBitQueue];
   if (*run_flag == 0) return;
@@ -306,7 +302,7 @@ __global__ void __launch_bounds__(kBitsWarps * 32)
        row += (int64_t)gridDim.x * kBitsWarps) {
     const int h = (int)(row / N);
     const int64_t g = row - (int64_t)h * N;
-    if (best[g * H + h] != kChainGaveUp) continue;
+    if (!emit.pending(g * H + h)) continue;
     int start = 0, len = 0;
     const int seq = find_segment(plan, g, &start, &len);
     const int i = (int)(g - start);                  // a row that gave up has earlier positions
@@ -330,9 +326,7 @@ template <typename T, typename OutT>
 __global__ void gather_output_kernel(Plan plan, const unsigned long long* __restrict__ best,
                                      const T* __restrict__ v, int64_t N, int H, int Hv, int Dv,
                                      int chunk, int vec, OutT* __restrict__ out,
-                                     int32_t* __restrict__ route_token,
-                                     const int32_t* __restrict__ run_flag) {
-  if (run_flag != nullptr && *run_flag == 0) return;
+                                     int32_t* __restrict__ route_token) {
   const int chunks = (Dv + chunk - 1) / chunk;
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= N * H * chunks) return;
@@ -370,31 +364,6 @@ __global__ void gather_output_kernel(Plan plan, const unsigned long long* __rest
   }
   for (int d = d0; d < d1; ++d)
     o[d] = src == nullptr ? (OutT)0 : positive<T>(src[d]) ? (OutT)1.0f : (OutT)-1.0f;
-}
-
-__global__ void inference_finish_kernel(Plan plan, const unsigned long long* __restrict__ best,
-                                        const float* __restrict__ payload, int64_t N, int H,
-                                        int Hp, int Dp, float* __restrict__ out,
-                                        int64_t* __restrict__ matched_end,
-                                        const int32_t* __restrict__ run_flag) {
-  if (*run_flag == 0) return;
-  const int64_t th = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (th >= N * H) return;
-  const int64_t token = th / H;
-  const int h = (int)(th - token * H);
-  const int route = (int)(best[th] & 0xffffffffull);
-  int start = 0, len = 0;
-  const bool hit = route > 0 && find_segment(plan, token, &start, &len) >= 0;
-  matched_end[th] = hit ? (int64_t)route - 1 : -1;
-  if (out) {
-    float* o = out + th * Dp;
-    if (hit) {
-      const float* src = payload + (((int64_t)start + route) * Hp + h / (H / Hp)) * Dp;
-      for (int d = 0; d < Dp; ++d) o[d] = src[d];
-    } else {
-      for (int d = 0; d < Dp; ++d) o[d] = 0.0f;
-    }
-  }
 }
 
 // Splits the winners into the selected route (local index a, 0 = null) and its match length.
@@ -461,36 +430,34 @@ int launch_match_bits(const FwdArgs& a, const int32_t* run_flag, cudaStream_t st
   return with_sign_emit(a, [&](auto emit) -> int {
     hard_match_bits_kernel<<<grid, kBitsWarps * 32, 0, stream>>>(
         a.plan, a.packed_q, a.match_masks, a.N, a.H, a.D, a.W, a.mask_words, a.sym_seq_stride,
-        a.sym_head_stride, a.best, run_flag, emit);
+        a.sym_head_stride, run_flag, emit);
     ROSA_CUDA_OK(cudaGetLastError());
     return 0;
   });
 }
 
-int launch_run_length_match(const FwdArgs& a, int items_upper, const int32_t* run_flag,
-                            cudaStream_t stream) {
+int launch_run_length_match(const FwdArgs& a, int items_upper, cudaStream_t stream) {
   if (items_upper <= 0) return 0;
   ProfileScope prof("hard_match_runs", stream);
   const int64_t max_len = a.plan.cu_seqlens == nullptr ? a.plan.uniform_len : a.N;
   if (a.W < 2048 && max_len < (1 << 21)) {
     // 32-bit candidate keys: run length in the top 11 bits, route in the low 21
     hard_match_fast_kernel<<<(unsigned)((int64_t)items_upper * a.H), kMatchThreads, 0, stream>>>(
-        a.plan, a.packed_q, a.packed_k, a.sym_seq_stride, a.sym_head_stride, a.H, a.W, a.best,
-        run_flag);
+        a.plan, a.packed_q, a.packed_k, a.sym_seq_stride, a.sym_head_stride, a.H, a.W, a.best);
     ROSA_CUDA_OK(cudaGetLastError());
     return 0;
   }
   dim3 grid((unsigned)items_upper, (unsigned)a.H);
   hard_match_kernel<<<grid, kFwdWarps * 32, 0, stream>>>(a.plan, a.packed_q, a.packed_k,
                                                         a.sym_seq_stride, a.sym_head_stride, a.H,
-                                                        a.W, a.best, run_flag);
+                                                        a.W, a.best);
   ROSA_CUDA_OK(cudaGetLastError());
   return 0;
 }
 
 namespace {
 template <typename T, typename OutT>
-int launch_gather_t(const FwdArgs& a, OutT* out, const int32_t* run_flag, cudaStream_t stream) {
+int launch_gather_t(const FwdArgs& a, OutT* out, cudaStream_t stream) {
   // vector path: a thread writes 16 bytes of output, i.e. 16 / sizeof(OutT) components, and
   // reads as many value components in 16-byte words
   constexpr int kOutPer = 16 / (int)sizeof(OutT);
@@ -502,35 +469,22 @@ int launch_gather_t(const FwdArgs& a, OutT* out, const int32_t* run_flag, cudaSt
   const int threads = 256;
   const int64_t blocks = (a.N * a.H * chunks + threads - 1) / threads;
   gather_output_kernel<T, OutT><<<(unsigned)blocks, threads, 0, stream>>>(
-      a.plan, a.best, (const T*)a.v, a.N, a.H, a.Hv, a.Dv, chunk, vec ? 1 : 0, out, a.route_token,
-      run_flag);
+      a.plan, a.best, (const T*)a.v, a.N, a.H, a.Hv, a.Dv, chunk, vec ? 1 : 0, out, a.route_token);
   ROSA_CUDA_OK(cudaGetLastError());
   return 0;
 }
 }  // namespace
 
-int launch_gather_output(const FwdArgs& a, const int32_t* run_flag, cudaStream_t stream) {
+int launch_gather_output(const FwdArgs& a, cudaStream_t stream) {
   ProfileScope prof("gather_output", stream);
   if (a.out_i8 != nullptr) {
-    if (a.dtype == ROSA_B200_F32) return launch_gather_t<float, int8_t>(a, a.out_i8, run_flag, stream);
-    if (a.dtype == ROSA_B200_F16) return launch_gather_t<__half, int8_t>(a, a.out_i8, run_flag, stream);
-    return launch_gather_t<__nv_bfloat16, int8_t>(a, a.out_i8, run_flag, stream);
+    if (a.dtype == ROSA_B200_F32) return launch_gather_t<float, int8_t>(a, a.out_i8, stream);
+    if (a.dtype == ROSA_B200_F16) return launch_gather_t<__half, int8_t>(a, a.out_i8, stream);
+    return launch_gather_t<__nv_bfloat16, int8_t>(a, a.out_i8, stream);
   }
-  if (a.dtype == ROSA_B200_F32) return launch_gather_t<float, float>(a, (float*)a.out, run_flag, stream);
-  if (a.dtype == ROSA_B200_F16) return launch_gather_t<__half, __half>(a, (__half*)a.out, run_flag, stream);
-  return launch_gather_t<__nv_bfloat16, __nv_bfloat16>(a, (__nv_bfloat16*)a.out, run_flag, stream);
-}
-
-int launch_inference_finish(const Plan& plan, const unsigned long long* best, const float* payload,
-                            int64_t N, int H, int Hp, int Dp, float* out, int64_t* matched_end,
-                            const int32_t* run_flag, cudaStream_t stream) {
-  ProfileScope prof("inference_finish", stream);
-  const int threads = 256;
-  const int64_t blocks = (N * H + threads - 1) / threads;
-  inference_finish_kernel<<<(unsigned)blocks, threads, 0, stream>>>(plan, best, payload, N, H, Hp,
-                                                                   Dp, out, matched_end, run_flag);
-  ROSA_CUDA_OK(cudaGetLastError());
-  return 0;
+  if (a.dtype == ROSA_B200_F32) return launch_gather_t<float, float>(a, (float*)a.out, stream);
+  if (a.dtype == ROSA_B200_F16) return launch_gather_t<__half, __half>(a, (__half*)a.out, stream);
+  return launch_gather_t<__nv_bfloat16, __nv_bfloat16>(a, (__nv_bfloat16*)a.out, stream);
 }
 
 }  // namespace rosa

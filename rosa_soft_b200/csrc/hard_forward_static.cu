@@ -113,6 +113,6 @@ extern "C" ROSA_B200_API int rosa_b200_hard_forward_static(
   if (int rc = launch_pack_symbols(query, key, dtype, N, H, D, dense, uniform_len, packed_query,
                                    packed_key, st))
     return rc;
-  if (int rc = launch_run_length_match(a, (int)items, nullptr, st)) return rc;
-  return launch_gather_output(a, nullptr, st);
+  if (int rc = launch_run_length_match(a, (int)items, st)) return rc;
+  return launch_gather_output(a, st);
 }

@@ -2,6 +2,7 @@
 // the winning match length and route (0, 0: no match).
 #pragma once
 
+#include "chain_match.cuh"
 #include "common.cuh"
 
 namespace rosa {
@@ -17,7 +18,10 @@ struct SignEmit {
   OutT* out;
   int32_t* route_token;
   unsigned long long* best;
-  int Hv, Dv, vec;
+  int Hv, group, Dv, vec;
+
+  // a row that the chained matcher gave up (length -1) and nobody has resolved yet
+  __device__ __forceinline__ bool pending(int64_t th) const { return best[th] == kChainGaveUp; }
 
   __device__ __forceinline__ void operator()(int64_t g, int h, int H, int start, int length,
                                              int route) const {
@@ -25,7 +29,7 @@ struct SignEmit {
     const int64_t src_token = route > 0 ? (int64_t)start + route : -1;
     best[th] = ((unsigned long long)(unsigned)length << 32) | (unsigned)route;
     if (route_token != nullptr) route_token[th] = (int32_t)src_token;
-    const T* src = v + (src_token * Hv + h / (H / Hv)) * Dv;
+    const T* src = v + (src_token * Hv + (group == 1 ? h : h / group)) * Dv;
     OutT* o = out + th * Dv;
     if (vec) {
       // 16 bytes of output at a time from as many value components
@@ -54,22 +58,22 @@ struct SignEmit {
   }
 };
 
-// Payload row of the successor and the position of the match.
+// Payload row of the successor and the position of the match (-2: the row is pending).
 struct PayloadEmit {
   const float* payload;
   float* out;
   int64_t* matched_end;
-  unsigned long long* best;
-  int Hp, Dp, vec;
+  int Hp, group, Dp, vec;
+
+  __device__ __forceinline__ bool pending(int64_t th) const { return matched_end[th] == -2; }
 
   __device__ __forceinline__ void operator()(int64_t g, int h, int H, int start, int length,
                                              int route) const {
     const int64_t th = g * H + h;
-    best[th] = ((unsigned long long)(unsigned)length << 32) | (unsigned)route;
-    matched_end[th] = route > 0 ? (int64_t)route - 1 : -1;
+    matched_end[th] = length < 0 ? -2 : (int64_t)route - 1;
     if (out == nullptr) return;
     float* o = out + th * Dp;
-    const float* src = payload + (((int64_t)start + route) * Hp + h / (H / Hp)) * Dp;
+    const float* src = payload + (((int64_t)start + route) * Hp + (group == 1 ? h : h / group)) * Dp;
     if (vec) {
       for (int d = 0; d < Dp; d += 4)
         *reinterpret_cast<float4*>(o + d) = route > 0
@@ -80,12 +84,19 @@ struct PayloadEmit {
   }
 };
 
+inline PayloadEmit make_payload_emit(const FwdArgs& a, const float* payload, float* out,
+                                     int64_t* matched_end) {
+  const auto aligned = [](const void* p) { return ((uintptr_t)p & 15u) == 0; };
+  return {payload, out, matched_end, a.Hv, a.H / a.Hv, a.Dv,
+          a.Dv % 4 == 0 && aligned(payload) && aligned(out)};
+}
+
 // Calls f with the functor of the call's value type and output form.
 template <typename T, typename OutT>
 inline SignEmit<T, OutT> make_sign_emit(const FwdArgs& a, OutT* out) {
   constexpr int kOutPer = 16 / (int)sizeof(OutT);
   const auto aligned = [](const void* p) { return ((uintptr_t)p & 15u) == 0; };
-  return {(const T*)a.v, out, a.route_token, a.best, a.Hv, a.Dv,
+  return {(const T*)a.v, out, a.route_token, a.best, a.Hv, a.H / a.Hv, a.Dv,
           a.Dv % kOutPer == 0 && aligned(a.v) && aligned(out) && (a.Dv * (int)sizeof(T)) % 16 == 0 &&
               kOutPer >= 16 / (int)sizeof(T)};
 }
