@@ -214,6 +214,44 @@ ROSA_B200_API int rosa_b200_stream_update(
     int64_t capacity, int64_t max_length_after, uint8_t* output, int64_t* matched_key_end,
     void* workspace, size_t workspace_bytes, void* stream);
 
+/* The same update over occurrence chains: the state holds the symbol histories, one link per key
+ * position and a table per (slot, head) instead of bitmaps, and an update costs the same whatever
+ * the length of the history.  It also takes logits (packed on the way in: bit d set iff component d
+ * is positive) and gives the result as +-1 values (0 for no match), so that a generation step is one
+ * kernel.  The caller owns the state (capacity a multiple of 32, pointers 16-byte aligned):
+ *   query_history, key_history  uint8  [slots, num_heads, capacity]
+ *   payload_history             uint8  [slots, num_payload_heads, capacity]
+ *   chain_links                 uint32 [slots, num_heads, capacity]
+ *   tables                      rosa_b200_stream_table_bytes() per (slot, head)
+ *   lengths / lengths_after     int32  [slots], two arrays that change places after every update
+ * A fresh or reset runtime is `lengths` = 0 and `tables` = 0.  Element types: -1 packed uint8
+ * symbols, otherwise a rosa_b200_dtype (logits [.., bits] in, values [.., payload_bits] out).
+ * `chunk_offsets` (device) NULL: every slot gets `max_chunk` tokens; the caller vouches for offsets
+ * that start at 0, do not decrease and end at chunk_tokens, and for max_chunk, the longest chunk.
+ * chunk_tokens = -1 rebuilds chain_links and tables (zeroed by the caller) from the histories, for
+ * a state that was loaded or whose table size changed with its capacity. */
+typedef struct rosa_b200_stream_call {
+  const void *query, *key, *payload;
+  int input_type, output_type;
+  const int32_t* chunk_offsets;
+  int64_t chunk_tokens, max_chunk, max_length_after;
+  int slots, num_heads, num_payload_heads, qk_bits, payload_bits;
+  int64_t max_suffix_length, capacity;
+  uint8_t *query_history, *key_history, *payload_history;
+  uint32_t* chain_links;
+  void* tables;
+  const int32_t* lengths;
+  int32_t* lengths_after;
+  void* output;
+  int64_t* matched_key_end;
+} rosa_b200_stream_call;
+
+ROSA_B200_API size_t rosa_b200_stream_table_bytes(int qk_bits, int64_t max_suffix_length,
+                                                  int64_t capacity);
+ROSA_B200_API size_t rosa_b200_stream_chained_workspace_bytes(int64_t chunk_tokens, int num_heads);
+ROSA_B200_API int rosa_b200_stream_update_chained(const rosa_b200_stream_call* update, void* workspace,
+                                                  size_t workspace_bytes, void* stream);
+
 /* Per-kernel timing for benchmarks (no counterpart in the reference, which times whole
  * steps with CUDA events in benchmarks/rosa_soft.py:151-173).  While enabled, every kernel
  * launch made by this library is bracketed by a CUDA event pair on the launching stream.

@@ -20,7 +20,8 @@ CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "librosa_soft_b200.so")
 EXT = os.path.join(PKG, "_C.so")
 
-CUDA_SOURCES = ["plan.cu", "hard_forward.cu", "hard_forward_static.cu", "chain_match.cu", "surrogate_vjp.cu", "vjp_tiled.cu", "vjp_tiled_sweep2.cu", "stream_runtime.cu", "api.cu"]
+CUDA_SOURCES = ["plan.cu", "hard_forward.cu", "hard_forward_static.cu", "chain_match.cu", "stream_chain.cu", "surrogate_vjp.cu", "vjp_tiled.cu", "vjp_tiled_sweep2.cu", "stream_runtime.cu", "api.cu"]
+EXT_SOURCES = ["torch_binding.cpp", "stream_binding.cpp"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "--use_fast_math", "-Xcompiler", "-fPIC,-fvisibility=hidden", "--expt-relaxed-constexpr",
@@ -45,6 +46,7 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
     deps = [os.path.join(CSRC, f) for f in CUDA_SOURCES] + [
         os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "bit_match.cuh"),
         os.path.join(CSRC, "chain_match.cuh"), os.path.join(CSRC, "row_emit.cuh"),
+        os.path.join(CSRC, "chain_kernels.cuh"),
         os.path.join(CSRC, "tcgen05.cuh"), os.path.join(CSRC, "vjp_shared.cuh"), os.path.join(CSRC, "vjp_tiled.cuh"), os.path.join(CSRC, "vjp_tiled_sweep2_kernel.inl"),
         os.path.join(ROOT, "include", "rosa_soft_b200.h")]
     if not force and _newer(LIB, deps):
@@ -70,8 +72,8 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
 
 
 def build_extension(force: bool = False, verbose: bool = False) -> str:
-    src = os.path.join(CSRC, "torch_binding.cpp")
-    deps = [src, os.path.join(ROOT, "include", "rosa_soft_b200.h"), LIB]
+    sources = [os.path.join(CSRC, f) for f in EXT_SOURCES]
+    deps = [*sources, os.path.join(ROOT, "include", "rosa_soft_b200.h"), LIB]
     if not force and _newer(EXT, deps):
         return EXT
     import torch
@@ -80,17 +82,31 @@ def build_extension(force: bool = False, verbose: bool = False) -> str:
     torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
     cuda_home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
-    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-DROSA_WITH_CUDA",
-           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
-           "-I" + os.path.join(ROOT, "include")]
+    compile_flags = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-DROSA_WITH_CUDA",
+                     "-DTORCH_EXTENSION_NAME=_C",
+                     "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
+                     "-I" + os.path.join(ROOT, "include")]
     for inc in cpp_extension.include_paths():
-        cmd += ["-isystem", inc]
-    cmd += ["-isystem", os.path.join(cuda_home, "include"),
-            "-isystem", sysconfig.get_paths()["include"]]
-    cmd += [src, "-o", EXT, "-L" + PKG, "-l:librosa_soft_b200.so", "-Wl,-rpath,$ORIGIN",
-            "-L" + torch_lib, "-Wl,-rpath," + torch_lib,
-            "-ltorch", "-ltorch_cpu", "-lc10", "-ltorch_cuda", "-lc10_cuda"]
-    _run(cmd, verbose)
+        compile_flags += ["-isystem", inc]
+    compile_flags += ["-isystem", os.path.join(cuda_home, "include"),
+                      "-isystem", sysconfig.get_paths()["include"]]
+    objdir = os.path.join(PKG, "build")
+    os.makedirs(objdir, exist_ok=True)
+    objs, procs = [], []
+    for src in sources:
+        obj = os.path.join(objdir, os.path.basename(src).replace(".cpp", ".cpp.o"))
+        objs.append(obj)
+        cmd = [cxx, *compile_flags, "-c", src, "-o", obj]
+        if verbose:
+            print(" ".join(cmd), flush=True)
+        procs.append((src, subprocess.Popen(cmd)))
+    for src, p in procs:
+        if p.wait() != 0:
+            raise RuntimeError(f"{cxx} failed on {src}")
+    _run([cxx, "-shared", "-o", EXT, *objs, "-L" + PKG, "-l:librosa_soft_b200.so", "-Wl,-rpath,$ORIGIN",
+          "-L" + torch_lib, "-Wl,-rpath," + torch_lib, "-L" + os.path.join(cuda_home, "lib64"),
+          "-ltorch", "-ltorch_cpu", "-lc10", "-ltorch_cuda", "-lc10_cuda", "-ltorch_python",
+          "-lcudart"], verbose)
     return EXT
 
 

@@ -29,6 +29,9 @@ EXPORTED_SYMBOLS = (
     "rosa_b200_hard_inference",
     "rosa_b200_stream_workspace_bytes",
     "rosa_b200_stream_update",
+    "rosa_b200_stream_table_bytes",
+    "rosa_b200_stream_chained_workspace_bytes",
+    "rosa_b200_stream_update_chained",
     "rosa_b200_read_status",
     "rosa_b200_decode_status",
     "rosa_b200_profile_enable",
@@ -81,6 +84,12 @@ def load() -> ctypes.CDLL:
     lib.rosa_b200_stream_update.restype = i32
     lib.rosa_b200_stream_update.argtypes = [vp, vp, vp, vp, i64, i32, i32, i32, i32, i32, i64, vp,
                                             vp, vp, vp, i64, i64, vp, vp, vp, sz, vp]
+    lib.rosa_b200_stream_table_bytes.restype = sz
+    lib.rosa_b200_stream_table_bytes.argtypes = [i32, i64, i64]
+    lib.rosa_b200_stream_chained_workspace_bytes.restype = sz
+    lib.rosa_b200_stream_chained_workspace_bytes.argtypes = [i64, i32]
+    lib.rosa_b200_stream_update_chained.restype = i32
+    lib.rosa_b200_stream_update_chained.argtypes = [vp, vp, sz, vp]
     lib.rosa_b200_read_status.restype = i32
     lib.rosa_b200_read_status.argtypes = [vp, vp, ctypes.POINTER(i32)]
     lib.rosa_b200_decode_status.restype = i32

@@ -1,0 +1,257 @@
+// Kernels of the chained matcher (chain_match.cuh), over whole sequences (chain_match.cu) or over
+// the histories of the streaming runtime (stream_chain.cu).
+//
+// An Axis says where a row lives: locate(g) gives the sequence (or slot) of token g, its `start`
+// (what the result functor wants to know of the sequence) and the position i inside it; symbols()
+// the offset of position 0 of a head in the symbol and link arrays; links() the offset of the row in
+// the arrays that the index pass wrote for the query positions.
+#pragma once
+
+#include "chain_match.cuh"
+#include "common.cuh"
+
+namespace rosa {
+namespace {
+
+// Indexes positions [begin, end) of one head for context length L; all lanes of a warp call.
+//
+// A warp takes 16 positions at a time: lanes 0..15 hold the key contexts that end there, lanes
+// 16..31 the query contexts.  A table entry is the last step in which a key context fell into the
+// bucket and the mask of its lanes in that step, so one read gives both the latest earlier position
+// and the equal lanes of the step itself.  A step reads the old entry, stores its own and reads back;
+// key lanes whose bit was overwritten by another lane of the same bucket then add it.  The links are
+// those of a strictly sequential pass.  What bounds it is the latency of that chain of three
+// shared-memory accesses times the number of steps (finding the equal lanes with match.any instead
+// took 330-380 ns a step); the symbols of the next eight steps are requested before the current ones
+// are processed, which keeps global latency out of it.  The results of a step are selected, not
+// branched on: 128 ns a step against 315 with branches (4096 tokens, 128 streams: 81 us before).
+//
+// kResume: the table holds the entries of the positions below `begin`, the first step may hold some.
+// kMerge: a shorter length leaves the larger of its own result and the one that is there (the longest
+// length that occurs wins).  q, k, key_links and query_links are addressed by position; query_links
+// null: the keys alone are indexed.
+template <typename Entry, bool kMerge, bool kResume, typename Sym>
+__device__ __forceinline__ void chain_index_warp(const Sym* q, const Sym* k, int begin, int end, int L,
+                                                 int bits, bool chained, int hash_bits, Entry* table,
+                                                 uint32_t* key_links, uint32_t* query_links) {
+  const int lane = threadIdx.x & 31;
+  const bool is_query = lane >= kChainStep;
+  const int l = lane & (kChainStep - 1);
+  const Sym* sym = is_query ? q : k;
+  const int context_bits = bits * L;
+  const uint32_t context_mask = context_bits >= 32 ? 0xffffffffu : (1u << context_bits) - 1u;
+  // a query at i needs a key context at j < i
+  const int first_valid = max(begin, is_query ? L : L - 1);
+  // bucket of the context that ends at p from its newest two symbols; ~0 where there is none
+  auto bucket_of = [&](int p, int newest, int second) -> uint32_t {
+    uint32_t w = (uint32_t)newest;
+    if (L > 1) w |= (uint32_t)second << bits;
+    for (int u = 2; u < L; ++u)
+      if (p >= first_valid && p < end) w |= (uint32_t)sym[p - u] << (bits * u);
+    w &= context_mask;
+    if (chained) w = chain_bucket(w, context_bits, hash_bits);
+    return p >= first_valid && p < end ? w : 0xffffffffu;
+  };
+  auto newest_at = [&](int p) { return p < end ? (int)sym[p] : 0; };
+  auto second_at = [&](int p) { return L > 1 && p >= 1 && p < end ? (int)sym[p - 1] : 0; };
+  uint32_t* dst = is_query ? query_links : key_links;
+  const bool writes = (chained || is_query) && dst != nullptr;
+  const uint32_t tag = chained ? 0u : (uint32_t)L << 28;
+  const int base = kResume ? begin / kChainStep * kChainStep : 0;
+  uint32_t bucket[kChainAhead];
+#pragma unroll
+  for (int s = 0; s < kChainAhead; ++s) {
+    const int p = base + s * kChainStep + l;
+    bucket[s] = bucket_of(p, newest_at(p), second_at(p));
+  }
+  const unsigned own_bit = 1u << l;
+  for (int p0 = base; p0 < end; p0 += kChainAhead * kChainStep) {
+    int a[kChainAhead], b[kChainAhead];
+#pragma unroll
+    for (int s = 0; s < kChainAhead; ++s) {
+      const int p = p0 + (kChainAhead + s) * kChainStep + l;
+      a[s] = newest_at(p);
+      b[s] = second_at(p);
+    }
+#pragma unroll
+    for (int s = 0; s < kChainAhead; ++s) {
+      if (s > 0 && p0 + s * kChainStep >= end) break;
+      const int p = p0 + s * kChainStep + l;
+      const bool valid = bucket[s] != 0xffffffffu;
+      const bool is_key = valid && !is_query;
+      Entry* slot = table + (valid ? bucket[s] : 0u);
+      const Entry step = (Entry)(p0 / kChainStep + s + 1) << 16;
+      const Entry old = *slot;
+      __syncwarp();
+      if (is_key) *slot = (kResume && (old >> 16) == (step >> 16) ? old : step) | own_bit;
+      __syncwarp();
+      Entry now = *slot;
+      if (__any_sync(0xffffffffu, is_key && ((unsigned)now & own_bit) == 0u)) {
+        if (is_key && ((unsigned)now & own_bit) == 0u) atomicOr(slot, (Entry)own_bit);
+        __syncwarp();
+        now = *slot;
+      }
+      // the newest key lane below this one, else the newest of the bucket's last step
+      const unsigned below = (now >> 16) == (step >> 16) ? (unsigned)now & (own_bit - 1u) : 0u;
+      // (an old entry of this very step holds positions before `begin`: they are in `below`)
+      const Entry from = below != 0u ? step | below : old;
+      // position + 1 of the predecessor: bit b of step n (from 1) is position 16 (n - 1) + b
+      uint32_t link = (uint32_t)(from >> 16) * kChainStep + 16u - (uint32_t)__clz((unsigned)from & 0xffffu);
+      link = from != 0 && valid ? link | tag : 0u;
+      if (writes && p >= begin && p < end) {
+        if (kMerge && !chained) {
+          if (link != 0u) atomicMax(dst + p, link);
+        } else {
+          dst[p] = link;
+        }
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < kChainAhead; ++s)
+      bucket[s] = bucket_of(p0 + (kChainAhead + s) * kChainStep + l, a[s], b[s]);
+  }
+}
+
+// Rows of whole sequences over packed symbols ([sequence][head][position] or [head][token]).
+struct SequenceAxis {
+  Plan plan;
+  int64_t seq_stride, head_stride;
+
+  __device__ __forceinline__ int locate(int64_t g, int* start, int* i) const {
+    int len = 0;
+    const int seq = find_segment(plan, g, start, &len);
+    *i = (int)(g - *start);
+    return seq;
+  }
+  __device__ __forceinline__ int64_t symbols(int seq, int h, int start) const {
+    return (int64_t)seq * seq_stride + (int64_t)h * head_stride +
+           (plan.cu_seqlens == nullptr ? 0 : start);
+  }
+  __device__ __forceinline__ int64_t links(int64_t base, int64_t, int, int i) const { return base + i; }
+};
+
+// One thread per row: a warp takes 32 consecutive tokens of one head (its symbol and link reads
+// coalesce), a CTA eight heads of them; the winners change places in shared memory so that the
+// results go out with the heads of a token side by side.  Bound by the latency and the sector
+// rate of the dependent chain reads in L2; many rows in flight hide it.
+constexpr int kChainRows = 32;
+constexpr int kChainHeads = 8;
+
+template <typename Sym, typename Axis, typename Emit>
+__global__ void __launch_bounds__(kChainRows * kChainHeads)
+    chain_match_kernel(Axis axis, const Sym* __restrict__ qsym, const Sym* __restrict__ ksym,
+                       int64_t N, int H, int W, int context, const uint32_t* __restrict__ start_link,
+                       const uint32_t* __restrict__ prev, const uint32_t* __restrict__ low,
+                       int head_blocks, int limit, int32_t* flag, Emit emit) {
+  __shared__ uint2 s_win[kChainRows][kChainHeads + 1];   // (length, route)
+  __shared__ int s_start[kChainRows];
+  const int heads = blockDim.x / kChainRows;             // heads of this CTA
+  const int tile = blockIdx.x / head_blocks;
+  const int h0 = (blockIdx.x - tile * head_blocks) * heads;
+  const int64_t g0 = (int64_t)tile * kChainRows;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int h = h0 + warp;
+  const int64_t g = g0 + lane;
+  int start = 0, i = 0, best_len = 0, best_route = 0;
+  int seq = -1;
+  if (g < N && h < H) seq = axis.locate(g, &start, &i);
+  int64_t base = 0;
+  uint32_t first = 0u, shorter = 0u;
+  if (seq >= 0) {
+    base = axis.symbols(seq, h, start);
+    const int64_t at = axis.links(base, g, h, i);
+    first = start_link[at];
+    if (context > 1) shorter = low[at];
+  }
+  if (chain_walk<Sym>(qsym + base, ksym + base, prev + base, first, seq, i, W, limit, lane, best_len,
+                      best_route)) {
+    best_len = (int)(kChainGaveUp >> 32);          // resolved by a matcher of whole warps
+    best_route = 0;
+    *flag = 1;
+  } else if (best_len < context) {
+    best_len = (int)(shorter >> 28);
+    best_route = (int)(shorter & 0x0fffffffu);
+  }
+  s_win[lane][warp] = make_uint2((unsigned)best_len, (unsigned)best_route);
+  if (warp == 0) s_start[lane] = start;
+  __syncthreads();
+  const int r = threadIdx.x / heads, hh = threadIdx.x - r * heads;
+  if (g0 + r < N && h0 + hh < H) {
+    const uint2 win = s_win[r][hh];
+    emit(g0 + r, h0 + hh, H, s_start[r], (int)win.x, (int)win.y);
+  }
+}
+
+template <typename Sym, typename Axis, typename Emit>
+int launch_chain_match_t(Axis axis, const Sym* q, const Sym* k, int64_t N, int H, int W, int context,
+                         const uint32_t* start, const uint32_t* prev, const uint32_t* low, int limit,
+                         int32_t* flag, Emit emit, cudaStream_t stream) {
+  const int heads = H < kChainHeads ? H : kChainHeads;
+  const int head_blocks = (H + heads - 1) / heads;
+  const int64_t tiles = (N + kChainRows - 1) / kChainRows;
+  chain_match_kernel<Sym, Axis, Emit><<<(unsigned)(tiles * head_blocks), kChainRows * heads, 0, stream>>>(
+      axis, q, k, N, H, W, context, start, prev, low, head_blocks, limit, flag, emit);
+  ROSA_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
+// A warp resolves one row by a look at every earlier position, newest first, 32 at a time: lanes
+// whose position agrees with the row here and at the distance of the best length so far extend it.
+// Cost: i / 32 coalesced reads, whatever the chains look like.  All lanes call and get the result.
+template <typename Sym>
+__device__ __forceinline__ void scan_row(const Sym* q, const Sym* k, int i, int W, int lane,
+                                         int& best_len, int& best_route) {
+  const Sym q_i = q[i];
+  best_len = best_route = 0;
+  for (int top = i - 1; top >= 0 && best_len < min(W, top + 1); top -= 32) {
+    const int j = top - lane;
+    int length = 0;
+    if (j >= best_len && k[j] == q_i && k[j - best_len] == q[i - best_len])
+      length = chain_extend<Sym>(q, k, i, j, 1, min(W, j + 1));
+    const int longest = __reduce_max_sync(0xffffffffu, length);
+    if (longest > best_len) {
+      best_len = longest;
+      best_route = __reduce_max_sync(0xffffffffu, length == longest ? j + 1 : 0);
+    }
+  }
+}
+
+// The rows that gave up, one warp each.
+constexpr int kScanWarps = 8;
+
+template <typename Sym, typename Axis, typename Emit>
+__global__ void __launch_bounds__(kScanWarps * 32)
+    scan_match_kernel(Axis axis, const Sym* __restrict__ qsym, const Sym* __restrict__ ksym, int64_t N,
+                      int H, int W, const int32_t* __restrict__ run_flag, Emit emit) {
+  if (*run_flag == 0) return;
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = (int64_t)gridDim.x * kScanWarps, count = N * H;
+  for (int64_t th0 = ((int64_t)blockIdx.x * kScanWarps + (threadIdx.x >> 5)) * 32; th0 < count;
+       th0 += warps * 32) {
+    const bool mine = th0 + lane < count && emit.pending(th0 + lane);
+    for (unsigned rows = __ballot_sync(0xffffffffu, mine); rows != 0u; rows &= rows - 1u) {
+      const int64_t th = th0 + __ffs(rows) - 1;
+      const int64_t g = th / H;
+      const int h = (int)(th - g * H);
+      int start = 0, i = 0, best_len, best_route;
+      const int seq = axis.locate(g, &start, &i);
+      const int64_t base = axis.symbols(seq, h, start);
+      scan_row<Sym>(qsym + base, ksym + base, i, W, lane, best_len, best_route);
+      if (lane == 0) emit(g, h, H, start, best_len, best_route);
+    }
+  }
+}
+
+template <typename Sym, typename Axis, typename Emit>
+int launch_scan_match_t(Axis axis, const Sym* q, const Sym* k, int64_t N, int H, int W,
+                        const int32_t* run_flag, Emit emit, cudaStream_t stream) {
+  ProfileScope prof("hard_match_scan", stream);
+  // a grid that fills the GPU: it is launched whether or not a row gave up
+  scan_match_kernel<Sym, Axis, Emit><<<148 * 8, kScanWarps * 32, 0, stream>>>(axis, q, k, N, H, W,
+                                                                             run_flag, emit);
+  ROSA_CUDA_OK(cudaGetLastError());
+  return 0;
+}
+
+}  // namespace
+}  // namespace rosa

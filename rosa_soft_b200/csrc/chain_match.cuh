@@ -22,6 +22,8 @@ namespace rosa {
 constexpr int kChainHashBits = 13;    // buckets of the chained contexts: at most 2^13
 constexpr int kChainStep = 16;        // positions a warp indexes at a time
 constexpr int kChainAhead = 8;        // steps between the request of a symbol and its use
+// Longest history whose step numbers fit a 32-bit table entry beside the mask of 16 lanes.
+constexpr int64_t kChainNarrow = (int64_t)65535 * kChainStep;
 // A row gives up after this many chain members (streams of few distinct symbols, or of passages
 // repeated very often) and is resolved by a whole warp.  Symbols of up to 8 bits have the
 // bit-parallel matcher for that, which is soon the cheaper way; wide ones a scan of all positions.
@@ -58,8 +60,8 @@ __host__ __device__ inline int chain_low_entries(int bits, int L) {
 // Number of equal symbols ending at k[j] and q[i], at most `cap`, of which `length` are known.
 // Four at a time: the loads of a group do not wait for one another.
 template <typename Sym>
-__device__ __forceinline__ int chain_extend(const Sym* __restrict__ q, const Sym* __restrict__ k, int i,
-                                            int j, int length, int cap) {
+__device__ __forceinline__ int chain_extend(const Sym* q, const Sym* k, int i, int j, int length,
+                                            int cap) {
   while (length + 4 <= cap) {
     const Sym* kp = k + (j - length);
     const Sym* qp = q + (i - length);
@@ -84,10 +86,9 @@ __device__ __forceinline__ int chain_extend(const Sym* __restrict__ q, const Sym
 // distance of the best length so far.  Returns the length and the route (position + 1) of the latest
 // among the longest; the result is true when the chain was longer than `limit`.  All lanes call.
 template <typename Sym>
-__device__ __forceinline__ bool chain_walk(const Sym* __restrict__ q, const Sym* __restrict__ k,
-                                           const uint32_t* __restrict__ prev, uint32_t first, int row,
-                                           int i, int W, int limit, int lane, int& best_len,
-                                           int& best_route) {
+__device__ __forceinline__ bool chain_walk(const Sym* q, const Sym* k, const uint32_t* prev,
+                                           uint32_t first, int row, int i, int W, int limit, int lane,
+                                           int& best_len, int& best_route) {
   best_len = 0;
   best_route = 0;
   int j = (int)first - 1;

@@ -14,18 +14,13 @@
 //
 // Also registered: rosa_soft::hard_inference (batched hard inference), the backward operator
 // rosa_soft::surrogate_vjp_sharded (dense or packed) that takes the dropout coordinate offsets
-// of a shard, and the custom class
-// torch.classes.rosa_soft.RosaRuntime (constructor and methods of the reference's class,
-// rosa_soft/csrc/rosa_runtime.cpp:570-582) over the streaming entry point of the C ABI.
+// of a shard.  The streaming runtime and the module itself are in stream_binding.cpp.
 //
 // One deliberate difference: the reference flags its backward as non-deterministic
 // (global float atomics).  This backward reduces in a fixed order and is bitwise
 // reproducible, so it does not raise under torch.use_deterministic_algorithms(True).
-#include <Python.h>
-
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
-#include <torch/custom_class.h>
 #include <torch/extension.h>
 
 #include <algorithm>
@@ -39,15 +34,6 @@
 #include <vector>
 
 #include "rosa_soft_b200.h"
-
-extern "C" {
-PyObject* PyInit__C(void) {
-  static struct PyModuleDef module_def = {
-      PyModuleDef_HEAD_INIT, "_C", "rosa_soft_b200 operator registration", -1, nullptr,
-  };
-  return PyModule_Create(&module_def);
-}
-}
 
 namespace {
 
@@ -413,164 +399,6 @@ std::tuple<Tensor, Tensor> hard_inference_op(Tensor query_symbols, Tensor key_sy
   return {out, matched};
 }
 
-// ------------------------------------------------------------------ RosaRuntime class
-// torch.classes.rosa_soft.RosaRuntime with the reference's constructor and methods
-// (rosa_soft/csrc/rosa_runtime.cpp:300-331, 333-482, 484-582): update_packed(cu_seqlens, query,
-// key, payload) -> (output uint8 [total, H], matched_key_end int64 [total, H]), reset, close,
-// stats.  The state (query / payload histories and one occurrence bitmap per key symbol) lives
-// on the GPU of the first update and every update is one rosa_b200_stream_update call on the
-// current stream; cu_seqlens is read on the host (int32 or int64, CPU or CUDA) like the
-// reference reads it, because the chunk lengths size the state.
-class RosaRuntimeClass : public torch::CustomClassHolder {
- public:
-  RosaRuntimeClass(int64_t num_heads, int64_t num_payload_heads, int64_t qk_bits,
-                   int64_t payload_bits, int64_t max_suffix_length)
-      : heads_(num_heads), payload_heads_(num_payload_heads), qk_bits_(qk_bits),
-        payload_bits_(payload_bits), horizon_(max_suffix_length) {
-    enforce({{heads_ > 0, "num_heads must be positive"},
-             {payload_heads_ > 0, "num_payload_heads must be positive"},
-             {payload_heads_ > 0 && heads_ % payload_heads_ == 0,
-              "num_heads must be divisible by num_payload_heads"},
-             {qk_bits_ > 0 && qk_bits_ <= 8, "qk_bits must be in [1, 8]"},
-             {payload_bits_ > 0 && payload_bits_ <= 8, "payload_bits must be in [1, 8]"},
-             {horizon_ > 0 && horizon_ <= kInt32Max, "max_suffix_length must be in [1, int32_max]"}});
-  }
-
-  std::tuple<Tensor, Tensor> update_packed(const Tensor& cu_seqlens, const Tensor& query,
-                                           const Tensor& key, const Tensor& payload) {
-    std::lock_guard<std::mutex> lock(mutex_);
-    TORCH_CHECK(!closed_, "RosaRuntime is closed");
-    enforce({{query.is_cuda() && key.is_cuda() && payload.is_cuda(),
-              "RosaRuntime keeps its state on the GPU: query, key and payload must be CUDA tensors"},
-             {query.scalar_type() == torch::kUInt8 && key.scalar_type() == torch::kUInt8 &&
-                  payload.scalar_type() == torch::kUInt8,
-              "query, key and payload must have dtype uint8"},
-             {query.dim() == 2 && key.dim() == 2 && payload.dim() == 2,
-              "query, key and payload must be two-dimensional (total_tokens, heads)"},
-             {cu_seqlens.dim() == 1 && cu_seqlens.numel() >= 2,
-              "cu_seqlens must be one-dimensional with at least two entries"},
-             {cu_seqlens.scalar_type() == torch::kInt32 || cu_seqlens.scalar_type() == torch::kInt64,
-              "cu_seqlens must be int32 or int64"}});
-    enforce({{query.sizes() == key.sizes(), "query/key shape mismatch"},
-             {query.size(1) == heads_, "query head count must equal num_heads"},
-             {payload.size(1) == payload_heads_, "payload head count must equal num_payload_heads"},
-             {payload.size(0) == query.size(0), "query/payload token mismatch"},
-             {query.device() == key.device() && query.device() == payload.device(),
-              "query, key and payload must be on the same CUDA device"}});
-    const Tensor host_cu = cu_seqlens.to(torch::kCPU, torch::kInt64).contiguous();
-    const int64_t* cu = host_cu.data_ptr<int64_t>();
-    const int64_t slots = host_cu.numel() - 1;
-    const int64_t total = query.size(0);
-    TORCH_CHECK(cu[0] == 0, "cu_seqlens must start at 0");
-    for (int64_t s = 0; s < slots; ++s)
-      TORCH_CHECK(cu[s + 1] >= cu[s], "cu_seqlens must be non-decreasing");
-    TORCH_CHECK(cu[slots] == total, "cu_seqlens[-1] must equal the total token count");
-    if (slots_ < 0) {
-      slots_ = slots;
-      device_ = query.device();
-      lengths_host_.assign(static_cast<size_t>(slots), 0);
-    } else {
-      TORCH_CHECK(slots == slots_, "RosaRuntime slot count is fixed after the first update");
-      TORCH_CHECK(query.device() == device_, "RosaRuntime state lives on another device");
-    }
-    std::vector<int64_t> after(lengths_host_);
-    int64_t needed = 0;
-    for (int64_t s = 0; s < slots; ++s) {
-      after[s] += cu[s + 1] - cu[s];
-      needed = std::max(needed, after[s]);
-    }
-    TORCH_CHECK(needed <= kInt32Max - 31, "ROSA sequence length exceeded int32 range");
-    const c10::cuda::CUDAGuard guard(device_);
-    grow(needed);
-    const auto u8 = query.options();
-    Tensor output = torch::empty({total, heads_}, u8);
-    Tensor matched = torch::empty({total, heads_}, u8.dtype(torch::kInt64));
-    const Tensor q = query.contiguous(), k = key.contiguous(), p = payload.contiguous();
-    const Tensor offsets = host_cu.to(torch::kInt32).to(device_);
-    const size_t bytes = rosa_b200_stream_workspace_bytes(total, (int)heads_);
-    Tensor ws = make_workspace(q, bytes);
-    check_rc(rosa_b200_stream_update(
-                 q.data_ptr<uint8_t>(), k.data_ptr<uint8_t>(), p.data_ptr<uint8_t>(),
-                 offsets.data_ptr<int32_t>(), total, (int)slots, (int)heads_, (int)payload_heads_,
-                 (int)qk_bits_, (int)payload_bits_, horizon_,
-                 reinterpret_cast<uint32_t*>(key_masks_.data_ptr<int32_t>()),
-                 query_history_.data_ptr<uint8_t>(), payload_history_.data_ptr<uint8_t>(),
-                 lengths_.data_ptr<int32_t>(), capacity_, needed, output.data_ptr<uint8_t>(),
-                 matched.data_ptr<int64_t>(), ws.data_ptr(), bytes,
-                 at::cuda::getCurrentCUDAStream().stream()),
-             "RosaRuntime.update_packed");
-    lengths_host_ = after;   // committed only once the update has been enqueued
-    return {output, matched};
-  }
-
-  void reset() {
-    std::lock_guard<std::mutex> lock(mutex_);
-    TORCH_CHECK(!closed_, "RosaRuntime is closed");
-    clear();
-  }
-
-  void close() {
-    std::lock_guard<std::mutex> lock(mutex_);
-    clear();
-    closed_ = true;
-  }
-
-  // (states, edges, payload_symbols, automata, sequences, logical_bytes): there is no
-  // automaton, so the first two are zero; the bytes are those of the histories and bitmaps.
-  std::tuple<int64_t, int64_t, int64_t, int64_t, int64_t, int64_t> stats() const {
-    std::lock_guard<std::mutex> lock(mutex_);
-    int64_t tokens = 0;
-    for (int64_t n : lengths_host_) tokens += n;
-    const int64_t slots = slots_ < 0 ? 0 : slots_;
-    const int64_t bytes =
-        tokens * (heads_ * (1 + ((int64_t)1 << qk_bits_) / 8) + payload_heads_);
-    return {0, 0, tokens * payload_heads_, slots * heads_, slots, bytes};
-  }
-
- private:
-  void clear() {
-    key_masks_ = Tensor();
-    query_history_ = Tensor();
-    payload_history_ = Tensor();
-    lengths_ = Tensor();
-    lengths_host_.clear();
-    slots_ = -1;
-    capacity_ = 0;
-  }
-
-  // Room for `needed` tokens per slot: the capacity doubles, old contents are kept.  All
-  // copies are enqueued on the current stream, which also orders them after earlier updates.
-  void grow(int64_t needed) {
-    if (needed <= capacity_ && capacity_ > 0) return;
-    int64_t capacity = std::max<int64_t>(256, capacity_);
-    while (capacity < needed) capacity *= 2;
-    const auto u8 = torch::TensorOptions().device(device_).dtype(torch::kUInt8);
-    Tensor masks = torch::zeros({slots_, heads_, (int64_t)1 << qk_bits_, capacity / 32},
-                                u8.dtype(torch::kInt32));
-    Tensor qh = torch::empty({slots_, heads_, capacity}, u8);
-    Tensor ph = torch::empty({slots_, payload_heads_, capacity}, u8);
-    if (capacity_ > 0) {
-      masks.narrow(3, 0, capacity_ / 32).copy_(key_masks_);
-      qh.narrow(2, 0, capacity_).copy_(query_history_);
-      ph.narrow(2, 0, capacity_).copy_(payload_history_);
-    } else {
-      lengths_ = torch::zeros({slots_}, u8.dtype(torch::kInt32));
-    }
-    key_masks_ = masks;
-    query_history_ = qh;
-    payload_history_ = ph;
-    capacity_ = capacity;
-  }
-
-  const int64_t heads_, payload_heads_, qk_bits_, payload_bits_, horizon_;
-  int64_t slots_ = -1, capacity_ = 0;
-  bool closed_ = false;
-  c10::Device device_{c10::kCPU};
-  std::vector<int64_t> lengths_host_;
-  Tensor key_masks_, query_history_, payload_history_, lengths_;
-  mutable std::mutex mutex_;
-};
-
 }  // namespace
 
 #ifdef ROSA_WITH_CUDA
@@ -581,12 +409,6 @@ TORCH_LIBRARY(rosa_soft, m) {
   m.def("surrogate_vjp_varlen_masked(Tensor query, Tensor key, Tensor value, Tensor cu_seqlens, Tensor grad_output, Tensor packed_query_symbols, Tensor packed_key_symbols, Tensor dropout_seed, int max_suffix_length, float scale, float dropout_p, float mismatch_scale, int gradient_mask) -> (Tensor grad_query, Tensor grad_key, Tensor grad_value)");
   m.def("surrogate_vjp_sharded(Tensor query, Tensor key, Tensor value, Tensor? cu_seqlens, Tensor grad_output, Tensor packed_query_symbols, Tensor packed_key_symbols, Tensor dropout_seed, int max_suffix_length, float scale, float dropout_p, float mismatch_scale, int gradient_mask, int batch_offset, int head_offset) -> (Tensor grad_query, Tensor grad_key, Tensor grad_value)");
   m.def("hard_inference(Tensor query_symbols, Tensor key_symbols, Tensor payload, Tensor? cu_seqlens, int max_suffix_length) -> (Tensor output, Tensor matched_key_end_positions)");
-  m.class_<RosaRuntimeClass>("RosaRuntime")
-      .def(torch::init<int64_t, int64_t, int64_t, int64_t, int64_t>())
-      .def("update_packed", &RosaRuntimeClass::update_packed)
-      .def("reset", &RosaRuntimeClass::reset)
-      .def("close", &RosaRuntimeClass::close)
-      .def("stats", &RosaRuntimeClass::stats);
 }
 
 TORCH_LIBRARY_IMPL(rosa_soft, CUDA, m) {

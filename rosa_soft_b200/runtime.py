@@ -5,11 +5,11 @@ rosa_soft/csrc/rosa_runtime.cpp:216-556) for the 1..8-bit packed deployment subs
 constructor, properties, ``update`` / ``update_packed`` signatures, slot fixing, ``sequence_ids``
 checks, ``reset`` / ``close`` life cycle and error texts.  The difference is where the state
 lives: the reference stages every update to the CPU, steps one suffix automaton per
-(slot, head) there and copies the result back (runtime.py:728-773); this class keeps the query
-and payload histories and one occurrence bitmap per key symbol in HBM and updates them with
-``rosa_b200_stream_update`` (a bit-parallel matcher), so a chunk never leaves the device and
-the call only enqueues work on a CUDA stream.  Results are identical to a one-shot pass
-whatever the chunking.
+(slot, head) there and copies the result back (runtime.py:728-773); this class keeps the symbol
+histories and their occurrence chains in HBM (``_C.StreamCore``) and updates them with
+``rosa_b200_stream_update_chained``, so a chunk never leaves the device and the call only enqueues
+work on a CUDA stream: one kernel for a generation step, from logits to unpacked values.  Results
+are identical to a one-shot pass whatever the chunking.
 """
 from __future__ import annotations
 
@@ -20,8 +20,10 @@ import torch
 from torch import Tensor
 
 from . import cabi
+from ._C import StreamCore
 
-_MIN_CAPACITY = 256
+# output types that the update kernels write themselves
+_NATIVE_OUTPUTS = (torch.float32, torch.float16, torch.bfloat16)
 
 
 def _as_index(name: str, value) -> int:
@@ -119,20 +121,14 @@ class RosaRuntime:
             raise ValueError("max_suffix_length must be >= 1")
         cabi.load()  # fail now, not at the first update, when the CUDA library is missing
         self._state = "OPEN"
+        self._core = StreamCore(self._num_heads, self._num_payload_heads, self._qk_bits,
+                                self._payload_bits, self._max_suffix_length)
         self._clear()
 
     def _clear(self) -> None:
-        self._device: Optional[torch.device] = None
-        self._slots = -1
-        self._capacity = 0
-        self._lengths_host: list = []
-        self._key_masks: Optional[Tensor] = None       # [slots, H, 2^qk_bits, capacity / 32]
-        self._query_history: Optional[Tensor] = None   # [slots, H, capacity]
-        self._payload_history: Optional[Tensor] = None  # [slots, Hp, capacity]
-        self._lengths: Optional[Tensor] = None
+        self._core.clear()
         self._sequence_ids: Optional[Tuple[int, ...]] = None
         self._ids_fixed = False
-        self._last_update: Optional[torch.cuda.Event] = None   # orders updates across streams
 
     # ------------------------------------------------------------------ configuration
     @property
@@ -184,21 +180,20 @@ class RosaRuntime:
         self._clear()
 
     def memory_stats(self) -> Dict[str, int]:
-        """Counts of what is held.  ``states`` / ``edges`` are zero: there is no automaton; the
-        matcher's state is one occurrence bit per key position and symbol
+        """Counts of what is held.  ``states`` / ``edges`` are zero: there is no automaton; a
+        token of a head is its query symbol, its key symbol and a chain link
         (reference runtime.py:557-576)."""
         self._require_open()
-        tokens = sum(self._lengths_host)
-        slots = max(self._slots, 0)
+        tokens = sum(self._core.lengths)
+        slots = max(self._core.slots, 0)
         return {
             "states": 0,
             "edges": 0,
             "payload_symbols": tokens * self._num_payload_heads,
             "automata": slots * self._num_heads,
             "sequences": slots,
-            "logical_bytes": tokens * (self._num_heads * (1 + (1 << self._qk_bits) // 8)
-                                       + self._num_payload_heads),
-            "capacity_tokens": self._capacity,
+            "logical_bytes": tokens * (self._num_heads * 6 + self._num_payload_heads),
+            "capacity_tokens": self._core.capacity,
         }
 
     def stats(self) -> Tuple[int, int, int]:
@@ -210,15 +205,13 @@ class RosaRuntime:
         declines to checkpoint its automata, runtime.py:590-603; plain arrays have no such
         problem.)"""
         self._require_open()
-        used = max(self._lengths_host, default=0)
         config = {name: getattr(self, name) for name in (
             "num_heads", "num_payload_heads", "qk_bits", "payload_bits", "max_suffix_length")}
-        state: Dict[str, Any] = {"config": config, "lengths": list(self._lengths_host),
+        state: Dict[str, Any] = {"config": config, "lengths": list(self._core.lengths),
                                  "sequence_ids": self._sequence_ids, "ids_fixed": self._ids_fixed}
-        if self._slots > 0:
-            state["key_masks"] = self._key_masks[..., :(used + 31) // 32].clone()
-            state["query_history"] = self._query_history[..., :used].clone()
-            state["payload_history"] = self._payload_history[..., :used].clone()
+        if self._core.slots > 0:
+            (state["query_history"], state["key_history"],
+             state["payload_history"]) = self._core.export_histories()
         return state
 
     def load_state_dict(self, state_dict: Dict[str, Any]) -> None:
@@ -236,40 +229,23 @@ class RosaRuntime:
         query_history = state_dict["query_history"]
         if not query_history.is_cuda:
             raise ValueError("state_dict tensors must be CUDA tensors")
-        self._device = query_history.device
-        self._slots = len(lengths)
-        self._lengths_host = lengths
-        self._grow(max(lengths))
-        used = query_history.shape[-1]
-        self._key_masks[..., :(used + 31) // 32] = state_dict["key_masks"]
-        self._query_history[..., :used] = query_history
-        self._payload_history[..., :used] = state_dict["payload_history"]
-        self._lengths.copy_(torch.tensor(lengths, dtype=torch.int32))
+        key_history = state_dict.get("key_history")
+        if key_history is None:     # saved as one occurrence bitmap per key symbol
+            key_history = self._keys_from_masks(state_dict["key_masks"], query_history.shape[-1])
+        self._core.import_histories(lengths, query_history, key_history,
+                                    state_dict["payload_history"])
+
+    @staticmethod
+    def _keys_from_masks(masks: Tensor, tokens: int) -> Tensor:
+        shifts = torch.arange(32, dtype=torch.int32, device=masks.device)
+        keys = torch.zeros((*masks.shape[:2], masks.shape[-1] * 32), dtype=torch.uint8,
+                           device=masks.device)
+        for symbol in range(1, masks.shape[2]):
+            bits = (masks[:, :, symbol, :, None] >> shifts) & 1
+            keys += bits.flatten(-2).to(torch.uint8) * symbol
+        return keys[..., :tokens].contiguous()
 
     # -------------------------------------------------------------------------- state
-    def _grow(self, needed: int) -> None:
-        """Makes room for `needed` tokens per slot (capacity doubles; old contents are kept)."""
-        if needed <= self._capacity and self._capacity > 0:
-            return      # (a first update without tokens still allocates the minimum capacity)
-        capacity = max(_MIN_CAPACITY, self._capacity)
-        while capacity < needed:
-            capacity *= 2
-        shape_m = (self._slots, self._num_heads, 1 << self._qk_bits, capacity // 32)
-        shape_q = (self._slots, self._num_heads, capacity)
-        shape_p = (self._slots, self._num_payload_heads, capacity)
-        key_masks = torch.zeros(shape_m, dtype=torch.int32, device=self._device)
-        query_history = torch.empty(shape_q, dtype=torch.uint8, device=self._device)
-        payload_history = torch.empty(shape_p, dtype=torch.uint8, device=self._device)
-        if self._capacity:
-            key_masks[..., :self._capacity // 32] = self._key_masks
-            query_history[..., :self._capacity] = self._query_history
-            payload_history[..., :self._capacity] = self._payload_history
-        else:
-            self._lengths = torch.zeros(self._slots, dtype=torch.int32, device=self._device)
-        self._key_masks, self._query_history, self._payload_history = (
-            key_masks, query_history, payload_history)
-        self._capacity = capacity
-
     def _check_sequence_ids(self, sequence_ids: Optional[Tuple[int, ...]]) -> None:
         if not self._ids_fixed:
             self._ids_fixed = True
@@ -291,6 +267,13 @@ class RosaRuntime:
                async_op: bool = False, return_packed: bool = False, sequence_ids=None):
         """Sign-binarises the logits and updates; dense [B, T, H, bits] or, with `cu_seqlens`,
         packed [N, H, bits] (reference runtime.py:605-651)."""
+        if (cu_seqlens is None and stream is None and not async_op and sequence_ids is None
+                and self._sequence_ids is None and self._state == "OPEN"
+                and query_logits.dtype in _NATIVE_OUTPUTS):
+            done = self._core.dense(query_logits, key_logits, payload_logits, return_packed, None)
+            if done is not None:
+                self._ids_fixed = True
+                return done
         if query_logits.shape != key_logits.shape:
             raise ValueError(f"query/key shapes differ: {query_logits.shape} vs {key_logits.shape}")
         if query_logits.size(-1) != self.qk_bits:
@@ -316,6 +299,14 @@ class RosaRuntime:
         whole history (-1 and payload 0 for no match); reference runtime.py:653-789,
         rosa_runtime.cpp:333-482.  Dense chunks are uint8 [B, T, H] / [B, T, Hp]; with
         `cu_seqlens` (int32/int64 [slots + 1]) they are packed [N, H] / [N, Hp]."""
+        if (cu_seqlens is None and stream is None and not async_op and sequence_ids is None
+                and self._sequence_ids is None and self._state == "OPEN"
+                and query_symbols.dtype == torch.uint8):
+            done = self._core.dense(query_symbols, key_symbols, payload_symbols, return_packed,
+                                    None if return_packed else output_dtype)
+            if done is not None:
+                self._ids_fixed = True
+                return done
         tensors = (query_symbols, key_symbols, payload_symbols)
         if any(t.dtype != torch.uint8 for t in tensors):
             raise TypeError("packed RosaRuntime inputs must have dtype torch.uint8")
@@ -369,53 +360,39 @@ class RosaRuntime:
             raise TypeError("output_dtype must be floating-point when unpacking")
         self._require_open()
 
-        if self._slots == -1:
-            self._slots, self._device = slots, device
-            self._lengths_host = [0] * slots
-        elif slots != self._slots:
-            raise RuntimeError("RosaRuntime slot count is fixed after the first update")
-        elif device != self._device:
-            raise ValueError("RosaRuntime state lives on another device")
+        core = self._core
+        if core.slots != -1:
+            if slots != core.slots:
+                raise RuntimeError("RosaRuntime slot count is fixed after the first update")
+            if not core.on(device):
+                raise ValueError("RosaRuntime state lives on another device")
         self._check_sequence_ids(ids)
 
-        chunk = [b - a for a, b in zip(offsets, offsets[1:])]
-        after = [held + n for held, n in zip(self._lengths_host, chunk)]
-        if max(after) > 2**31 - 1:
+        held = core.lengths or [0] * slots
+        if max(n + b - a for n, a, b in zip(held, offsets, offsets[1:])) > 2**31 - 1:
             raise RuntimeError("ROSA sequence length exceeded int32 range")
         current = torch.cuda.current_stream(device)
         run_on = stream if stream is not None else current
         if stream is not None:
             stream.wait_stream(current)   # the inputs were produced on the caller's stream
-        if self._last_update is not None:
-            # the state is shared by all updates: whatever stream the previous one ran on, this
-            # one starts after it (the C ABI wants calls that share a state ordered)
-            run_on.wait_event(self._last_update)
+        # values of a type that the kernels do not write are unpacked from the symbols here
+        native = return_packed or output_dtype in _NATIVE_OUTPUTS
+        # offsets that are on the device already are used there
+        on_device = (cu_seqlens if not dense and cu_seqlens.device == device
+                     and cu_seqlens.dtype == torch.int32 else None)
         with torch.cuda.stream(run_on):
-            self._grow(max(after))
-            flat_q = query_symbols.reshape(-1, heads).contiguous()
-            flat_k = key_symbols.reshape(-1, heads).contiguous()
-            flat_p = payload_symbols.reshape(-1, payload_heads).contiguous()
-            dev_offsets = torch.tensor(offsets, dtype=torch.int32).to(device, non_blocking=True)
-            packed, end, workspace = cabi.stream_update(
-                flat_q, flat_k, flat_p, dev_offsets, self.qk_bits, self.payload_bits,
-                self.max_suffix_length, self._key_masks, self._query_history, self._payload_history,
-                self._lengths, max(after), stream=run_on.cuda_stream)
-            self._lengths_host = after
-            if dense:
-                packed = packed.reshape(slots, tokens, heads)
-                end = end.reshape(slots, tokens, heads)
-            if return_packed:
-                result = (packed, end)
-            else:
+            result = core.packed(query_symbols, key_symbols, payload_symbols, offsets, on_device,
+                                 None if return_packed or not native else output_dtype,
+                                 list(query_symbols.shape))
+            if not native:
+                packed, end = result
                 values = unpack_sign_bits(packed, self.payload_bits, output_dtype)
                 values = torch.where(end.unsqueeze(-1) >= 0, values,
                                      torch.zeros((), dtype=output_dtype, device=device))
                 result = (values, end)
-            for tensor in (flat_q, flat_k, flat_p, dev_offsets, workspace, self._key_masks,
-                           self._query_history, self._payload_history, self._lengths):
-                tensor.record_stream(run_on)
-            self._last_update = torch.cuda.Event()
-            self._last_update.record(run_on)
+            if stream is not None:
+                for tensor in (*tensors, *((on_device,) if on_device is not None else ())):
+                    tensor.record_stream(run_on)
         if stream is None:
             if async_op:
                 event = torch.cuda.Event()
