@@ -42,37 +42,46 @@ __device__ __forceinline__ void chain_index_warp(const Sym* q, const Sym* k, int
   const uint32_t context_mask = context_bits >= 32 ? 0xffffffffu : (1u << context_bits) - 1u;
   // a query at i needs a key context at j < i
   const int first_valid = max(begin, is_query ? L : L - 1);
-  // bucket of the context that ends at p from its newest two symbols; ~0 where there is none
-  auto bucket_of = [&](int p, int newest, int second) -> uint32_t {
-    uint32_t w = (uint32_t)newest;
-    if (L > 1) w |= (uint32_t)second << bits;
-    for (int u = 2; u < L; ++u)
-      if (p >= first_valid && p < end) w |= (uint32_t)sym[p - u] << (bits * u);
-    w &= context_mask;
-    if (chained) w = chain_bucket(w, context_bits, hash_bits);
-    return p >= first_valid && p < end ? w : 0xffffffffu;
+  // buckets of the contexts of the next steps from their newest two symbols (requested earlier) and
+  // the older ones, all steps of one distance at a time; ~0 where there is no context
+  uint32_t bucket[kChainAhead];
+  auto fill_buckets = [&](int p0, const int (&newest)[kChainAhead], const int (&second)[kChainAhead]) {
+#pragma unroll
+    for (int s = 0; s < kChainAhead; ++s)
+      bucket[s] = (uint32_t)newest[s] | (L > 1 ? (uint32_t)second[s] << bits : 0u);
+    for (int u = 2; u < L; ++u) {
+#pragma unroll
+      for (int s = 0; s < kChainAhead; ++s) {
+        const int p = p0 + s * kChainStep + l;
+        if (p >= first_valid && p < end) bucket[s] |= (uint32_t)sym[p - u] << (bits * u);
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < kChainAhead; ++s) {
+      const int p = p0 + s * kChainStep + l;
+      const uint32_t w = bucket[s] & context_mask;
+      bucket[s] = p < first_valid || p >= end ? 0xffffffffu
+                  : chained ? chain_bucket(w, context_bits, hash_bits) : w;
+    }
   };
-  auto newest_at = [&](int p) { return p < end ? (int)sym[p] : 0; };
-  auto second_at = [&](int p) { return L > 1 && p >= 1 && p < end ? (int)sym[p - 1] : 0; };
+  auto request = [&](int p0, int (&newest)[kChainAhead], int (&second)[kChainAhead]) {
+#pragma unroll
+    for (int s = 0; s < kChainAhead; ++s) {
+      const int p = p0 + s * kChainStep + l;
+      newest[s] = p < end ? (int)sym[p] : 0;
+      second[s] = L > 1 && p >= 1 && p < end ? (int)sym[p - 1] : 0;
+    }
+  };
   uint32_t* dst = is_query ? query_links : key_links;
   const bool writes = (chained || is_query) && dst != nullptr;
   const uint32_t tag = chained ? 0u : (uint32_t)L << 28;
-  const int base = kResume ? begin / kChainStep * kChainStep : 0;
-  uint32_t bucket[kChainAhead];
-#pragma unroll
-  for (int s = 0; s < kChainAhead; ++s) {
-    const int p = base + s * kChainStep + l;
-    bucket[s] = bucket_of(p, newest_at(p), second_at(p));
-  }
+  const int base = begin / kChainStep * kChainStep;
+  int newest[kChainAhead], second[kChainAhead];
+  request(base, newest, second);
+  fill_buckets(base, newest, second);
   const unsigned own_bit = 1u << l;
   for (int p0 = base; p0 < end; p0 += kChainAhead * kChainStep) {
-    int a[kChainAhead], b[kChainAhead];
-#pragma unroll
-    for (int s = 0; s < kChainAhead; ++s) {
-      const int p = p0 + (kChainAhead + s) * kChainStep + l;
-      a[s] = newest_at(p);
-      b[s] = second_at(p);
-    }
+    request(p0 + kChainAhead * kChainStep, newest, second);
 #pragma unroll
     for (int s = 0; s < kChainAhead; ++s) {
       if (s > 0 && p0 + s * kChainStep >= end) break;
@@ -106,10 +115,87 @@ __device__ __forceinline__ void chain_index_warp(const Sym* q, const Sym* k, int
         }
       }
     }
-#pragma unroll
-    for (int s = 0; s < kChainAhead; ++s)
-      bucket[s] = bucket_of(p0 + (kChainAhead + s) * kChainStep + l, a[s], b[s]);
+    fill_buckets(p0 + kChainAhead * kChainStep, newest, second);
   }
+}
+
+// Indexes positions [begin, end) of one head by a whole CTA of context * segments warps.  `tables`
+// are `segments` table sets of `entries` entries each; the first holds the positions below `begin`.
+//
+// One warp per context length is all the parallelism a sequential pass has, so a call with few heads
+// leaves the GPU idle for len / 16 steps.  With more segments the positions are cut into as many
+// pieces: all threads together leave the newest key position of every bucket and piece in the table
+// set of the next piece (a maximum, in any order), the sets are made cumulative, and every piece
+// then runs its own pass from the table of everything before it.
+template <typename Entry, bool kMerge, bool kResume, typename Sym>
+__device__ __forceinline__ void chain_index_block(const Sym* q, const Sym* k, int begin, int end,
+                                                  int context, int bits, int hash_bits, int entries,
+                                                  int segments, Entry* tables, uint32_t* key_links,
+                                                  uint32_t* start, uint32_t* low) {
+  const int first_step = begin / kChainStep, steps = (end - 1) / kChainStep - first_step + 1;
+  const int per = (steps + segments - 1) / segments;
+  const auto piece = [&](int g) { return max(begin, (first_step + g * per) * kChainStep); };
+  const auto table_at = [&](int g, int L) {
+    return tables + (int64_t)g * entries +
+           (L == context ? 0 : (1 << hash_bits) + chain_low_entries(bits, L));
+  };
+  if (segments > 1) {
+    for (int e = threadIdx.x; e < (segments - 1) * entries; e += blockDim.x) tables[entries + e] = 0;
+    __syncthreads();
+    const int last = min(end, piece(segments - 1));
+    constexpr int kBatch = 4;                        // positions of a thread whose loads overlap
+    for (int p0 = begin + threadIdx.x; p0 < last; p0 += kBatch * blockDim.x) {
+      uint32_t w[kBatch] = {0u, 0u, 0u, 0u};
+      for (int L = 1; L <= context; ++L) {
+        const int context_bits = bits * L;
+        int symbol[kBatch];
+#pragma unroll
+        for (int x = 0; x < kBatch; ++x) {
+          const int p = p0 + x * blockDim.x;
+          symbol[x] = p < last && p >= L - 1 ? (int)k[p - L + 1] : 0;
+        }
+#pragma unroll
+        for (int x = 0; x < kBatch; ++x) {
+          const int p = p0 + x * blockDim.x;
+          w[x] |= (uint32_t)symbol[x] << (context_bits - bits);
+          if (p >= last || p < L - 1) continue;
+          const int g = (p / kChainStep - first_step) / per + 1;
+          const Entry entry = (Entry)(p / kChainStep + 1) << 16 | 1u << (p & (kChainStep - 1));
+          const uint32_t c = context_bits >= 32 ? w[x] : w[x] & ((1u << context_bits) - 1u);
+          atomicMax(table_at(g, L) + (L == context ? chain_bucket(c, context_bits, hash_bits) : c), entry);
+        }
+      }
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < entries; e += blockDim.x) {
+      Entry newest = tables[e];
+      for (int g = 1; g < segments; ++g) {
+        Entry* t = tables + (int64_t)g * entries + e;
+        newest = max(newest, *t);
+        *t = newest;
+      }
+    }
+    __syncthreads();
+  }
+  const int warp = threadIdx.x >> 5;
+  const int level = warp / segments, g = warp - level * segments;
+  const int L = context - level;                     // level 0: the chained length
+  const int from = piece(g), to = g + 1 < segments ? min(end, piece(g + 1)) : end;
+  if (from < to)
+    chain_index_warp<Entry, kMerge, kResume>(q, k, from, to, L, bits, level == 0, hash_bits, table_at(g, L),
+                                             key_links, level == 0 ? start : low);
+}
+
+// How many pieces per head: as many warps as the GPU holds of these CTAs, pieces of at least 256
+// positions, at most 8 (a table set each in shared memory), at most 768 threads a CTA (registers).
+constexpr int kChainSharedBytes = 200 * 1024;
+
+inline int chain_segments(int64_t heads, int64_t positions, size_t set_bytes, int context) {
+  int n = 1;
+  while (n < 8 && heads * n * 2 <= 148 * 8 && positions >= 256 * n * 2 &&
+         (size_t)n * 2 * set_bytes <= kChainSharedBytes && context * n * 2 <= 24)
+    n *= 2;
+  return n;
 }
 
 // Rows of whole sequences over packed symbols ([sequence][head][position] or [head][token]).

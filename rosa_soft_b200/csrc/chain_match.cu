@@ -8,12 +8,12 @@ namespace rosa {
 
 namespace {
 
-// One CTA per (sequence, head), one warp per context length; the tables of a CTA in shared memory.
+// One CTA per (sequence, head), one warp per context length and piece; the tables in shared memory.
 template <typename Entry, bool kMerge>
 __global__ void chain_index_kernel(Plan plan, const int32_t* __restrict__ qsym,
                                    const int32_t* __restrict__ ksym, int64_t sym_seq_stride,
                                    int64_t sym_head_stride, int H, int bits, int context,
-                                   int hash_bits, uint32_t* __restrict__ start,
+                                   int hash_bits, int segments, uint32_t* __restrict__ start,
                                    uint32_t* __restrict__ prev, uint32_t* __restrict__ low) {
   extern __shared__ unsigned long long table_words[];
   Entry* tables = reinterpret_cast<Entry*>(table_words);
@@ -29,11 +29,9 @@ __global__ void chain_index_kernel(Plan plan, const int32_t* __restrict__ qsym,
   const int entries = (1 << hash_bits) + chain_low_entries(bits, context);
   for (int e = threadIdx.x; e < entries; e += blockDim.x) tables[e] = 0;
   __syncthreads();
-  const int warp = threadIdx.x >> 5;
-  const int L = context - warp;                    // warp 0: the chained length
-  Entry* table = warp == 0 ? tables : tables + (1 << hash_bits) + chain_low_entries(bits, L);
-  chain_index_warp<Entry, kMerge, false>(qsym + base, ksym + base, 0, len, L, bits, warp == 0, hash_bits,
-                                         table, prev + base, (warp == 0 ? start : low) + base);
+  chain_index_block<Entry, kMerge, false>(qsym + base, ksym + base, 0, len, context, bits, hash_bits,
+                                          entries, segments, tables, prev + base, start + base,
+                                          low + base);
 }
 
 SequenceAxis sequence_axis(const FwdArgs& a) {
@@ -58,20 +56,31 @@ int scan_rows(const FwdArgs& a, const int32_t* run_flag, Emit emit, cudaStream_t
 
 int launch_chain_index(const FwdArgs& a, int64_t max_len, cudaStream_t stream) {
   ProfileScope prof("chain_index", stream);
-  const int hash_bits = chain_hash_bits(a.D, a.context, max_len);
-  if (a.context > 2)   // several shorter lengths merge their results into zeroed words
-    ROSA_CUDA_OK(cudaMemsetAsync(a.chain_low, 0, (size_t)a.N * a.H * sizeof(uint32_t), stream));
-  const size_t entries = (size_t)(1 << hash_bits) + chain_low_entries(a.D, a.context);
   const bool merge = a.context > 2, wide = max_len > kChainNarrow;
-  const size_t bytes = entries * (wide ? sizeof(unsigned long long) : sizeof(uint32_t));
+  int hash_bits = chain_hash_bits(a.D, a.context, max_len);
+  const auto set_bytes = [&] {
+    return ((size_t)(1 << hash_bits) + chain_low_entries(a.D, a.context)) *
+           (wide ? sizeof(unsigned long long) : sizeof(uint32_t));
+  };
+  const int64_t heads = (int64_t)a.plan.S * a.H;
+  int segments = chain_segments(heads, max_len, set_bytes(), a.context);
+  if (hash_bits == kChainHashBits && segments > 1 && segments < 8) {
+    // half the buckets, if that doubles the pieces
+    hash_bits = kChainHashBits - 1;
+    const int more = chain_segments(heads, max_len, set_bytes(), a.context);
+    if (more > segments) segments = more; else hash_bits = kChainHashBits;
+  }
+  if (merge)   // several shorter lengths merge their results into zeroed words
+    ROSA_CUDA_OK(cudaMemsetAsync(a.chain_low, 0, (size_t)a.N * a.H * sizeof(uint32_t), stream));
+  const size_t bytes = set_bytes() * segments;
   auto kernel = wide ? (merge ? chain_index_kernel<unsigned long long, true>
                               : chain_index_kernel<unsigned long long, false>)
                      : (merge ? chain_index_kernel<uint32_t, true> : chain_index_kernel<uint32_t, false>);
   if (bytes > 48 * 1024)
     ROSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  kernel<<<(unsigned)(a.plan.S * a.H), 32 * a.context, bytes, stream>>>(
+  kernel<<<(unsigned)heads, 32 * a.context * segments, bytes, stream>>>(
       a.plan, a.packed_q, a.packed_k, a.sym_seq_stride, a.sym_head_stride, a.H, a.D, a.context,
-      hash_bits, a.chain_start, a.chain_prev, a.chain_low);
+      hash_bits, segments, a.chain_start, a.chain_prev, a.chain_low);
   ROSA_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -218,8 +218,8 @@ __global__ void __launch_bounds__(256) stream_append_chunk_kernel(StreamCall c, 
 // One CTA per (slot, head), one warp per context length: the tables of the pair are staged in
 // shared memory for the chunk.  tokens < 0: the whole histories (after they were loaded or moved).
 template <typename Entry, bool kMerge>
-__global__ void stream_index_kernel(StreamCall c, uint32_t* __restrict__ start, uint32_t* __restrict__ low,
-                                    int32_t* flag) {
+__global__ void stream_index_kernel(StreamCall c, int segments, uint32_t* __restrict__ start,
+                                    uint32_t* __restrict__ low, int32_t* flag) {
   extern __shared__ uint4 staged_words[];
   Entry* staged = reinterpret_cast<Entry*>(staged_words);
   const int pair = blockIdx.x;
@@ -241,21 +241,22 @@ __global__ void stream_index_kernel(StreamCall c, uint32_t* __restrict__ start, 
     for (int e = threadIdx.x; e < c.entries / kPer; e += blockDim.x) staged_words[e] = outside[e];
   }
   __syncthreads();
-  const int warp = threadIdx.x >> 5;
-  const int L = c.context - warp;
-  Entry* table = warp == 0 ? staged : staged + (1 << c.hash_bits) + chain_low_entries(c.qk_bits, L);
   const int64_t at = (int64_t)pair * c.capacity;
-  uint32_t* query_links = (warp == 0 ? start : low) + ((int64_t)h * c.tokens + off - len);
+  const int64_t row = (int64_t)h * c.tokens + off - len;
   if (!whole)
-    chain_index_warp<Entry, kMerge, true>(c.query_history + at, c.key_history + at, begin, end, L,
-                                          c.qk_bits, warp == 0, c.hash_bits, table, c.prev + at,
-                                          query_links);
+    chain_index_block<Entry, kMerge, true>(c.query_history + at, c.key_history + at, begin, end, c.context,
+                                           c.qk_bits, c.hash_bits, c.entries, segments, staged, c.prev + at,
+                                           start + row, low + row);
   else   // keys only: the query lanes index the keys a second time and leave nothing
-    chain_index_warp<Entry, false, true>(c.key_history + at, c.key_history + at, begin, end, L, c.qk_bits,
-                                         warp == 0, c.hash_bits, table, c.prev + at,
-                                         (uint32_t*)nullptr);
+    chain_index_block<Entry, false, true>(c.key_history + at, c.key_history + at, begin, end, c.context,
+                                          c.qk_bits, c.hash_bits, c.entries, segments, staged, c.prev + at,
+                                          (uint32_t*)nullptr, (uint32_t*)nullptr);
   __syncthreads();
-  for (int e = threadIdx.x; e < c.entries / kPer; e += blockDim.x) outside[e] = staged_words[e];
+  // the set of the last piece has seen everything (of the pieces that are not empty)
+  const int steps = (end - 1) / kChainStep - begin / kChainStep + 1;
+  const int per = (steps + segments - 1) / segments;
+  const uint4* newest = staged_words + (int64_t)((steps - 1) / per) * (c.entries / kPer);
+  for (int e = threadIdx.x; e < c.entries / kPer; e += blockDim.x) outside[e] = newest[e];
 }
 
 // Rows of a chunk over the histories of their slots.
@@ -322,11 +323,14 @@ int run_chunk(const StreamCall& c, int out_type, int vec_out, int max_chunk, cha
   {
     ProfileScope prof("stream_index", stream);
     if (c.context > 2) ROSA_CUDA_OK(cudaMemsetAsync(low, 0, (size_t)rows * sizeof(uint32_t), stream));
-    const int bytes = c.entries * (int)sizeof(Entry);
+    const int set_bytes = c.entries * (int)sizeof(Entry);
+    const int segments = chain_segments((int64_t)c.slots * c.H, max_chunk, set_bytes, c.context);
+    const int bytes = set_bytes * segments;
     auto kernel = c.context > 2 ? stream_index_kernel<Entry, true> : stream_index_kernel<Entry, false>;
     if (bytes > 48 * 1024)
       ROSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    kernel<<<(unsigned)(c.slots * c.H), 32 * c.context, bytes, stream>>>(c, start, low, flag);
+    kernel<<<(unsigned)(c.slots * c.H), 32 * c.context * segments, bytes, stream>>>(c, segments, start, low,
+                                                                                  flag);
     ROSA_CUDA_OK(cudaGetLastError());
   }
   auto match = [&](auto emit) -> int {
@@ -444,7 +448,7 @@ ROSA_B200_API int rosa_b200_stream_update_chained(const rosa_b200_stream_call* u
     auto kernel = wide ? stream_index_kernel<unsigned long long, false> : stream_index_kernel<uint32_t, false>;
     if (bytes > 48 * 1024)
       ROSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    kernel<<<(unsigned)(c.slots * c.H), 32 * c.context, bytes, st>>>(c, nullptr, nullptr, nullptr);
+    kernel<<<(unsigned)(c.slots * c.H), 32 * c.context, bytes, st>>>(c, 1, nullptr, nullptr, nullptr);
     ROSA_CUDA_OK(cudaGetLastError());
     return 0;
   }
