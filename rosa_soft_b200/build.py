@@ -21,7 +21,7 @@ LIB = os.path.join(PKG, "librosa_soft_b200.so")
 EXT = os.path.join(PKG, "_C.so")
 
 CUDA_SOURCES = ["plan.cu", "hard_forward.cu", "hard_forward_static.cu", "chain_match.cu", "stream_chain.cu", "surrogate_vjp.cu", "vjp_tiled.cu", "vjp_tiled_sweep2.cu", "stream_runtime.cu", "api.cu"]
-EXT_SOURCES = ["torch_binding.cpp", "stream_binding.cpp"]
+EXT_SOURCES = ["torch_binding.cpp", "autograd_binding.cpp", "stream_binding.cpp"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "--use_fast_math", "-Xcompiler", "-fPIC,-fvisibility=hidden", "--expt-relaxed-constexpr",
@@ -73,7 +73,8 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
 
 def build_extension(force: bool = False, verbose: bool = False) -> str:
     sources = [os.path.join(CSRC, f) for f in EXT_SOURCES]
-    deps = [*sources, os.path.join(ROOT, "include", "rosa_soft_b200.h"), LIB]
+    deps = [*sources, os.path.join(CSRC, "autograd_binding.h"),
+            os.path.join(ROOT, "include", "rosa_soft_b200.h"), LIB]
     if not force and _newer(EXT, deps):
         return EXT
     import torch

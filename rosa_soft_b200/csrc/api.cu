@@ -254,13 +254,16 @@ int run_hard_forward(const void* query, const void* key, const void* value, int 
     launch_build_plan(a.plan, st);
     ROSA_CUDA_OK(cudaGetLastError());
   }
-  if (query != nullptr)
+  if (query != nullptr) {
     if (int rc = launch_pack_symbols(query, key, dtype, N, H, D, dense, uniform_len, packed_query,
-                                     packed_key, st))
+                                     packed_key, a.context > 2 ? a.chain_low : nullptr, st))
       return rc;
+    a.low_is_zero = 1;
+  }
   if (int rc = launch_chain_index(a, max_len, st)) return rc;
   const bool bits = D <= kMaskSymbolBits;
-  const int limit = bits ? kChainLimitBits : kChainLimitScan;
+  // a short sequence walks its chains to the end: the stand-by launches would cost more
+  const int limit = max_len <= 512 ? 512 : bits ? kChainLimitBits : kChainLimitScan;
   if (int rc = launch_chain_forward(a, limit, st)) return rc;
   if (max_len <= limit) return 0;              // no chain is longer than its sequence
   return bits ? launch_match_bits(a, a.plan.status + 2, st)
@@ -294,7 +297,7 @@ ROSA_B200_API int rosa_b200_pack_symbols(const void* logits, int dtype, int64_t 
   if (dense)
     ROSA_REQUIRE(num_seq * uniform_len == N, "dense description needs num_seq * uniform_len == N");
   return launch_pack_symbols(logits, nullptr, dtype, N, H, D, dense, uniform_len, packed, nullptr,
-                             as_stream(stream));
+                             nullptr, as_stream(stream));
 }
 
 ROSA_B200_API int rosa_b200_hard_forward_packed(
@@ -369,8 +372,8 @@ ROSA_B200_API int rosa_b200_hard_inference(const uint32_t* query_symbols, const 
                                         st))
     return rc;
   if (int rc = launch_chain_index(a, max_len, st)) return rc;
-  if (int rc = launch_chain_inference(a, payload, out, matched_end, kChainLimitScan, st)) return rc;
-  if (max_len <= kChainLimitScan) return 0;
+  if (int rc = launch_chain_inference(a, payload, out, matched_end, max_len <= 512 ? 512 : kChainLimitScan, st)) return rc;
+  if (max_len <= 512) return 0;
   return launch_scan_inference(a, payload, out, matched_end, a.plan.status + 2, st);
 }
 
@@ -437,13 +440,28 @@ struct VjpCall {
   const int64_t* dropout_seed;
   float scale, dropout_p, mismatch_scale;
   int gradient_mask;
-  bool force_cuda_cores;
+  bool force_cuda_cores, typed_gradients;
   int64_t batch_offset, head_offset;
-  float *grad_query, *grad_key, *grad_value;
+  void *grad_query, *grad_key, *grad_value;
   void* workspace;
   size_t workspace_bytes;
   cudaStream_t stream;
 };
+
+// Largest mismatch-count sum of a window whose product P = exp(-m sum / D) is kept; smaller products
+// are taken as zero, in the evidence and in the adjoint alike.  What that leaves out, relative to
+// the largest adjoint of the diagonal: the evidence S_n >= exp(-m) changes by at most P (1 + W),
+// the cell adjoint C_n by the sum of W terms Sbar P with |Sbar| <= (1 + W) max|dS|, while the largest
+// |C| is at least exp(-m) max|dS|.  With P < 2^-30 exp(-m) / (1 + W)^2 both are below 2^-30, a
+// 64th of the last bit of float32; the logit error carries the factor scale as well.  (Products
+// below exp(-88) are zero in float32 with flush-to-zero anyway.)  The horizon of 32 tokens with
+// m = 3 has a typical product of exp(-50): it used to keep the windows of random symbols alive.
+int window_cutoff(float mismatch_scale, int D, int64_t W, float scale) {
+  const double lim = 30.0 * std::log(2.0) + mismatch_scale + 2.0 * std::log1p((double)W) +
+                     std::log1p((double)scale);
+  const double sum = std::min(88.0, lim) * D / mismatch_scale;
+  return sum < 1.0e9 ? (int)sum : 1000000000;
+}
 
 // The backward of `S` whole sequences (`N` tokens) starting at sequence `first_seq` of the call
 // (`first_seq` > 0 only for dense layouts, where it is also the token and dropout batch offset).
@@ -485,6 +503,7 @@ int run_vjp_slice(const VjpCall& c, int64_t first_seq, int64_t N, int64_t S, boo
   a.dropout_p = c.dropout_p;
   a.inv_keep = 1.0f / (1.0f - c.dropout_p);
   a.mismatch_scale = c.mismatch_scale;
+  a.window_cut = window_cutoff(c.mismatch_scale, D, c.W, c.scale);
   a.mask = c.gradient_mask;
   a.force_cuda_core_contraction = c.force_cuda_cores;
   a.batch_offset = (uint32_t)(c.batch_offset + first_seq);
@@ -498,14 +517,22 @@ int run_vjp_slice(const VjpCall& c, int64_t first_seq, int64_t N, int64_t S, boo
   a.dq_part = reinterpret_cast<float*>(ws + l.dq_off);
   a.dk_part = reinterpret_cast<float*>(ws + l.dk_off);
   a.dv_part = reinterpret_cast<float*>(ws + l.dv_off);
-  a.dq = c.grad_query ? c.grad_query + tok * H * D : nullptr;
-  a.dk = c.grad_key ? c.grad_key + tok * H * D : nullptr;
-  a.dv = c.grad_value ? c.grad_value + tok * Hv * Dv : nullptr;
+  a.typed_gradients = c.typed_gradients;
+  const size_t gsz = c.typed_gradients ? esz : sizeof(float);
+  auto grad_at = [&](void* p, size_t elements) {
+    return p != nullptr ? static_cast<void*>(static_cast<char*>(p) + elements * gsz) : nullptr;
+  };
+  a.dq = grad_at(c.grad_query, (size_t)tok * H * D);
+  a.dk = grad_at(c.grad_key, (size_t)tok * H * D);
+  a.dv = grad_at(c.grad_value, (size_t)tok * Hv * Dv);
 
-  launch_build_plan(a.plan, st);
-  ROSA_CUDA_OK(cudaGetLastError());
-  if (l.ring_bytes) ROSA_CUDA_OK(cudaMemsetAsync(a.ring, 0, l.ring_bytes, st));
-  if (int rc = launch_pack_value_bits(a.v, c.dtype, N, Hv, Dv, a.vbits, a.vwords, st)) return rc;
+  if (!dense) {   // dense batches need no tables
+    launch_build_plan(a.plan, st);
+    ROSA_CUDA_OK(cudaGetLastError());
+  }
+  if (l.ring_bytes && !vjp_tiled_applies(a))   // the tiled kernels read what they wrote only
+    ROSA_CUDA_OK(cudaMemsetAsync(a.ring, 0, l.ring_bytes, st));
+  if (int rc = launch_pack_value_bits(a, st)) return rc;
   if (int rc = launch_vjp_sweep1(a, (int)l.items_upper, st)) return rc;
   if (int rc = launch_vjp_rowstats(a, st)) return rc;
   if (int rc = launch_vjp_sweep2(a, (int)l.items_upper, st)) return rc;
@@ -518,7 +545,7 @@ ROSA_B200_API size_t rosa_b200_surrogate_vjp_workspace_bytes(int64_t N, int H, i
                                                int64_t max_suffix_length, int gradient_mask) {
   const bool dense = uniform_len > 0;
   const int64_t W = std::min<int64_t>(max_suffix_length, dense ? uniform_len : N);
-  gradient_mask &= ~ROSA_B200_MASK_CUDA_CORE_CONTRACTION;
+  gradient_mask &= ~(ROSA_B200_MASK_CUDA_CORE_CONTRACTION | ROSA_B200_MASK_TYPED_GRADIENTS);
   if (dense) {
     // the largest slice (slice 0) sizes the workspace that all slices share
     const int64_t n = vjp_dense_slices(H, D, Dv, num_seq, uniform_len, W, gradient_mask);
@@ -542,7 +569,8 @@ ROSA_B200_API int rosa_b200_surrogate_vjp(const void* query, const void* key, co
                              dtype))
     return rc;
   const int force_cuda_cores = gradient_mask & ROSA_B200_MASK_CUDA_CORE_CONTRACTION;
-  gradient_mask &= ~ROSA_B200_MASK_CUDA_CORE_CONTRACTION;
+  const bool typed = (gradient_mask & ROSA_B200_MASK_TYPED_GRADIENTS) != 0;
+  gradient_mask &= ~(ROSA_B200_MASK_CUDA_CORE_CONTRACTION | ROSA_B200_MASK_TYPED_GRADIENTS);
   ROSA_REQUIRE(gradient_mask >= 1 && gradient_mask <= 7,
                "gradient_mask must be an integer bit mask in [1, 7]");
   ROSA_REQUIRE(query && key && value && grad_output && packed_query && packed_key && workspace,
@@ -561,7 +589,7 @@ ROSA_B200_API int rosa_b200_surrogate_vjp(const void* query, const void* key, co
   const int64_t W = std::min<int64_t>(max_suffix_length, dense ? uniform_len : N);
   VjpCall c{query, key, value, grad_output, dtype, H, D, Hv, Dv, cu_seqlens, uniform_len, W,
             packed_query, packed_key, dropout_seed, scale, dropout_p, mismatch_scale,
-            gradient_mask, force_cuda_cores != 0, dropout_batch_offset, dropout_head_offset,
+            gradient_mask, force_cuda_cores != 0, typed, dropout_batch_offset, dropout_head_offset,
             grad_query, grad_key, grad_value, workspace, workspace_bytes, as_stream(stream)};
   if (!dense) return run_vjp_slice(c, 0, N, num_seq, false);
   // dense: slices of whole sequences (one slice unless the partial rows exceed their budget)

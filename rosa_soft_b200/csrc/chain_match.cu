@@ -70,7 +70,7 @@ int launch_chain_index(const FwdArgs& a, int64_t max_len, cudaStream_t stream) {
     const int more = chain_segments(heads, max_len, set_bytes(), a.context);
     if (more > segments) segments = more; else hash_bits = kChainHashBits;
   }
-  if (merge)   // several shorter lengths merge their results into zeroed words
+  if (merge && !a.low_is_zero)   // several shorter lengths merge their results into zeroed words
     ROSA_CUDA_OK(cudaMemsetAsync(a.chain_low, 0, (size_t)a.N * a.H * sizeof(uint32_t), stream));
   const size_t bytes = set_bytes() * segments;
   auto kernel = wide ? (merge ? chain_index_kernel<unsigned long long, true>

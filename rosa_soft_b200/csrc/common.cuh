@@ -143,6 +143,22 @@ __host__ __device__ __forceinline__ int dense_items(const Plan& plan) {
   return plan.uniform_len >= 2 ? (plan.uniform_len - 2 + plan.item_diagonals) / plan.item_diagonals : 0;
 }
 
+// Items of one sequence and the items, partial rows and checkpoint blocks (per head) before it.
+__device__ __forceinline__ void sequence_offsets(const Plan& plan, int s, int len, int* nitems,
+                                                 int64_t* items, int64_t* rows, int64_t* cks) {
+  if (plan.cu_seqlens == nullptr) {
+    *nitems = dense_items(plan);
+    *items = (int64_t)s * *nitems;
+    *rows = *items * len;
+    *cks = (int64_t)s * vjp_ck_count(len);
+  } else {
+    *items = plan.item_prefix[s];
+    *nitems = plan.item_prefix[s + 1] - plan.item_prefix[s];
+    *rows = plan.row_prefix[s];
+    *cks = plan.ck_prefix[s];
+  }
+}
+
 // Work item -> (sequence, item index inside the sequence); false when the slot is unused.
 __device__ __forceinline__ bool find_item(const Plan& plan, int slot, int* seq, int* local) {
   if (plan.cu_seqlens == nullptr) {   // dense: the same number of items in every sequence
@@ -300,6 +316,7 @@ struct FwdArgs {
   // chain_start null selects the run-length matcher alone (no workspace).
   uint32_t *chain_start, *chain_prev, *chain_low;
   int context;                    // chained context length
+  int low_is_zero;                // chain_low was cleared by an earlier kernel of the call
   // Per-symbol occurrence bitmaps of the key symbols, [H][2^D][mask_words] over the packed
   // token axis (bit g of row (h, s) set iff key symbol of token g, head h is s), for the rows
   // that the chained matcher gives up (D <= 8); they take the place of its scratch.
@@ -309,7 +326,7 @@ struct FwdArgs {
 
 int launch_pack_symbols(const void* q, const void* k, int dtype, int64_t N, int H, int D,
                         int dense, int64_t uniform_len, int32_t* packed_q, int32_t* packed_k,
-                        cudaStream_t stream);
+                        uint32_t* zeroed, cudaStream_t stream);
 // chained matcher (chain_match.cu): index, then match and results; a row whose chain is longer than
 // `limit` raises status[2] and stays pending
 int launch_chain_index(const FwdArgs& a, int64_t max_len, cudaStream_t stream);
@@ -369,6 +386,7 @@ struct VjpArgs {
   int vwords;
   const int64_t* seed;
   float scale, dropout_p, inv_keep, mismatch_scale;
+  int window_cut;                  // largest mismatch-count sum whose window product counts
   int mask;
   int force_cuda_core_contraction;  // debugging aid: contract on CUDA cores even when tcgen05 applies
   uint32_t batch_offset, head_offset;
@@ -382,13 +400,13 @@ struct VjpArgs {
   float* dq_part;                  // [item rows][D]
   float* dk_part;
   float* dv_part;                  // [item rows][Dv]
-  float* dq;
-  float* dk;
-  float* dv;
+  void* dq;                        // float32, or the input type with typed_gradients
+  void* dk;
+  void* dv;
+  int typed_gradients;
 };
 
-int launch_pack_value_bits(const void* v, int dtype, int64_t N, int Hv, int Dv, uint32_t* vbits,
-                           int vwords, cudaStream_t stream);
+int launch_pack_value_bits(const VjpArgs& a, cudaStream_t stream);
 int launch_vjp_sweep1(const VjpArgs& a, int items_upper, cudaStream_t stream);
 // register-tiled sweeps (vjp_tiled.cu): four diagonals per thread
 bool vjp_tiled_applies(const VjpArgs& a);

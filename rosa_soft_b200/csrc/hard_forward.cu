@@ -58,9 +58,11 @@ __device__ __forceinline__ uint32_t sign_word(const T* __restrict__ row, int D, 
 template <typename T>
 __global__ void pack_symbols_kernel(const T* __restrict__ q, const T* __restrict__ k, int64_t N,
                                     int H, int D, int dense, int64_t uniform_len, int vec,
-                                    int32_t* __restrict__ pq, int32_t* __restrict__ pk) {
+                                    int32_t* __restrict__ pq, int32_t* __restrict__ pk,
+                                    uint32_t* __restrict__ zeroed) {
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= N * H) return;
+  if (zeroed != nullptr) zeroed[idx] = 0u;         // scratch of the matcher, one word per token-head
   const int64_t token = idx / H;
   const int h = (int)(idx - token * H);
   const uint32_t wq = sign_word<T>(q + idx * D, D, vec != 0);
@@ -389,7 +391,7 @@ int launch_route_inspect(const unsigned long long* best, int64_t count, int32_t*
 }
 
 int launch_pack_symbols(const void* q, const void* k, int dtype, int64_t N, int H, int D,
-                        int dense, int64_t uniform_len, int32_t* pq, int32_t* pk,
+                        int dense, int64_t uniform_len, int32_t* pq, int32_t* pk, uint32_t* zeroed,
                         cudaStream_t stream) {
   ProfileScope prof("pack_symbols", stream);
   const int threads = 256;
@@ -399,13 +401,13 @@ int launch_pack_symbols(const void* q, const void* k, int dtype, int64_t N, int 
   const int vec = (D * esize) % 16 == 0 && aligned(q) && aligned(k);
   if (dtype == ROSA_B200_F32)
     pack_symbols_kernel<float><<<(unsigned)blocks, threads, 0, stream>>>(
-        (const float*)q, (const float*)k, N, H, D, dense, uniform_len, vec, pq, pk);
+        (const float*)q, (const float*)k, N, H, D, dense, uniform_len, vec, pq, pk, zeroed);
   else if (dtype == ROSA_B200_F16)
     pack_symbols_kernel<__half><<<(unsigned)blocks, threads, 0, stream>>>(
-        (const __half*)q, (const __half*)k, N, H, D, dense, uniform_len, vec, pq, pk);
+        (const __half*)q, (const __half*)k, N, H, D, dense, uniform_len, vec, pq, pk, zeroed);
   else
     pack_symbols_kernel<__nv_bfloat16><<<(unsigned)blocks, threads, 0, stream>>>(
-        (const __nv_bfloat16*)q, (const __nv_bfloat16*)k, N, H, D, dense, uniform_len, vec, pq, pk);
+        (const __nv_bfloat16*)q, (const __nv_bfloat16*)k, N, H, D, dense, uniform_len, vec, pq, pk, zeroed);
   ROSA_CUDA_OK(cudaGetLastError());
   return 0;
 }

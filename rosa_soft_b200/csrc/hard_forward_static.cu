@@ -111,7 +111,7 @@ extern "C" ROSA_B200_API int rosa_b200_hard_forward_static(
   // the winner table still holds the previous call's results: start every row from "no match"
   ROSA_CUDA_OK(cudaMemsetAsync(a.best, 0, (size_t)N * H * sizeof(unsigned long long), st));
   if (int rc = launch_pack_symbols(query, key, dtype, N, H, D, dense, uniform_len, packed_query,
-                                   packed_key, st))
+                                   packed_key, nullptr, st))
     return rc;
   if (int rc = launch_run_length_match(a, (int)items, st)) return rc;
   return launch_gather_output(a, st);

@@ -18,6 +18,7 @@
 #include <tuple>
 #include <vector>
 
+#include "autograd_binding.h"
 #include "rosa_soft_b200.h"
 
 namespace {
@@ -391,7 +392,8 @@ TORCH_LIBRARY_FRAGMENT(rosa_soft, m) {
 }
 
 PYBIND11_MODULE(_C, m) {
-  m.doc() = "rosa_soft_b200 operator registration and streaming state";
+  m.doc() = "rosa_soft_b200 operator registration, differentiable operator and streaming state";
+  bind_autograd(m);
   py::class_<StreamCore>(m, "StreamCore")
       .def(py::init<int64_t, int64_t, int64_t, int64_t, int64_t>())
       .def_property_readonly("slots", &StreamCore::slots)

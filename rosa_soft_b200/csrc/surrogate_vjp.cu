@@ -44,8 +44,11 @@ namespace {
 // ------------------------------------------------------------ value sign bits
 template <typename T>
 __global__ void pack_value_bits_kernel(const T* __restrict__ v, int64_t N, int Hv, int Dv,
-                                       uint32_t* __restrict__ vbits, int vwords) {
+                                       uint32_t* __restrict__ vbits, int vwords,
+                                       int32_t* __restrict__ status, int keep_mma_status) {
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  // without a plan kernel (dense batches) the first kernel of the call clears the status words
+  if (status != nullptr && idx < 4 && !(idx == 1 && keep_mma_status)) status[idx] = 0;
   if (idx >= N * Hv * vwords) return;
   const int wd = (int)(idx % vwords);
   const int64_t tv = idx / vwords;
@@ -180,8 +183,8 @@ __device__ __forceinline__ void fill_block_windows(const SweepSmem& sm, const It
 
 // Forward step of one diagonal: gate, window product, evidence.  Inactive cells (before the
 // diagonal starts) leave S and hs at zero.  With kSkipDeadWindow the exponential of the window
-// product is skipped when no lane of the warp has a sum small enough to survive flush-to-zero
-// (all lanes of the warp must then call together); that pays where the special-function unit
+// product is skipped when no lane of the warp has a sum small enough to count (VjpArgs::window_cut;
+// all lanes of the warp must then call together); that pays where the special-function unit
 // is loaded (sweep 2) and costs where integer issue binds (sweep 1).
 template <bool kSkipDeadWindow>
 __device__ __forceinline__ float forward_cell(float& S, int& hs, bool act, int qi, int kj,
@@ -193,9 +196,10 @@ __device__ __forceinline__ float forward_cell(float& S, int& hs, bool act, int q
   if (windowed) {
     hs += act ? ham : 0;
     hs -= (j > W) ? __popc(qold ^ kold) : 0;
-    if (!kSkipDeadWindow || __any_sync(0xffffffffu, j >= W && hs <= hs_cut)) {
+    const bool on = j >= W && hs <= hs_cut;
+    if (!kSkipDeadWindow || __any_sync(0xffffffffu, on)) {
       const float pw = __expf(neg_md * (float)hs);
-      P = (j >= W) ? pw : 0.0f;
+      P = on ? pw : 0.0f;
     }
   }
   const float Sn = x * (1.0f + S) - P;
@@ -243,7 +247,7 @@ __global__ void __launch_bounds__(kVjpBand) vjp_sweep1_kernel(VjpArgs a) {
   const int W = a.W;
   const float scale = a.scale, inv_keep = a.inv_keep;
   const float neg_md = -a.mismatch_scale / (float)a.D;
-  const int hs_cut = window_sum_cutoff(neg_md);
+  const int hs_cut = a.window_cut;
   constexpr bool windowed = kWindowed;
   constexpr bool use_dropout = kDropout;
   const DropoutKey dkey = make_dropout_key((uint32_t)it.h + a.head_offset,
@@ -423,8 +427,10 @@ __global__ void vjp_rowstats_kernel(VjpArgs a) {
   if (seq >= 0) {
     const int i = (int)(token - start);
     if (i >= 1) {
-      const int nitems = a.plan.item_prefix[seq + 1] - a.plan.item_prefix[seq];
-      const int64_t base = a.plan.row_prefix[seq] * a.H + (int64_t)h * nitems * (int64_t)len;
+      int nitems;
+      int64_t items_before, rows_before, cks_before;
+      sequence_offsets(a.plan, seq, len, &nitems, &items_before, &rows_before, &cks_before);
+      const int64_t base = rows_before * a.H + (int64_t)h * nitems * (int64_t)len;
       float m = 0.5f * a.scale, z = 1.0f, e = 0.0f;  // the null route
       for (int t = 0; t < nitems && 1 + (int64_t)t * a.plan.item_diagonals <= i; ++t) {
         const float4 p = a.stat_part[base + (int64_t)t * len + i];
@@ -483,7 +489,7 @@ __global__ void __launch_bounds__(kVjpBand, 2) vjp_sweep2_kernel(VjpArgs a) {
   const int W = a.W, D = a.D, mask = a.mask, ring_slots = a.ring_slots;
   const float scale = a.scale, inv_keep = a.inv_keep;
   const float neg_md = -a.mismatch_scale / (float)a.D;
-  const int hs_cut = window_sum_cutoff(neg_md);
+  const int hs_cut = a.window_cut;
   const bool windowed = W <= it.len - 2;
   const bool use_dropout = a.dropout_p > 0.0f;
   const float4* __restrict__ rowstat = a.rowstat + (int64_t)it.h * a.N + it.start;
@@ -850,7 +856,7 @@ __global__ void __launch_bounds__(kVjpBand, 2) vjp_sweep2_tc_kernel(VjpArgs a) {
   const int W = a.W, D = a.D, Dv = a.Dv, mask = a.mask, ring_slots = a.ring_slots;
   const float scale = a.scale, inv_keep = a.inv_keep;
   const float neg_md = -a.mismatch_scale / (float)a.D;
-  const int hs_cut = window_sum_cutoff(neg_md);
+  const int hs_cut = a.window_cut;
   const bool has_glo = a.dtype != ROSA_B200_BF16;   // bf16 grad_output is exact in one term
   const float4* __restrict__ rowstat = a.rowstat + (int64_t)it.h * a.N + it.start;
   float* ring = ring_slots ? a.ring + it.item_linear * (int64_t)ring_slots * kVjpBand + tid
@@ -1332,7 +1338,7 @@ __global__ void __launch_bounds__(kVjpBand, 2) vjp_sweep2_tc_kernel(VjpArgs a) {
         const int c = cbase + r, j = jbase + r;
         const float Sv = Sbuf[r * kVjpBand + tid];
         const int ham = __popc(sm.s_q[r] ^ sm.s_k[c]);
-        const float P = (act && j >= W) ? __expf(neg_md * (float)hs) : 0.0f;
+        const float P = (act && j >= W && hs <= hs_cut) ? __expf(neg_md * (float)hs) : 0.0f;
         hs += ((act && j > W) ? __popc(sm.s_qold[r] ^ sm.s_kold[c]) : 0) - (act ? ham : 0);
         const float x = sm.glut[ham];
         float pd;
@@ -1455,18 +1461,23 @@ __global__ void __launch_bounds__(kVjpBand, 2) vjp_sweep2_tc_kernel(VjpArgs a) {
 }
 
 // ------------------------------------------------------------------ finalize
-// Sums the per-item partials in item order and applies the softsign Jacobian.
-// which: 0 = query, 1 = key, 2 = value.  VEC = 4: a thread owns four consecutive components
-// (128-bit loads of the partial rows); VEC = 1 for rows that are not a multiple of four.
-template <int VEC>
-__global__ void vjp_finalize_kernel(VjpArgs a, int which) {
+// Sums the per-item partials in item order and applies the softsign Jacobian, for the query, key
+// and value gradients of one launch (`first_block` of each, in that order).  VEC = 4: a thread owns
+// four consecutive components (128-bit loads of the partial rows); VEC = 1 for rows that are not a
+// multiple of four.  Grad is float or the input type: the operator's gradients are float32, autograd
+// wants the input's type, and rounding here saves three passes over them.
+struct FinalizeBlocks {
+  unsigned first_block[3];
+};
+
+template <int VEC, typename Grad>
+__device__ __forceinline__ void finalize_one(const VjpArgs& a, int which, int64_t lin) {
   const int dim = which == 2 ? a.Dv : a.D;
   const int heads = which == 2 ? a.Hv : a.H;
   const int dimv = dim / VEC;
   // Threads run head-major over (head, token, component): the partial rows of one head and item
   // are contiguous over (token, component), so the reads of a warp coalesce; only the final
   // element access is strided by the head count.
-  const int64_t lin = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (lin >= a.N * heads * dimv) return;
   const int hh = (int)(lin / (a.N * dimv));
   const int64_t rem = lin - (int64_t)hh * a.N * dimv;
@@ -1493,8 +1504,10 @@ __global__ void vjp_finalize_kernel(VjpArgs a, int which) {
   };
   if (seq >= 0 && len >= 2) {
     const int i = (int)(token - start);
-    const int nitems = a.plan.item_prefix[seq + 1] - a.plan.item_prefix[seq];
-    const int64_t seq_base = a.plan.row_prefix[seq] * a.H;
+    int nitems;
+    int64_t items_before, rows_before, cks_before;
+    sequence_offsets(a.plan, seq, len, &nitems, &items_before, &rows_before, &cks_before);
+    const int64_t seq_base = rows_before * a.H;
     const int64_t id = a.plan.item_diagonals;
     // item t covers diagonals 1 + t id ..: query row i meets it iff 1 + t id <= i, key / value
     // row iff t id <= len - 2 - i (value rows are shifted by one)
@@ -1519,22 +1532,33 @@ __global__ void vjp_finalize_kernel(VjpArgs a, int which) {
   }
   const void* src = which == 0 ? a.q : which == 1 ? a.k : a.v;
   const float coef = which == 2 ? 1.0f : a.mismatch_scale / (2.0f * (float)a.D);
-  float* dst = which == 0 ? a.dq : which == 1 ? a.dk : a.dv;
+  Grad* dst = static_cast<Grad*>(which == 0 ? a.dq : which == 1 ? a.dk : a.dv);
   // the last position of a sequence is never a key: exact zero, whatever the input holds
   const bool never_key = which == 1 && seq >= 0 && token - start == len - 1;
-  float out[VEC];
+  alignas(sizeof(Grad) * VEC) Grad out[VEC];
 #pragma unroll
   for (int x = 0; x < VEC; ++x) {
     const float xv = load_as_float(src, idx + x, a.dtype);
     const float den = 1.0f + fabsf(xv);
-    out[x] = never_key ? 0.0f : coef * sum[x] / (den * den);
+    out[x] = (Grad)(never_key ? 0.0f : coef * sum[x] / (den * den));
   }
-  if (VEC == 4) {
-    *reinterpret_cast<float4*>(dst + idx) = make_float4(out[0], out[VEC > 1 ? 1 : 0],
-                                                        out[VEC > 2 ? 2 : 0], out[VEC > 3 ? 3 : 0]);
-  } else {
+  if constexpr (VEC == 1) {
     dst[idx] = out[0];
+  } else if constexpr (sizeof(Grad) == 4) {
+    *reinterpret_cast<float4*>(dst + idx) = *reinterpret_cast<const float4*>(out);
+  } else {
+    *reinterpret_cast<uint2*>(dst + idx) = *reinterpret_cast<const uint2*>(out);
   }
+}
+
+template <typename Grad>
+__global__ void __launch_bounds__(256) vjp_finalize_kernel(VjpArgs a, FinalizeBlocks blocks, int vec) {
+  const int which = blockIdx.x >= blocks.first_block[2] ? 2 : blockIdx.x >= blocks.first_block[1] ? 1 : 0;
+  const int64_t lin = (int64_t)(blockIdx.x - blocks.first_block[which]) * blockDim.x + threadIdx.x;
+  if (vec >> which & 1)
+    finalize_one<4, Grad>(a, which, lin);
+  else
+    finalize_one<1, Grad>(a, which, lin);
 }
 
 template <int DPAD, int DVPAD>
@@ -1597,21 +1621,19 @@ int launch_sweep2_d(const VjpArgs& a, int items_upper, cudaStream_t stream) {
 
 }  // namespace
 
-int launch_pack_value_bits(const void* v, int dtype, int64_t N, int Hv, int Dv, uint32_t* vbits,
-                           int vwords, cudaStream_t stream) {
+int launch_pack_value_bits(const VjpArgs& a, cudaStream_t stream) {
   ProfileScope prof("pack_value_bits", stream);
   const int threads = 256;
-  const int64_t total = N * Hv * vwords;
+  const int64_t total = a.N * a.Hv * a.vwords;
   const int64_t blocks = (total + threads - 1) / threads;
-  if (dtype == ROSA_B200_F32)
-    pack_value_bits_kernel<float><<<(unsigned)blocks, threads, 0, stream>>>((const float*)v, N, Hv,
-                                                                            Dv, vbits, vwords);
-  else if (dtype == ROSA_B200_F16)
-    pack_value_bits_kernel<__half><<<(unsigned)blocks, threads, 0, stream>>>((const __half*)v, N,
-                                                                             Hv, Dv, vbits, vwords);
-  else
-    pack_value_bits_kernel<__nv_bfloat16><<<(unsigned)blocks, threads, 0, stream>>>(
-        (const __nv_bfloat16*)v, N, Hv, Dv, vbits, vwords);
+  int32_t* status = a.plan.cu_seqlens == nullptr ? a.plan.status : nullptr;
+#define ROSA_PACK_VALUES(T)                                                                         \
+  pack_value_bits_kernel<T><<<(unsigned)blocks, threads, 0, stream>>>(                              \
+      (const T*)a.v, a.N, a.Hv, a.Dv, a.vbits, a.vwords, status, a.plan.keep_mma_status)
+  if (a.dtype == ROSA_B200_F32) ROSA_PACK_VALUES(float);
+  else if (a.dtype == ROSA_B200_F16) ROSA_PACK_VALUES(__half);
+  else ROSA_PACK_VALUES(__nv_bfloat16);
+#undef ROSA_PACK_VALUES
   ROSA_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -1681,22 +1703,33 @@ int launch_vjp_sweep2(const VjpArgs& a, int items_upper, cudaStream_t stream) {
 int launch_vjp_finalize(const VjpArgs& a, cudaStream_t stream) {
   ProfileScope prof("vjp_finalize", stream);
   const int threads = 256;
+  const int size = !a.typed_gradients || a.dtype == ROSA_B200_F32 ? 4 : 2;
+  FinalizeBlocks blocks{};
+  int vec = 0;
+  unsigned at = 0;
   for (int which = 0; which < 3; ++which) {
+    blocks.first_block[which] = at;
     if (!(a.mask >> which & 1)) continue;
     const int dim = which == 2 ? a.Dv : a.D;
-    float* dst = which == 0 ? a.dq : which == 1 ? a.dk : a.dv;
+    const void* dst = which == 0 ? a.dq : which == 1 ? a.dk : a.dv;
     const float* part = which == 0 ? a.dq_part : which == 1 ? a.dk_part : a.dv_part;
-    // whole float4 groups and 16-byte aligned rows on both sides: four components per thread
-    const bool vec = dim % 4 == 0 && ((reinterpret_cast<uintptr_t>(dst) |
-                                       reinterpret_cast<uintptr_t>(part)) & 15) == 0;
-    const int64_t total = a.N * (which == 2 ? (int64_t)a.Hv : (int64_t)a.H) * (vec ? dim / 4 : dim);
-    const int64_t blocks = (total + threads - 1) / threads;
-    if (vec)
-      vjp_finalize_kernel<4><<<(unsigned)blocks, threads, 0, stream>>>(a, which);
-    else
-      vjp_finalize_kernel<1><<<(unsigned)blocks, threads, 0, stream>>>(a, which);
-    ROSA_CUDA_OK(cudaGetLastError());
+    // whole groups of four and aligned rows on both sides: four components per thread
+    const bool whole = dim % 4 == 0 && reinterpret_cast<uintptr_t>(dst) % (4 * size) == 0 &&
+                       reinterpret_cast<uintptr_t>(part) % 16 == 0;
+    if (whole) vec |= 1 << which;
+    const int64_t total = a.N * (which == 2 ? (int64_t)a.Hv : (int64_t)a.H) * (whole ? dim / 4 : dim);
+    const int64_t count = (total + threads - 1) / threads;
+    ROSA_REQUIRE(at + count <= 0x7fffffff, "the gradients exceed the CUDA grid limit");
+    at += (unsigned)count;
   }
+  // a gradient that is not wanted starts where the next one does: no block falls to it
+  if (size == 4)
+    vjp_finalize_kernel<float><<<at, threads, 0, stream>>>(a, blocks, vec);
+  else if (a.dtype == ROSA_B200_F16)
+    vjp_finalize_kernel<__half><<<at, threads, 0, stream>>>(a, blocks, vec);
+  else
+    vjp_finalize_kernel<__nv_bfloat16><<<at, threads, 0, stream>>>(a, blocks, vec);
+  ROSA_CUDA_OK(cudaGetLastError());
   return 0;
 }
 

@@ -273,17 +273,17 @@ Triple run_surrogate_vjp(const Tensor& query, const Tensor& key, const Tensor& v
                          const Tensor& cu, const Tensor& grad_output, const Tensor& packed_q,
                          const Tensor& packed_k, const Tensor& seed, int64_t max_suffix_length,
                          double scale, double dropout_p, double mismatch_scale, int64_t mask,
-                         int64_t batch_offset, int64_t head_offset) {
+                         int64_t batch_offset, int64_t head_offset, bool typed) {
   const Call c = describe_call(query, key, value, cu, max_suffix_length);
   check_backward_extras(c, query, grad_output, packed_q, packed_k, seed, dropout_p, mask);
   const Controls sc = narrow_controls(c.horizon, scale, dropout_p, mismatch_scale);
   const c10::cuda::CUDAGuard guard(query.device());
   const Tensor go = grad_output.contiguous();
   const Tensor pq = packed_q.contiguous(), pk = packed_k.contiguous(), sd = seed.contiguous();
-  const auto f32 = c.q.options().dtype(torch::kFloat32);
-  Tensor dq = (mask & 1) ? torch::empty(c.q.sizes(), f32) : torch::empty({0}, f32);
-  Tensor dk = (mask & 2) ? torch::empty(c.k.sizes(), f32) : torch::empty({0}, f32);
-  Tensor dv = (mask & 4) ? torch::empty(c.v.sizes(), f32) : torch::empty({0}, f32);
+  const auto options = typed ? c.q.options() : c.q.options().dtype(torch::kFloat32);
+  Tensor dq = (mask & 1) ? torch::empty(c.q.sizes(), options) : torch::empty({0}, options);
+  Tensor dk = (mask & 2) ? torch::empty(c.k.sizes(), options) : torch::empty({0}, options);
+  Tensor dv = (mask & 4) ? torch::empty(c.v.sizes(), options) : torch::empty({0}, options);
   const size_t bytes = rosa_b200_surrogate_vjp_workspace_bytes(
       c.tokens, (int)c.heads, (int)c.bits, (int)c.value_heads, (int)c.value_dim, c.sequences,
       c.uniform_len, c.horizon, (int)mask);
@@ -293,10 +293,11 @@ Triple run_surrogate_vjp(const Tensor& query, const Tensor& key, const Tensor& v
                (int)c.heads, (int)c.bits, (int)c.value_heads, (int)c.value_dim, c.offsets(),
                c.sequences, c.uniform_len, c.horizon, pq.data_ptr<int32_t>(),
                pk.data_ptr<int32_t>(), sc.dropout_p > 0.0f ? sd.data_ptr<int64_t>() : nullptr,
-               sc.scale, sc.dropout_p, sc.mismatch_scale, (int)mask, batch_offset, head_offset,
-               (mask & 1) ? dq.data_ptr<float>() : nullptr,
-               (mask & 2) ? dk.data_ptr<float>() : nullptr,
-               (mask & 4) ? dv.data_ptr<float>() : nullptr, ws.data_ptr(), bytes,
+               sc.scale, sc.dropout_p, sc.mismatch_scale,
+               (int)mask | (typed ? ROSA_B200_MASK_TYPED_GRADIENTS : 0), batch_offset, head_offset,
+               (mask & 1) ? static_cast<float*>(dq.data_ptr()) : nullptr,
+               (mask & 2) ? static_cast<float*>(dk.data_ptr()) : nullptr,
+               (mask & 4) ? static_cast<float*>(dv.data_ptr()) : nullptr, ws.data_ptr(), bytes,
                at::cuda::getCurrentCUDAStream().stream()),
            "surrogate_vjp");
   maybe_check_status(ws, "surrogate_vjp");
@@ -318,7 +319,7 @@ Triple surrogate_vjp_masked_op(Tensor query, Tensor key, Tensor value, Tensor gr
                                double dropout_p, double mismatch_scale, int64_t gradient_mask) {
   return run_surrogate_vjp(query, key, value, Tensor(), grad_output, packed_query_symbols,
                            packed_key_symbols, dropout_seed, max_suffix_length, scale, dropout_p,
-                           mismatch_scale, gradient_mask, 0, 0);
+                           mismatch_scale, gradient_mask, 0, 0, false);
 }
 
 Triple surrogate_vjp_varlen_masked_op(Tensor query, Tensor key, Tensor value, Tensor cu_seqlens,
@@ -328,7 +329,13 @@ Triple surrogate_vjp_varlen_masked_op(Tensor query, Tensor key, Tensor value, Te
                                       double mismatch_scale, int64_t gradient_mask) {
   return run_surrogate_vjp(query, key, value, cu_seqlens, grad_output, packed_query_symbols,
                            packed_key_symbols, dropout_seed, max_suffix_length, scale, dropout_p,
-                           mismatch_scale, gradient_mask, 0, 0);
+                           mismatch_scale, gradient_mask, 0, 0, false);
+}
+
+void check_shard_offsets(int64_t batch_offset, int64_t head_offset) {
+  TORCH_CHECK(batch_offset >= 0 && head_offset >= 0 && batch_offset <= kInt32Max &&
+                  head_offset <= kInt32Max,
+              "shard offsets must be non-negative 32-bit values");
 }
 
 // A shard of a larger problem: same as the masked operators plus the global coordinates of
@@ -339,13 +346,25 @@ Triple surrogate_vjp_sharded_op(Tensor query, Tensor key, Tensor value,
                                 Tensor dropout_seed, int64_t max_suffix_length, double scale,
                                 double dropout_p, double mismatch_scale, int64_t gradient_mask,
                                 int64_t batch_offset, int64_t head_offset) {
-  TORCH_CHECK(batch_offset >= 0 && head_offset >= 0 && batch_offset <= kInt32Max &&
-                  head_offset <= kInt32Max,
-              "shard offsets must be non-negative 32-bit values");
+  check_shard_offsets(batch_offset, head_offset);
   return run_surrogate_vjp(query, key, value, cu_seqlens.has_value() ? *cu_seqlens : Tensor(),
                            grad_output, packed_query_symbols, packed_key_symbols, dropout_seed,
                            max_suffix_length, scale, dropout_p, mismatch_scale, gradient_mask,
-                           batch_offset, head_offset);
+                           batch_offset, head_offset, false);
+}
+
+// The backward that autograd calls: dense or packed, shard offsets, gradients in the input's type.
+Triple surrogate_vjp_typed_op(Tensor query, Tensor key, Tensor value, std::optional<Tensor> cu_seqlens,
+                              Tensor grad_output, Tensor packed_query_symbols,
+                              Tensor packed_key_symbols, Tensor dropout_seed,
+                              int64_t max_suffix_length, double scale, double dropout_p,
+                              double mismatch_scale, int64_t gradient_mask, int64_t batch_offset,
+                              int64_t head_offset) {
+  check_shard_offsets(batch_offset, head_offset);
+  return run_surrogate_vjp(query, key, value, cu_seqlens.has_value() ? *cu_seqlens : Tensor(),
+                           grad_output, packed_query_symbols, packed_key_symbols, dropout_seed,
+                           max_suffix_length, scale, dropout_p, mismatch_scale, gradient_mask,
+                           batch_offset, head_offset, true);
 }
 
 // Batched hard inference: query/key symbols int32 [streams, T, H] (or packed [N, H] with
@@ -408,6 +427,7 @@ TORCH_LIBRARY(rosa_soft, m) {
   m.def("surrogate_vjp_masked(Tensor query, Tensor key, Tensor value, Tensor grad_output, Tensor packed_query_symbols, Tensor packed_key_symbols, Tensor dropout_seed, int max_suffix_length, float scale, float dropout_p, float mismatch_scale, int gradient_mask) -> (Tensor grad_query, Tensor grad_key, Tensor grad_value)");
   m.def("surrogate_vjp_varlen_masked(Tensor query, Tensor key, Tensor value, Tensor cu_seqlens, Tensor grad_output, Tensor packed_query_symbols, Tensor packed_key_symbols, Tensor dropout_seed, int max_suffix_length, float scale, float dropout_p, float mismatch_scale, int gradient_mask) -> (Tensor grad_query, Tensor grad_key, Tensor grad_value)");
   m.def("surrogate_vjp_sharded(Tensor query, Tensor key, Tensor value, Tensor? cu_seqlens, Tensor grad_output, Tensor packed_query_symbols, Tensor packed_key_symbols, Tensor dropout_seed, int max_suffix_length, float scale, float dropout_p, float mismatch_scale, int gradient_mask, int batch_offset, int head_offset) -> (Tensor grad_query, Tensor grad_key, Tensor grad_value)");
+  m.def("surrogate_vjp_typed(Tensor query, Tensor key, Tensor value, Tensor? cu_seqlens, Tensor grad_output, Tensor packed_query_symbols, Tensor packed_key_symbols, Tensor dropout_seed, int max_suffix_length, float scale, float dropout_p, float mismatch_scale, int gradient_mask, int batch_offset, int head_offset) -> (Tensor grad_query, Tensor grad_key, Tensor grad_value)");
   m.def("hard_inference(Tensor query_symbols, Tensor key_symbols, Tensor payload, Tensor? cu_seqlens, int max_suffix_length) -> (Tensor output, Tensor matched_key_end_positions)");
 }
 
@@ -417,6 +437,7 @@ TORCH_LIBRARY_IMPL(rosa_soft, CUDA, m) {
   m.impl("surrogate_vjp_masked", &surrogate_vjp_masked_op);
   m.impl("surrogate_vjp_varlen_masked", &surrogate_vjp_varlen_masked_op);
   m.impl("surrogate_vjp_sharded", &surrogate_vjp_sharded_op);
+  m.impl("surrogate_vjp_typed", &surrogate_vjp_typed_op);
   m.impl("hard_inference", &hard_inference_op);
 }
 #endif

@@ -60,14 +60,6 @@ __device__ __forceinline__ float warp_reduce8(const float (&v)[8], int lane) {
   return c;
 }
 
-// Largest mismatch-count sum whose window product exp(-m * hs / D) is not flushed to zero
-// (the kernels are compiled with flush-to-zero: exp(x) == 0 for x <= -88).
-__device__ __forceinline__ int window_sum_cutoff(float neg_md) {
-  if (!(neg_md < 0.0f)) return 1000000000;
-  const float lim = -88.0f / neg_md;
-  return lim < 1.0e9f ? (int)lim : 1000000000;
-}
-
 // Work item of a 1-D grid.  Heads vary fastest; for a dense batch the sequences vary next and
 // the item index slowest, so that the longest items (the bands next to the main diagonal) of ALL
 // sequences and heads are scheduled first and the tail of the launch consists of the shortest
@@ -76,8 +68,7 @@ __device__ __forceinline__ int window_sum_cutoff(float neg_md) {
 __device__ __forceinline__ bool load_item_1d(const VjpArgs& a, Item* o) {
   const int slot = blockIdx.x / a.H;
   if (a.plan.cu_seqlens == nullptr) {
-    if (a.plan.status[0] != 0) return false;
-    const int per = a.plan.item_prefix[1];          // items of every sequence
+    const int per = dense_items(a.plan);            // items of every sequence
     if (per <= 0 || slot >= per * a.plan.S) return false;
     o->it = slot / a.plan.S;
     o->seq = slot - o->it * a.plan.S;
@@ -85,16 +76,16 @@ __device__ __forceinline__ bool load_item_1d(const VjpArgs& a, Item* o) {
     return false;
   }
   o->h = blockIdx.x - slot * a.H;
-  o->start = a.plan.seg_start[o->seq];
-  o->len = a.plan.seg_len[o->seq];
-  o->nitems = a.plan.item_prefix[o->seq + 1] - a.plan.item_prefix[o->seq];
+  segment_bounds(a.plan, o->seq, &o->start, &o->len);
+  int64_t items_before, rows_before, cks_before;
+  sequence_offsets(a.plan, o->seq, o->len, &o->nitems, &items_before, &rows_before, &cks_before);
   const int nbands = (int)vjp_bands(o->len);
   o->w_begin = o->it * a.bands_per_item;
   o->w_end = min(nbands, o->w_begin + a.bands_per_item);
-  o->rowslot = a.plan.row_prefix[o->seq] * a.H +
+  o->rowslot = rows_before * a.H +
                ((int64_t)o->h * o->nitems + o->it) * (int64_t)o->len;
-  o->ck_base = a.plan.ck_prefix[o->seq] * a.H + (int64_t)o->h * vjp_ck_count(o->len);
-  o->item_linear = (int64_t)a.plan.item_prefix[o->seq] * a.H + (int64_t)o->h * o->nitems + o->it;
+  o->ck_base = cks_before * a.H + (int64_t)o->h * vjp_ck_count(o->len);
+  o->item_linear = items_before * a.H + (int64_t)o->h * o->nitems + o->it;
   return true;
 }
 

@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kTThreads, 8) vjp_sweep1_tiled_kernel(VjpArgs 
   p.W = W;
   p.len = it.len;
   p.neg_md = -a.mismatch_scale / (float)a.D;
-  p.hs_cut = window_sum_cutoff(p.neg_md);
+  p.hs_cut = a.window_cut;
   const float logit_mul = kSqrtScale * a.scale;
   const float ref_top = a.scale * kSqrtScale * (sqrtf(1.0f + (float)W) - 1.0f);
   p.mul2 = logit_mul * 1.4426950408889634f;

@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(kS2Threads) vjp_sweep2_tiled_pair_kernel(VjpAr
   const int W = a.W, D = a.D, Dv = a.Dv, mask = a.mask, ring_slots = a.ring_slots;
   const bool windowed = ring_slots > 0;
   const float neg_md = -a.mismatch_scale / (float)a.D;
-  const int hs_cut = window_sum_cutoff(neg_md);
+  const int hs_cut = a.window_cut;
   const float4* __restrict__ rowstat = a.rowstat + (int64_t)it.h * a.N + it.start;
   float* ring = ring_slots ? a.ring + it.item_linear * (int64_t)ring_slots * kS2Band + kS2R * tid
                            : nullptr;
@@ -392,8 +392,8 @@ __global__ void __launch_bounds__(kS2Threads) vjp_sweep2_tiled_pair_kernel(VjpAr
   // per-band state of the thread's two diagonals
   float sb[2] = {0.f, 0.f}, xnext[2] = {0.f, 0.f};
   double Sbar[2] = {0.0, 0.0}, Y[2] = {0.0, 0.0};
-  int live = 0;
-  bool ring_dirty = false;
+  int live = 0;          // rows until the last live window product has left the window
+  int age = 0;           // rows since the live stretch began
   Prefetch pf;
   {
     prefetch_load(geom_of(w, rb), pf);
@@ -410,7 +410,6 @@ __global__ void __launch_bounds__(kS2Threads) vjp_sweep2_tiled_pair_kernel(VjpAr
       sb[0] = sb[1] = xnext[0] = xnext[1] = 0.0f;
       Sbar[0] = Sbar[1] = Y[0] = Y[1] = 0.0;
       live = 0;
-      ring_dirty = false;
       // the bottom block of a band refills the whole kz^T ring: the last block of the previous
       // band must have released it
       if (prev_pending) {
@@ -575,12 +574,12 @@ __global__ void __launch_bounds__(kS2Threads) vjp_sweep2_tiled_pair_kernel(VjpAr
         const int qo = s_qold[r];
         float Cv[2], pd[2], Pv[2], gate[2], dS[2];
         bool act[2];
-        // the ring line of this row is requested first: while no window product has been alive
-        // for W + 2 rows the ring holds zeros and nothing is read
+        // the ring line of this row is requested first; it was written W + 1 rows ago, or not at
+        // all if the live stretch is younger than that (the ring needs no clearing)
         float* line = ring + (int64_t)slot * kS2Band;
         slot = (slot == 0 ? ring_slots : slot) - 1;
         float2 old_t = make_float2(0.0f, 0.0f);
-        if (live > 0) old_t = *reinterpret_cast<const float2*>(line);
+        if (live > 0 && age > W) old_t = *reinterpret_cast<const float2*>(line);
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const int c = r + kS2Band - 1 - kS2R * tid - e;
@@ -589,7 +588,7 @@ __global__ void __launch_bounds__(kS2Threads) vjp_sweep2_tiled_pair_kernel(VjpAr
           const uint32_t hoff = (hb >> (8 * ((r & 1) * 2 + e))) & 0xffu;
           const int ham = (int)(hoff >> 2);
           gate[e] = glut[ham];
-          Pv[e] = (act[e] && j >= W) ? __expf(neg_md * (float)hs[e]) : 0.0f;
+          Pv[e] = (act[e] && j >= W && hs[e] <= hs_cut) ? __expf(neg_md * (float)hs[e]) : 0.0f;
           hs[e] += ((act[e] && j > W) ? __popc(qo ^ s_kold[c]) : 0) - (act[e] ? ham : 0);
           const float Se = e == 0 ? Sv2.x : Sv2.y;
           const float t = 1.0f + Se;
@@ -604,8 +603,8 @@ __global__ void __launch_bounds__(kS2Threads) vjp_sweep2_tiled_pair_kernel(VjpAr
         }
         const bool any_p = __any_sync(0xffffffffu, Pv[0] != 0.0f || Pv[1] != 0.0f);
         if (any_p) {
+          if (live == 0) age = 0;
           live = W + 2;
-          ring_dirty = true;
         }
         if (live > 0) {
 #pragma unroll
@@ -616,6 +615,7 @@ __global__ void __launch_bounds__(kS2Threads) vjp_sweep2_tiled_pair_kernel(VjpAr
               line[e] = tf;
               Y[e] += (double)tf - (double)old;
             }
+          ++age;
           if (--live == 0) Y[0] = Y[1] = 0.0;
         }
 #pragma unroll
@@ -711,12 +711,6 @@ __global__ void __launch_bounds__(kS2Threads) vjp_sweep2_tiled_pair_kernel(VjpAr
     }
 #endif /* ROSA_S2_PAIR */
     buf ^= 1;
-    // leave the ring zeroed for the next band of this item
-    if (!next_same && ring != nullptr && ring_dirty && has_next)
-      for (int sl = 0; sl < ring_slots; ++sl) {
-        ring[(int64_t)sl * kS2Band] = 0.0f;
-        ring[(int64_t)sl * kS2Band + 1] = 0.0f;
-      }
     if (!has_next) break;
     band_start = !next_same;
     if (next_same) {
