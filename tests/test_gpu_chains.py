@@ -1,0 +1,205 @@
+"""The chained matcher and the streaming state that is built on it, where they can go wrong: lengths
+around a step of 16 positions and a tile of 32 rows, every context length, horizons below it, rows on
+chains too long to follow, histories whose step numbers need wide table entries; and the native form
+of the differentiable call against the Python one.  All results are exact."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import rosa_oracle as orc
+from tests.helpers import nonzero_randn
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _streams(n, heads, bits, seed, alphabet=None, copies=True):
+    """Query and key symbols [n, heads] (uint32); the query stream repeats passages of the key's."""
+    rng = np.random.default_rng(seed)
+    letters = rng.integers(0, 1 << bits, size=alphabet or 1 << min(bits, 16), dtype=np.uint64)
+    if alphabet is None and bits <= 16:
+        letters = np.arange(1 << bits, dtype=np.uint64)
+    q, k = (letters[rng.integers(0, len(letters), size=(n, heads))].astype(np.uint32) for _ in range(2))
+    if copies:
+        for _ in range(max(1, n // 64)):
+            length = int(rng.integers(1, 41))
+            if n > 2 * length:
+                src, dst = (int(x) for x in rng.integers(0, n - length, size=2))
+                q[dst:dst + length] = k[src:src + length]
+    return q, k
+
+
+def _logits(symbols, bits):
+    ones = (symbols[..., None] >> np.arange(bits, dtype=np.uint32)) & 1
+    return torch.from_numpy(np.where(ones == 1, 0.7, -0.7).astype(np.float32)).to(DEV)
+
+
+LENGTHS = (1, 15, 16, 17, 31, 33, 129, 256, 511)
+
+
+@pytest.mark.parametrize("bits,W,alphabet", [
+    (1, 300, None), (1, 5, None), (2, 64, None), (3, 2, None), (3, 64, None), (4, 3, None), (5, 32, None),
+    (6, 1, None), (7, 16, None), (8, 32, None), (11, 32, None), (12, 32, 40), (16, 20, 300), (32, 32, 60),
+    (1, 40, 1), (8, 300, 2), (20, 300, 2)])          # the last three: chains too long to follow
+def test_routes_of_packed_sequences_equal_the_oracle(bits, W, alphabet):
+    from rosa_soft_b200 import cabi
+    H = 3
+    cu = np.concatenate([[0], np.cumsum(LENGTHS)])
+    q, k = _streams(int(cu[-1]), H, bits, 17 * bits + W, alphabet)
+    v = nonzero_randn((int(cu[-1]), 1, 3), 5).to(DEV)
+    _, _, _, routes, _ = cabi.hard_forward(_logits(q, bits), _logits(k, bits), v,
+                                           torch.from_numpy(cu.astype(np.int32)).to(DEV), W)
+    _, want = orc.hard_forward(_logits(q, bits).cpu().numpy(), _logits(k, bits).cpu().numpy(),
+                               v.cpu().numpy(), cu, W)
+    starts = np.repeat(cu[:-1], LENGTHS)[:, None]
+    assert np.array_equal(routes.cpu().numpy(), np.where(want > 0, want + starts, -1))
+
+
+@pytest.mark.parametrize("T", (2047, 4096, 4113))
+@pytest.mark.parametrize("bits,W", [(2, 200), (8, 32), (32, 32)])
+def test_long_sequences_of_few_heads_are_indexed_in_pieces(bits, W, T):
+    import rosa_soft_b200 as rs
+    from rosa_soft_b200 import cabi
+    H = 2
+    q, k = _streams(T, H, bits, T + bits, None if bits <= 8 else 500)
+    pay = np.random.default_rng(3).standard_normal((T, 1, 4)).astype(np.float32)
+    want_out, want_end = orc.hard_inference(q, k, pay, np.array([0, T]), W)
+    as_int = lambda x: torch.from_numpy(x.view(np.int32))[None].to(DEV)  # noqa: E731
+    out, end = rs.rosa_hard_inference(as_int(q), as_int(k), torch.from_numpy(pay)[None].to(DEV),
+                                      max_suffix_length=W)
+    assert np.array_equal(end[0].cpu().numpy(), want_end)
+    assert np.array_equal(out[0].cpu().numpy(), want_out)
+    if bits <= 8:
+        routes = cabi.hard_forward(_logits(q, bits), _logits(k, bits), torch.from_numpy(pay).to(DEV), (1, T),
+                                   W)[3]
+        assert np.array_equal(routes.cpu().numpy(), np.where(want_end >= 0, want_end + 1, -1))
+
+
+def _latest_longest(q, k, i, W):
+    """End position of the latest longest match of row i, by a look at all earlier positions."""
+    j = np.flatnonzero(k[:i] == q[i])
+    length = 1
+    while len(j) and length < W:
+        longer = j[j >= length]
+        longer = longer[k[longer - length] == q[i - length]]
+        if len(longer) == 0:
+            break
+        j, length = longer, length + 1
+    return int(j[-1]) if len(j) else -1
+
+
+def test_histories_beyond_the_narrow_table_entries():
+    """More than 65535 steps of 16 positions: training forward, batched inference and stream."""
+    import rosa_soft_b200 as rs
+    from rosa_soft_b200 import cabi
+    T, W, bits = 65535 * 16 + 200, 24, 8
+    q, k = _streams(T, 1, bits, 9)
+    q[T - 120:T - 80] = k[1000:1040]
+    q[T - 60:T - 30] = k[T - 150:T - 120]
+    rows = np.concatenate([np.arange(T - 300, T), np.arange(40)])
+    want = np.array([_latest_longest(q[:, 0], k[:, 0], int(i), W) for i in rows])
+    v = torch.randn(T, 1, 4, device=DEV)
+    routes = cabi.hard_forward(_logits(q, bits), _logits(k, bits), v, (1, T), W)[3].cpu().numpy()[rows, 0]
+    assert np.array_equal(routes, np.where(want >= 0, want + 1, -1))
+    as_int = lambda x: torch.from_numpy(x.view(np.int32))[None].to(DEV)  # noqa: E731
+    _, end = rs.rosa_hard_inference(as_int(q), as_int(k), v[None], max_suffix_length=W)
+    assert np.array_equal(end[0, :, 0].cpu().numpy()[rows], want)
+    byte = lambda x: torch.from_numpy(x.astype(np.uint8))[None].to(DEV)  # noqa: E731
+    tq, tk = byte(q), byte(k)
+    ends = []
+    with rs.RosaRuntime(1, 1, bits, bits, W) as runtime:
+        cuts = [0, 5000, 65535 * 16 - 8, T - 120, *range(T - 60, T, 7), T]   # prompts, then steps
+        for a, b in zip(cuts[:-1], cuts[1:]):
+            ends.append(runtime.update_packed(tq[:, a:b], tk[:, a:b], tk[:, a:b])[1])
+    assert np.array_equal(torch.cat(ends, dim=1)[0, :, 0].cpu().numpy()[rows], want)
+
+
+@pytest.mark.parametrize("bits,W,alphabet", [(1, 40, None), (1, 200, 1), (3, 2, None), (8, 32, 30), (8, 1, None)])
+@pytest.mark.parametrize("form", ("packed", "float32", "bfloat16"))
+def test_steps_and_chunks_of_a_stream_equal_one_pass(form, bits, W, alphabet):
+    """Chunks on both sides of the 16 tokens of the one-kernel step, over two growths of the state."""
+    from rosa_soft_b200 import RosaRuntime
+    H, Hp, B, pay_bits = 4, 2, 2, 5
+    chunks = [1, 16, 17, 15, 1, 33, 16, 16, 2, 120, 16, 1, 40, 250, 5, 16, 17]
+    T = sum(chunks)
+    q, k = _streams(B * T, H, bits, 3 * bits + W, alphabet)
+    pay = np.random.default_rng(1).integers(0, 1 << pay_bits, size=(B * T, Hp)).astype(np.uint32)
+    cu = np.arange(B + 1) * T
+    want, want_end = orc.hard_inference(q, k, pay.astype(np.float32)[..., None], cu, W)
+    shape = lambda x, n: x.reshape(B, T, n)  # noqa: E731
+    got, ends = [], []
+    runtime = RosaRuntime(H, Hp, bits, pay_bits, W)
+    at = 0
+    for n in chunks:
+        part = [shape(x, heads)[:, at:at + n] for x, heads in ((q, H), (k, H), (pay, Hp))]
+        if form == "packed":
+            out, end = runtime.update_packed(*(torch.from_numpy(x.astype(np.uint8)).to(DEV) for x in part))
+        else:
+            dt = getattr(torch, form)
+            out, end = runtime.update(_logits(part[0], bits).to(dt), _logits(part[1], bits).to(dt),
+                                      _logits(part[2], pay_bits).to(dt))
+            assert out.dtype == dt
+        got.append(out)
+        ends.append(end)
+        at += n
+    end = torch.cat(ends, dim=1).cpu().numpy().reshape(-1, H)
+    out = torch.cat(got, dim=1).float().cpu().numpy()
+    assert np.array_equal(end, want_end)
+    if form == "packed":
+        assert np.array_equal(out.reshape(-1, H), want[:, :, 0])
+    else:
+        signs = 2.0 * ((want.astype(np.int64) >> np.arange(pay_bits)) & 1) - 1.0
+        signs[want_end < 0] = 0.0
+        assert np.array_equal(out.reshape(-1, H, pay_bits), signs)
+
+
+@pytest.mark.parametrize("dtype", (torch.float32, torch.float16, torch.bfloat16))
+@pytest.mark.parametrize("packed", (False, True))
+def test_native_call_equals_the_python_form(dtype, packed):
+    import rosa_soft_b200 as rs
+    from rosa_soft_b200 import soft
+    H, D, Hv, Dv, W = 4, 5, 2, 3, 9
+    lead = (70,) if packed else (2, 35)
+    cu = torch.tensor([0, 20, 21, 70], dtype=torch.int32, device=DEV) if packed else None
+    q, k, v, go = (nonzero_randn((*lead, *s), 40 + n, dtype).to(DEV)
+                   for n, s in enumerate(((H, D), (H, D), (Hv, Dv), (H, Dv))))
+
+    def grads(call, wanted):
+        leaves = [t.clone().requires_grad_(n in wanted) for n, t in enumerate((q, k, v))]
+        torch.cuda.manual_seed(11)
+        out = call(*leaves)
+        return [out.detach(), *torch.autograd.grad(out, [t for n, t in enumerate(leaves) if n in wanted], go)]
+
+    controls = dict(max_suffix_length=W, scale=1.2, dropout_p=0.2, mismatch_scale=3.0)
+    native = (lambda *t: rs.rosa_soft_varlen(*t, cu, **controls)) if packed else (
+        lambda *t: rs.rosa_soft(*t, **controls))
+    python = lambda *t: soft._run(*t, cu, min(W, lead[-1]), 1.2, 0.2, 3.0)  # noqa: E731
+    for wanted in ((0, 1, 2), (0,), (2,), (1, 2)):
+        for a, b in zip(grads(native, wanted), grads(python, wanted)):
+            assert a.dtype == dtype and torch.equal(a, b)
+
+
+def test_native_call_keeps_the_rules_of_autograd():
+    import rosa_soft_b200 as rs
+    q, k = (nonzero_randn((1, 24, 2, 4), s).to(DEV).requires_grad_(True) for s in (1, 2))
+    v = nonzero_randn((1, 24, 2, 3), 3).to(DEV).requires_grad_(True)
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.shape) or t.cpu(),
+                                                  lambda t: t.to(DEV)):
+        out = rs.rosa_soft(q, k, v, max_suffix_length=8)
+    assert len(packed) >= 5                              # q, k, v and the packed symbols
+    want = torch.autograd.grad(rs.rosa_soft(q, k, v, max_suffix_length=8).sum(), (q, k, v))
+    for a, b in zip(torch.autograd.grad(out.sum(), (q, k, v)), want):
+        assert torch.equal(a, b)
+    # once differentiable
+    go = torch.ones_like(out, requires_grad=True)
+    dq, = torch.autograd.grad(rs.rosa_soft(q, k, v, max_suffix_length=8), q, go, create_graph=True)
+    with pytest.raises(RuntimeError, match="once_differentiable"):
+        dq.sum().backward()
+    # an input that was changed in place after the forward is noticed
+    w = q.detach().clone().requires_grad_(True)
+    leaf = w * 1.0
+    out = rs.rosa_soft(leaf, k, v, max_suffix_length=8)
+    leaf.add_(1.0)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        out.sum().backward()
