@@ -89,6 +89,20 @@ __device__ __forceinline__ bool load_item_1d(const VjpArgs& a, Item* o) {
   return true;
 }
 
+// How much work a launch of one CTA per item holds: the row blocks of all items per SM over those of
+// the longest item.  Items run next to each other but a block of an item follows the block before it,
+// so a launch of little work is as long as the longest item takes by itself (few, short blocks are
+// what counts), one of much work as long as the SMs are busy.  The lengths of a packed batch are on
+// the GPU: its longest sequence is taken to be twice as long as the average.
+inline float vjp_fill(const VjpArgs& a) {
+  const int64_t N = a.plan.N > 0 ? a.plan.N : 1;
+  const int64_t S = a.plan.S > 0 ? a.plan.S : 1;
+  int64_t longest = a.plan.cu_seqlens == nullptr ? a.plan.uniform_len : 2 * N / S;
+  longest = longest < 2 ? 2 : longest > N ? N : longest;
+  const float items = (float)vjp_bands(longest) / (float)a.bands_per_item;
+  return (float)a.H * (float)N / (float)longest * 0.5f * (items + 1.0f) / 148.0f;
+}
+
 }  // namespace
 
 // Adds four accumulator values to a partial gradient row that this CTA alone writes: the first

@@ -3,8 +3,9 @@
 // thread and 128 threads per band of 256 diagonals.
 //
 // Per row block (16 rows, bottom-up): the forward recurrence is re-run from the block's
-// checkpoint (evidence S kept in a thread-private shared-memory column, the mismatch counts
-// packed into bytes), the adjoint recurrence runs backwards over it and writes the cell adjoint
+// checkpoint (evidence S kept every four rows in a thread-private shared-memory column, the
+// mismatch counts packed into bytes), the adjoint recurrence runs backwards over it, four rows at
+// a time whose S it rebuilds from the kept one, and writes the cell adjoint
 // C and the weighted probability p*d as bf16 terms into one un-skewed [row][window column]
 // operand area, and tcgen05.mma contracts that area three ways (column sums C^T qz and
 // (p d)^T gO, row sums C kz) into fp32 accumulators in tensor memory.  The MMAs of block b run
@@ -17,8 +18,8 @@
 // What the two-diagonal tiling buys: key-side tables of four rows are six consecutive columns
 // held in registers (64-bit shared loads), row-only values are loaded once for two cells, on
 // even rows the two cells of a thread are one aligned 32-bit operand store per term, S and the
-// packed mismatch counts move as 64-bit words, and blocks whose cells are all active and past
-// the horizon run without per-cell predicates.
+// packed mismatch counts move as 64-bit words once per four rows, and blocks whose cells are all
+// active and past the horizon run without per-cell predicates.
 //
 // Operand precision follows the input dtype: float32 inputs keep three bf16 terms of C (24
 // mantissa bits, the row sums cancel heavily) and two of p*d; float16 inputs two and two;
@@ -51,6 +52,8 @@ __host__ __device__ constexpr int tile_cols(int NV) {
   return pairs_blocks(NV) ? kS2Win + kS2Rows : kS2Win;
 }
 constexpr int kS2NK = 16;                            // symbol bits padded to one MMA N
+// ... and of the row sums, whose M = 64 tiles go down to N = 8
+__host__ __device__ constexpr int kz_bits(int D) { return D <= 8 ? 8 : kS2NK; }
 static_assert(kS2Threads * kS2R == kS2Band && kS2Rows == 16, "tile geometry");
 
 // Operand area: core matrices of 8 rows x 16 bytes, ordered [column group][term][row group],
@@ -61,9 +64,10 @@ constexpr int kRowGroupBytes = 144;
 constexpr int kTermBytes = 2 * kRowGroupBytes;
 __host__ __device__ constexpr int col_group_bytes(int nterms) { return nterms * kTermBytes + 16; }
 __host__ __device__ constexpr int operand_bytes(int nterms, int cols = kS2Win) {
-  // the K-major view with M = 64 reads eight cores (1152 bytes) from every column group start:
-  // keep that much readable after the last group
-  return (cols / 8) * col_group_bytes(nterms) + 8 * kRowGroupBytes;
+  // (the K-major view with M = 64 reads eight cores, 1152 bytes, from every column group start, and
+  // the third chunk of the column sums more columns than there are: rows and lanes that are never
+  // used, read from the buffers that follow)
+  return (cols / 8) * col_group_bytes(nterms);
 }
 __host__ __device__ constexpr int chunk_start(int ch, int cols = kS2Win) {
   return ch == 0 ? 0 : ch == 1 ? 128 : cols - 128;
@@ -159,8 +163,8 @@ template <int NV, int NG, int kPrec>
 struct S2Smem {
   static constexpr int kTerms = Terms<kPrec>::C + Terms<kPrec>::P;
   static constexpr int kCg = col_group_bytes(kTerms);
-  static constexpr int kKzSlots = kS2Win / 16 + 2;              // circular k-steps of kz^T
-  static constexpr int kKzSlotBytes = kS2NK * 32;               // [NK][16] bf16
+  // circular k-steps of kz^T: the window's, and the one that the next block adds while they are read
+  static constexpr int kKzSlots = kS2Win / 16 + 1;
   static constexpr int kQzBytes = kS2NK * kS2Rows * 2;
   static constexpr int kGBytes = NV * kS2Rows * 2;
   static constexpr int oTile = 0;
@@ -168,37 +172,46 @@ struct S2Smem {
   static constexpr int oQz = operand_bytes(kTerms, kTileCols);  // two buffers
   static constexpr int oGhi = oQz + 2 * kQzBytes;               // two buffers
   static constexpr int oGlo = oGhi + 2 * kGBytes;               // two buffers
-  static constexpr int oKz = oGlo + 2 * kGBytes;
-  static constexpr int oBar = oKz + kKzSlots * kKzSlotBytes;    // mbarrier, tmem pointer
-  static constexpr int oDq = oBar + 16;                         // row-sum terms of two warps
-  static constexpr int oS = oDq + 2 * kS2Rows * 16 * 4;         // [16][128] float2 evidence
-  static constexpr int oHam = oS + kS2Rows * kS2Threads * 8;    // [4][128] uint2 packed counts
+  static constexpr int oBar = oGlo + (Terms<kPrec>::glo ? 2 * kGBytes : 0);  // mbarrier, tmem pointer
+  static constexpr int oDq = oBar + 16;                         // row-sum terms of the other warps
+  static constexpr int oS = oDq + (Terms<kPrec>::C - 1) * kS2Rows * 16 * 4;
+  // [3][128] float2 evidence at rows 4, 8 and 12 (that of row 0 is the checkpoint, in registers)
+  static constexpr int oHam = oS + (kS2Rows / 4 - 1) * kS2Threads * 8;  // [4][128] uint2 packed counts
   static constexpr int oK = oHam + 4 * kS2Threads * 8;          // int tables from here
   static constexpr int oKold = oK + kS2Win * 4;
   static constexpr int oVb0 = oKold + kS2Win * 4;
-  static constexpr int oVb1 = oVb0 + kS2Win * 4;
-  static constexpr int oQ = oVb1 + kS2Win * 4;
+  static constexpr int oVb1 = oVb0 + kS2Win * 4;                // only wide value rows have one
+  static constexpr int oQ = oVb1 + (NG > 4 ? kS2Win * 4 : 0);
   static constexpr int oQold = oQ + kS2Rows * 4;
-  static constexpr int oKeep = oQold + kS2Rows * 4;             // [16][8] keep ballots
-  static constexpr int oRstat = oKeep + kS2Rows * kVjpWarps * 4;  // [16] float4
-  static constexpr int oGlut = oRstat + kS2Rows * 16;           // [64] float
-  static constexpr int oUlut = oGlut + 64 * 4;                  // [16][NG][16] float
-  static constexpr int kBytes = oUlut + kS2Rows * NG * 16 * 4;
-  static_assert(oQz % 16 == 0 && oS % 16 == 0 && oK % 16 == 0 && oRstat % 16 == 0, "alignment");
+  static constexpr int oRstat = oQold + kS2Rows * 4;            // [16] float4
+  static constexpr int oGlut = oRstat + kS2Rows * 16;           // [kS2NK + 1] float
+  static constexpr int oUlut = oGlut + (kS2NK + 4) * 4;         // [16][NG][16] float
+  static constexpr int oKz = oUlut + kS2Rows * NG * 16 * 4;     // circular k-steps of kz^T
+  // Shared memory decides how many CTAs an SM holds (value rows of up to 16 components): bfloat16
+  // inputs 4, otherwise 3.  It was 3 and 2 with S kept for every row, which left the schedulers 3
+  // or 2 warps with a dependent chain each (0.59 issued per cycle).  2 x 1024 x 64 float32: 595 us
+  // with two, 495 with three.
+  // the k-steps hold 8 or 16 symbol bits (kz_bits) of 16 columns as bf16
+  __host__ __device__ static constexpr int bytes(int D) { return oKz + kKzSlots * kz_bits(D) * 32; }
+  static_assert(oQz % 16 == 0 && oS % 16 == 0 && oK % 16 == 0 && oRstat % 16 == 0 && oUlut % 16 == 0 &&
+                oKz % 16 == 0, "alignment");
+  // what is read past the operand area stays inside
+  static_assert((224 + 128) / 8 * kCg + kTerms * kTermBytes <= oKz, "operand reads leave shared memory");
 };
 
 
 // ---- forward phase: four rows x two diagonals from the running state.  kw / kow hold the key
 // symbols (and the symbols leaving the horizon) of window columns cb .. cb + 5, cb the column of
-// (row r0, diagonal 1); cell (rr, e) reads entry rr + 1 - e.  Stores S per row and the eight
-// mismatch counts (times four: byte offsets into the gate table) as one 64-bit word.  Returns
+// (row r0, diagonal 1); cell (rr, e) reads entry rr + 1 - e.  Stores the S that the group starts
+// from and the eight mismatch counts (times four: byte offsets into the gate table) as one 64-bit
+// word each.  Returns
 // whether any window product of the thread may be non-zero.
 template <bool kEdge>
 __device__ __forceinline__ bool s2_forward_group(const int* s_q, const int* s_qold,
                                                  const float* glut, const int (&kw)[6],
                                                  const int (&kow)[6], bool windowed, int r0, int i0,
                                                  int j1, int W, int len, int hs_cut, float neg_md,
-                                                 float (&S)[2], int (&hs)[2], float2* s_row,
+                                                 float (&S)[2], int (&hs)[2], float2* s_start,
                                                  uint2* ham_out) {
   const int4 q4 = *reinterpret_cast<const int4*>(s_q + r0);
   const int q[4] = {q4.x, q4.y, q4.z, q4.w};
@@ -245,18 +258,18 @@ __device__ __forceinline__ bool s2_forward_group(const int* s_q, const int* s_qo
       }
   }
   uint32_t hw[2] = {0u, 0u};
+  if (r0 > 0) *s_start = make_float2(S[0], S[1]);
 #pragma unroll
   for (int rr = 0; rr < 4; ++rr) {
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const float x = glut[ham[rr][e]];
-      const float Sn = x * (1.0f + S[e]) - P[rr][e];
+      const float Sn = fmaf(x, 1.0f + S[e], -P[rr][e]);
       bool act = true;
       if (kEdge) act = (j1 + rr + 1 - e) >= 0 && i0 + r0 + rr <= len - 1;
       S[e] = act ? Sn : 0.0f;
       hw[rr >> 1] |= (uint32_t)(ham[rr][e] * 4) << (8 * ((rr & 1) * 2 + e));
     }
-    s_row[rr * kS2Threads] = make_float2(S[0], S[1]);
   }
   *ham_out = make_uint2(hw[0], hw[1]);
   return any_alive;
@@ -264,12 +277,14 @@ __device__ __forceinline__ bool s2_forward_group(const int* s_q, const int* s_qo
 
 // ---- adjoint phase, no window product alive: four rows (descending) x two diagonals.
 // sb is the running adjoint of S in float32 (a contraction here), xnext the gate one row
-// further down the diagonal.  Writes C and p*d into the operand area.
+// further down the diagonal.  S of the four rows is rebuilt from the one the group starts from (one
+// multiplication a cell: 1 + S is needed anyway), the same operations as in the forward phase.
+// Writes C and p*d into the operand area.
 template <int NG, int NC, int NP, bool kRound, bool kDropout, bool kEdge>
 __device__ __forceinline__ void s2_adjoint_group(
     unsigned char* tC, unsigned char* tP, int cg, const float4* s_rstat, uint2 keepw,
     const float* glut, const float* ulut, const uint32_t (&v0)[6], const uint32_t (&v1)[6],
-    const float2* s_row, uint2 hamw, int r0, int i0, int j1, int len, int skew, int cb, float mul2,
+    float2 s_start, uint2 hamw, int r0, int i0, int j1, int len, int skew, int cb, float mul2,
     int keep_shift, float (&sb)[2], float (&xnext)[2]) {
   // keep flags of the group's four rows, this thread's two diagonals at bits 4 rr, 4 rr + 1
   const uint32_t kgroup = (r0 < 8 ? keepw.x : keepw.y) >> (4 * (r0 & 7) + keep_shift);
@@ -281,21 +296,32 @@ __device__ __forceinline__ void s2_adjoint_group(
   o[4] = col_off(cb + 4, cg) + row_off(r0);
   o[1] = o[0] + 2;
   o[3] = o[2] + 2;
+  float gate[4][2], S[4][2];
+  {
+    float t[2] = {1.0f + s_start.x, 1.0f + s_start.y};
+#pragma unroll
+    for (int rr = 0; rr < 4; ++rr)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const uint32_t hoff = ((rr < 2 ? hamw.x : hamw.y) >> (8 * ((rr & 1) * 2 + e))) & 0xffu;
+        gate[rr][e] = *reinterpret_cast<const float*>(reinterpret_cast<const char*>(glut) + hoff);
+        float Sn = gate[rr][e] * t[e];
+        if (kEdge) Sn = (j1 + rr + 1 - e) >= 0 && i0 + r0 + rr <= len - 1 ? Sn : 0.0f;
+        S[rr][e] = Sn;
+        t[e] = 1.0f + Sn;
+      }
+  }
 #pragma unroll
   for (int rr = 3; rr >= 0; --rr) {
     const int r = r0 + rr;
     const float4 st = s_rstat[r];          // (exponent bias, 1/Z, E * ds, 1/Z / keep probability)
-    const float2 Sv = s_row[rr * kS2Threads];
-    const uint32_t hb = rr < 2 ? hamw.x : hamw.y;
     uint32_t kbits = 3u;
     if (kDropout) kbits = kgroup >> (4 * rr);
     float Cv[2], pd[2];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int x = rr + 1 - e;
-      const float Se = e == 0 ? Sv.x : Sv.y;
-      const uint32_t hoff = (hb >> (8 * ((rr & 1) * 2 + e))) & 0xffu;
-      const float gate = *reinterpret_cast<const float*>(reinterpret_cast<const char*>(glut) + hoff);
+      const float Se = S[rr][e];
       const float t = 1.0f + Se;
       const float rs = rsqrtf(t);
       float ex = exp2f(fmaf(t * rs, mul2, st.x));
@@ -312,7 +338,7 @@ __device__ __forceinline__ void s2_adjoint_group(
       const float dS = (pd[e] * u - pr * st.z) * rs;
       sb[e] = fmaf(xnext[e], sb[e], dS);
       Cv[e] = act ? Se * sb[e] : 0.0f;
-      xnext[e] = gate;
+      xnext[e] = gate[rr][e];
     }
     // diagonal 1 sits on the lower column (cb + rr), diagonal 0 on the next one
     const bool aligned = (rr & 1) == 0;
@@ -332,9 +358,20 @@ struct S2Geom {
 #include "vjp_tiled_sweep2_kernel.inl"
 #undef ROSA_S2_PAIR
 
+constexpr float kS2FourCtasFill = 5.0f;
+constexpr int kS2ThreeCtas = 60 * 1024;     // shared memory of which a fourth CTA does not find enough
+constexpr int kS2TwoCtas = 78 * 1024;       // ... a third
+
 template <int NV, int NG, bool kDropout, int kPrec>
 int launch_s2_tiled_t(const VjpArgs& a, unsigned grid, cudaStream_t stream) {
-  constexpr int bytes = S2Smem<NV, NG, kPrec>::kBytes;
+  int bytes = S2Smem<NV, NG, kPrec>::bytes(a.D);
+  // A fourth CTA per SM raises the throughput of a full GPU and slows down every CTA; where the longest
+  // item decides (vjp_fill), the SMs keep to three.  Three against four: 2 x 1024 x 64 (fill 2.2) 472 /
+  // 505 us, 4 x 1024 x 64 (4.3) 817 / 823 us, 32 x 256 x 32 (6.9) 416 / 364 us, 16 x 8192 x 64 in
+  // slices (14) 149.9 / 139.5 ms.  Paired blocks take 256 of the 512 tensor-memory columns: a third
+  // CTA would only wait for them (packed 32768 x 16 float16: 19 - 21 ms against 16.5).
+  const int least = pairs_blocks(NV) ? kS2TwoCtas : vjp_fill(a) < kS2FourCtasFill ? kS2ThreeCtas : 0;
+  if (bytes < least) bytes = least;
   if constexpr (pairs_blocks(NV)) {
     auto kernel = vjp_sweep2_tiled_pair_kernel<NV, NG, kDropout, kPrec>;
     ROSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));

@@ -19,7 +19,7 @@
 
 template <int NV, int NG, bool kDropout, int kPrec>
 #ifndef ROSA_S2_PAIR
-__global__ void __launch_bounds__(kS2Threads, 3) vjp_sweep2_tiled_kernel(VjpArgs a) {
+__global__ void __launch_bounds__(kS2Threads, kPrec == 2 ? 4 : 3) vjp_sweep2_tiled_kernel(VjpArgs a) {
 #else /* ROSA_S2_PAIR */
 __global__ void __launch_bounds__(kS2Threads) vjp_sweep2_tiled_pair_kernel(VjpArgs a) {
 #endif /* ROSA_S2_PAIR */
@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(kS2Threads) vjp_sweep2_tiled_pair_kernel(VjpAr
   __syncthreads();
   tc::fence_after_thread_sync();
   const uint32_t tmem = *tmem_ptr;
+  const int kz_n = kz_bits(D), kz_slot = kz_n * 32;      // bits of a kz^T k-step, its bytes
   uint32_t mma_phase = 0;
   bool mma_timed_out = false;
   int buf = 0;
@@ -445,15 +446,15 @@ __global__ void __launch_bounds__(kS2Threads) vjp_sweep2_tiled_pair_kernel(VjpAr
     if (mask & 1) {
       const int g0 = (g.jwin + (1 << 20)) >> 4;        // absolute group of window column 0
       const int nfill = band_start ? kS2Win / 16 : 1;
-      for (int e = tid; e < nfill * NK * 16; e += kS2Threads) {
-        const int ks = e / (NK * 16), rem = e - ks * (NK * 16);
+      for (int e = tid; e < nfill * kz_n * 16; e += kS2Threads) {
+        const int ks = kz_n == 8 ? e >> 7 : e >> 8, rem = e - ks * kz_n * 16;
         const int d = rem >> 4, cc = rem & 15;
         const int c = ks * 16 + cc;
         const int j = g.jwin + c;
         const float v = (d < D && j >= 0 && j < it.len - 1)
                             ? ((s_k[c] >> d & 1) ? 1.0f : -1.0f) : 0.0f;
         const int sl = (g0 + ks) % L::kKzSlots;
-        *reinterpret_cast<__nv_bfloat16*>(bKz + sl * L::kKzSlotBytes + b_off(d, cc, NK)) =
+        *reinterpret_cast<__nv_bfloat16*>(bKz + sl * kz_slot + b_off(d, cc, kz_n)) =
             __float2bfloat16_rn(v);
       }
     }
@@ -484,14 +485,14 @@ __global__ void __launch_bounds__(kS2Threads) vjp_sweep2_tiled_pair_kernel(VjpAr
           kow[2] = b1.x; kow[3] = b1.y; kow[4] = b2.x; kow[5] = b2.y;
         }
         const int j1 = g.jwin + cb;                    // key column of (row r0, diagonal 1)
-        float2* s_row = Sbuf + r0 * kS2Threads + tid;
+        float2* s_start = Sbuf + ((r0 >> 2) - 1) * kS2Threads + tid;      // not written at r0 = 0
         uint2* ham_out = Hbuf + (r0 >> 2) * kS2Threads + tid;
         if (interior)
           has_p |= s2_forward_group<false>(s_q, s_qold, glut, kw, kow, windowed, r0, g.i0, j1, W,
-                                           it.len, hs_cut, neg_md, S, hs, s_row, ham_out);
+                                           it.len, hs_cut, neg_md, S, hs, s_start, ham_out);
         else
           has_p |= s2_forward_group<true>(s_q, s_qold, glut, kw, kow, windowed, r0, g.i0, j1, W,
-                                          it.len, hs_cut, neg_md, S, hs, s_row, ham_out);
+                                          it.len, hs_cut, neg_md, S, hs, s_start, ham_out);
         kw[0] = kw[4]; kw[1] = kw[5];
         kow[0] = kow[4]; kow[1] = kow[5];
       }
@@ -526,6 +527,7 @@ __global__ void __launch_bounds__(kS2Threads) vjp_sweep2_tiled_pair_kernel(VjpAr
 #endif /* ROSA_S2_PAIR */
     // ---- phase B: adjoint recurrence, rows descending; C and p*d go to the operand area
     const bool warp_p = windowed && ring != nullptr && has_p;
+    const float2 s_top = make_float2(__int_as_float(ck.x), __int_as_float(ck.z));
     if (!warp_p && live == 0) {
       sb[0] = (float)Sbar[0];
       sb[1] = (float)Sbar[1];
@@ -542,16 +544,16 @@ __global__ void __launch_bounds__(kS2Threads) vjp_sweep2_tiled_pair_kernel(VjpAr
             v1[2 * x2] = t1.x; v1[2 * x2 + 1] = t1.y;
           }
         }
-        const float2* s_row = Sbuf + r0 * kS2Threads + tid;
+        const float2 s_start = r0 > 0 ? Sbuf[((r0 >> 2) - 1) * kS2Threads + tid] : s_top;
         const uint2 hamw = Hbuf[(r0 >> 2) * kS2Threads + tid];
         const int j1 = g.jwin + cb;
         if (interior)
           s2_adjoint_group<NG, NC, NP, kPrec == 0, kDropout, false>(S2_TILE_C, S2_TILE_P, CG, s_rstat, keepw, glut, ulut, v0,
-                                                        v1, s_row, hamw, r0, g.i0, j1, it.len,
+                                                        v1, s_start, hamw, r0, g.i0, j1, it.len,
                                                         g.skew, cb, mul2, keep_shift, sb, xnext);
         else
           s2_adjoint_group<NG, NC, NP, kPrec == 0, kDropout, true>(S2_TILE_C, S2_TILE_P, CG, s_rstat, keepw, glut, ulut, v0,
-                                                       v1, s_row, hamw, r0, g.i0, j1, it.len,
+                                                       v1, s_start, hamw, r0, g.i0, j1, it.len,
                                                        g.skew, cb, mul2, keep_shift, sb, xnext);
       }
       Sbar[0] = (double)sb[0];
@@ -563,75 +565,90 @@ __global__ void __launch_bounds__(kS2Threads) vjp_sweep2_tiled_pair_kernel(VjpAr
       // reads and writes one contiguous line per row.
       int slot = (g.i0 + kS2Rows - 1) % ring_slots;    // ring line of the row, walked downwards
 #pragma unroll 1
-      for (int r = kS2Rows - 1; r >= 0; --r) {
-        const int i = g.i0 + r;
-        const float4 st = s_rstat[r];
-        const float2 Sv2 = Sbuf[r * kS2Threads + tid];
-        const uint2 hamw = Hbuf[(r >> 2) * kS2Threads + tid];
-        const uint32_t hb = (r & 3) < 2 ? hamw.x : hamw.y;
-        uint32_t kbits = 3u;
-        if (kDropout) kbits = (r < 8 ? keepw.x : keepw.y) >> (4 * (r & 7) + keep_shift);
-        const int qo = s_qold[r];
-        float Cv[2], pd[2], Pv[2], gate[2], dS[2];
-        bool act[2];
-        // the ring line of this row is requested first; it was written W + 1 rows ago, or not at
-        // all if the live stretch is younger than that (the ring needs no clearing)
-        float* line = ring + (int64_t)slot * kS2Band;
-        slot = (slot == 0 ? ring_slots : slot) - 1;
-        float2 old_t = make_float2(0.0f, 0.0f);
-        if (live > 0 && age > W) old_t = *reinterpret_cast<const float2*>(line);
+      for (int r0 = kS2Rows - 4; r0 >= 0; r0 -= 4) {
+        const uint2 hamw = Hbuf[(r0 >> 2) * kS2Threads + tid];
+        const float2 s_start = r0 > 0 ? Sbuf[((r0 >> 2) - 1) * kS2Threads + tid] : s_top;
+        // the four rows' window products, downwards, then their S, upwards, as in phase A
+        float Pv[4][2], gate[4][2], S4[4][2];
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int c = r + kS2Band - 1 - kS2R * tid - e;
-          const int j = g.jwin + c;
-          act[e] = j >= 0 && i <= it.len - 1;
-          const uint32_t hoff = (hb >> (8 * ((r & 1) * 2 + e))) & 0xffu;
-          const int ham = (int)(hoff >> 2);
-          gate[e] = glut[ham];
-          Pv[e] = (act[e] && j >= W && hs[e] <= hs_cut) ? __expf(neg_md * (float)hs[e]) : 0.0f;
-          hs[e] += ((act[e] && j > W) ? __popc(qo ^ s_kold[c]) : 0) - (act[e] ? ham : 0);
-          const float Se = e == 0 ? Sv2.x : Sv2.y;
-          const float t = 1.0f + Se;
-          const float rs = rsqrtf(t);
-          const float ex = act[e] ? exp2f(fmaf(t * rs, mul2, st.x)) : 0.0f;
-          const float pr = ex * st.y;
-          pd[e] = ex * st.w;
-          if (kDropout) pd[e] = (kbits >> e & 1u) ? pd[e] : 0.0f;
-          const float u = tiled_utility<NG>(ulut + r * NG * 16, s_vb0[c], NG > 4 ? s_vb1[c] : 0u);
-          dS[e] = (pd[e] * u - pr * st.z) * rs;
-          if (act[e]) Sbar[e] = (double)dS[e] + (double)xnext[e] * Sbar[e];
-        }
-        const bool any_p = __any_sync(0xffffffffu, Pv[0] != 0.0f || Pv[1] != 0.0f);
-        if (any_p) {
-          if (live == 0) age = 0;
-          live = W + 2;
-        }
-        if (live > 0) {
+        for (int rr = 3; rr >= 0; --rr) {
+          const int r = r0 + rr, qo = s_qold[r];
+          const uint32_t hb = rr < 2 ? hamw.x : hamw.y;
 #pragma unroll
-          for (int e = 0; e < 2; ++e)
-            if (act[e]) {
-              const float tf = (float)(Sbar[e] * (double)Pv[e]);
-              const float old = e == 0 ? old_t.x : old_t.y;
-              line[e] = tf;
-              Y[e] += (double)tf - (double)old;
-            }
-          ++age;
-          if (--live == 0) Y[0] = Y[1] = 0.0;
+          for (int e = 0; e < 2; ++e) {
+            const int c = r + kS2Band - 1 - kS2R * tid - e;
+            const int j = g.jwin + c;
+            const bool act = j >= 0 && g.i0 + r <= it.len - 1;
+            const int ham = (int)((hb >> (8 * ((rr & 1) * 2 + e) + 2)) & 0x3fu);
+            gate[rr][e] = glut[ham];
+            Pv[rr][e] = (act && j >= W && hs[e] <= hs_cut) ? __expf(neg_md * (float)hs[e]) : 0.0f;
+            hs[e] += ((act && j > W) ? __popc(qo ^ s_kold[c]) : 0) - (act ? ham : 0);
+          }
         }
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const float Se = e == 0 ? Sv2.x : Sv2.y;
-          Cv[e] = act[e] ? (float)((double)(Se + Pv[e]) * Sbar[e] - Y[e]) : 0.0f;
-          if (act[e]) xnext[e] = gate[e];
+          float Sn = e == 0 ? s_start.x : s_start.y;
+#pragma unroll
+          for (int rr = 0; rr < 4; ++rr) {
+            const int j = g.jwin + r0 + rr + kS2Band - 1 - kS2R * tid - e;
+            Sn = fmaf(gate[rr][e], 1.0f + Sn, -Pv[rr][e]);
+            S4[rr][e] = Sn = j >= 0 && g.i0 + r0 + rr <= it.len - 1 ? Sn : 0.0f;
+          }
         }
-        const int c1 = r + kS2Band - 2 - kS2R * tid;           // column of diagonal 1
-        const int off_lo = col_off(c1, CG) + row_off(r), off_hi = col_off(c1 + 1, CG) + row_off(r);
-        if ((r & 1) == 0) {
-          store_pair<NC, kPrec == 0>(S2_TILE_C, off_lo, off_hi, true, Cv[1], Cv[0]);
-          store_pair<NP, kPrec == 0>(S2_TILE_P, off_lo, off_hi, true, pd[1], pd[0]);
-        } else {
-          store_pair<NC, kPrec == 0>(S2_TILE_C, off_lo, off_hi, false, Cv[1], Cv[0]);
-          store_pair<NP, kPrec == 0>(S2_TILE_P, off_lo, off_hi, false, pd[1], pd[0]);
+#pragma unroll
+        for (int rr = 3; rr >= 0; --rr) {
+          const int r = r0 + rr, i = g.i0 + r;
+          const float4 st = s_rstat[r];
+          uint32_t kbits = 3u;
+          if (kDropout) kbits = (r0 < 8 ? keepw.x : keepw.y) >> (4 * (r & 7) + keep_shift);
+          float Cv[2], pd[2];
+          bool act[2];
+          // the ring line of this row is requested first; it was written W + 1 rows ago, or not at
+          // all if the live stretch is younger than that (the ring needs no clearing)
+          float* line = ring + (int64_t)slot * kS2Band;
+          slot = (slot == 0 ? ring_slots : slot) - 1;
+          float2 old_t = make_float2(0.0f, 0.0f);
+          if (live > 0 && age > W) old_t = *reinterpret_cast<const float2*>(line);
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int c = r + kS2Band - 1 - kS2R * tid - e;
+            act[e] = g.jwin + c >= 0 && i <= it.len - 1;
+            const float t = 1.0f + S4[rr][e];
+            const float rs = rsqrtf(t);
+            const float ex = act[e] ? exp2f(fmaf(t * rs, mul2, st.x)) : 0.0f;
+            const float pr = ex * st.y;
+            pd[e] = ex * st.w;
+            if (kDropout) pd[e] = (kbits >> e & 1u) ? pd[e] : 0.0f;
+            const float u = tiled_utility<NG>(ulut + r * NG * 16, s_vb0[c], NG > 4 ? s_vb1[c] : 0u);
+            const float dS = (pd[e] * u - pr * st.z) * rs;
+            if (act[e]) Sbar[e] = (double)dS + (double)xnext[e] * Sbar[e];
+          }
+          const bool any_p = __any_sync(0xffffffffu, Pv[rr][0] != 0.0f || Pv[rr][1] != 0.0f);
+          if (any_p) {
+            if (live == 0) age = 0;
+            live = W + 2;
+          }
+          if (live > 0) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+              if (act[e]) {
+                const float tf = (float)(Sbar[e] * (double)Pv[rr][e]);
+                const float old = e == 0 ? old_t.x : old_t.y;
+                line[e] = tf;
+                Y[e] += (double)tf - (double)old;
+              }
+            ++age;
+            if (--live == 0) Y[0] = Y[1] = 0.0;
+          }
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            Cv[e] = act[e] ? (float)((double)(S4[rr][e] + Pv[rr][e]) * Sbar[e] - Y[e]) : 0.0f;
+            if (act[e]) xnext[e] = gate[rr][e];
+          }
+          const int c1 = r + kS2Band - 2 - kS2R * tid;           // column of diagonal 1
+          const int off_lo = col_off(c1, CG) + row_off(r), off_hi = col_off(c1 + 1, CG) + row_off(r);
+          store_pair<NC, kPrec == 0>(S2_TILE_C, off_lo, off_hi, (rr & 1) == 0, Cv[1], Cv[0]);
+          store_pair<NP, kPrec == 0>(S2_TILE_P, off_lo, off_hi, (rr & 1) == 0, pd[1], pd[0]);
         }
       }
     }
@@ -654,7 +671,7 @@ __global__ void __launch_bounds__(kS2Threads) vjp_sweep2_tiled_pair_kernel(VjpAr
       tc::fence_after_thread_sync();
       constexpr uint32_t idK = tc::idesc_bf16_f32(128, NK, true, false);
       constexpr uint32_t idV = tc::idesc_bf16_f32(128, NV, true, false);
-      constexpr uint32_t idQ = tc::idesc_bf16_f32(64, NK, false, false);
+      const uint32_t idQ = tc::idesc_bf16_f32(64, kz_n, false, false);
       if (warp == 0 && (mask & 2)) {
         const uint64_t dQz = tc::smem_desc(tc::smem_addr(bQz), NK / 8 * 128, 128);
         const uint64_t c0 = tc::smem_desc(tc::smem_addr(tC), kRowGroupBytes, CG);
@@ -683,7 +700,7 @@ __global__ void __launch_bounds__(kS2Threads) vjp_sweep2_tiled_pair_kernel(VjpAr
         // K-major view (row sums): K direction = column groups, M direction = the row groups of
         // the C terms of a column group (M = 64: the rows past the last term alias p*d cores)
         const uint64_t kC = tc::smem_desc(tc::smem_addr(S2_TILE_C), CG, kRowGroupBytes);
-        const uint64_t dKz0 = tc::smem_desc(tc::smem_addr(bKz), NK / 8 * 128, 128);
+        const uint64_t dKz0 = tc::smem_desc(tc::smem_addr(bKz), kz_n / 8 * 128, 128);
         constexpr int kSteps = kS2Win / 16;
         const int part = warp - 2;
         const int ks0 = part * kSteps / NQ, ks1 = (part + 1) * kSteps / NQ;
@@ -692,7 +709,7 @@ __global__ void __launch_bounds__(kS2Threads) vjp_sweep2_tiled_pair_kernel(VjpAr
         int sl = (g0 + ks0) % L::kKzSlots;
 #pragma unroll 1
         for (int ks = ks0; ks < ks1; ++ks) {
-          const uint64_t dKz = dKz0 + (uint64_t)((sl * L::kKzSlotBytes) >> 4);
+          const uint64_t dKz = dKz0 + (uint64_t)((sl * kz_slot) >> 4);
           const uint64_t shift = (uint64_t)((ks * 2 * CG) >> 4);
           tc::mma_bf16(acc, kC + shift, dKz, idQ, ks > ks0);
           sl = sl + 1 == L::kKzSlots ? 0 : sl + 1;
