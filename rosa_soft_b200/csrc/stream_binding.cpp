@@ -62,6 +62,22 @@ class StreamCore {
     ordered_ = false;
   }
 
+  // The first update fixes the slots of a fresh runtime, unless it fails.
+  struct Opening {
+    Opening(StreamCore* core, int64_t slots, const c10::Device& device)
+        : core_(core->slots_ == -1 ? core : nullptr) {
+      if (core_ != nullptr) core_->open(slots, device);
+    }
+    ~Opening() {
+      if (core_ != nullptr) core_->clear();
+    }
+    Pair done(Pair result) const {
+      core_ = nullptr;
+      return result;
+    }
+    mutable StreamCore* core_;
+  };
+
   // Fixes the slots of a fresh runtime.
   void open(int64_t slots, const c10::Device& device) {
     slots_ = slots;
@@ -142,9 +158,9 @@ class StreamCore {
         B * T * heads_ > kInt32Max || (slots_ != -1 && (slots_ != B || device != device_)))
       return std::nullopt;
     const c10::cuda::OptionalCUDAGuard guard(device);
-    if (slots_ == -1) open(B, device);
-    return append(query, key, payload, Tensor(), nullptr, B * T, T, out,
-                  query.sizes().slice(0, 3));
+    const Opening opening(this, B, device);
+    return opening.done(append(query, key, payload, Tensor(), nullptr, B * T, T, out,
+                               query.sizes().slice(0, 3)));
   }
 
   // Chunks of host-known lengths: offsets[s] .. offsets[s + 1] of the token axis; `device_offsets`
@@ -155,7 +171,7 @@ class StreamCore {
     const c10::Device device = query.device();
     const c10::cuda::OptionalCUDAGuard guard(device);
     const int64_t slots = (int64_t)offsets.size() - 1;
-    if (slots_ == -1) open(slots, device);
+    const Opening opening(this, slots, device);
     std::vector<int64_t> chunk(static_cast<size_t>(slots));
     int64_t longest = 0, shortest = kInt32Max;
     for (int64_t s = 0; s < slots; ++s) {
@@ -173,7 +189,7 @@ class StreamCore {
         dev = host.to(device, /*non_blocking=*/true);
       }
     }
-    return append(query, key, payload, dev, &chunk, offsets.back(), longest, out_type, shape);
+    return opening.done(append(query, key, payload, dev, &chunk, offsets.back(), longest, out_type, shape));
   }
 
   std::tuple<Tensor, Tensor, Tensor> export_histories() const {
@@ -249,21 +265,23 @@ class StreamCore {
       }
       return t;
     };
-    query_ = moved(query_, heads_, u8);
-    key_ = moved(key_, heads_, u8);
-    payload_ = moved(payload_, payload_heads_, u8);
-    links_ = moved(links_, heads_, i32);
+    Tensor query = moved(query_, heads_, u8), key = moved(key_, heads_, u8);
+    Tensor payload = moved(payload_, payload_heads_, u8), links = moved(links_, heads_, i32);
     const int64_t table = (int64_t)rosa_b200_stream_table_bytes((int)qk_bits_, horizon_, capacity);
     const bool rebuilt = capacity_ > 0 && table != table_bytes_;
+    Tensor tables = tables_, lens = lens_, scratch = scratch_;
     if (capacity_ == 0) {
-      lens_ = torch::zeros({2, slots_}, i32);
-      scratch_ = torch::empty({kScratchBytes}, u8);
+      lens = torch::zeros({2, slots_}, i32);
+      scratch = torch::empty({kScratchBytes}, u8);
     } else if (stream != *home_) {
-      lens_ = lens_.clone();
-      scratch_ = torch::empty({kScratchBytes}, u8);
-      if (!rebuilt) tables_ = tables_.clone();
+      lens = lens_.clone();
+      scratch = torch::empty({kScratchBytes}, u8);
+      if (!rebuilt) tables = tables_.clone();
     }
-    if (capacity_ == 0 || rebuilt) tables_ = torch::zeros({slots_, heads_, table}, u8);
+    if (capacity_ == 0 || rebuilt) tables = torch::zeros({slots_, heads_, table}, u8);
+    // everything is allocated: an update that runs out of memory leaves the state as it was
+    query_ = query; key_ = key; payload_ = payload; links_ = links;
+    tables_ = tables; lens_ = lens; scratch_ = scratch;
     table_bytes_ = table;
     capacity_ = capacity;
     home_ = stream;
