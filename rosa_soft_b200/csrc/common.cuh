@@ -408,7 +408,8 @@ struct VjpArgs {
 
 int launch_pack_value_bits(const VjpArgs& a, cudaStream_t stream);
 int launch_vjp_sweep1(const VjpArgs& a, int items_upper, cudaStream_t stream);
-// register-tiled sweeps (vjp_tiled.cu): four diagonals per thread
+// register-tiled sweeps (vjp_tiled.cu, vjp_tiled_sweep2.cu): the first, both
+bool vjp_sweep1_tiled_applies(const VjpArgs& a);
 bool vjp_tiled_applies(const VjpArgs& a);
 int launch_vjp_sweep1_tiled(const VjpArgs& a, int items_upper, cudaStream_t stream);
 int launch_vjp_sweep2_tiled(const VjpArgs& a, int items_upper, cudaStream_t stream);

@@ -1641,7 +1641,7 @@ int launch_pack_value_bits(const VjpArgs& a, cudaStream_t stream) {
 int launch_vjp_sweep1(const VjpArgs& a, int items_upper, cudaStream_t stream) {
   if (items_upper <= 0) return 0;
   ProfileScope prof("vjp_sweep1", stream);
-  if (vjp_tiled_applies(a)) return launch_vjp_sweep1_tiled(a, items_upper, stream);
+  if (vjp_sweep1_tiled_applies(a)) return launch_vjp_sweep1_tiled(a, items_upper, stream);
   const bool small_dv = a.Dv <= 32;
   const size_t bytes = sweep_common_floats(small_dv ? (a.Dv + 3) / 4 : 0) * sizeof(float);
   const unsigned grid = (unsigned)((int64_t)items_upper * a.H);

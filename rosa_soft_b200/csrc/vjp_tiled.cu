@@ -2,16 +2,16 @@
 // surrogate_vjp.cu: evidence recurrence along diagonals, online softmax with the analytic
 // reference, dropout counter, checkpoints every 16 rows).
 //
-// One thread owns FOUR consecutive diagonals and walks them down the rows together.  On block
-// row r the four cells of a thread sit on four consecutive key columns, and one row further
-// down the same four diagonals sit one column to the right, so the key-side tables (key
-// symbol, the symbol leaving the horizon window, value sign bits, first dropout hash round) of
-// a group of four rows are seven consecutive columns: two aligned 128-bit shared-memory loads
-// per table and sixteen cells, kept in registers and indexed at compile time.  Everything that
-// depends on the row only (query symbols, hash word of the query position, utility table base)
-// is loaded once per row and thread and shared by four cells; the row sums of four cells are
-// added in registers before the warp reduction.  Rows of a block always start at a multiple of
-// 16 (rows that do not exist are masked), interior blocks -- every cell active and past the
+// One thread owns R = FOUR (or two, or one: see launch_s1_tiled) consecutive diagonals and walks
+// them down the rows together.  On block row r the R cells of a thread sit on R consecutive key
+// columns, and one row further down the same diagonals sit one column to the right, so the
+// key-side tables (key symbol, the symbol leaving the horizon window, value sign bits, first
+// dropout hash round) of a group of four rows are R + 3 consecutive columns: for R = 4 two aligned
+// 128-bit shared-memory loads per table and sixteen cells, kept in registers and indexed at
+// compile time.  Everything that depends on the row only (query symbols, hash word of the query
+// position, utility table base) is loaded once per row and thread and shared by R cells; the row
+// sums of R cells are added in registers before the warp reduction.  Rows of a block always start
+// at a multiple of 16 (rows that do not exist are masked), interior blocks -- every cell active and past the
 // horizon -- run without any per-cell predicate.
 #include "common.cuh"
 #include "vjp_shared.cuh"
@@ -21,10 +21,8 @@ namespace rosa {
 
 namespace {
 
-constexpr int kTR = 4;                          // diagonals per thread
 constexpr int kTBand = kVjpBand;                // diagonals per band
-constexpr int kTThreads = kTBand / kTR;         // threads per CTA
-constexpr int kTWarps = kTThreads / 32;
+constexpr int s1_threads(int R) { return kTBand / R; }         // threads per CTA, R diagonals each
 constexpr int kTRows = kVjpRows;                // rows per checkpointed block
 constexpr int kTWin = kTBand + kTRows;          // window columns of a block
 // The column tables of a block (key symbols, symbols leaving the horizon, first hash round of the
@@ -46,15 +44,15 @@ struct S1Smem {
   int* s_q;          // [kTRows]
   int* s_qold;       // [kTRows]
   float* glut;       // [64] gate per mismatch count
-  float2* wstat;     // [kTRows][kTWarps] per-warp (sum e, sum e d u)
+  float2* wstat;     // [kTRows][warps] per-warp (sum e, sum e d u)
   float* ulut;       // [kTRows][NG][16]
 };
 
-__host__ __device__ constexpr int s1_smem_words(int ng) {
-  return 5 * kTTab + 2 * kTRows + 64 + 2 * kTRows * kTWarps + kTRows * ng * 16;
+__host__ __device__ constexpr int s1_smem_words(int ng, int warps) {
+  return 5 * kTTab + 2 * kTRows + 64 + 2 * kTRows * warps + kTRows * ng * 16;
 }
 
-__device__ __forceinline__ S1Smem s1_carve(float* base, int ng) {
+__device__ __forceinline__ S1Smem s1_carve(float* base, int warps) {
   S1Smem s;
   int* w = reinterpret_cast<int*>(base);
   s.s_k = w;                                        w += kTTab;
@@ -65,42 +63,59 @@ __device__ __forceinline__ S1Smem s1_carve(float* base, int ng) {
   s.s_q = w;                                        w += kTRows;
   s.s_qold = w;                                     w += kTRows;
   s.glut = reinterpret_cast<float*>(w);             w += 64;
-  s.wstat = reinterpret_cast<float2*>(w);           w += 2 * kTRows * kTWarps;
+  s.wstat = reinterpret_cast<float2*>(w);           w += 2 * kTRows * warps;
   s.ulut = reinterpret_cast<float*>(w);
-  (void)ng;
   return s;
 }
 
-// The column windows of one group of four rows: eight consecutive table entries per table,
-// cell (row rr, diagonal e) reads entry rr + 3 - e.
-template <int NG, bool kWindowed, bool kDropout>
+// bits 0 .. 15 of x on the even bits
+__device__ __forceinline__ uint32_t spread_bits(uint32_t x) {
+  x &= 0xffffu;
+  x = (x | x << 8) & 0x00ff00ffu;
+  x = (x | x << 4) & 0x0f0f0f0fu;
+  x = (x | x << 2) & 0x33333333u;
+  return (x | x << 1) & 0x55555555u;
+}
+
+// The column windows of one group of four rows: consecutive table entries, cell (row rr, diagonal e)
+// reads entry rr + R - 1 - e.  The last kept(R) entries are the first ones of the next group.
+__host__ __device__ constexpr int s1_kept(int R) { return R == 1 ? 0 : R; }
+
+template <int NG, int R, bool kWindowed, bool kDropout>
 struct ColWindow {
-  int k[8];
-  int kold[kWindowed ? 8 : 1];
-  uint32_t h1[kDropout ? 8 : 1];
-  uint32_t v0[8];
-  uint32_t v1[NG > 4 ? 8 : 1];
+  static constexpr int E = 4 + s1_kept(R);
+  int k[E];
+  int kold[kWindowed ? E : 1];
+  uint32_t h1[kDropout ? E : 1];
+  uint32_t v0[E];
+  uint32_t v1[NG > 4 ? E : 1];
 };
 
-template <int NG, bool kWindowed, bool kDropout>
-__device__ __forceinline__ void load_quad(ColWindow<NG, kWindowed, kDropout>& cw, const S1Smem& sm,
-                                          int col, int at) {
-  const int4 kq = *reinterpret_cast<const int4*>(sm.s_k + col);
-  cw.k[at] = kq.x; cw.k[at + 1] = kq.y; cw.k[at + 2] = kq.z; cw.k[at + 3] = kq.w;
-  if (kWindowed) {
-    const int4 ko = *reinterpret_cast<const int4*>(sm.s_kold + col);
-    cw.kold[at] = ko.x; cw.kold[at + 1] = ko.y; cw.kold[at + 2] = ko.z; cw.kold[at + 3] = ko.w;
+// n entries from column `src` (a multiple of R) with loads of R entries
+template <int R, typename T>
+__device__ __forceinline__ void load_cols(T* dst, const T* src, int n) {
+#pragma unroll
+  for (int x = 0; x < n; x += R) {
+    if constexpr (R == 4) {
+      const int4 w = *reinterpret_cast<const int4*>(src + x);
+      dst[x] = (T)w.x; dst[x + 1] = (T)w.y; dst[x + 2] = (T)w.z; dst[x + 3] = (T)w.w;
+    } else if constexpr (R == 2) {
+      const int2 w = *reinterpret_cast<const int2*>(src + x);
+      dst[x] = (T)w.x; dst[x + 1] = (T)w.y;
+    } else {
+      dst[x] = src[x];
+    }
   }
-  if (kDropout) {
-    const uint4 hq = *reinterpret_cast<const uint4*>(sm.s_h1 + col);
-    cw.h1[at] = hq.x; cw.h1[at + 1] = hq.y; cw.h1[at + 2] = hq.z; cw.h1[at + 3] = hq.w;
-  }
-  const uint4 va = *reinterpret_cast<const uint4*>(sm.s_vb0 + col);
-  cw.v0[at] = va.x; cw.v0[at + 1] = va.y; cw.v0[at + 2] = va.z; cw.v0[at + 3] = va.w;
-  if (NG > 4) {
-    const uint4 vb = *reinterpret_cast<const uint4*>(sm.s_vb1 + col);
-    cw.v1[at] = vb.x; cw.v1[at + 1] = vb.y; cw.v1[at + 2] = vb.z; cw.v1[at + 3] = vb.w;
-  }
+}
+
+template <int NG, int R, bool kWindowed, bool kDropout>
+__device__ __forceinline__ void load_window(ColWindow<NG, R, kWindowed, kDropout>& cw, const S1Smem& sm,
+                                            int col, int at, int n) {
+  load_cols<R>(cw.k + at, sm.s_k + col, n);
+  if (kWindowed) load_cols<R>(cw.kold + at, sm.s_kold + col, n);
+  if (kDropout) load_cols<R>(cw.h1 + at, sm.s_h1 + col, n);
+  load_cols<R>(cw.v0 + at, sm.s_vb0 + col, n);
+  if (NG > 4) load_cols<R>(cw.v1 + at, sm.s_vb1 + col, n);
 }
 
 struct S1Params {
@@ -108,15 +123,50 @@ struct S1Params {
   float neg_md, mul2, bias2;
 };
 
-// Sixteen cells: rows r0 .. r0 + 3 of the block, the thread's four diagonals.  kEdge adds the
+// The sums of a row are formed in one order whatever R is, a binary tree over neighbouring diagonals:
+// inside the thread, across the lanes of a warp from the nearest to the farthest, across the warps.  A
+// sequence then gives the same bits in a launch of any size, alone, in a batch or in a slice.
+template <int N, typename T>
+__device__ __forceinline__ T tree_sum(const T (&v)[N]) {
+  if constexpr (N == 1) return v[0];
+  else if constexpr (N == 2) return v[0] + v[1];
+  else {
+    T half[N / 2];
+#pragma unroll
+    for (int x = 0; x < N / 2; ++x) half[x] = v[2 * x] + v[2 * x + 1];
+    return tree_sum<N / 2>(half);
+  }
+}
+
+// warp_reduce8 with the nearest lanes first: lane L holds the total of value s1_value(L).
+__device__ __forceinline__ int s1_value(int lane) {
+  return (lane & 1) * 4 + (lane & 2) + ((lane >> 2) & 1);
+}
+
+__device__ __forceinline__ float s1_reduce8(const float (&v)[8], int lane) {
+  const bool h1 = lane & 1, h2 = lane & 2, h4 = lane & 4;
+  float a[4], b[2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    a[i] = (h1 ? v[i + 4] : v[i]) + __shfl_xor_sync(0xffffffffu, h1 ? v[i] : v[i + 4], 1);
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    b[i] = (h2 ? a[i + 2] : a[i]) + __shfl_xor_sync(0xffffffffu, h2 ? a[i] : a[i + 2], 2);
+  float c = (h4 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, h4 ? b[0] : b[1], 4);
+  c += __shfl_xor_sync(0xffffffffu, c, 8);
+  c += __shfl_xor_sync(0xffffffffu, c, 16);
+  return c;
+}
+
+// 4 R cells: rows r0 .. r0 + 3 of the block, the thread's R diagonals.  kEdge adds the
 // predicates of blocks that touch the start of a diagonal, the first W + 1 key columns or the
-// end of the sequence.  Returns the keep flags as 16 bits (row rr, diagonal e at bit 4 rr + e)
-// and adds the row sums to es / eds.
-template <int NG, bool kWindowed, bool kDropout, bool kEdge>
-__device__ __forceinline__ uint32_t s1_group(const ColWindow<NG, kWindowed, kDropout>& cw,
+// end of the sequence.  Returns the keep flags as bits (row rr, diagonal e at bit 4 rr + e)
+// and the row sums in es / eds.
+template <int NG, int R, bool kWindowed, bool kDropout, bool kEdge>
+__device__ __forceinline__ uint32_t s1_group(const ColWindow<NG, R, kWindowed, kDropout>& cw,
                                              const S1Smem& sm, const S1Params& p,
                                              const DropoutKey& dkey, int r0, int i0, int j_first,
-                                             uint32_t qword0, float (&S)[kTR], int (&hs)[kTR],
+                                             uint32_t qword0, float (&S)[R], int (&hs)[R],
                                              float (&es)[4], float (&eds)[4]) {
   int q[4], qo[4];
   {
@@ -127,16 +177,16 @@ __device__ __forceinline__ uint32_t s1_group(const ColWindow<NG, kWindowed, kDro
       qo[0] = o4.x; qo[1] = o4.y; qo[2] = o4.z; qo[3] = o4.w;
     }
   }
-  // mismatch counts and the sliding window sums of all sixteen cells first: whether any window
+  // mismatch counts and the sliding window sums of all cells first: whether any window
   // product of the warp survives flush-to-zero is decided once per group
-  int ham[4][kTR];
-  int hsv[4][kTR];
+  int ham[4][R];
+  int hsv[4][R];
   bool alive = false;
 #pragma unroll
   for (int rr = 0; rr < 4; ++rr) {
 #pragma unroll
-    for (int e = 0; e < kTR; ++e) {
-      const int idx = rr + 3 - e;
+    for (int e = 0; e < R; ++e) {
+      const int idx = rr + R - 1 - e;
       ham[rr][e] = __popc(q[rr] ^ cw.k[idx]);
       if (kWindowed) {
         const int old = __popc(qo[rr] ^ cw.kold[idx]);
@@ -153,16 +203,16 @@ __device__ __forceinline__ uint32_t s1_group(const ColWindow<NG, kWindowed, kDro
       }
     }
   }
-  float P[4][kTR];
+  float P[4][R];
 #pragma unroll
   for (int rr = 0; rr < 4; ++rr)
 #pragma unroll
-    for (int e = 0; e < kTR; ++e) P[rr][e] = 0.0f;
+    for (int e = 0; e < R; ++e) P[rr][e] = 0.0f;
   if (kWindowed && __any_sync(0xffffffffu, alive)) {
 #pragma unroll
     for (int rr = 0; rr < 4; ++rr)
 #pragma unroll
-      for (int e = 0; e < kTR; ++e) {
+      for (int e = 0; e < R; ++e) {
         bool on = hsv[rr][e] <= p.hs_cut;
         if (kEdge) on = on && (j_first + rr - e) >= p.W;
         P[rr][e] = on ? __expf(p.neg_md * (float)hsv[rr][e]) : 0.0f;
@@ -173,9 +223,10 @@ __device__ __forceinline__ uint32_t s1_group(const ColWindow<NG, kWindowed, kDro
   for (int rr = 0; rr < 4; ++rr) {
     const float* lut = sm.ulut + (r0 + rr) * NG * 16;
     const uint32_t qword = qword0 ^ (uint32_t)(r0 + rr);   // block rows start at a multiple of 16
+    float part_e[R], part_d[R];
 #pragma unroll
-    for (int e = 0; e < kTR; ++e) {
-      const int idx = rr + 3 - e;
+    for (int e = 0; e < R; ++e) {
+      const int idx = rr + R - 1 - e;
       const float x = sm.glut[ham[rr][e]];
       const float Sn = x * (1.0f + S[e]) - P[rr][e];
       bool act = true;
@@ -185,28 +236,29 @@ __device__ __forceinline__ uint32_t s1_group(const ColWindow<NG, kWindowed, kDro
       float ex = exp2f(fmaf(sqrtf(1.0f + S[e]), p.mul2, p.bias2));
       if (kEdge) ex = act ? ex : 0.0f;
       const float du = tiled_utility<NG>(lut, cw.v0[idx], NG > 4 ? cw.v1[idx] : 0u);
-      es[rr] += ex;
+      part_e[e] = ex;
+      part_d[e] = __fmul_rn(ex, du);      // not fused with the sums, whose grouping depends on R
       if (kDropout) {
         const bool keep = act && dropout_keep_open(dkey, cw.h1[idx], qword);
-        if (keep) {     // predicated: one logic operation and one fused multiply-add
-          keepbits |= 1u << (4 * rr + e);
-          eds[rr] = fmaf(ex, du, eds[rr]);
-        }
-      } else {
-        eds[rr] = fmaf(ex, du, eds[rr]);
+        part_d[e] = keep ? part_d[e] : 0.0f;
+        keepbits |= keep ? 1u << (4 * rr + e) : 0u;
       }
     }
+    es[rr] = tree_sum<R>(part_e);
+    eds[rr] = tree_sum<R>(part_d);
   }
   return keepbits;
 }
 
-// Sweep 1, four diagonals per thread.  Writes the same checkpoints and per-item row partials as
+// Sweep 1, R diagonals per thread.  Writes the same checkpoints and per-item row partials as
 // vjp_sweep1_kernel<NG, true, ...> (analytic softmax reference only); the dropout keep flags go
-// out as one 64-bit word per thread and block, the layout vjp_sweep2_tiled_kernel reads.
-template <int NG, bool kWindowed, bool kDropout>
-__global__ void __launch_bounds__(kTThreads, 8) vjp_sweep1_tiled_kernel(VjpArgs a) {
+// out as one 64-bit word per four diagonals and block, the layout vjp_sweep2_tiled_kernel reads, or
+// (kBallot) as the row ballots that the one-diagonal-per-thread second sweep reads.
+template <int NG, int R, bool kWindowed, bool kDropout, bool kBallot>
+__global__ void __launch_bounds__(s1_threads(R), 2 * R) vjp_sweep1_tiled_kernel(VjpArgs a) {
+  constexpr int kTThreads = s1_threads(R), kTWarps = kTThreads / 32;
   extern __shared__ float4 smem_raw[];
-  const S1Smem sm = s1_carve(reinterpret_cast<float*>(smem_raw), NG);
+  const S1Smem sm = s1_carve(reinterpret_cast<float*>(smem_raw), kTWarps);
   Item it;
   if (!load_item_1d(a, &it)) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -230,15 +282,15 @@ __global__ void __launch_bounds__(kTThreads, 8) vjp_sweep1_tiled_kernel(VjpArgs 
   const DropoutKey dkey = make_dropout_key((uint32_t)it.h + a.head_offset,
                                            (uint32_t)it.seq + a.batch_offset, a.seed, a.dropout_p);
   if (tid <= a.D) sm.glut[tid] = expf(p.neg_md * (float)tid);
-  const int vslot = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+  const int vslot = s1_value(lane);
 
   for (int w = it.w_begin; w < it.w_end; ++w) {
     const int dmin = 1 + w * kTBand;
     const int dmax = dmin + kTBand - 1;
-    float S[kTR];
-    int hs[kTR];
+    float S[R];
+    int hs[R];
 #pragma unroll
-    for (int e = 0; e < kTR; ++e) {
+    for (int e = 0; e < R; ++e) {
       S[e] = 0.0f;
       hs[e] = 0;
     }
@@ -323,8 +375,8 @@ __global__ void __launch_bounds__(kTThreads, 8) vjp_sweep1_tiled_kernel(VjpArgs 
         qold_new = (kWindowed && in && i - W - 1 >= 0) ? __ldg(q + i - W - 1) : 0;
       }
       uint32_t go_first[4];
-      // the per-block chores are spread over both warps: warp 0 fetches the entering columns and
-      // the row symbols, warp 1 builds the utility tables and closes the block's row sums
+      // the per-block chores are spread over the warps: the first fetches the entering columns and
+      // the row symbols, the upper half builds the utility tables and closes the block's row sums
       const int ue = (tid + kTThreads / 2) & (kTThreads - 1);
       load_go4(ue, go_first);
       // -- shared-memory side
@@ -365,34 +417,61 @@ __global__ void __launch_bounds__(kTThreads, 8) vjp_sweep1_tiled_kernel(VjpArgs 
         store_ulut(e, raw);
       }
       __syncthreads();
-      // ---- checkpoint of the thread's four diagonals
+      // ---- checkpoint of the thread's diagonals
       {
-        int4* ck = reinterpret_cast<int4*>(a.ckpt + ck_idx * kTBand + kTR * tid);
-        ck[0] = make_int4(__float_as_int(S[0]), hs[0], __float_as_int(S[1]), hs[1]);
-        ck[1] = make_int4(__float_as_int(S[2]), hs[2], __float_as_int(S[3]), hs[3]);
+        auto* ck = a.ckpt + ck_idx * kTBand + R * tid;
+        if constexpr (R == 1) {
+          *reinterpret_cast<int2*>(ck) = make_int2(__float_as_int(S[0]), hs[0]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < R; e += 2)
+            reinterpret_cast<int4*>(ck)[e / 2] =
+                make_int4(__float_as_int(S[e]), hs[e], __float_as_int(S[e + 1]), hs[e + 1]);
+        }
       }
       const bool interior = jwin0 >= (kWindowed ? W + 1 : 0) && i0 + kTRows - 1 <= it.len - 1;
       const uint32_t qword0 = dropout_query_word((uint32_t)i0);
-      // window column of (row 0, diagonal 3 of this thread); a multiple of 4
-      const int col0 = kTBand - kTR - kTR * tid;
-      ColWindow<NG, kWindowed, kDropout> cw;
-      load_quad<NG, kWindowed, kDropout>(cw, win, col0, 0);
+      // window column of (row 0, last diagonal of this thread); a multiple of R
+      const int col0 = kTBand - R - R * tid;
+      constexpr int kKept = s1_kept(R);
+      ColWindow<NG, R, kWindowed, kDropout> cw;
+      load_window<NG, R, kWindowed, kDropout>(cw, win, col0, 0, kKept);
       uint32_t keep_lo = 0u, keep_hi = 0u;
 #pragma unroll 1
       for (int r0 = 0; r0 < kTRows; r0 += 4) {
-        load_quad<NG, kWindowed, kDropout>(cw, win, col0 + r0 + 4 < kTWin ? col0 + r0 + 4 : col0 + r0, 4);
+        load_window<NG, R, kWindowed, kDropout>(cw, win, col0 + r0 + kKept, kKept, 4);
         float es[4] = {0.0f, 0.0f, 0.0f, 0.0f}, eds[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         // key column of (row r0, diagonal 0 of this thread)
-        const int j_first = jwin0 + col0 + r0 + 3;
+        const int j_first = jwin0 + col0 + r0 + R - 1;
         uint32_t keep;
         if (interior)
-          keep = s1_group<NG, kWindowed, kDropout, false>(cw, sm, p, dkey, r0, i0, j_first, qword0, S,
+          keep = s1_group<NG, R, kWindowed, kDropout, false>(cw, sm, p, dkey, r0, i0, j_first, qword0, S,
                                                           hs, es, eds);
         else
-          keep = s1_group<NG, kWindowed, kDropout, true>(cw, sm, p, dkey, r0, i0, j_first, qword0, S,
+          keep = s1_group<NG, R, kWindowed, kDropout, true>(cw, sm, p, dkey, r0, i0, j_first, qword0, S,
                                                          hs, es, eds);
-        if (kDropout) {
-          // 16 keep flags of this group: bit 4 r + e of the thread's 64-bit word of the block
+        if constexpr (kDropout && kBallot) {
+          // a word per row and 32 diagonals: [row][diagonal / 32], lane L writes row L / R (R = 2: the
+          // even diagonals' flags and the odd ones' are interleaved)
+          static_assert(R <= 2, "a word holds the flags of whole lanes of one or two diagonals");
+          const int mine = (lane / R) & 3;
+          uint32_t word[R];
+#pragma unroll
+          for (int rr = 0; rr < 4; ++rr)
+#pragma unroll
+            for (int e = 0; e < R; ++e) {
+              const uint32_t ballot = __ballot_sync(0xffffffffu, keep >> (4 * rr + e) & 1u);
+              if (rr == 0 || mine == rr) word[e] = ballot;
+            }
+          if constexpr (R == 2) {
+            const int half = 16 * (lane & 1);
+            word[0] = spread_bits(word[0] >> half) | spread_bits(word[1] >> half) << 1;
+          }
+          const int row = r0 + mine - skew;     // there the rows of a block count from its first one
+          if (lane < 4 * R && row >= 0)
+            a.keepbits[(ck_idx * kTRows + row) * (kTBand / 32) + R * warp + lane % R] = word[0];
+        } else if (kDropout) {
+          // the keep flags of this group: bit 4 r + e of the 64-bit word of the block
           if (r0 < 8) keep_lo |= keep << (4 * r0);
           else keep_hi |= keep << (4 * (r0 - 8));
         }
@@ -402,12 +481,12 @@ __global__ void __launch_bounds__(kTThreads, 8) vjp_sweep1_tiled_kernel(VjpArgs 
           v[2 * rr] = es[rr];
           v[2 * rr + 1] = eds[rr];
         }
-        const float total = warp_reduce8(v, lane);
-        if ((lane & 3) == 0)
+        const float total = s1_reduce8(v, lane);
+        if (lane < 8)
           reinterpret_cast<float*>(sm.wstat + (r0 + (vslot >> 1)) * kTWarps + warp)[vslot & 1] = total;
-        // the upper quad becomes the lower one of the next group
+        // the upper entries become the lower ones of the next group
 #pragma unroll
-        for (int x = 0; x < 4; ++x) {
+        for (int x = 0; x < kKept; ++x) {
           cw.k[x] = cw.k[x + 4];
           if (kWindowed) cw.kold[x] = cw.kold[x + 4];
           if (kDropout) cw.h1[x] = cw.h1[x + 4];
@@ -415,21 +494,37 @@ __global__ void __launch_bounds__(kTThreads, 8) vjp_sweep1_tiled_kernel(VjpArgs 
           if (NG > 4) cw.v1[x] = cw.v1[x + 4];
         }
       }
-      // keep flags of the block: one 64-bit word per thread (row r, diagonal e at bit 4 r + e)
-      if (kDropout)
-        reinterpret_cast<uint2*>(a.keepbits)[ck_idx * kTThreads + tid] = make_uint2(keep_lo, keep_hi);
+      // keep flags of the block: one 64-bit word per four diagonals (row r, diagonal e at bit
+      // 4 r + e), put together by the 4 / R threads that own them
+      if (kDropout && !kBallot) {
+        if constexpr (R < 4) {
+          const int part = tid & (4 / R - 1);
+          keep_lo <<= R * part;
+          keep_hi <<= R * part;
+#pragma unroll
+          for (int x = 1; x < 4 / R; x *= 2) {
+            keep_lo |= __shfl_xor_sync(0xffffffffu, keep_lo, x);
+            keep_hi |= __shfl_xor_sync(0xffffffffu, keep_hi, x);
+          }
+        }
+        if ((tid & (4 / R - 1)) == 0)
+          reinterpret_cast<uint2*>(a.keepbits)[ck_idx * (kTBand / 4) + tid / (4 / R)] =
+              make_uint2(keep_lo, keep_hi);
+      }
       __syncthreads();
-      const int tr = tid - kTThreads / 2;         // row of the tail, on warp 1
+      const int tr = tid - kTThreads / 2;         // row of the tail
       if (tr >= 0 && tr < kTRows) {
         const int i = i0 + tr;
         if (i >= first_row && i <= it.len - 1) {
-          float m = ref_top - logf((float)i), z = 0.0f, e = 0.0f;
+          float m = ref_top - logf((float)i);
+          float zs[kTWarps], es[kTWarps];
 #pragma unroll
           for (int ww = 0; ww < kTWarps; ++ww) {
             const float2 part = sm.wstat[tr * kTWarps + ww];
-            z += part.x;
-            e += part.y;
+            zs[ww] = part.x;
+            es[ww] = part.y;
           }
+          float z = tree_sum<kTWarps>(zs), e = tree_sum<kTWarps>(es);
           e *= a.inv_keep;
           const int64_t slot = it.rowslot + i;
           if (w > it.w_begin) {
@@ -443,32 +538,64 @@ __global__ void __launch_bounds__(kTThreads, 8) vjp_sweep1_tiled_kernel(VjpArgs 
   }
 }
 
-template <int NG>
-int launch_s1_tiled(const VjpArgs& a, unsigned grid, cudaStream_t stream) {
-  const size_t smem = (size_t)s1_smem_words(NG) * sizeof(float);
+template <int NG, int R, bool kBallot>
+int launch_s1_tiled_r(const VjpArgs& a, unsigned grid, cudaStream_t stream) {
+  constexpr int threads = s1_threads(R);
+  constexpr size_t smem = (size_t)s1_smem_words(NG, threads / 32) * sizeof(float);
   const bool windowed = a.ring_slots > 0;
   const bool dropout = a.dropout_p > 0.0f;
   if (windowed && dropout)
-    vjp_sweep1_tiled_kernel<NG, true, true><<<grid, kTThreads, smem, stream>>>(a);
+    vjp_sweep1_tiled_kernel<NG, R, true, true, kBallot><<<grid, threads, smem, stream>>>(a);
   else if (windowed)
-    vjp_sweep1_tiled_kernel<NG, true, false><<<grid, kTThreads, smem, stream>>>(a);
+    vjp_sweep1_tiled_kernel<NG, R, true, false, false><<<grid, threads, smem, stream>>>(a);
   else if (dropout)
-    vjp_sweep1_tiled_kernel<NG, false, true><<<grid, kTThreads, smem, stream>>>(a);
+    vjp_sweep1_tiled_kernel<NG, R, false, true, kBallot><<<grid, threads, smem, stream>>>(a);
   else
-    vjp_sweep1_tiled_kernel<NG, false, false><<<grid, kTThreads, smem, stream>>>(a);
+    vjp_sweep1_tiled_kernel<NG, R, false, false, false><<<grid, threads, smem, stream>>>(a);
   ROSA_CUDA_OK(cudaGetLastError());
   return 0;
 }
 
+// Diagonals per thread.  Four share the most work (row values, column loads, row reductions), but a
+// CTA is then two warps that need 7 us for a block of 16 rows; two or one have more warps work on a
+// block.  Where the longest item decides that is the faster way (time with four / two / one):
+//   1 x 256 x 4 float32 (fill 0.03)                    52 / 44 / 39 us
+//   1 x 4096 x 16 (fill 0.9)                          1219 / 807 / 782 us
+//   packed 3001 x 16, sequences up to 257             165 / 100 / 79 us
+//   2 x 1024 x 64 (fill 2.2)                          472 / 329 / 370 us
+//   4 x 1024 x 64 (fill 4.3)                          599 / 548 / 642 us
+//   2 x 4096 x 64 (fill 7.4)                          3.01 / 3.06 / 3.98 ms
+//   16 x 8192 x 64 in slices (fill 14)                76.1 / 81.1 / 111 ms
+// Value rows of more than 16 components (two sign tables) never take four: their column windows and
+// four sets of diagonals leave no registers to overlap anything (packed 32768 x 16, 32 components:
+// 14.0 / 8.1 / 10.2 ms).
+template <int NG>
+int launch_s1_tiled(const VjpArgs& a, unsigned grid, cudaStream_t stream) {
+  const float fill = vjp_fill(a);
+  if (!vjp_tiled_applies(a)) {      // the second sweep is the one that reads ballots
+    if (fill < 1.8f) return launch_s1_tiled_r<NG, 1, true>(a, grid, stream);
+    return launch_s1_tiled_r<NG, 2, true>(a, grid, stream);
+  }
+  if (fill < 1.8f) return launch_s1_tiled_r<NG, 1, false>(a, grid, stream);
+  if constexpr (NG > 4) {
+    return launch_s1_tiled_r<NG, 2, false>(a, grid, stream);
+  } else {
+    if (fill < 7.0f) return launch_s1_tiled_r<NG, 2, false>(a, grid, stream);
+    return launch_s1_tiled_r<NG, 4, false>(a, grid, stream);
+  }
+}
+
 }  // namespace
 
-bool vjp_tiled_applies(const VjpArgs& a) {
-  // value rows of up to 32 components (nibble tables), symbols of up to 16 bits (one MMA N of the
-  // second sweep), the analytic softmax reference, and not the testing flag that selects the
-  // one-diagonal-per-thread kernels
+// Value rows of up to 32 components (nibble tables), the analytic softmax reference, and not the
+// testing flag that selects the one-diagonal-per-thread kernels.
+bool vjp_sweep1_tiled_applies(const VjpArgs& a) {
   const float top = a.scale * kSqrtScale * (sqrtf(1.0f + (float)a.W) - 1.0f);
-  return a.Dv <= 32 && a.D <= 16 && top <= 80.0f && !a.force_cuda_core_contraction;
+  return a.Dv <= 32 && top <= 80.0f && !a.force_cuda_core_contraction;
 }
+
+// The second sweep takes symbols of up to 16 bits (one MMA N).
+bool vjp_tiled_applies(const VjpArgs& a) { return vjp_sweep1_tiled_applies(a) && a.D <= 16; }
 
 int launch_vjp_sweep1_tiled(const VjpArgs& a, int items_upper, cudaStream_t stream) {
   const unsigned grid = (unsigned)((int64_t)items_upper * a.H);
