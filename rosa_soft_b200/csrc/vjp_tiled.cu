@@ -10,7 +10,7 @@
 // 128-bit shared-memory loads per table and sixteen cells, kept in registers and indexed at
 // compile time.  Everything that depends on the row only (query symbols, hash word of the query
 // position, utility table base) is loaded once per row and thread and shared by R cells; the row
-// sums of R cells are added in registers before the warp reduction.  Rows of a block always start
+// sums of four cells are added in registers before the warp reduction.  Rows of a block always start
 // at a multiple of 16 (rows that do not exist are masked), interior blocks -- every cell active and past the
 // horizon -- run without any per-cell predicate.
 #include "common.cuh"
@@ -44,15 +44,19 @@ struct S1Smem {
   int* s_q;          // [kTRows]
   int* s_qold;       // [kTRows]
   float* glut;       // [64] gate per mismatch count
-  float2* wstat;     // [kTRows][warps] per-warp (sum e, sum e d u)
+  float2* wstat;     // four diagonals a thread: [kTRows][warps] sums of (e, e d u); else the cells'
+                     // (e, d u), [kTRows][kTBand] in the order of s1_cell
   float* ulut;       // [kTRows][NG][16]
 };
 
-__host__ __device__ constexpr int s1_smem_words(int ng, int warps) {
-  return 5 * kTTab + 2 * kTRows + 64 + 2 * kTRows * warps + kTRows * ng * 16;
+__host__ __device__ constexpr int s1_stat_words(int R) {
+  return 2 * kTRows * (R == 4 ? s1_threads(R) / 32 : kTBand);
+}
+__host__ __device__ constexpr int s1_smem_words(int ng, int R) {
+  return 5 * kTTab + 2 * kTRows + 64 + s1_stat_words(R) + kTRows * ng * 16;
 }
 
-__device__ __forceinline__ S1Smem s1_carve(float* base, int warps) {
+__device__ __forceinline__ S1Smem s1_carve(float* base, int R) {
   S1Smem s;
   int* w = reinterpret_cast<int*>(base);
   s.s_k = w;                                        w += kTTab;
@@ -63,7 +67,7 @@ __device__ __forceinline__ S1Smem s1_carve(float* base, int warps) {
   s.s_q = w;                                        w += kTRows;
   s.s_qold = w;                                     w += kTRows;
   s.glut = reinterpret_cast<float*>(w);             w += 64;
-  s.wstat = reinterpret_cast<float2*>(w);           w += 2 * kTRows * warps;
+  s.wstat = reinterpret_cast<float2*>(w);           w += s1_stat_words(R);
   s.ulut = reinterpret_cast<float*>(w);
   return s;
 }
@@ -123,51 +127,67 @@ struct S1Params {
   float neg_md, mul2, bias2;
 };
 
-// The sums of a row are formed in one order whatever R is, a binary tree over neighbouring diagonals:
-// inside the thread, across the lanes of a warp from the nearest to the farthest, across the warps.  A
-// sequence then gives the same bits in a launch of any size, alone, in a batch or in a slice.
-template <int N, typename T>
-__device__ __forceinline__ T tree_sum(const T (&v)[N]) {
-  if constexpr (N == 1) return v[0];
-  else if constexpr (N == 2) return v[0] + v[1];
-  else {
-    T half[N / 2];
+// The sums of a row are formed in one order whatever R is: four neighbouring diagonals one after the
+// other, then 32 such groups as warp_reduce8 pairs its lanes, then the two halves of the band.  A
+// sequence then gives the same bits in a launch of any size, alone, in a batch or in a slice.  With
+// four diagonals a thread holds a group and a warp half a band; with fewer the cells go to shared
+// memory and the sums are formed behind the barrier that closes the block (s1_row_sums).
+//
+// Where the cells of a row lie: neighbouring pairs change places in half of the groups, those that
+// the lanes of a quarter warp would otherwise read from the same banks in s1_row_sums.
+template <int R>
+__device__ __forceinline__ int s1_swap(int group) {
+  return (R == 1 ? group >> 2 : group >> 5) & 1;
+}
+template <int R>
+__device__ __forceinline__ int s1_cell(int diagonal) {
+  return diagonal ^ 2 * s1_swap<R>(diagonal >> 2);
+}
+
+// Sum of e and of e d u over 4 neighbouring diagonals from their (e, d u); a dropped cell's d u is 0
+// and leaves the second sum as it is.
+template <int R>
+__device__ __forceinline__ float2 s1_group_sums(const float4* row, int group) {
+  const int swap = s1_swap<R>(group);
+  const float4 a = row[2 * group + swap], b = row[2 * group + 1 - swap];
+  return make_float2(a.x + a.z + b.x + b.z,
+                     fmaf(b.z, b.w, fmaf(b.x, b.y, fmaf(a.z, a.w, a.x * a.y))));
+}
+
+// Totals of row `row` of the block by 16 / R neighbouring lanes, half of them for each half of the
+// band; every lane gets them.  The pairing is that of warp_reduce8: 16, 8, 4, 2, 1 groups apart.
+template <int R>
+__device__ __forceinline__ float2 s1_row_sums(const float2* wstat, int row, int lane) {
+  constexpr int kHalf = 8 / R, kGroups = 32 / kHalf;
+  const int u = lane & (kHalf - 1), half = (lane / kHalf) & 1;
+  const float4* cells = reinterpret_cast<const float4*>(wstat + row * kTBand);
+  float2 v[kGroups];                       // groups u, u + kHalf, ...
 #pragma unroll
-    for (int x = 0; x < N / 2; ++x) half[x] = v[2 * x] + v[2 * x + 1];
-    return tree_sum<N / 2>(half);
+  for (int g = 0; g < kGroups; ++g) v[g] = s1_group_sums<R>(cells, 32 * half + u + kHalf * g);
+#pragma unroll
+  for (int n = kGroups / 2; n >= 1; n /= 2)
+#pragma unroll
+    for (int g = 0; g < n; ++g) v[g] = make_float2(v[g].x + v[g + n].x, v[g].y + v[g + n].y);
+  float2 t = v[0];
+#pragma unroll
+  for (int x = kHalf / 2; x >= 1; x /= 2) {
+    t.x += __shfl_xor_sync(0xffffffffu, t.x, x);
+    t.y += __shfl_xor_sync(0xffffffffu, t.y, x);
   }
-}
-
-// warp_reduce8 with the nearest lanes first: lane L holds the total of value s1_value(L).
-__device__ __forceinline__ int s1_value(int lane) {
-  return (lane & 1) * 4 + (lane & 2) + ((lane >> 2) & 1);
-}
-
-__device__ __forceinline__ float s1_reduce8(const float (&v)[8], int lane) {
-  const bool h1 = lane & 1, h2 = lane & 2, h4 = lane & 4;
-  float a[4], b[2];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-    a[i] = (h1 ? v[i + 4] : v[i]) + __shfl_xor_sync(0xffffffffu, h1 ? v[i] : v[i + 4], 1);
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-    b[i] = (h2 ? a[i + 2] : a[i]) + __shfl_xor_sync(0xffffffffu, h2 ? a[i] : a[i + 2], 2);
-  float c = (h4 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, h4 ? b[0] : b[1], 4);
-  c += __shfl_xor_sync(0xffffffffu, c, 8);
-  c += __shfl_xor_sync(0xffffffffu, c, 16);
-  return c;
+  return make_float2(t.x + __shfl_xor_sync(0xffffffffu, t.x, kHalf),
+                     t.y + __shfl_xor_sync(0xffffffffu, t.y, kHalf));
 }
 
 // 4 R cells: rows r0 .. r0 + 3 of the block, the thread's R diagonals.  kEdge adds the
 // predicates of blocks that touch the start of a diagonal, the first W + 1 key columns or the
-// end of the sequence.  Returns the keep flags as bits (row rr, diagonal e at bit 4 rr + e)
-// and the row sums in es / eds.
+// end of the sequence.  Returns the keep flags as bits (row rr, diagonal e at bit 4 rr + e); R = 4
+// adds the row sums to es / eds, fewer diagonals store the thread's cells at `cells`.
 template <int NG, int R, bool kWindowed, bool kDropout, bool kEdge>
 __device__ __forceinline__ uint32_t s1_group(const ColWindow<NG, R, kWindowed, kDropout>& cw,
                                              const S1Smem& sm, const S1Params& p,
                                              const DropoutKey& dkey, int r0, int i0, int j_first,
                                              uint32_t qword0, float (&S)[R], int (&hs)[R],
-                                             float (&es)[4], float (&eds)[4]) {
+                                             float (&es)[4], float (&eds)[4], float2* cells) {
   int q[4], qo[4];
   {
     const int4 q4 = *reinterpret_cast<const int4*>(sm.s_q + r0);
@@ -223,7 +243,7 @@ __device__ __forceinline__ uint32_t s1_group(const ColWindow<NG, R, kWindowed, k
   for (int rr = 0; rr < 4; ++rr) {
     const float* lut = sm.ulut + (r0 + rr) * NG * 16;
     const uint32_t qword = qword0 ^ (uint32_t)(r0 + rr);   // block rows start at a multiple of 16
-    float part_e[R], part_d[R];
+    float ev[R], dv[R];
 #pragma unroll
     for (int e = 0; e < R; ++e) {
       const int idx = rr + R - 1 - e;
@@ -236,16 +256,22 @@ __device__ __forceinline__ uint32_t s1_group(const ColWindow<NG, R, kWindowed, k
       float ex = exp2f(fmaf(sqrtf(1.0f + S[e]), p.mul2, p.bias2));
       if (kEdge) ex = act ? ex : 0.0f;
       const float du = tiled_utility<NG>(lut, cw.v0[idx], NG > 4 ? cw.v1[idx] : 0u);
-      part_e[e] = ex;
-      part_d[e] = __fmul_rn(ex, du);      // not fused with the sums, whose grouping depends on R
-      if (kDropout) {
-        const bool keep = act && dropout_keep_open(dkey, cw.h1[idx], qword);
-        part_d[e] = keep ? part_d[e] : 0.0f;
-        keepbits |= keep ? 1u << (4 * rr + e) : 0u;
+      const bool keep = !kDropout || (act && dropout_keep_open(dkey, cw.h1[idx], qword));
+      if constexpr (R == 4) {
+        es[rr] += ex;
+        if (keep) {       // predicated: one logic operation and one fused multiply-add
+          if (kDropout) keepbits |= 1u << (4 * rr + e);
+          eds[rr] = fmaf(ex, du, eds[rr]);
+        }
+      } else {
+        if (kDropout) keepbits |= keep ? 1u << (4 * rr + e) : 0u;
+        ev[e] = ex;
+        dv[e] = keep ? du : 0.0f;
       }
     }
-    es[rr] = tree_sum<R>(part_e);
-    eds[rr] = tree_sum<R>(part_d);
+    if constexpr (R == 2)
+      *reinterpret_cast<float4*>(cells + rr * kTBand) = make_float4(ev[0], dv[0], ev[1], dv[1]);
+    if constexpr (R == 1) cells[rr * kTBand] = make_float2(ev[0], dv[0]);
   }
   return keepbits;
 }
@@ -258,7 +284,7 @@ template <int NG, int R, bool kWindowed, bool kDropout, bool kBallot>
 __global__ void __launch_bounds__(s1_threads(R), 2 * R) vjp_sweep1_tiled_kernel(VjpArgs a) {
   constexpr int kTThreads = s1_threads(R), kTWarps = kTThreads / 32;
   extern __shared__ float4 smem_raw[];
-  const S1Smem sm = s1_carve(reinterpret_cast<float*>(smem_raw), kTWarps);
+  const S1Smem sm = s1_carve(reinterpret_cast<float*>(smem_raw), R);
   Item it;
   if (!load_item_1d(a, &it)) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -276,13 +302,14 @@ __global__ void __launch_bounds__(s1_threads(R), 2 * R) vjp_sweep1_tiled_kernel(
   p.neg_md = -a.mismatch_scale / (float)a.D;
   p.hs_cut = a.window_cut;
   const float logit_mul = kSqrtScale * a.scale;
-  const float ref_top = a.scale * kSqrtScale * (sqrtf(1.0f + (float)W) - 1.0f);
+  const float top_root = sqrtf(1.0f + (float)W) - 1.0f;
+  const float ref_top = a.scale * kSqrtScale * top_root;
   p.mul2 = logit_mul * 1.4426950408889634f;
   p.bias2 = -(logit_mul + ref_top) * 1.4426950408889634f;
   const DropoutKey dkey = make_dropout_key((uint32_t)it.h + a.head_offset,
                                            (uint32_t)it.seq + a.batch_offset, a.seed, a.dropout_p);
   if (tid <= a.D) sm.glut[tid] = expf(p.neg_md * (float)tid);
-  const int vslot = s1_value(lane);
+  const int vslot = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
 
   for (int w = it.w_begin; w < it.w_end; ++w) {
     const int dmin = 1 + w * kTBand;
@@ -304,8 +331,8 @@ __global__ void __launch_bounds__(s1_threads(R), 2 * R) vjp_sweep1_tiled_kernel(
       const int skew = first_row - i0;
       const int64_t ck_idx = ck_band + (rb - rb_lo);
       // No barrier here: every warp has passed the barrier that closes the previous block (all
-      // table reads done), and the threads that still read the per-warp row sums after it are
-      // through before they reach the barrier below, ahead of which nobody writes new sums.
+      // table reads done), and the threads that still read the sums or cells of its rows after it
+      // are through before they reach the barrier below, ahead of which nobody writes new ones.
       // ---- block tables: entry `at` of the buffers describes window column c.  Every global
       // load of the block (entering columns, row symbols, grad_output of the utility tables) is
       // issued before the first result is used, so the section costs one round trip to L2, not
@@ -443,13 +470,14 @@ __global__ void __launch_bounds__(s1_threads(R), 2 * R) vjp_sweep1_tiled_kernel(
         float es[4] = {0.0f, 0.0f, 0.0f, 0.0f}, eds[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         // key column of (row r0, diagonal 0 of this thread)
         const int j_first = jwin0 + col0 + r0 + R - 1;
+        float2* cells = R == 4 ? nullptr : sm.wstat + r0 * kTBand + s1_cell<R>(R * tid);
         uint32_t keep;
         if (interior)
           keep = s1_group<NG, R, kWindowed, kDropout, false>(cw, sm, p, dkey, r0, i0, j_first, qword0, S,
-                                                          hs, es, eds);
+                                                          hs, es, eds, cells);
         else
           keep = s1_group<NG, R, kWindowed, kDropout, true>(cw, sm, p, dkey, r0, i0, j_first, qword0, S,
-                                                         hs, es, eds);
+                                                         hs, es, eds, cells);
         if constexpr (kDropout && kBallot) {
           // a word per row and 32 diagonals: [row][diagonal / 32], lane L writes row L / R (R = 2: the
           // even diagonals' flags and the odd ones' are interleaved)
@@ -475,15 +503,17 @@ __global__ void __launch_bounds__(s1_threads(R), 2 * R) vjp_sweep1_tiled_kernel(
           if (r0 < 8) keep_lo |= keep << (4 * r0);
           else keep_hi |= keep << (4 * (r0 - 8));
         }
-        float v[8];
+        if constexpr (R == 4) {
+          float v[8];
 #pragma unroll
-        for (int rr = 0; rr < 4; ++rr) {
-          v[2 * rr] = es[rr];
-          v[2 * rr + 1] = eds[rr];
+          for (int rr = 0; rr < 4; ++rr) {
+            v[2 * rr] = es[rr];
+            v[2 * rr + 1] = eds[rr];
+          }
+          const float total = warp_reduce8(v, lane);
+          if ((lane & 3) == 0)
+            reinterpret_cast<float*>(sm.wstat + (r0 + (vslot >> 1)) * kTWarps + warp)[vslot & 1] = total;
         }
-        const float total = s1_reduce8(v, lane);
-        if (lane < 8)
-          reinterpret_cast<float*>(sm.wstat + (r0 + (vslot >> 1)) * kTWarps + warp)[vslot & 1] = total;
         // the upper entries become the lower ones of the next group
 #pragma unroll
         for (int x = 0; x < kKept; ++x) {
@@ -512,20 +542,25 @@ __global__ void __launch_bounds__(s1_threads(R), 2 * R) vjp_sweep1_tiled_kernel(
               make_uint2(keep_lo, keep_hi);
       }
       __syncthreads();
-      const int tr = tid - kTThreads / 2;         // row of the tail
-      if (tr >= 0 && tr < kTRows) {
+      // row of the tail: R = 4 one thread of the second warp each, else 16 or 8 lanes each
+      constexpr int kLanes = R == 4 ? 2 : kTThreads / kTRows;
+      const int tr = R == 4 ? tid - kTThreads / 2 : tid / kLanes;
+      float2 sum = make_float2(0.0f, 0.0f);
+      if constexpr (R < 4) sum = s1_row_sums<R>(sm.wstat, tr, lane);
+      if (tr >= 0 && tr < kTRows && (R == 4 || tid % kLanes == 0)) {
         const int i = i0 + tr;
         if (i >= first_row && i <= it.len - 1) {
-          float m = ref_top - logf((float)i);
-          float zs[kTWarps], es[kTWarps];
-#pragma unroll
-          for (int ww = 0; ww < kTWarps; ++ww) {
-            const float2 part = sm.wstat[tr * kTWarps + ww];
-            zs[ww] = part.x;
-            es[ww] = part.y;
+          if constexpr (R == 4) {
+            const float2 upper = sm.wstat[tr * kTWarps], lower = sm.wstat[tr * kTWarps + 1];
+            sum = make_float2(upper.x + lower.x, upper.y + lower.y);
           }
-          float z = tree_sum<kTWarps>(zs), e = tree_sum<kTWarps>(es);
-          e *= a.inv_keep;
+          // ref_top - log i, rounded once; where both factors of ref_top are at hand the product
+          // is fused and log i rounded, elsewhere log i is.  (One last bit of m is 2e-6 of a row's
+          // sums: each variant keeps its rounding, so that gradients keep their bits.)
+          constexpr bool kFusedTop = kWindowed && (kDropout || NG > 4);
+          float m = kFusedTop ? fmaf(a.scale * kSqrtScale, top_root, -logf((float)i))
+                              : fmaf(-__log2f((float)i), 0.69314718f, ref_top);
+          float z = sum.x, e = sum.y * a.inv_keep;
           const int64_t slot = it.rowslot + i;
           if (w > it.w_begin) {
             const float4 prev = a.stat_part[slot];
@@ -541,17 +576,16 @@ __global__ void __launch_bounds__(s1_threads(R), 2 * R) vjp_sweep1_tiled_kernel(
 template <int NG, int R, bool kBallot>
 int launch_s1_tiled_r(const VjpArgs& a, unsigned grid, cudaStream_t stream) {
   constexpr int threads = s1_threads(R);
-  constexpr size_t smem = (size_t)s1_smem_words(NG, threads / 32) * sizeof(float);
+  constexpr int smem = s1_smem_words(NG, R) * (int)sizeof(float);
   const bool windowed = a.ring_slots > 0;
   const bool dropout = a.dropout_p > 0.0f;
-  if (windowed && dropout)
-    vjp_sweep1_tiled_kernel<NG, R, true, true, kBallot><<<grid, threads, smem, stream>>>(a);
-  else if (windowed)
-    vjp_sweep1_tiled_kernel<NG, R, true, false, false><<<grid, threads, smem, stream>>>(a);
-  else if (dropout)
-    vjp_sweep1_tiled_kernel<NG, R, false, true, kBallot><<<grid, threads, smem, stream>>>(a);
-  else
-    vjp_sweep1_tiled_kernel<NG, R, false, false, false><<<grid, threads, smem, stream>>>(a);
+  auto kernel = windowed ? (dropout ? vjp_sweep1_tiled_kernel<NG, R, true, true, kBallot>
+                                    : vjp_sweep1_tiled_kernel<NG, R, true, false, false>)
+                         : (dropout ? vjp_sweep1_tiled_kernel<NG, R, false, true, kBallot>
+                                    : vjp_sweep1_tiled_kernel<NG, R, false, false, false>);
+  if (smem > 48 * 1024)
+    ROSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  kernel<<<grid, threads, smem, stream>>>(a);
   ROSA_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -3,6 +3,8 @@ a block of 16 rows and a band of 256 diagonals, symbols on both sides of 8 bits 
 holds 8 or 16), all value widths, launches of little and of much work (one, two or four diagonals per
 thread), and streams whose window products stay alive (S rebuilt from every fourth row together with
 the products)."""
+import hashlib
+
 import numpy as np
 import pytest
 import torch
@@ -59,3 +61,26 @@ def test_live_window_products(T, D, Dv, W, p, dtype):
     (33, 32, 129, 6, 12, 20, 0.1), (33, 32, 146, 8, 4, 200, 0.1), (33, 32, 100, 9, 20, 7, 0.05)])  # four, four, two
 def test_launches_of_every_size(B, H, T, D, Dv, W, p, dtype):
     _random(B, T, H, D, 1, Dv, W, p, dtype)
+
+
+# sha256 of the float32 gradients (dq, dk, dv) of heads 0 and 1 of sequence 0, as the sweep with four
+# diagonals per thread gave them before there were others.  No window product is alive here.
+ROW_SUM_BITS = {
+    (8, 0.0): "06e1d9c03c593cb661cc5a2ffafa681bbd012a46286ddcd7a991cb0187fd1e16",
+    (8, 0.1): "4245b35eeb36ebe843df237814b20e7384b4a9d709be7167e5379488741a90e1",
+    (16, 0.1): "9d38878ae149926d4f5f5513b906890efed4f8822f673d9ef63a730a2ec79c05",
+    (24, 0.0): "c474b1a2f15a05974865e01d01a14666bcaa9df7901daee8027ab75b6ca4a24f"}
+
+
+@pytest.mark.parametrize("B,H", [(1, 4), (1, 256), (32, 64)])       # one, two, four diagonals per thread
+@pytest.mark.parametrize("Dv,p", sorted(ROW_SUM_BITS))
+def test_row_sums_have_the_same_bits_in_launches_of_every_size(B, H, Dv, p):
+    from rosa_soft_b200 import cabi
+    T, D, W = 530, 8, 128
+    whole = lambda x: x.repeat(B, H // 2, 1).to(DEV)  # noqa: E731
+    q, k, v, go = (whole(nonzero_randn((T, 2, n), s)) for s, n in ((1, D), (2, D), (3, Dv), (4, Dv)))
+    _, pq, pk, _, _ = cabi.hard_forward(q, k, v, (B, T), W)
+    seed = torch.tensor(7, dtype=torch.int64, device=DEV) if p > 0 else None
+    got = cabi.surrogate_vjp(q, k, v, go, (B, T), pq, pk, W, 1.0, p, 3.0, seed, 7)[:3]
+    bits = hashlib.sha256(b"".join(g[:T, :2].contiguous().cpu().numpy().tobytes() for g in got)).hexdigest()
+    assert bits == ROW_SUM_BITS[Dv, p]
