@@ -127,9 +127,7 @@ class StreamCore {
     }
     longest_ = after;
     phase_ ^= 1;
-    if (stream != *home_)   // the state was allocated on another stream
-      for (const Tensor& t : {query_, key_, payload_, links_, tables_, lens_, scratch_})
-        c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), stream);
+    used_on(stream);
     last_.record(stream);
     last_stream_ = stream;
     ordered_ = true;
@@ -237,6 +235,14 @@ class StreamCore {
     return u;
   }
 
+  // Work on `stream` touches the state: its memory, allocated on another stream perhaps, may not be
+  // handed out again before that work is done.
+  void used_on(const c10::cuda::CUDAStream& stream) const {
+    if (stream == *home_) return;
+    for (const Tensor& t : {query_, key_, payload_, links_, tables_, lens_, scratch_})
+      c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), stream);
+  }
+
   void reindex(const c10::cuda::CUDAStream& stream) {
     rosa_b200_stream_call u = state_of_call();
     u.chunk_tokens = -1;
@@ -260,8 +266,6 @@ class StreamCore {
         C10_CUDA_CHECK(cudaMemcpy2DAsync(t.data_ptr(), capacity * item, old.data_ptr(), capacity_ * item,
                                          capacity_ * item, slots_ * heads, cudaMemcpyDeviceToDevice,
                                          stream.stream()));
-        if (stream != *home_)
-          c10::cuda::CUDACachingAllocator::recordStream(old.storage().data_ptr(), stream);
       }
       return t;
     };
@@ -279,7 +283,9 @@ class StreamCore {
       if (!rebuilt) tables = tables_.clone();
     }
     if (capacity_ == 0 || rebuilt) tables = torch::zeros({slots_, heads_, table}, u8);
-    // everything is allocated: an update that runs out of memory leaves the state as it was
+    // everything is allocated: an update that runs out of memory leaves the state as it was.  The old
+    // tensors are read by copies on this stream, whatever stream they go back to.
+    if (capacity_ > 0) used_on(stream);
     query_ = query; key_ = key; payload_ = payload; links_ = links;
     tables_ = tables; lens_ = lens; scratch_ = scratch;
     table_bytes_ = table;

@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(128) stream_step_kernel(StreamCall c, int vec_
   chunk_of(c, s, &off, &n);
   const int len = c.lengths[s];
   if (h == 0 && lane == 0) c.lengths_after[s] = len + n;
-  if (n <= 0 || n > kStepTokens || (int64_t)len + n > c.capacity) return;
+  if (len < 0 || n <= 0 || n > kStepTokens || (int64_t)len + n > c.capacity) return;
   uint8_t* q = c.query_history + (int64_t)pair * c.capacity;
   uint8_t* k = c.key_history + (int64_t)pair * c.capacity;
   uint32_t* prev = c.prev + (int64_t)pair * c.capacity;
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(256) stream_append_chunk_kernel(StreamCall c, 
   const int step = len / kChainStep + (int)(st - (int64_t)s * steps_upper);
   if (col == 0 && st == (int64_t)s * steps_upper) c.lengths_after[s] = len + n;
   const int begin = max(len, step * kChainStep), end = min(len + n, (step + 1) * kChainStep);
-  if (begin >= end || (int64_t)len + n > c.capacity) return;
+  if (len < 0 || begin >= end || (int64_t)len + n > c.capacity) return;
   const void* src;
   uint8_t* dst;
   int heads, head, bits, vec;
@@ -230,7 +230,7 @@ __global__ void stream_index_kernel(StreamCall c, int segments, uint32_t* __rest
   if (!whole) chunk_of(c, s, &off, &n);
   const int len = c.lengths[s];
   const int begin = whole ? 0 : len, end = whole ? len : len + n;
-  if (begin >= end || (int64_t)end > c.capacity) return;
+  if (len < 0 || begin >= end || (int64_t)end > c.capacity) return;
   Entry* tables = static_cast<Entry*>(c.tables) + (int64_t)pair * c.entries;
   constexpr int kPer = 16 / (int)sizeof(Entry);       // c.entries is a multiple of it
   uint4* outside = reinterpret_cast<uint4*>(tables);
@@ -279,7 +279,7 @@ struct StreamAxis {
     }
     *start = s;
     *i = c.lengths[s] + (int)(g - off);
-    return (int64_t)*i < c.capacity ? s : -1;
+    return *i >= 0 && (int64_t)*i < c.capacity ? s : -1;
   }
   __device__ __forceinline__ int64_t symbols(int s, int h, int) const {
     return ((int64_t)s * c.H + h) * c.capacity;

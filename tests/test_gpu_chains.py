@@ -203,3 +203,48 @@ def test_native_call_keeps_the_rules_of_autograd():
     leaf.add_(1.0)
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         out.sum().backward()
+
+
+def _held(stream):
+    """Queues some milliseconds of work on a stream (bounded: a spin of a fixed count of cycles)."""
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(20_000_000)
+
+
+def _stream_case(T, seed):
+    """Packed symbols [2, T, 4] (4 bits) and the result of one pass over them."""
+    B, H, bits, W = 2, 4, 4, 32
+    q, k = _streams(B * T, H, bits, seed)
+    want, want_end = orc.hard_inference(q, k, k.astype(np.float32)[..., None], np.arange(B + 1) * T, W)
+    byte = lambda x: torch.from_numpy(x.astype(np.uint8)).reshape(B, T, H).to(DEV)  # noqa: E731
+    return byte(q), byte(k), want[..., 0].reshape(B, T, H), want_end.reshape(B, T, H)
+
+
+def _feed(runtime, q, k, a, b, **how):
+    return runtime.update_packed(q[:, a:b], k[:, a:b], k[:, a:b], **how)
+
+
+def _check_stream(results, want, want_end):
+    assert np.array_equal(torch.cat([r[1] for r in results], dim=1).cpu().numpy(), want_end)
+    assert np.array_equal(torch.cat([r[0] for r in results], dim=1).cpu().numpy(), want)
+
+
+def test_a_growth_on_another_stream_keeps_the_old_state_until_it_is_copied():
+    """The growing update waits on a second stream while the first one allocates and fills blocks of
+    the sizes that the old state had."""
+    from rosa_soft_b200 import RosaRuntime
+    T = 700
+    q, k, want, want_end = _stream_case(T, 3)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    runtime = RosaRuntime(4, 4, 4, 4, 32)
+    first = _feed(runtime, q, k, 0, 200)
+    side = torch.cuda.Stream()
+    _held(side)
+    work = _feed(runtime, q, k, 200, T, stream=side, async_op=True)
+    noise = [torch.full((n,), 255, dtype=torch.uint8, device=DEV)
+             for n in (8, 16, 512, 2048, 8192, 16384, 65536, 131072, 262144) for _ in range(8)]
+    second = work.wait()
+    torch.cuda.synchronize()
+    assert len(noise) == 72
+    _check_stream([first, second], want, want_end)
