@@ -60,6 +60,9 @@ class StreamCore {
     phase_ = 0;
     longest_ = 0;
     ordered_ = false;
+    last_ = at::cuda::CUDAEvent();   // an event stays with the device of its first record
+    home_.reset();
+    last_stream_.reset();
   }
 
   // The first update fixes the slots of a fresh runtime, unless it fails.
@@ -119,6 +122,10 @@ class StreamCore {
     u.output = out.data_ptr(); u.matched_key_end = end.data_ptr<int64_t>();
     const int rc = rosa_b200_stream_update_chained(&u, ws.data_ptr(), (size_t)ws.numel(), stream.stream());
     TORCH_CHECK(rc == 0, "RosaRuntime update: ", rosa_b200_last_error());
+    used_on(stream);
+    last_.record(stream);
+    last_stream_ = stream;
+    ordered_ = true;
     // committed only once the update has been enqueued
     if (chunk == nullptr) {
       for (auto& n : lengths_) n += max_chunk;
@@ -127,10 +134,6 @@ class StreamCore {
     }
     longest_ = after;
     phase_ ^= 1;
-    used_on(stream);
-    last_.record(stream);
-    last_stream_ = stream;
-    ordered_ = true;
     return {out, end};
   }
 

@@ -248,3 +248,26 @@ def test_a_growth_on_another_stream_keeps_the_old_state_until_it_is_copied():
     torch.cuda.synchronize()
     assert len(noise) == 72
     _check_stream([first, second], want, want_end)
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
+@pytest.mark.parametrize("how", ("reset", "load"))
+def test_a_runtime_that_was_reset_or_loaded_may_go_on_on_another_gpu(how):
+    from rosa_soft_b200 import RosaRuntime
+    T = 300
+    q, k, want, want_end = _stream_case(T, 4)
+    runtime = RosaRuntime(4, 4, 4, 4, 32)
+    first = _feed(runtime, q, k, 0, 100)
+    if how == "reset":
+        runtime.reset()
+        results = []
+        at = 0
+    else:
+        state = {n: x.to("cuda:1") if isinstance(x, torch.Tensor) else x
+                 for n, x in runtime.state_dict().items()}
+        runtime.load_state_dict(state)
+        results = [tuple(x.cpu() for x in first)]
+        at = 100
+    for a, b in ((at, 150), (150, T)):
+        results.append(tuple(x.cpu() for x in _feed(runtime, q.to("cuda:1"), k.to("cuda:1"), a, b)))
+    _check_stream(results, want, want_end)
