@@ -122,10 +122,7 @@ class StreamCore {
     u.output = out.data_ptr(); u.matched_key_end = end.data_ptr<int64_t>();
     const int rc = rosa_b200_stream_update_chained(&u, ws.data_ptr(), (size_t)ws.numel(), stream.stream());
     TORCH_CHECK(rc == 0, "RosaRuntime update: ", rosa_b200_last_error());
-    used_on(stream);
-    last_.record(stream);
-    last_stream_ = stream;
-    ordered_ = true;
+    touched_on(stream);
     // committed only once the update has been enqueued
     if (chunk == nullptr) {
       for (auto& n : lengths_) n += max_chunk;
@@ -217,9 +214,7 @@ class StreamCore {
     lengths_ = lengths;
     longest_ = *std::max_element(lengths.begin(), lengths.end());
     reindex(stream);
-    last_.record(stream);
-    last_stream_ = stream;
-    ordered_ = true;
+    touched_on(stream);
   }
 
  private:
@@ -244,6 +239,14 @@ class StreamCore {
     if (stream == *home_) return;
     for (const Tensor& t : {query_, key_, payload_, links_, tables_, lens_, scratch_})
       c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), stream);
+  }
+
+  // ... and whatever touches the state next starts after it.
+  void touched_on(const c10::cuda::CUDAStream& stream) {
+    used_on(stream);
+    last_.record(stream);
+    last_stream_ = stream;
+    ordered_ = true;
   }
 
   void reindex(const c10::cuda::CUDAStream& stream) {
@@ -294,7 +297,13 @@ class StreamCore {
     table_bytes_ = table;
     capacity_ = capacity;
     home_ = stream;
-    if (rebuilt) reindex(stream);
+    // recorded here, not only by the update that grows: if that one fails after this, the next may come
+    // on the stream of the one before
+    touched_on(stream);
+    if (rebuilt) {
+      reindex(stream);
+      touched_on(stream);
+    }
   }
 
   // workspace of an update that is one kernel, and of any update of up to 8000 token-heads

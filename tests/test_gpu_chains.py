@@ -271,3 +271,23 @@ def test_a_runtime_that_was_reset_or_loaded_may_go_on_on_another_gpu(how):
     for a, b in ((at, 150), (150, T)):
         results.append(tuple(x.cpu() for x in _feed(runtime, q.to("cuda:1"), k.to("cuda:1"), a, b)))
     _check_stream(results, want, want_end)
+
+
+def test_an_update_after_one_that_failed_in_its_growth_waits_for_the_copies():
+    """The failing update grows the state on a held-back stream and then cannot allocate its result; the
+    next one comes on the stream of the update before it."""
+    from rosa_soft_b200 import RosaRuntime
+    T = 900
+    q, k, want, want_end = _stream_case(T, 5)
+    runtime = RosaRuntime(4, 4, 4, 4, 32)
+    first = _feed(runtime, q, k, 0, 250)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    _held(side)
+    part = [x[:, 250:T].contiguous() for x in (q, k, k)]
+    with torch.cuda.stream(side), pytest.raises(RuntimeError):
+        runtime._core.packed(*part, [0, T - 250, 2 * (T - 250)], None, None, [-7, 4])
+    assert runtime._core.capacity >= T
+    second = _feed(runtime, q, k, 250, T)
+    torch.cuda.synchronize()
+    _check_stream([first, second], want, want_end)
