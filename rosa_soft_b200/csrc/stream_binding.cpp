@@ -74,8 +74,9 @@ class StreamCore {
     ~Opening() {
       if (core_ != nullptr) core_->clear();
     }
+    void keep() const { core_ = nullptr; }
     Pair done(Pair result) const {
-      core_ = nullptr;
+      keep();
       return result;
     }
     mutable StreamCore* core_;
@@ -201,7 +202,7 @@ class StreamCore {
     clear();
     const c10::Device device = query.device();
     const c10::cuda::OptionalCUDAGuard guard(device);
-    open((int64_t)lengths.size(), device);
+    const Opening opening(this, (int64_t)lengths.size(), device);   // a load that fails leaves nothing
     const int64_t used = query.size(2);
     const auto stream = at::cuda::getCurrentCUDAStream(device_.index());
     grow(std::max(used, *std::max_element(lengths.begin(), lengths.end())), stream);
@@ -215,6 +216,7 @@ class StreamCore {
     longest_ = *std::max_element(lengths.begin(), lengths.end());
     reindex(stream);
     touched_on(stream);
+    opening.keep();
   }
 
  private:

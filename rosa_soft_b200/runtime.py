@@ -222,10 +222,12 @@ class RosaRuntime:
             raise ValueError("state_dict was produced by a differently configured RosaRuntime")
         self._clear()
         lengths = [int(v) for v in state_dict["lengths"]]
+        if lengths:
+            self._load_histories(lengths, state_dict)
         self._sequence_ids = state_dict.get("sequence_ids")
         self._ids_fixed = bool(state_dict.get("ids_fixed", False))
-        if not lengths:
-            return
+
+    def _load_histories(self, lengths: list, state_dict: Dict[str, Any]) -> None:
         query_history = state_dict["query_history"]
         if not query_history.is_cuda:
             raise ValueError("state_dict tensors must be CUDA tensors")

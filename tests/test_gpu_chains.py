@@ -291,3 +291,19 @@ def test_an_update_after_one_that_failed_in_its_growth_waits_for_the_copies():
     second = _feed(runtime, q, k, 250, T)
     torch.cuda.synchronize()
     _check_stream([first, second], want, want_end)
+
+
+def test_a_load_that_fails_leaves_a_fresh_runtime():
+    from rosa_soft_b200 import RosaRuntime
+    T = 120
+    q, k, want, want_end = _stream_case(T, 6)
+    source = RosaRuntime(4, 4, 4, 4, 32)
+    source.update_packed(*(torch.cat([x, x]) for x in (q, k, k)), sequence_ids=[3, 4, 5, 6])    # four slots
+    state = source.state_dict()
+    runtime = RosaRuntime(4, 4, 4, 4, 32)
+    for broken in ({"payload_history": state["payload_history"][..., :-1]},
+                   {"key_history": state["key_history"][:2]}, {"lengths": [T] * 3}):
+        with pytest.raises(RuntimeError):
+            runtime.load_state_dict({**state, **broken})
+        assert runtime.memory_stats()["sequences"] == 0
+    _check_stream([_feed(runtime, q, k, 0, 50), _feed(runtime, q, k, 50, T)], want, want_end)    # two slots, no IDs
