@@ -191,10 +191,16 @@ class StreamCore {
     return opening.done(append(query, key, payload, dev, &chunk, offsets.back(), longest, out_type, shape));
   }
 
-  std::tuple<Tensor, Tensor, Tensor> export_histories() const {
+  // Copies on the current stream, after the last update and before the next.
+  std::tuple<Tensor, Tensor, Tensor> export_histories() {
+    const c10::cuda::OptionalCUDAGuard guard(device_);
+    const auto stream = at::cuda::getCurrentCUDAStream(device_.index());
+    if (ordered_ && stream != *last_stream_) last_.block(stream);
     const int64_t used = longest_;
     auto cut = [&](const Tensor& t) { return t.narrow(2, 0, used).clone(); };
-    return {cut(query_), cut(key_), cut(payload_)};
+    std::tuple<Tensor, Tensor, Tensor> copies{cut(query_), cut(key_), cut(payload_)};
+    touched_on(stream);
+    return copies;
   }
 
   void import_histories(const std::vector<int64_t>& lengths, const Tensor& query, const Tensor& key,

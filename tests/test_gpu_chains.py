@@ -307,3 +307,21 @@ def test_a_load_that_fails_leaves_a_fresh_runtime():
             runtime.load_state_dict({**state, **broken})
         assert runtime.memory_stats()["sequences"] == 0
     _check_stream([_feed(runtime, q, k, 0, 50), _feed(runtime, q, k, 50, T)], want, want_end)    # two slots, no IDs
+
+
+def test_a_state_is_saved_between_the_updates_around_it_whatever_their_streams():
+    from rosa_soft_b200 import RosaRuntime
+    T = 400
+    q, k, want, want_end = _stream_case(T, 8)
+    runtime = RosaRuntime(4, 4, 4, 4, 32)
+    first = _feed(runtime, q, k, 0, 100)
+    side = torch.cuda.Stream()
+    _held(side)
+    second = _feed(runtime, q, k, 100, 250, stream=side, async_op=True)     # no growth: capacity 256
+    state = runtime.state_dict()                                            # not ordered by the caller
+    loaded = RosaRuntime(4, 4, 4, 4, 32)
+    loaded.load_state_dict(state)
+    rest = [_feed(r, q, k, 250, T) for r in (runtime, loaded)]
+    done = second.wait()
+    for r in rest:
+        _check_stream([first, done, r], want, want_end)
