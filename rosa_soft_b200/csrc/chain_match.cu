@@ -77,7 +77,7 @@ int launch_chain_index(const FwdArgs& a, int64_t max_len, cudaStream_t stream) {
                               : chain_index_kernel<unsigned long long, false>)
                      : (merge ? chain_index_kernel<uint32_t, true> : chain_index_kernel<uint32_t, false>);
   if (bytes > 48 * 1024)
-    ROSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    ROSA_CUDA_OK(allow_shared(kernel));
   kernel<<<(unsigned)heads, 32 * a.context * segments, bytes, stream>>>(
       a.plan, a.packed_q, a.packed_k, a.sym_seq_stride, a.sym_head_stride, a.H, a.D, a.context,
       hash_bits, segments, a.chain_start, a.chain_prev, a.chain_low);

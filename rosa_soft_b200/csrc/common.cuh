@@ -294,6 +294,14 @@ struct ProfileScope {
     }                                                                             \
   } while (0)
 
+// Lets a kernel (without static shared memory) be launched with any amount a block may have.  The limit
+// belongs to the function and the device, not to the call: set to what one call needs, it would refuse
+// the launch of a larger call that another thread has just set it for.
+template <typename Kernel>
+inline cudaError_t allow_shared(Kernel* kernel) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+}
+
 // ------------------------------------------------------- kernel entry points
 struct FwdArgs {
   Plan plan;

@@ -328,7 +328,7 @@ int run_chunk(const StreamCall& c, int out_type, int vec_out, int max_chunk, cha
     const int bytes = set_bytes * segments;
     auto kernel = c.context > 2 ? stream_index_kernel<Entry, true> : stream_index_kernel<Entry, false>;
     if (bytes > 48 * 1024)
-      ROSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+      ROSA_CUDA_OK(allow_shared(kernel));
     kernel<<<(unsigned)(c.slots * c.H), 32 * c.context * segments, bytes, stream>>>(c, segments, start, low,
                                                                                   flag);
     ROSA_CUDA_OK(cudaGetLastError());
@@ -447,7 +447,7 @@ ROSA_B200_API int rosa_b200_stream_update_chained(const rosa_b200_stream_call* u
     const int bytes = c.entries * (wide ? 8 : 4);
     auto kernel = wide ? stream_index_kernel<unsigned long long, false> : stream_index_kernel<uint32_t, false>;
     if (bytes > 48 * 1024)
-      ROSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+      ROSA_CUDA_OK(allow_shared(kernel));
     kernel<<<(unsigned)(c.slots * c.H), 32 * c.context, bytes, st>>>(c, 1, nullptr, nullptr, nullptr);
     ROSA_CUDA_OK(cudaGetLastError());
     return 0;

@@ -1569,12 +1569,10 @@ int launch_sweep2_t(const VjpArgs& a, int items_upper, bool small_dv, cudaStream
   const size_t bytes = floats * sizeof(float);
   const unsigned grid = (unsigned)((int64_t)items_upper * a.H);
   if (small_dv) {
-    ROSA_CUDA_OK(cudaFuncSetAttribute(vjp_sweep2_kernel<DPAD, DVPAD, true>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    ROSA_CUDA_OK(allow_shared(vjp_sweep2_kernel<DPAD, DVPAD, true>));
     vjp_sweep2_kernel<DPAD, DVPAD, true><<<grid, kVjpBand, bytes, stream>>>(a);
   } else {
-    ROSA_CUDA_OK(cudaFuncSetAttribute(vjp_sweep2_kernel<DPAD, DVPAD, false>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    ROSA_CUDA_OK(allow_shared(vjp_sweep2_kernel<DPAD, DVPAD, false>));
     vjp_sweep2_kernel<DPAD, DVPAD, false><<<grid, kVjpBand, bytes, stream>>>(a);
   }
   ROSA_CUDA_OK(cudaGetLastError());
@@ -1587,7 +1585,7 @@ int launch_sweep2_tc_t(const VjpArgs& a, int items_upper, cudaStream_t stream) {
                  (2 * tc_table_floats(NG, NV) + kVjpRows * kVjpBand) * sizeof(float);
   const unsigned grid = (unsigned)((int64_t)items_upper * a.H);
   auto kernel = vjp_sweep2_tc_kernel<NK, NV, NG, kWindowed, kDropout>;
-  ROSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  ROSA_CUDA_OK(allow_shared(kernel));
   kernel<<<grid, kVjpBand, bytes, stream>>>(a);
   ROSA_CUDA_OK(cudaGetLastError());
   return 0;

@@ -584,7 +584,7 @@ int launch_s1_tiled_r(const VjpArgs& a, unsigned grid, cudaStream_t stream) {
                          : (dropout ? vjp_sweep1_tiled_kernel<NG, R, false, true, kBallot>
                                     : vjp_sweep1_tiled_kernel<NG, R, false, false, false>);
   if (smem > 48 * 1024)
-    ROSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    ROSA_CUDA_OK(allow_shared(kernel));
   kernel<<<grid, threads, smem, stream>>>(a);
   ROSA_CUDA_OK(cudaGetLastError());
   return 0;

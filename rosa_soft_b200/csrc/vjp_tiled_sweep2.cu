@@ -374,11 +374,11 @@ int launch_s2_tiled_t(const VjpArgs& a, unsigned grid, cudaStream_t stream) {
   if (bytes < least) bytes = least;
   if constexpr (pairs_blocks(NV)) {
     auto kernel = vjp_sweep2_tiled_pair_kernel<NV, NG, kDropout, kPrec>;
-    ROSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    ROSA_CUDA_OK(allow_shared(kernel));
     kernel<<<grid, kS2Threads, bytes, stream>>>(a);
   } else {
     auto kernel = vjp_sweep2_tiled_kernel<NV, NG, kDropout, kPrec>;
-    ROSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    ROSA_CUDA_OK(allow_shared(kernel));
     kernel<<<grid, kS2Threads, bytes, stream>>>(a);
   }
   ROSA_CUDA_OK(cudaGetLastError());

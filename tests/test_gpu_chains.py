@@ -325,3 +325,37 @@ def test_a_state_is_saved_between_the_updates_around_it_whatever_their_streams()
     done = second.wait()
     for r in rest:
         _check_stream([first, done, r], want, want_end)
+
+
+def test_host_threads_with_calls_of_different_sizes_do_not_disturb_each_other():
+    """The kernels of two threads need different amounts of shared memory."""
+    import threading
+
+    import rosa_soft_b200 as rs
+
+    def inputs(T, D, seed):
+        return [nonzero_randn((1, T, 1, n), seed + s).to(DEV) for s, n in enumerate((D, D, 8))]
+
+    # few heads are indexed in pieces: tables of 75 to 140 KB a block
+    cases = [inputs(T, D, 11 * n) for n, (T, D) in enumerate([(2048, 8), (4096, 8), (8192, 8), (4096, 3)])]
+    call = lambda case: rs.rosa_soft(*case, max_suffix_length=20)  # noqa: E731
+    want = [call(case) for case in cases]
+    torch.cuda.synchronize()
+    failed = []
+
+    def work(n):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(3000):
+                    got = call(cases[n])
+                torch.cuda.current_stream().synchronize()
+                assert torch.equal(got, want[n])
+        except Exception as error:  # noqa: BLE001
+            failed.append((n, error))
+
+    threads = [threading.Thread(target=work, args=(n,)) for n in range(len(cases))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
