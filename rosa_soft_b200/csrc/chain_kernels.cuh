@@ -13,6 +13,20 @@
 namespace rosa {
 namespace {
 
+// How many pieces per head: as many warps as the GPU holds of these CTAs, pieces of at least 256
+// positions, at most 8 (a table set each in shared memory), at most kChainIndexWarps warps a CTA:
+// the index kernels are compiled for as many, with the 80 registers a thread that this leaves.
+constexpr int kChainSharedBytes = 200 * 1024;
+constexpr int kChainIndexWarps = 24;
+
+inline int chain_segments(int64_t heads, int64_t positions, size_t set_bytes, int context) {
+  int n = 1;
+  while (n < 8 && heads * n * 2 <= 148 * 8 && positions >= 256 * n * 2 &&
+         (size_t)n * 2 * set_bytes <= kChainSharedBytes && context * n * 2 <= kChainIndexWarps)
+    n *= 2;
+  return n;
+}
+
 // Indexes positions [begin, end) of one head for context length L; all lanes of a warp call.
 //
 // A warp takes 16 positions at a time: lanes 0..15 hold the key contexts that end there, lanes
@@ -184,18 +198,6 @@ __device__ __forceinline__ void chain_index_block(const Sym* q, const Sym* k, in
   if (from < to)
     chain_index_warp<Entry, kMerge, kResume>(q, k, from, to, L, bits, level == 0, hash_bits, table_at(g, L),
                                              key_links, level == 0 ? start : low);
-}
-
-// How many pieces per head: as many warps as the GPU holds of these CTAs, pieces of at least 256
-// positions, at most 8 (a table set each in shared memory), at most 768 threads a CTA (registers).
-constexpr int kChainSharedBytes = 200 * 1024;
-
-inline int chain_segments(int64_t heads, int64_t positions, size_t set_bytes, int context) {
-  int n = 1;
-  while (n < 8 && heads * n * 2 <= 148 * 8 && positions >= 256 * n * 2 &&
-         (size_t)n * 2 * set_bytes <= kChainSharedBytes && context * n * 2 <= 24)
-    n *= 2;
-  return n;
 }
 
 // Rows of whole sequences over packed symbols ([sequence][head][position] or [head][token]).

@@ -10,11 +10,11 @@ namespace {
 
 // One CTA per (sequence, head), one warp per context length and piece; the tables in shared memory.
 template <typename Entry, bool kMerge>
-__global__ void chain_index_kernel(Plan plan, const int32_t* __restrict__ qsym,
-                                   const int32_t* __restrict__ ksym, int64_t sym_seq_stride,
-                                   int64_t sym_head_stride, int H, int bits, int context,
-                                   int hash_bits, int segments, uint32_t* __restrict__ start,
-                                   uint32_t* __restrict__ prev, uint32_t* __restrict__ low) {
+__global__ void __launch_bounds__(32 * kChainIndexWarps)
+    chain_index_kernel(Plan plan, const int32_t* __restrict__ qsym, const int32_t* __restrict__ ksym,
+                       int64_t sym_seq_stride, int64_t sym_head_stride, int H, int bits, int context,
+                       int hash_bits, int segments, uint32_t* __restrict__ start,
+                       uint32_t* __restrict__ prev, uint32_t* __restrict__ low) {
   extern __shared__ unsigned long long table_words[];
   Entry* tables = reinterpret_cast<Entry*>(table_words);
   if (plan.cu_seqlens == nullptr && blockIdx.x == 0 && threadIdx.x < 4) plan.status[threadIdx.x] = 0;

@@ -359,3 +359,22 @@ def test_host_threads_with_calls_of_different_sizes_do_not_disturb_each_other():
     for t in threads:
         t.join()
     assert not failed
+
+
+@pytest.mark.parametrize("bits", (1, 2))
+def test_chunks_of_long_histories_of_few_heads_take_the_largest_index_blocks(bits):
+    """Wide table entries, all shorter lengths, two or four pieces: 24 warps a block."""
+    from rosa_soft_b200 import RosaRuntime
+    held, n, W = 65535 * 16 + 40, 1100, 24
+    q, k = _streams(held + n, 1, bits, 5, copies=False)
+    q[held + 500:held + 560] = k[held + 100:held + 160]
+    q[held + 700:held + 790] = k[3000:3090]
+    byte = lambda x: torch.from_numpy(x.astype(np.uint8).reshape(1, 1, -1)).to(DEV)  # noqa: E731
+    runtime = RosaRuntime(1, 1, bits, bits, W)
+    config = runtime.state_dict()["config"]
+    runtime.load_state_dict({"config": config, "lengths": [held], "query_history": byte(q[:held]),
+                             "key_history": byte(k[:held]), "payload_history": byte(k[:held])})
+    tq, tk = (byte(x[held:]).reshape(1, n, 1) for x in (q, k))
+    end = runtime.update_packed(tq, tk, tk)[1][0, :, 0].cpu().numpy()
+    rows = np.concatenate([np.arange(0, n, 16), np.arange(540, 560), np.arange(770, 790)])
+    assert np.array_equal(end[rows], [_latest_longest(q[:, 0], k[:, 0], held + int(i), W) for i in rows])
