@@ -84,3 +84,16 @@ def test_row_sums_have_the_same_bits_in_launches_of_every_size(B, H, Dv, p):
     got = cabi.surrogate_vjp(q, k, v, go, (B, T), pq, pk, W, 1.0, p, 3.0, seed, 7)[:3]
     bits = hashlib.sha256(b"".join(g[:T, :2].contiguous().cpu().numpy().tobytes() for g in got)).hexdigest()
     assert bits == ROW_SUM_BITS[Dv, p]
+
+
+@pytest.mark.parametrize("W,m", [(2, 3.0), (3, 9.0), (5, 6.0), (16, 3.0)])
+def test_runs_of_matches_far_longer_than_the_horizon(W, m):
+    """Lone mismatches between long runs: products on both sides of the cut-off, and an adjoint that adds up
+    over a whole run."""
+    T, H, D = 1200, 2, 2
+    rng = np.random.default_rng(W)
+    tokens = np.repeat(rng.integers(0, 4, size=(T // 8, H)), 8, axis=0)
+    tokens[rng.integers(0, T, size=40), 0] ^= 3
+    q = torch.from_numpy(np.where((tokens[..., None] >> np.arange(D)) & 1, 0.7, -0.7).astype(np.float32))
+    _check(q, q.clone(), nonzero_randn((T, H, 8), 3), nonzero_randn((T, H, 8), 4), (1, T), W, 0.0, m,
+           torch.float32)
