@@ -33,16 +33,10 @@ size_t partial_budget_bytes() {
 
 struct FwdLayout {
   PlanLayout plan;
-  size_t best_off, qt_off, kt_off, start_off, prev_off, low_off, masks_off;
-  int64_t mask_words;
+  size_t best_off, qt_off, kt_off, start_off, prev_off, low_off;
   size_t bytes;
 };
 
-constexpr int kMaskSymbolBits = 8;   // widest symbol served by the bit-parallel matcher
-
-// The sizing function knows neither D nor the lengths: both matchers get the most they may need.
-// The bitmaps of the bit-parallel matcher (rows that the chained matcher gave up, H * 2^8 rows of
-// ceil(N / 32) + 1 words) are built after the chains have been walked and take their place.
 FwdLayout fwd_layout(int64_t N, int H, int64_t S, bool transposed_symbols) {
   FwdLayout l;
   l.plan = plan_layout(0, S);
@@ -57,17 +51,12 @@ FwdLayout fwd_layout(int64_t N, int H, int64_t S, bool transposed_symbols) {
     l.kt_off = off;
     off = align_up(off + word_rows);
   }
-  l.mask_words = (N + 31) / 32 + 1;
-  l.masks_off = off;
   l.start_off = off;
   off = align_up(off + word_rows);
   l.prev_off = off;
   off = align_up(off + word_rows);
   l.low_off = off;
   off = align_up(off + word_rows);
-  if (!transposed_symbols)
-    off = std::max(off, align_up(l.masks_off + ((size_t)H << kMaskSymbolBits) *
-                                                   (size_t)l.mask_words * sizeof(uint32_t)));
   l.bytes = off;
   return l;
 }
@@ -247,8 +236,6 @@ int run_hard_forward(const void* query, const void* key, const void* value, int 
   a.sym_head_stride = dense ? uniform_len : N;
   const int64_t max_len = dense ? uniform_len : N;
   set_chain_scratch(a, ws, l, max_len);
-  a.match_masks = reinterpret_cast<uint32_t*>(ws + l.masks_off);
-  a.mask_words = l.mask_words;
 
   if (!dense) {   // a dense batch needs no tables: its sequences and items are arithmetic
     launch_build_plan(a.plan, st);
@@ -261,13 +248,9 @@ int run_hard_forward(const void* query, const void* key, const void* value, int 
     a.low_is_zero = 1;
   }
   if (int rc = launch_chain_index(a, max_len, st)) return rc;
-  const bool bits = D <= kMaskSymbolBits;
-  // a short sequence walks its chains to the end: the stand-by launches would cost more
-  const int limit = max_len <= 512 ? 512 : bits ? kChainLimitBits : kChainLimitScan;
-  if (int rc = launch_chain_forward(a, limit, st)) return rc;
-  if (max_len <= limit) return 0;              // no chain is longer than its sequence
-  return bits ? launch_match_bits(a, a.plan.status + 2, st)
-              : launch_scan_forward(a, a.plan.status + 2, st);
+  if (int rc = launch_chain_forward(a, max_len, st)) return rc;
+  if (max_len <= kChainShort) return 0;
+  return launch_pending_forward(a, a.plan.status + 2, st);
 }
 }  // namespace
 
@@ -372,9 +355,9 @@ ROSA_B200_API int rosa_b200_hard_inference(const uint32_t* query_symbols, const 
                                         st))
     return rc;
   if (int rc = launch_chain_index(a, max_len, st)) return rc;
-  if (int rc = launch_chain_inference(a, payload, out, matched_end, max_len <= 512 ? 512 : kChainLimitScan, st)) return rc;
-  if (max_len <= 512) return 0;
-  return launch_scan_inference(a, payload, out, matched_end, a.plan.status + 2, st);
+  if (int rc = launch_chain_inference(a, payload, out, matched_end, max_len, st)) return rc;
+  if (max_len <= kChainShort) return 0;
+  return launch_pending_inference(a, payload, out, matched_end, a.plan.status + 2, st);
 }
 
 ROSA_B200_API size_t rosa_b200_stream_workspace_bytes(int64_t chunk_tokens, int num_heads) {

@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(kChainRows * kChainHeads)
     chain_match_kernel(Axis axis, const Sym* __restrict__ qsym, const Sym* __restrict__ ksym,
                        int64_t N, int H, int W, int context, const uint32_t* __restrict__ start_link,
                        const uint32_t* __restrict__ prev, const uint32_t* __restrict__ low,
-                       int head_blocks, int limit, int32_t* flag, Emit emit) {
+                       int head_blocks, ChainPatience patience, int32_t* flag, Emit emit) {
   __shared__ uint2 s_win[kChainRows][kChainHeads + 1];   // (length, route)
   __shared__ int s_start[kChainRows];
   const int heads = blockDim.x / kChainRows;             // heads of this CTA
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(kChainRows * kChainHeads)
     first = start_link[at];
     if (context > 1) shorter = low[at];
   }
-  if (chain_walk<Sym>(qsym + base, ksym + base, prev + base, first, seq, i, W, limit, lane, best_len,
+  if (chain_walk<Sym>(qsym + base, ksym + base, prev + base, first, seq, i, W, patience, lane, best_len,
                       best_route)) {
     best_len = (int)(kChainGaveUp >> 32);          // resolved by a matcher of whole warps
     best_route = 0;
@@ -272,71 +272,281 @@ __global__ void __launch_bounds__(kChainRows * kChainHeads)
 
 template <typename Sym, typename Axis, typename Emit>
 int launch_chain_match_t(Axis axis, const Sym* q, const Sym* k, int64_t N, int H, int W, int context,
-                         const uint32_t* start, const uint32_t* prev, const uint32_t* low, int limit,
-                         int32_t* flag, Emit emit, cudaStream_t stream) {
+                         const uint32_t* start, const uint32_t* prev, const uint32_t* low,
+                         ChainPatience patience, int32_t* flag, Emit emit, cudaStream_t stream) {
   const int heads = H < kChainHeads ? H : kChainHeads;
   const int head_blocks = (H + heads - 1) / heads;
   const int64_t tiles = (N + kChainRows - 1) / kChainRows;
   chain_match_kernel<Sym, Axis, Emit><<<(unsigned)(tiles * head_blocks), kChainRows * heads, 0, stream>>>(
-      axis, q, k, N, H, W, context, start, prev, low, head_blocks, limit, flag, emit);
+      axis, q, k, N, H, W, context, start, prev, low, head_blocks, patience, flag, emit);
   ROSA_CUDA_OK(cudaGetLastError());
   return 0;
 }
 
-// A warp resolves one row by a look at every earlier position, newest first, 32 at a time: lanes
-// whose position agrees with the row here and at the distance of the best length so far extend it.
-// Cost: i / 32 coalesced reads, whatever the chains look like.  All lanes call and get the result.
+// ------------------------------------------------------------ rows that gave up
+// The newest kSymbols symbols that end at a position, compared at once.
+template <typename Sym>
+struct Probe;
+
+template <>
+struct Probe<uint8_t> {
+  static constexpr int kSymbols = 8;
+  uint32_t older, newer;
+  // the eight bytes that end at p[0], from the aligned words that hold one of them or the byte after it
+  __device__ __forceinline__ static Probe of(const uint8_t* p) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(p - 7);
+    const uint32_t* words = reinterpret_cast<const uint32_t*>(at & ~(uintptr_t)3);
+    const unsigned shift = 8u * (unsigned)(at & 3);
+    const uint32_t a = words[0], b = words[1], c = words[2];
+    return {__funnelshift_r(a, b, shift), __funnelshift_r(b, c, shift)};
+  }
+  // whether the newest n symbols agree (n from 1 to 8)
+  __device__ __forceinline__ bool agrees(const Probe& o, int n) const {
+    const uint32_t lo = n <= 4 ? 0u : ~0u << (64 - 8 * n), hi = n >= 4 ? ~0u : ~0u << (32 - 8 * n);
+    return (((older ^ o.older) & lo) | ((newer ^ o.newer) & hi)) == 0u;
+  }
+};
+
+template <>
+struct Probe<int32_t> {
+  static constexpr int kSymbols = 4;
+  int32_t w[4];
+  __device__ __forceinline__ static Probe of(const int32_t* p) { return {{p[0], p[-1], p[-2], p[-3]}}; }
+  __device__ __forceinline__ bool agrees(const Probe& o, int n) const {
+    return w[0] == o.w[0] && (n < 2 || w[1] == o.w[1]) && (n < 3 || w[2] == o.w[2]) &&
+           (n < 4 || w[3] == o.w[3]);
+  }
+};
+
+// A warp resolves one row by a look at every earlier position, newest first, 128 at a time: a position
+// is worth extending only if it agrees in one symbol more than the best match has so far, which a probe
+// or the symbol at that distance decides.  Cost: i / 128 rounds of coalesced reads, whatever the chains
+// look like.  (A byte history is a row of whole words.)  All lanes call and get the result.
 template <typename Sym>
 __device__ __forceinline__ void scan_row(const Sym* q, const Sym* k, int i, int W, int lane,
                                          int& best_len, int& best_route) {
+  constexpr int kProbe = Probe<Sym>::kSymbols;
   const Sym q_i = q[i];
+  Probe<Sym> newest{};
+  if (i >= kProbe) newest = Probe<Sym>::of(q + i);
   best_len = best_route = 0;
-  for (int top = i - 1; top >= 0 && best_len < min(W, top + 1); top -= 32) {
-    const int j = top - lane;
-    int length = 0;
-    if (j >= best_len && k[j] == q_i && k[j - best_len] == q[i - best_len])
-      length = chain_extend<Sym>(q, k, i, j, 1, min(W, j + 1));
+  const auto take = [&](int j, int length) {
     const int longest = __reduce_max_sync(0xffffffffu, length);
     if (longest > best_len) {
       best_len = longest;
       best_route = __reduce_max_sync(0xffffffffu, length == longest ? j + 1 : 0);
     }
+  };
+  int top = i - 1;
+  while (top >= 0 && best_len < min(W, top + 1)) {
+    if (top - 127 >= max(best_len, kProbe)) {
+      const int n = min(best_len + 1, kProbe);
+      const Sym q_b = q[i - best_len];
+      bool candidate[4], any = false;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int j = top - 32 * u - lane;
+        candidate[u] = Probe<Sym>::of(k + j).agrees(newest, n) && k[j - best_len] == q_b;
+        any = any || candidate[u];
+      }
+      if (__any_sync(0xffffffffu, any)) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int j = top - 32 * u - lane;
+          take(j, candidate[u] ? chain_extend<Sym>(q, k, i, j, n, min(W, j + 1)) : 0);
+        }
+      }
+      top -= 128;
+    } else {
+      const int j = top - lane;
+      int length = 0;
+      if (j >= best_len && k[j] == q_i && k[j - best_len] == q[i - best_len])
+        length = chain_extend<Sym>(q, k, i, j, 1, min(W, j + 1));
+      take(j, length);
+      top -= 32;
+    }
   }
 }
 
-// The rows that gave up, one warp each.
-constexpr int kScanWarps = 8;
+// Tiles of up to 256 rows of one sequence in which many rows gave up: the run-length recurrence
+//     len(i, j) = (q_i == k_j) ? min(len(i - 1, j - 1) + 1, W) : 0
+// along the diagonals, newest first in bands of 2048.  A thread owns eight neighbouring diagonals, so
+// that the key symbols of eight rows are fifteen consecutive ones in registers; a pair costs a compare, an
+// add with the cap, a select and a maximum over (run << 11 | how late the diagonal is), whatever the data
+// are.  The run that enters the tile is counted backwards once per diagonal.  A band is the last when no
+// older match can be longer.  What bounds it is instruction issue.  Streams of two symbols, against the
+// matchers that took these rows before (a scan per row; bitmaps of the symbols, of up to 8 bits):
+//   8 x 8192 x 32 inference, wide symbols       43.9 -> 3.1 ms
+//   4 x 4096 x 32 scoring, 8 bits               1.48 -> 0.52 ms, 4 x 4096 x 16, 24 bits 3.59 -> 0.30 ms
+//   16 x 8192 x 32 stream in chunks of 1024     78.1 -> 6.5 ms
+constexpr int kRunRows = 256;          // most rows of a tile, threads of the CTA
+constexpr int kRunPer = 8;
+constexpr int kRunBits = 11;
+constexpr int kRunBand = kRunRows * kRunPer;
+static_assert(kRunBand == 1 << kRunBits, "a key holds the diagonal of a band");
+constexpr int kRunMaxHorizon = 1 << 19;      // runs of a 32-bit key
+// With at most this many pending rows a warp scans for each instead (a row of a scan costs as much as
+// 6 to 40 rows of the runs, as the symbols go).
+constexpr int kRunFew = 12;
 
+// run[e]: key of the thread's diagonal e, its run << 11 | how late it is in the band.
+__device__ __forceinline__ void run_rows(const int* s_q, const int* s_k, unsigned* s_best, int nrows, int W,
+                                         int tid, int (&run)[kRunPer]) {
+  const int lane = tid & 31;
+  const int base = kRunBand - kRunPer - kRunPer * tid;       // column of (row 0, the oldest diagonal)
+  int none[kRunPer], most[kRunPer], kw[2 * kRunPer];
+#pragma unroll
+  for (int e = 0; e < kRunPer; ++e) {
+    none[e] = base + kRunPer - 1 - e;
+    most[e] = none[e] + (W << kRunBits);
+  }
+  const auto load = [&](int at, int column) {
+#pragma unroll
+    for (int x = 0; x < kRunPer; x += 4) {
+      const int4 w = *reinterpret_cast<const int4*>(s_k + column + x);
+      kw[at + x] = w.x; kw[at + x + 1] = w.y; kw[at + x + 2] = w.z; kw[at + x + 3] = w.w;
+    }
+  };
+  load(0, base);
+#pragma unroll 1
+  for (int r0 = 0; r0 < nrows; r0 += kRunPer) {
+    load(kRunPer, base + r0 + kRunPer);
+    int q[kRunPer];
+#pragma unroll
+    for (int x = 0; x < kRunPer; ++x) q[x] = s_q[r0 + x];
+    unsigned mine = 0u;
+#pragma unroll
+    for (int rr = 0; rr < kRunPer; ++rr) {
+      int key = 0;
+#pragma unroll
+      for (int e = 0; e < kRunPer; ++e) {
+        run[e] = kw[rr + kRunPer - 1 - e] == q[rr] ? min(run[e] + kRunBand, most[e]) : none[e];
+        key = max(key, run[e]);
+      }
+      const unsigned longest = __reduce_max_sync(0xffffffffu, (unsigned)key);
+      if (lane == rr) mine = longest;
+    }
+    if (lane < kRunPer && mine >= (unsigned)kRunBand) atomicMax(s_best + r0 + lane, mine);
+#pragma unroll
+    for (int x = 0; x < kRunPer; ++x) kw[x] = kw[x + kRunPer];
+  }
+}
+
+// The rows that gave up, tile by tile: longest first, as many CTAs as fill the GPU.
 template <typename Sym, typename Axis, typename Emit>
-__global__ void __launch_bounds__(kScanWarps * 32)
-    scan_match_kernel(Axis axis, const Sym* __restrict__ qsym, const Sym* __restrict__ ksym, int64_t N,
-                      int H, int W, const int32_t* __restrict__ run_flag, Emit emit) {
+__global__ void __launch_bounds__(kRunRows, 2)
+    run_match_kernel(Axis axis, const Sym* __restrict__ qsym, const Sym* __restrict__ ksym, int64_t N,
+                     int H, int W, int tile_rows, const int32_t* __restrict__ run_flag, Emit emit) {
+  __shared__ __align__(16) int s_k[kRunBand + kRunRows];
+  __shared__ int s_q[kRunRows];
+  __shared__ unsigned s_best[kRunRows];
+  __shared__ bool s_mine[kRunRows];
+  __shared__ unsigned s_used[kRunRows / 32];
+  __shared__ int s_first, s_last, s_count, s_seq, s_start, s_i0;
   if (*run_flag == 0) return;
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * kScanWarps, count = N * H;
-  for (int64_t th0 = ((int64_t)blockIdx.x * kScanWarps + (threadIdx.x >> 5)) * 32; th0 < count;
-       th0 += warps * 32) {
-    const bool mine = th0 + lane < count && emit.pending(th0 + lane);
-    for (unsigned rows = __ballot_sync(0xffffffffu, mine); rows != 0u; rows &= rows - 1u) {
-      const int64_t th = th0 + __ffs(rows) - 1;
-      const int64_t g = th / H;
-      const int h = (int)(th - g * H);
-      int start = 0, i = 0, best_len, best_route;
-      const int seq = axis.locate(g, &start, &i);
-      const int64_t base = axis.symbols(seq, h, start);
-      scan_row<Sym>(qsym + base, ksym + base, i, W, lane, best_len, best_route);
-      if (lane == 0) emit(g, h, H, start, best_len, best_route);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t tiles = (N + tile_rows - 1) / tile_rows;
+  for (int64_t task = blockIdx.x; task < tiles * H; task += gridDim.x) {
+    const int h = (int)(task % H);
+    const int64_t g0 = (tiles - 1 - task / H) * tile_rows;
+    int seq = -1, start = 0, row = 0;
+    bool pending = false;
+    if (tid < tile_rows && g0 + tid < N && emit.pending((g0 + tid) * H + h)) {
+      seq = axis.locate(g0 + tid, &start, &row);
+      pending = seq >= 0;
+    }
+    // one sequence (or slot) of the tile at a time
+    while (__syncthreads_or(pending)) {
+      if (tid == 0) {
+        s_first = kRunRows;
+        s_last = s_count = 0;
+      }
+      __syncthreads();
+      if (pending) atomicMin(&s_first, tid);
+      __syncthreads();
+      const int first = s_first;
+      if (tid == first) {
+        s_seq = seq;
+        s_start = start;
+        s_i0 = row;
+      }
+      __syncthreads();
+      const bool mine = pending && seq == s_seq;
+      s_mine[tid] = mine;
+      if (mine) {
+        atomicMax(&s_last, tid);
+        atomicAdd(&s_count, 1);
+      }
+      __syncthreads();
+      const int n = s_last - first + 1, i0 = s_i0;
+      const int64_t at = axis.symbols(s_seq, h, s_start);
+      const Sym* q = qsym + at;
+      const Sym* k = ksym + at;
+      if (s_count <= kRunFew || W > kRunMaxHorizon) {
+        for (int r = first + warp; r <= s_last; r += kRunRows / 32) {
+          if (!s_mine[r]) continue;
+          int length, route;
+          scan_row<Sym>(q, k, i0 + r - first, W, lane, length, route);
+          if (lane == 0) emit(g0 + r, h, H, s_start, length, route);
+        }
+      } else {
+        // thread t owns row i0 + t of the sequence as well as diagonals db + 8 t .. db + 8 t + 7
+        const bool own = tid < n && s_mine[min(first + tid, kRunRows - 1)];
+        const int i = i0 + tid, newest_row = i0 + n - 1;
+        int best_len = 0, best_route = 0;
+        // positions before the sequence hold a symbol that no row of the tile has: one of 0 .. 256
+        if (tid < kRunRows / 32) s_used[tid] = 0u;
+        __syncthreads();
+        const int symbol = tid < n ? (int)q[i] : 0;
+        s_q[tid] = symbol;
+        if (symbol >= 0 && symbol < kRunRows) atomicOr(s_used + (symbol >> 5), 1u << (symbol & 31));
+        __syncthreads();
+        int absent = kRunRows;
+        for (int x = kRunRows / 32 - 1; x >= 0; --x)
+          if (~s_used[x] != 0u) absent = 32 * x + __ffs(~s_used[x]) - 1;
+        for (int db = 1; db <= newest_row; db += kRunBand) {
+          const int j0 = i0 - db - (kRunBand - 1);        // key position of column 0
+          s_best[tid] = 0u;
+          for (int c = tid; c < kRunBand + n; c += kRunRows) {
+            const int j = j0 + c;
+            s_k[c] = j >= 0 && j < newest_row ? (int)k[j] : absent;
+          }
+          __syncthreads();
+          if (db + kRunPer * 32 * warp <= newest_row) {    // a warp of diagonals that exist
+            int run[kRunPer];
+#pragma unroll
+            for (int e = 0; e < kRunPer; ++e) {
+              const int d = db + kRunPer * tid + e;
+              run[e] = kRunBand - 1 - kRunPer * tid - e;
+              if (d < i0)
+                run[e] += chain_extend<Sym>(q, k, i0 - 1, i0 - 1 - d, 0, min(W, i0 - d)) << kRunBits;
+            }
+            run_rows(s_q, s_k, s_best, n, W, tid, run);
+          }
+          __syncthreads();
+          const int key = (int)s_best[tid];
+          if (own && key >> kRunBits > best_len) {         // older bands only with a longer match
+            best_len = key >> kRunBits;
+            best_route = i - (db + kRunBand - 1 - (key & (kRunBand - 1))) + 1;
+          }
+          // the matches of the next band start at position i - db - 2048 at best
+          if (__syncthreads_and(!own || best_len >= W || best_len >= i - db - kRunBand + 1)) break;
+        }
+        if (own) emit(g0 + first + tid, h, H, s_start, best_len, best_route);
+      }
+      pending = pending && !mine;
     }
   }
 }
 
 template <typename Sym, typename Axis, typename Emit>
-int launch_scan_match_t(Axis axis, const Sym* q, const Sym* k, int64_t N, int H, int W,
-                        const int32_t* run_flag, Emit emit, cudaStream_t stream) {
-  ProfileScope prof("hard_match_scan", stream);
-  // a grid that fills the GPU: it is launched whether or not a row gave up
-  scan_match_kernel<Sym, Axis, Emit><<<148 * 8, kScanWarps * 32, 0, stream>>>(axis, q, k, N, H, W,
-                                                                             run_flag, emit);
+int launch_run_match_t(Axis axis, const Sym* q, const Sym* k, int64_t N, int H, int W,
+                       const int32_t* run_flag, Emit emit, cudaStream_t stream) {
+  ProfileScope prof("hard_match_runs", stream);
+  // launched whether or not a row gave up; short tiles where the tall ones would not fill the GPU
+  const int tile_rows = (N + kRunRows - 1) / kRunRows * H < 148 * 2 ? 64 : kRunRows;
+  run_match_kernel<Sym, Axis, Emit><<<148 * 2, kRunRows, 0, stream>>>(axis, q, k, N, H, W, tile_rows,
+                                                                      run_flag, emit);
   ROSA_CUDA_OK(cudaGetLastError());
   return 0;
 }

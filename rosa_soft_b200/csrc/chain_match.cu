@@ -39,17 +39,17 @@ SequenceAxis sequence_axis(const FwdArgs& a) {
 }
 
 template <typename Emit>
-int match_rows(const FwdArgs& a, int limit, Emit emit, cudaStream_t stream) {
+int match_rows(const FwdArgs& a, ChainPatience patience, Emit emit, cudaStream_t stream) {
   ProfileScope prof("hard_match", stream);
   return launch_chain_match_t(sequence_axis(a), a.packed_q, a.packed_k, a.N, a.H, a.W, a.context,
-                              a.chain_start, a.chain_prev, a.chain_low, limit, a.plan.status + 2, emit,
+                              a.chain_start, a.chain_prev, a.chain_low, patience, a.plan.status + 2, emit,
                               stream);
 }
 
 template <typename Emit>
-int scan_rows(const FwdArgs& a, const int32_t* run_flag, Emit emit, cudaStream_t stream) {
-  return launch_scan_match_t(sequence_axis(a), a.packed_q, a.packed_k, a.N, a.H, a.W, run_flag, emit,
-                             stream);
+int run_rows_of(const FwdArgs& a, const int32_t* run_flag, Emit emit, cudaStream_t stream) {
+  return launch_run_match_t(sequence_axis(a), a.packed_q, a.packed_k, a.N, a.H, a.W, run_flag, emit,
+                            stream);
 }
 
 }  // namespace
@@ -85,22 +85,24 @@ int launch_chain_index(const FwdArgs& a, int64_t max_len, cudaStream_t stream) {
   return 0;
 }
 
-int launch_chain_forward(const FwdArgs& a, int limit, cudaStream_t stream) {
-  return with_sign_emit(a, [&](auto emit) { return match_rows(a, limit, emit, stream); });
+int launch_chain_forward(const FwdArgs& a, int64_t max_len, cudaStream_t stream) {
+  const ChainPatience patience = chain_patience(a.D, a.context, max_len);
+  return with_sign_emit(a, [&](auto emit) { return match_rows(a, patience, emit, stream); });
 }
 
 int launch_chain_inference(const FwdArgs& a, const float* payload, float* out, int64_t* matched_end,
-                           int limit, cudaStream_t stream) {
-  return match_rows(a, limit, make_payload_emit(a, payload, out, matched_end), stream);
+                           int64_t max_len, cudaStream_t stream) {
+  return match_rows(a, chain_patience(a.D, a.context, max_len),
+                    make_payload_emit(a, payload, out, matched_end), stream);
 }
 
-int launch_scan_forward(const FwdArgs& a, const int32_t* run_flag, cudaStream_t stream) {
-  return with_sign_emit(a, [&](auto emit) { return scan_rows(a, run_flag, emit, stream); });
+int launch_pending_forward(const FwdArgs& a, const int32_t* run_flag, cudaStream_t stream) {
+  return with_sign_emit(a, [&](auto emit) { return run_rows_of(a, run_flag, emit, stream); });
 }
 
-int launch_scan_inference(const FwdArgs& a, const float* payload, float* out, int64_t* matched_end,
-                          const int32_t* run_flag, cudaStream_t stream) {
-  return scan_rows(a, run_flag, make_payload_emit(a, payload, out, matched_end), stream);
+int launch_pending_inference(const FwdArgs& a, const float* payload, float* out, int64_t* matched_end,
+                             const int32_t* run_flag, cudaStream_t stream) {
+  return run_rows_of(a, run_flag, make_payload_emit(a, payload, out, matched_end), stream);
 }
 
 }  // namespace rosa

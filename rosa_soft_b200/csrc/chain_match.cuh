@@ -1,5 +1,5 @@
 // Latest-longest suffix matching through occurrence chains, shared by the training forward, the
-// batched inference (hard_forward.cu) and the streaming runtime (stream_runtime.cu).
+// batched inference (chain_match.cu) and the streaming runtime (stream_chain.cu).
 //
 // The context of length c at position p is the c symbols that end there.  Every key position is
 // linked to the previous key position whose context falls into the same bucket, every query
@@ -24,11 +24,20 @@ constexpr int kChainStep = 16;        // positions a warp indexes at a time
 constexpr int kChainAhead = 8;        // steps between the request of a symbol and its use
 // Longest history whose step numbers fit a 32-bit table entry beside the mask of 16 lanes.
 constexpr int64_t kChainNarrow = (int64_t)65535 * kChainStep;
-// A row gives up after this many chain members (streams of few distinct symbols, or of passages
-// repeated very often) and is resolved by a whole warp.  Symbols of up to 8 bits have the
-// bit-parallel matcher for that, which is soon the cheaper way; wide ones a scan of all positions.
-constexpr int kChainLimitBits = 64;
-constexpr int kChainLimitScan = 256;
+// When a row leaves its chain to the matchers whose cost does not depend on the data (run_match_kernel,
+// scan_row): after `steps` members, or when they lie close together (streams of few distinct symbols): at
+// the 24th less than 6 positions apart, at the `trial`-th (24th or 64th) or a later one less than 20;
+// `trial` 0: the first rule alone.  A member is two dependent reads, 4 to 9 ps with all rows of a launch in
+// flight, a position of the run matcher 0.3 ps, on short sequences 0.8.  Alphabet of 16, 8 x 8192 x 32
+// inference: 3.2 ms when the rows leave, 5.0 when they walk on; 16 x 1024 x 16 scoring: 160 us when they
+// leave after 24 members, 105 after 64.
+struct ChainPatience {
+  int steps, trial;
+};
+constexpr int kChainTrial = 24;
+// Sequences up to here walk their chains to the end: the launch that stands by for the rows that give up
+// would cost more.
+constexpr int64_t kChainShort = 512;
 // Winner that such a row leaves behind (a match length no real row has).
 constexpr unsigned long long kChainGaveUp = 0xffffffffull << 32;
 
@@ -44,6 +53,12 @@ __host__ __device__ inline int chain_hash_bits(int bits, int c, int64_t len) {
   int n = 8;
   while (n < kChainHashBits && ((int64_t)1 << n) < len) ++n;
   return bits * c < n ? bits * c : n;
+}
+
+inline ChainPatience chain_patience(int bits, int c, int64_t len) {
+  if (len <= kChainShort) return {0x7fffffff, 0};
+  const int64_t expected = len >> chain_hash_bits(bits, c, len);    // members without structure
+  return {(int)(4 * expected > 1024 ? 4 * expected : 1024), len <= 2048 ? 64 : kChainTrial};
 }
 
 __host__ __device__ inline uint32_t chain_bucket(uint32_t context, int context_bits, int hash_bits) {
@@ -84,10 +99,10 @@ __device__ __forceinline__ int chain_extend(const Sym* q, const Sym* k, int i, i
 // every lane walks the rest of its chain: candidates come newest first, so only a strictly longer
 // match replaces the best one, and a candidate is worth extending only if it also agrees at the
 // distance of the best length so far.  Returns the length and the route (position + 1) of the latest
-// among the longest; the result is true when the chain was longer than `limit`.  All lanes call.
+// among the longest; the result is true when the row ran out of patience.  All lanes call.
 template <typename Sym>
 __device__ __forceinline__ bool chain_walk(const Sym* q, const Sym* k, const uint32_t* prev,
-                                           uint32_t first, int row, int i, int W, int limit, int lane,
+                                           uint32_t first, int row, int i, int W, ChainPatience patience, int lane,
                                            int& best_len, int& best_route) {
   best_len = 0;
   best_route = 0;
@@ -109,7 +124,7 @@ __device__ __forceinline__ bool chain_walk(const Sym* q, const Sym* k, const uin
     best_len = min(W, counted);
     best_route = j + 1;
   }
-  int steps = 0;
+  int steps = 0, check = patience.trial > 0 ? kChainTrial : patience.steps;
   while (first != 0u && best_len < W) {
     j = (int)first - 1;
     const int cap = min(W, j + 1);                 // a match cannot start before the sequence
@@ -122,7 +137,10 @@ __device__ __forceinline__ bool chain_walk(const Sym* q, const Sym* k, const uin
         best_route = j + 1;
       }
     }
-    if (++steps == limit) return first != 0u;
+    if (++steps == check) {                        // now and then: the loop is as long as its chain
+      if (steps >= patience.steps || i - j < (steps < patience.trial ? 6 : 20) * steps) return first != 0u;
+      check += 40;
+    }
   }
   return false;
 }

@@ -325,27 +325,21 @@ struct FwdArgs {
   uint32_t *chain_start, *chain_prev, *chain_low;
   int context;                    // chained context length
   int low_is_zero;                // chain_low was cleared by an earlier kernel of the call
-  // Per-symbol occurrence bitmaps of the key symbols, [H][2^D][mask_words] over the packed
-  // token axis (bit g of row (h, s) set iff key symbol of token g, head h is s), for the rows
-  // that the chained matcher gives up (D <= 8); they take the place of its scratch.
-  uint32_t* match_masks;
-  int64_t mask_words;
 };
 
 int launch_pack_symbols(const void* q, const void* k, int dtype, int64_t N, int H, int D,
                         int dense, int64_t uniform_len, int32_t* packed_q, int32_t* packed_k,
                         uint32_t* zeroed, cudaStream_t stream);
-// chained matcher (chain_match.cu): index, then match and results; a row whose chain is longer than
-// `limit` raises status[2] and stays pending
+// chained matcher (chain_match.cu): index, then match and results; a row that gives up its chain raises
+// status[2] and stays pending (sequences of up to kChainShort tokens: none)
 int launch_chain_index(const FwdArgs& a, int64_t max_len, cudaStream_t stream);
-int launch_chain_forward(const FwdArgs& a, int limit, cudaStream_t stream);
+int launch_chain_forward(const FwdArgs& a, int64_t max_len, cudaStream_t stream);
 int launch_chain_inference(const FwdArgs& a, const float* payload, float* out, int64_t* matched_end,
-                           int limit, cudaStream_t stream);
+                           int64_t max_len, cudaStream_t stream);
 // matchers of the pending rows: they do nothing while *run_flag is zero
-int launch_match_bits(const FwdArgs& a, const int32_t* run_flag, cudaStream_t stream);
-int launch_scan_forward(const FwdArgs& a, const int32_t* run_flag, cudaStream_t stream);
-int launch_scan_inference(const FwdArgs& a, const float* payload, float* out, int64_t* matched_end,
-                          const int32_t* run_flag, cudaStream_t stream);
+int launch_pending_forward(const FwdArgs& a, const int32_t* run_flag, cudaStream_t stream);
+int launch_pending_inference(const FwdArgs& a, const float* payload, float* out, int64_t* matched_end,
+                             const int32_t* run_flag, cudaStream_t stream);
 // all rows of a call without a workspace
 int launch_run_length_match(const FwdArgs& a, int items_upper, cudaStream_t stream);
 int launch_gather_output(const FwdArgs& a, cudaStream_t stream);

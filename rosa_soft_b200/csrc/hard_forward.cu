@@ -4,16 +4,13 @@
 // merge_hard_route and hard_forward_kernel of the reference
 // (rosa_soft/csrc/cuda/rosa_soft_kernels.cu:202-241, 311-531).
 //
-// Rows are resolved by the chained matcher (chain_match.cu).  Here: packing, and the matchers whose
-// cost does not depend on the data, for the rows that it gives up and for the entry point without a
-// workspace.  Symbols of up to 8 bits: bitmaps of every symbol's occurrences (bit_match.cuh).  Any
-// width: the exact diagonal run-length recurrence
+// Rows are resolved by the chained matcher (chain_match.cu).  Here: packing, and the matcher of the
+// entry point without a workspace, the exact diagonal run-length recurrence
 //     len(i, a) = (q_i == k_{a-1}) ? min(len(i-1, a-1) + 1, W) : 0
 // where one thread owns several diagonals, a warp sits on one query row at a time, the per-row
 // winner is reduced with redux.sync and merged across bands with one 64-bit integer atomicMax
 // (order independent, hence exact and deterministic).
 #include "common.cuh"
-#include "bit_match.cuh"
 #include "chain_match.cuh"
 #include "row_emit.cuh"
 
@@ -248,77 +245,6 @@ __global__ void __launch_bounds__(kMatchThreads)
   }
 }
 
-// ------------------------------------------------- bit-parallel matcher (D <= 8)
-// The matcher itself is bit_match_row (bit_match.cuh).  Here: the occurrence bitmaps of the
-// key symbols over the packed token axis, [H][2^D][mask_words], and the kernel that gives one
-// warp to every row that the chained matcher gave up.
-
-// Occurrence bitmaps: one warp per 32 consecutive tokens of one head writes the word column of
-// all symbols; the lanes that share a symbol are found with match.any and the lowest of them
-// stores the word.
-__global__ void build_match_masks_kernel(Plan plan, const int32_t* __restrict__ ksym, int64_t N,
-                                         int H, int D, int64_t sym_seq_stride,
-                                         int64_t sym_head_stride, uint32_t* __restrict__ masks,
-                                         int64_t mask_words, const int32_t* __restrict__ run_flag) {
-  if (*run_flag == 0) return;
-  const int lane = threadIdx.x & 31;
-  const int64_t words = (N + 31) >> 5, warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t warp_id = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; warp_id < words * H;
-       warp_id += warps) {
-    const int h = (int)(warp_id / words);
-    const int64_t word = warp_id - (int64_t)h * words;
-    const int64_t g = word * 32 + lane;
-    // lanes past the end get distinct out-of-range symbols so that they match nobody
-    unsigned sym = 0x80000000u | (unsigned)lane;
-    if (g < N) {
-      int start = 0, len = 0;
-      const int seq = find_segment(plan, g, &start, &len);
-      if (seq >= 0) {
-        const bool dense = plan.cu_seqlens == nullptr;
-        const int64_t idx = (int64_t)seq * sym_seq_stride + (int64_t)h * sym_head_stride +
-                            (dense ? g - start : g);
-        sym = (unsigned)ksym[idx];
-      }
-    }
-    uint32_t* __restrict__ column = masks + ((int64_t)h << D) * mask_words + word;
-    for (int e = lane; e < 1 << D; e += 32) column[e * mask_words] = 0u;
-    const unsigned peers = __match_any_sync(0xffffffffu, sym);
-    __syncwarp();
-    if (sym < (1u << D) && lane == __ffs(peers) - 1) column[(int64_t)sym * mask_words] = peers;
-  }
-}
-
-constexpr int kBitsWarps = 8;
-
-template <typename Emit>
-__global__ void __launch_bounds__(kBitsWarps * 32)
-    hard_match_bits_kernel(Plan plan, const int32_t* __restrict__ qsym,
-                           const uint32_t* __restrict__ masks, int64_t N, int H, int D, int W,
-                           int64_t mask_words, int64_t sym_seq_stride, int64_t sym_head_stride,
-                           const int32_t* __restrict__ run_flag, Emit emit) {
-  __shared__ BitCandidate queues[kBitsWarps][kBitQueue];
-  if (*run_flag == 0) return;
-  const int lane = threadIdx.x & 31;
-  // head-major order: neighbouring warps work on neighbouring rows of one head's bitmaps
-  for (int64_t row = (int64_t)blockIdx.x * kBitsWarps + (threadIdx.x >> 5); row < N * H;
-       row += (int64_t)gridDim.x * kBitsWarps) {
-    const int h = (int)(row / N);
-    const int64_t g = row - (int64_t)h * N;
-    if (!emit.pending(g * H + h)) continue;
-    int start = 0, len = 0;
-    const int seq = find_segment(plan, g, &start, &len);
-    const int i = (int)(g - start);                  // a row that gave up has earlier positions
-    const bool dense = plan.cu_seqlens == nullptr;
-    const int32_t* __restrict__ q = qsym + (int64_t)seq * sym_seq_stride +
-                                    (int64_t)h * sym_head_stride + (dense ? 0 : start);
-    const unsigned long long key =
-        bit_match_row(q, masks + ((int64_t)h << D) * mask_words, mask_words, start, i, W, lane,
-                      queues[threadIdx.x >> 5]);
-    if (lane == 0) emit(g, h, H, start, (int)(key >> 32), (int)(key & 0xffffffffull));
-    __syncwarp();
-  }
-}
-
 // ------------------------------------------------------------------- gather
 // One thread per (token, head, chunk of value components): 16 bytes of output per thread when
 // the rows allow it (128-bit loads of the value row, one 128-bit store), else element by element.
@@ -419,23 +345,6 @@ int launch_transpose_symbols(const uint32_t* q, const uint32_t* k, int64_t N, in
   transpose_symbols_kernel<<<grid, block, 0, stream>>>(q, k, N, H, qt, kt);
   ROSA_CUDA_OK(cudaGetLastError());
   return 0;
-}
-
-int launch_match_bits(const FwdArgs& a, const int32_t* run_flag, cudaStream_t stream) {
-  ProfileScope prof("hard_match_bits", stream);
-  // one grid that fills the GPU: it is launched whether or not a row gave up
-  const unsigned grid = 148 * 8;
-  build_match_masks_kernel<<<grid, 256, 0, stream>>>(a.plan, a.packed_k, a.N, a.H, a.D,
-                                                     a.sym_seq_stride, a.sym_head_stride,
-                                                     a.match_masks, a.mask_words, run_flag);
-  ROSA_CUDA_OK(cudaGetLastError());
-  return with_sign_emit(a, [&](auto emit) -> int {
-    hard_match_bits_kernel<<<grid, kBitsWarps * 32, 0, stream>>>(
-        a.plan, a.packed_q, a.match_masks, a.N, a.H, a.D, a.W, a.mask_words, a.sym_seq_stride,
-        a.sym_head_stride, run_flag, emit);
-    ROSA_CUDA_OK(cudaGetLastError());
-    return 0;
-  });
 }
 
 int launch_run_length_match(const FwdArgs& a, int items_upper, cudaStream_t stream) {

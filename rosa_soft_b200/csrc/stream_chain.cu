@@ -28,8 +28,9 @@ struct StreamCall {
   void* tables;                        // [slots][H][table entries]
   const int32_t* lengths;
   int32_t* lengths_after;
-  int64_t capacity;
+  int64_t capacity, longest;           // longest: of the histories after the update
   int context, hash_bits, entries;
+  ChainPatience patience;
   int vec_qk, vec_payload;             // logit rows are whole aligned 16-byte words
   void* output;
   int64_t* matched_end;
@@ -99,7 +100,7 @@ __device__ __forceinline__ void store_symbol(void* base, int64_t index, int bits
 // One warp per (slot, head).  The tables stay in global memory: a few entries are touched.  What
 // bounds it is the latency of about ten dependent reads.
 template <typename Entry, typename In, typename Out>
-__global__ void __launch_bounds__(128) stream_step_kernel(StreamCall c, int vec_out) {
+__global__ void __launch_bounds__(128, 4) stream_step_kernel(StreamCall c, int vec_out) {
   __shared__ uint32_t links[4][2][2 * kStepTokens];      // per warp: chained, shorter lengths
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int pair = blockIdx.x * 4 + warp;
@@ -138,7 +139,7 @@ __global__ void __launch_bounds__(128) stream_step_kernel(StreamCall c, int vec_
   const int i = len + lane;
   int best_len, best_route;
   const bool gave_up = chain_walk<uint8_t>(q, k, prev, lane < n ? chained[lane] : 0u, lane < n ? 0 : -1, i,
-                                           c.W, kChainLimitScan, lane, best_len, best_route);
+                                           c.W, c.patience, lane, best_len, best_route);
   if (!gave_up && best_len < c.context) {
     best_route = (int)(shorter[lane] & 0x0fffffffu);
   }
@@ -338,12 +339,13 @@ int run_chunk(const StreamCall& c, int out_type, int vec_out, int max_chunk, cha
     {
       ProfileScope prof("stream_match", stream);
       if (int rc = launch_chain_match_t<uint8_t>(StreamAxis{c}, c.query_history, c.key_history, c.tokens,
-                                                 c.H, c.W, c.context, start, c.prev, low,
-                                                 kChainLimitScan, flag, emit, stream))
+                                                 c.H, c.W, c.context, start, c.prev, low, c.patience,
+                                                 flag, emit, stream))
         return rc;
     }
-    return launch_scan_match_t<uint8_t>(StreamAxis{c}, c.query_history, c.key_history, c.tokens, c.H,
-                                        c.W, flag, emit, stream);
+    if (c.longest <= kChainShort) return 0;        // nobody gives up
+    return launch_run_match_t<uint8_t>(StreamAxis{c}, c.query_history, c.key_history, c.tokens, c.H, c.W,
+                                       flag, emit, stream);
   };
   if (out_type == kPacked) return match(SymbolEmit<uint8_t>{c, vec_out});
   if (out_type == ROSA_B200_F32) return match(SymbolEmit<float>{c, vec_out});
@@ -465,6 +467,12 @@ ROSA_B200_API int rosa_b200_stream_update_chained(const rosa_b200_stream_call* u
   ROSA_REQUIRE(u->max_chunk >= 0 && u->max_chunk <= u->max_length_after, "max_chunk exceeds max_length_after");
   ROSA_REQUIRE(u->chunk_offsets != nullptr || u->max_chunk * (int64_t)u->slots == u->chunk_tokens,
                "without chunk_offsets every slot gets max_chunk tokens");
+  c.longest = u->max_length_after;
+  c.patience = chain_patience(c.qk_bits, c.context, c.longest);
+  // A step is one kernel with a warp per row: a member (two reads one after the other) takes as long as a
+  // round of 128 positions of the scan.
+  if (u->max_chunk <= kStepTokens)
+    c.patience = {(int)std::max<int64_t>(32, 4 * (c.longest >> c.hash_bits)), 0};
   c.query = u->query; c.key = u->key; c.payload = u->payload;
   c.offsets = u->chunk_offsets;
   c.uniform_chunk = (int)std::max<int64_t>(1, u->max_chunk);

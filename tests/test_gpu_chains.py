@@ -378,3 +378,85 @@ def test_chunks_of_long_histories_of_few_heads_take_the_largest_index_blocks(bit
     end = runtime.update_packed(tq, tk, tk)[1][0, :, 0].cpu().numpy()
     rows = np.concatenate([np.arange(0, n, 16), np.arange(540, 560), np.arange(770, 790)])
     assert np.array_equal(end[rows], [_latest_longest(q[:, 0], k[:, 0], held + int(i), W) for i in rows])
+
+
+def _few_symbols(n, heads, bits, seed, alphabet, top=None):
+    """Key symbols of a small alphabet (with `top`: one symbol that often, the rest wide) and a query stream
+    of other positions of the same heads."""
+    rng = np.random.default_rng(seed)
+    letters = rng.choice(1 << min(bits, 20), size=alphabet, replace=False).astype(np.uint32)
+    k = letters[rng.integers(0, alphabet, size=(n, heads))]
+    if top is not None:
+        k = np.where(rng.random((n, heads)) < top, letters[0], k)
+    return np.roll(k, n // 3, axis=0).astype(np.uint32), k.astype(np.uint32)
+
+
+RUN_LENGTHS = (513, 40, 767, 769, 2303, 2306, 4400, 1, 600)     # around tiles of 256 rows, bands of 2048
+
+
+@pytest.mark.parametrize("bits,W,alphabet,top", [
+    (8, 40, 2, None), (8, 4000, 3, None), (3, 2, 2, None), (24, 128, 2, None), (16, 32, 7, None),
+    (16, 32, 500, 0.9), (8, 64, 200, 0.6), (24, 600000, 2, None)])
+def test_rows_on_chains_too_long_to_follow(bits, W, alphabet, top):
+    """Forward over packed sequences and batched inference over the longest of them."""
+    import rosa_soft_b200 as rs
+    from rosa_soft_b200 import cabi
+    H = 8 if bits <= 16 else 2          # tiles of 256 rows, or of 64 where those are too few
+    cu = np.concatenate([[0], np.cumsum(RUN_LENGTHS)])
+    parts = [_few_symbols(n, H, bits, n + W, alphabet, top) for n in RUN_LENGTHS]
+    q, k = (np.concatenate([p[x] for p in parts]) for x in (0, 1))
+    pay = np.random.default_rng(3).standard_normal((int(cu[-1]), 1, 4)).astype(np.float32)
+    want_out, want_end = orc.hard_inference(q, k, pay, cu, W)
+    device_cu = torch.from_numpy(cu.astype(np.int32)).to(DEV)
+    routes = cabi.hard_forward(_logits(q, bits), _logits(k, bits), torch.from_numpy(pay).to(DEV), device_cu,
+                               W)[3].cpu().numpy()
+    starts = np.repeat(cu[:-1], RUN_LENGTHS)[:, None]
+    assert np.array_equal(routes, np.where(want_end >= 0, want_end + 1 + starts, -1))
+    s = slice(cu[6], cu[7])
+    as_int = lambda x: torch.from_numpy(x[s].view(np.int32))[None].to(DEV)  # noqa: E731
+    out, end = rs.rosa_hard_inference(as_int(q), as_int(k), torch.from_numpy(pay[s])[None].to(DEV),
+                                      max_suffix_length=W)
+    assert np.array_equal(end[0].cpu().numpy(), want_end[s]) and np.array_equal(out[0].cpu().numpy(), want_out[s])
+
+
+def test_lone_rows_on_long_chains():
+    """A symbol that is frequent among the keys and rare among the queries: a few pending rows a tile."""
+    from rosa_soft_b200 import cabi
+    T, H, bits, W = 3000, 2, 16, 32
+    rng = np.random.default_rng(1)
+    k = rng.integers(0, 1 << bits, size=(T, H)).astype(np.uint32)
+    q = rng.integers(0, 1 << bits, size=(T, H)).astype(np.uint32)
+    k[rng.random((T, H)) < 0.3] = 77
+    q[::60] = 77
+    q[1200:1215] = k[300:315]
+    v = nonzero_randn((T, 1, 3), 5).to(DEV)
+    routes = cabi.hard_forward(_logits(q, bits), _logits(k, bits), v, (1, T), W)[3]
+    _, want = orc.hard_forward(_logits(q, bits).cpu().numpy(), _logits(k, bits).cpu().numpy(), v.cpu().numpy(),
+                               np.array([0, T]), W)
+    assert np.array_equal(routes.cpu().numpy(), np.where(want > 0, want, -1))
+
+
+@pytest.mark.parametrize("bits,W,alphabet,top", [(8, 32, 2, None), (8, 300, 3, None), (2, 5, 2, None),
+                                                 (8, 32, 200, 0.8)])
+def test_streams_of_few_symbols_equal_one_pass(bits, W, alphabet, top):
+    """Chunks around the tiles of the run matcher and single steps, slots of different lengths."""
+    from rosa_soft_b200 import RosaRuntime
+    H, B = 40 if bits == 2 else 3, 2
+    chunks = [(700, 650), (300, 0), (1, 1), (16, 16), (17, 40), (257, 255), (2200, 2306), (40, 300), (1, 1), (7, 0)]
+    T = [sum(c[s] for c in chunks) for s in range(B)]
+    data = [_few_symbols(T[s], H, bits, 5 * s + W, alphabet, top) for s in range(B)]
+    runtime = RosaRuntime(H, H, bits, bits, W)
+    got, at = [[], []], [0, 0]
+    for n in chunks:
+        part = [torch.from_numpy(np.concatenate([data[s][x][at[s]:at[s] + n[s]] for s in range(B)]).astype(np.uint8))
+                for x in (0, 1)]
+        cu = torch.tensor([0, n[0], n[0] + n[1]], dtype=torch.int32, device=DEV)
+        out, end = runtime.update_packed(part[0].to(DEV), part[1].to(DEV), part[1].to(DEV), cu)
+        for s, rows in enumerate((slice(0, n[0]), slice(n[0], n[0] + n[1]))):
+            got[s].append((out[rows].cpu().numpy(), end[rows].cpu().numpy()))
+            at[s] += n[s]
+    for s in range(B):
+        q, k = data[s]
+        want, want_end = orc.hard_inference(q, k, k.astype(np.float32)[..., None], np.array([0, T[s]]), W)
+        assert np.array_equal(np.concatenate([g[1] for g in got[s]]), want_end)
+        assert np.array_equal(np.concatenate([g[0] for g in got[s]]), want[..., 0])
