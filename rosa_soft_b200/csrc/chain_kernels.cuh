@@ -15,9 +15,12 @@ namespace {
 
 // How many pieces per head: as many warps as the GPU holds of these CTAs, pieces of at least 256
 // positions, at most 8 (a table set each in shared memory), at most kChainIndexWarps warps a CTA:
-// the index kernels are compiled for as many, with the 80 registers a thread that this leaves.
+// the index kernels are compiled for the registers a thread that this leaves.  (As a bound on the threads
+// the same limit made the pass 19 % slower: 0.70 -> 0.83 ms at 64 x 16384 x 64 wide symbols.)
 constexpr int kChainSharedBytes = 200 * 1024;
 constexpr int kChainIndexWarps = 24;
+constexpr int kChainIndexRegisters = 80;
+static_assert(32 * kChainIndexWarps * kChainIndexRegisters <= 65536, "more registers than an SM has");
 
 inline int chain_segments(int64_t heads, int64_t positions, size_t set_bytes, int context) {
   int n = 1;

@@ -10,7 +10,7 @@ namespace {
 
 // One CTA per (sequence, head), one warp per context length and piece; the tables in shared memory.
 template <typename Entry, bool kMerge>
-__global__ void __launch_bounds__(32 * kChainIndexWarps)
+__global__ void __maxnreg__(kChainIndexRegisters)
     chain_index_kernel(Plan plan, const int32_t* __restrict__ qsym, const int32_t* __restrict__ ksym,
                        int64_t sym_seq_stride, int64_t sym_head_stride, int H, int bits, int context,
                        int hash_bits, int segments, uint32_t* __restrict__ start,

@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(256) stream_append_chunk_kernel(StreamCall c, 
 // One CTA per (slot, head), one warp per context length: the tables of the pair are staged in
 // shared memory for the chunk.  tokens < 0: the whole histories (after they were loaded or moved).
 template <typename Entry, bool kMerge>
-__global__ void __launch_bounds__(32 * kChainIndexWarps)
+__global__ void __maxnreg__(kChainIndexRegisters)
     stream_index_kernel(StreamCall c, int segments, uint32_t* __restrict__ start,
                         uint32_t* __restrict__ low, int32_t* flag) {
   extern __shared__ uint4 staged_words[];
