@@ -196,6 +196,7 @@ __device__ __forceinline__ void chain_index_block(const Sym* q, const Sym* k, in
   }
   const int warp = threadIdx.x >> 5;
   const int level = warp / segments, g = warp - level * segments;
+  if (level >= context) return;                      // a short sequence of a pack takes fewer pieces
   const int L = context - level;                     // level 0: the chained length
   const int from = piece(g), to = g + 1 < segments ? min(end, piece(g + 1)) : end;
   if (from < to)

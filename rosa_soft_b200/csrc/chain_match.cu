@@ -25,6 +25,10 @@ __global__ void __maxnreg__(kChainIndexRegisters)
     if (plan.status[0] != 0) return;
     base += plan.seg_start[seq];
     len = plan.seg_len[seq];
+    // the launch is sized for the longest sequence that the pack could hold: buckets (which the CTA has
+    // to clear) and pieces by its own length
+    hash_bits = min(hash_bits, chain_hash_bits(bits, context, len));
+    if (len < 512) segments = 1;
   }
   const int entries = (1 << hash_bits) + chain_low_entries(bits, context);
   for (int e = threadIdx.x; e < entries; e += blockDim.x) tables[e] = 0;

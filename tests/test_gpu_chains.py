@@ -460,3 +460,27 @@ def test_streams_of_few_symbols_equal_one_pass(bits, W, alphabet, top):
         want, want_end = orc.hard_inference(q, k, k.astype(np.float32)[..., None], np.array([0, T[s]]), W)
         assert np.array_equal(np.concatenate([g[1] for g in got[s]]), want_end)
         assert np.array_equal(np.concatenate([g[0] for g in got[s]]), want[..., 0])
+
+
+@pytest.mark.parametrize("bits", (1, 8, 16))
+@pytest.mark.parametrize("heads", (1, 12))        # indexed in pieces, in one
+def test_packs_of_one_long_and_many_short_sequences(bits, heads):
+    """Every sequence has buckets, pieces and a share of the launch by its own length: forward and gradients."""
+    import rosa_soft_b200 as rs
+    from tests.helpers import normalised_error, oracle_grads
+    rng = np.random.default_rng(bits)
+    lengths = np.concatenate([rng.integers(0, 20, size=150), [1700, 511, 512], rng.integers(1, 40, size=50)])
+    cu = np.concatenate([[0], np.cumsum(lengths)])
+    N, W = int(cu[-1]), 24
+    q, k = _streams(N, heads, bits, 7)
+    leaves = [t.requires_grad_(True) for t in (_logits(q, bits), _logits(k, bits),
+                                               nonzero_randn((N, 1, 4), 5).to(DEV))]
+    out = rs.rosa_soft_varlen(*leaves, torch.from_numpy(cu.astype(np.int32)).to(DEV), max_suffix_length=W,
+                              dropout_p=0.0)
+    go = nonzero_randn((N, heads, 4), 6).to(DEV)
+    got = torch.autograd.grad(out, leaves, go)
+    host = [t.detach().cpu().numpy() for t in leaves]
+    assert np.array_equal(out.detach().cpu().numpy(), orc.hard_forward(*host, cu, W)[0])
+    want = oracle_grads(*leaves, go, cu, W, 1.0, 0.0, 3.0, 0)
+    for mine, ref in zip(got, want):
+        assert normalised_error(mine.cpu().numpy(), ref) <= 1e-4       # the bound of float32 inputs
