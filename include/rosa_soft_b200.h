@@ -218,8 +218,10 @@ ROSA_B200_API int rosa_b200_stream_update(
     void* workspace, size_t workspace_bytes, void* stream);
 
 /* The same update over occurrence chains: the state holds the symbol histories, one link per key
- * position and a table per (slot, head) instead of bitmaps, and an update costs the same whatever
- * the length of the history.  It also takes logits (packed on the way in: bit d set iff component d
+ * position and a table per (slot, head) instead of bitmaps.  A new token is linked in constant time;
+ * its row then walks the chain of its context, about length / 2^13 members in a stream without
+ * structure, and where the members lie closer (few distinct symbols) looks at the whole history
+ * once (length / 128 rounds of a warp, or its share of a tile of rows).  The call also takes logits (packed on the way in: bit d set iff component d
  * is positive) and gives the result as +-1 values (0 for no match), so that a generation step is one
  * kernel.  The caller owns the state (capacity a multiple of 32, pointers 16-byte aligned):
  *   query_history, key_history  uint8  [slots, num_heads, capacity]

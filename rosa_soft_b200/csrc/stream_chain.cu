@@ -1,8 +1,10 @@
 // Streaming hard inference over occurrence chains: the state of a (slot, head) is its query and key
 // symbol histories, the chain links of its keys and the tables of chain_match.cuh, all of which only
-// grow, so an update of n tokens costs n steps whatever the length of the history (the bitmaps of
-// rosa_b200_stream_update cost n * length / 32 word reads).  Semantics as there: reference
-// rosa_soft/csrc/rosa_runtime.cpp:333-482 (chunked update_packed), :103-133, :455-467.
+// grow.  Indexing n tokens costs n steps whatever the length of the history; a row then walks the chain of
+// its context, length / 2^13 members in a stream without structure, and looks at the whole history once
+// where they lie closer (the bitmaps of rosa_b200_stream_update cost n * length / 32 word reads always).
+// Semantics as there: reference rosa_soft/csrc/rosa_runtime.cpp:333-482 (chunked update_packed),
+// :103-133, :455-467.
 //
 // Two schedules.  Up to kStepTokens tokens per slot (generation): ONE kernel, one warp per (slot,
 // head), does everything from the logits to the unpacked result.  More (prompts): pack and append,
@@ -382,11 +384,25 @@ int run_update(const StreamCall& c, int in_type, int out_type, int vec_out, int 
 #undef ROSA_STREAM_IN
 }
 
-// The tables follow the horizon as it was asked for: their layout changes only where a position
-// outgrows the entries or the shorter lengths' results.
+// The tables follow the horizon as it was asked for and the capacity: a state of up to 512 tokens per slot
+// holds contexts of 9 bits in 512 buckets (8-bit symbols: 3 KB per slot and head), a larger one the full
+// tables (34 KB), with wider entries where a position outgrows them.  The state's owner indexes the
+// histories anew when the size of the tables changes.
+constexpr int64_t kSmallState = 512;
+
+int stream_context(int qk_bits, int64_t W, int64_t capacity) {
+  if (capacity > kSmallState) return chain_context(qk_bits, W, capacity);
+  const int c = (9 + qk_bits - 1) / qk_bits;
+  return (int64_t)c < W ? c : (int)W;
+}
+
+int stream_hash_bits(int qk_bits, int context, int64_t capacity) {
+  return chain_hash_bits(qk_bits, context, capacity <= kSmallState ? kSmallState : (int64_t)1 << 30);
+}
+
 int table_entries(int qk_bits, int64_t W, int64_t capacity) {
-  const int context = chain_context(qk_bits, W, capacity);
-  const int n = (1 << chain_hash_bits(qk_bits, context, (int64_t)1 << 30)) + chain_low_entries(qk_bits, context);
+  const int context = stream_context(qk_bits, W, capacity);
+  const int n = (1 << stream_hash_bits(qk_bits, context, capacity)) + chain_low_entries(qk_bits, context);
   return (n + 3) / 4 * 4;
 }
 
@@ -441,8 +457,8 @@ ROSA_B200_API int rosa_b200_stream_update_chained(const rosa_b200_stream_call* u
   c.prev = u->chain_links; c.tables = u->tables;
   c.lengths = u->lengths; c.lengths_after = u->lengths_after;
   c.capacity = u->capacity;
-  c.context = chain_context(u->qk_bits, u->max_suffix_length, u->capacity);
-  c.hash_bits = chain_hash_bits(u->qk_bits, c.context, (int64_t)1 << 30);
+  c.context = stream_context(u->qk_bits, u->max_suffix_length, u->capacity);
+  c.hash_bits = stream_hash_bits(u->qk_bits, c.context, u->capacity);
   c.entries = table_entries(u->qk_bits, u->max_suffix_length, u->capacity);
   const bool wide = u->capacity > kChainNarrow;
   cudaStream_t st = static_cast<cudaStream_t>(stream);

@@ -35,6 +35,19 @@ def test_workspace_sizes_are_pure_functions_of_shapes():
     assert 0 < small < large
 
 
+def test_state_of_a_short_stream_is_small():
+    """Per slot and head: no more than the 8.4 KB that bitmaps of 8-bit symbols took for 256 tokens; full
+    tables from 1024 tokens on, wide entries from 65536 steps of 16 positions."""
+    from rosa_soft_b200 import cabi
+    table = cabi.load().rosa_b200_stream_table_bytes
+    for bits in range(1, 9):
+        for horizon in (1, 5, 32, 4096):
+            assert 256 * 7 + table(bits, horizon, 256) <= 8600
+            assert table(bits, horizon, 256) == table(bits, horizon, 512) <= table(bits, horizon, 1024)
+            assert 2 * table(bits, horizon, 1024) == table(bits, horizon, 2 ** 21)
+    assert table(8, 32, 1024) == 4 * (2 ** 13 + 2 ** 8)
+
+
 def test_status_word_decoding():
     """The plan's code wins; a set tensor-core word alone reads as the timeout status."""
     from rosa_soft_b200 import cabi
