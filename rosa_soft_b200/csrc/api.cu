@@ -432,24 +432,26 @@ struct VjpCall {
 };
 
 // Largest mismatch-count sum of a window whose product P = exp(-m sum / D) is kept; smaller products
-// are taken as zero, in the evidence and in the adjoint alike.  With every dropped product below c, on
-// a diagonal of n < T cells with gates in [exp(-m), 1]:
-//   S_n = x_n (1 + S_n-1) - P_n is off by the dropped products times gates, less than T c in all, and is
-//     at least exp(-m);
-//   Sbar_n = dS_n + x_n+1 Sbar_n+1 does not contain P, is at most T max|dS|, and some |Sbar| is at least
-//     max|dS| / 2 (that of the largest dS, or else the next one);
-//   C_n = (S_n + P_n) Sbar_n - (the sum of Sbar P over W + 1 cells) is off by less than (W + 2) c T max|dS|
-//     on top of what S is off by, and the largest |S Sbar| is at least exp(-m) max|dS| / 2.
-// With c = 2^-28 exp(-m) / (2 (W + 2) T) all of that stays below 2^-28 of the largest term of the diagonal,
-// a sixteenth of its last bit in float32; the logits carry the factor scale (sqrt(2) + 1) / 2 as well.
-// (Products below exp(-88) are zero in float32 with flush-to-zero anyway.)
+// are taken as zero, in the evidence and in the adjoint alike.  On a diagonal of n < T cells with gates x
+// in [exp(-m), 1], let every dropped product be below c.
+//   Adjoint: Sbar_n = dS_n + x_n+1 Sbar_n+1 does not contain P.  C_n = (S_n + P_n) Sbar_n - (the sum of
+//     Sbar P over W + 1 cells) is off by at most (W + 2) c M, M the largest |Sbar|, while the largest
+//     |S Sbar| is at least exp(-m) M, because S_n >= exp(-m).
+//   Evidence: the dropped products reach S_n = x_n (1 + S_n-1) - P_n weighted with X_k, the product of the
+//     k gates up to n; X_1 .. X_W add up to S_n, and a later X_k is at most P_n <= S_n / W where that is
+//     kept and less than c where not.  S_n is off by at most c (1 + S_n) (1 + T / W), the logit
+//     scale (sqrt(2) + 1) (sqrt(1 + S_n) - 1) by 1.21 scale sqrt(1 + W) times c (1 + T / W).
+// With c = 2^-30 / max(exp(m) (W + 2), (1 + T / W) (1 + 1.21 scale sqrt(1 + W))) all of it stays below a 64th
+// of a last bit of the diagonal's largest term in float32.  (Products below exp(-88) are zero in float32 with
+// flush-to-zero anyway.)
 // Why drop any: live products keep the second sweep on its float64 path, and the horizon of 32 tokens with
-// m = 3 has a typical product of exp(-50).  1 x 256 x 4 float32, W = 32: 187 us a step against 297 with
-// every product above exp(-88); packed 3001 x 16 bfloat16: 296 against 399.  The error against float64 is
-// the same within 0.5 % in both (1 x 256 x 4 float32: 1.04 and 1.05e-6 for dQ, 2.74 and 2.76e-6 for dK).
+// m = 3 has a typical product of exp(-50).  1 x 256 x 4 float32, W = 32: 176 us a step against 297 with
+// every product above exp(-88); packed 3001 x 16 bfloat16: 284 against 399.  The error against float64 is
+// the same within 0.6 % in both (1 x 256 x 4 float32: 1.04 and 1.05e-6 for dQ, 2.74 and 2.76e-6 for dK).
 int window_cutoff(float mismatch_scale, int D, int64_t W, int64_t T, float scale) {
-  const double lim = 29.0 * std::log(2.0) + mismatch_scale + std::log((double)W + 2.0) + std::log((double)T) +
-                     std::log1p((double)scale * 1.21);
+  const double adjoint = mismatch_scale + std::log((double)W + 2.0);
+  const double evidence = std::log1p((double)T / W) + std::log1p(1.21 * scale * std::sqrt(1.0 + W));
+  const double lim = 30.0 * std::log(2.0) + std::max(adjoint, evidence);
   const double sum = std::min(88.0, lim) * D / mismatch_scale;
   return sum < 1.0e9 ? (int)sum : 1000000000;
 }
