@@ -609,8 +609,8 @@ def rooflines(case, timing, peaks, name):
     s = 2 if cfg["dtype"] not in ("float32",) else 4
     per_unit = (80 if case.kind == "inference" else 12 if case.kind == "stream" else
                 2 * cfg["D"] * s + cfg["Dv"] * s * cfg["Hv"] / cfg["H"] + cfg["Dv"] * s + 8)
-    names = ("pack_symbols", "transpose_symbols", "chain_index", "hard_match", "hard_match_bits",
-             "hard_match_scan", "stream_append", "stream_index", "stream_match", "stream_step")
+    names = ("pack_symbols", "transpose_symbols", "chain_index", "hard_match", "hard_match_runs",
+             "stream_append", "stream_index", "stream_match", "stream_step")
     fwd_ms = sum(kernels.get(n, (0.0, 0))[0] for n in names) / steps
     hbm_peak = peaks.get("hbm_gbs", 6650.0)
     gbs = per_unit * case.local_units / (fwd_ms / 1e3) / 1e9 if fwd_ms else None
@@ -619,7 +619,7 @@ def rooflines(case, timing, peaks, name):
         "frac": (gbs / hbm_peak) if gbs else None, "forward_ms": fwd_ms,
         "bytes_per_token_head": per_unit,
         "kernels": ("stream_append+index+match" if case.kind == "stream" else
-                    "pack_symbols+chain_index+hard_match(+bits/scan of rows on long chains)")}
+                    "pack_symbols+chain_index+hard_match(+runs of rows on long chains)")}
     return out
 
 

@@ -24,7 +24,7 @@ static_assert(32 * kChainIndexWarps * kChainIndexRegisters <= 65536, "more regis
 
 inline int chain_segments(int64_t heads, int64_t positions, size_t set_bytes, int context) {
   int n = 1;
-  while (n < 8 && heads * n * 2 <= 148 * 8 && positions >= 256 * n * 2 &&
+  while (n < 8 && heads * n * 2 <= kSMs * 8 && positions >= 256 * n * 2 &&
          (size_t)n * 2 * set_bytes <= kChainSharedBytes && context * n * 2 <= kChainIndexWarps)
     n *= 2;
   return n;
@@ -548,8 +548,8 @@ int launch_run_match_t(Axis axis, const Sym* q, const Sym* k, int64_t N, int H, 
                        const int32_t* run_flag, Emit emit, cudaStream_t stream) {
   ProfileScope prof("hard_match_runs", stream);
   // launched whether or not a row gave up; short tiles where the tall ones would not fill the GPU
-  const int tile_rows = (N + kRunRows - 1) / kRunRows * H < 148 * 2 ? 64 : kRunRows;
-  run_match_kernel<Sym, Axis, Emit><<<148 * 2, kRunRows, 0, stream>>>(axis, q, k, N, H, W, tile_rows,
+  const int tile_rows = (N + kRunRows - 1) / kRunRows * H < kSMs * 2 ? 64 : kRunRows;
+  run_match_kernel<Sym, Axis, Emit><<<kSMs * 2, kRunRows, 0, stream>>>(axis, q, k, N, H, W, tile_rows,
                                                                       run_flag, emit);
   ROSA_CUDA_OK(cudaGetLastError());
   return 0;

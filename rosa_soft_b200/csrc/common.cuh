@@ -294,6 +294,8 @@ struct ProfileScope {
     }                                                                             \
   } while (0)
 
+constexpr int kSMs = 148;      // of a B200
+
 // Lets a kernel (without static shared memory) be launched with any amount a block may have.  The limit
 // belongs to the function and the device, not to the call: set to what one call needs, it would refuse
 // the launch of a larger call that another thread has just set it for.

@@ -100,7 +100,7 @@ inline float vjp_fill(const VjpArgs& a) {
   int64_t longest = a.plan.cu_seqlens == nullptr ? a.plan.uniform_len : 2 * N / S;
   longest = longest < 2 ? 2 : longest > N ? N : longest;
   const float items = (float)vjp_bands(longest) / (float)a.bands_per_item;
-  return (float)a.H * (float)N / (float)longest * 0.5f * (items + 1.0f) / 148.0f;
+  return (float)a.H * (float)N / (float)longest * 0.5f * (items + 1.0f) / kSMs;
 }
 
 }  // namespace

@@ -593,16 +593,17 @@ int launch_s1_tiled_r(const VjpArgs& a, unsigned grid, cudaStream_t stream) {
 // Diagonals per thread.  Four share the most work (row values, column loads, row reductions), but a
 // CTA is then two warps that need 7 us for a block of 16 rows; two or one have more warps work on a
 // block.  Where the longest item decides that is the faster way (time with four / two / one):
-//   1 x 256 x 4 float32 (fill 0.03)                    52 / 44 / 39 us
-//   1 x 4096 x 16 (fill 0.9)                          1219 / 807 / 782 us
-//   packed 3001 x 16, sequences up to 257             165 / 100 / 79 us
-//   2 x 1024 x 64 (fill 2.2)                          472 / 329 / 370 us
-//   4 x 1024 x 64 (fill 4.3)                          599 / 548 / 642 us
-//   2 x 4096 x 64 (fill 7.4)                          3.01 / 3.06 / 3.98 ms
-//   16 x 8192 x 64 in slices (fill 14)                76.1 / 81.1 / 111 ms
+//   1 x 256 x 4 float32 (fill 0.03)                    56 / 53 / 44 us
+//   1 x 4096 x 16 (fill 0.9)                          1192 / 856 / 793 us
+//   packed 3001 x 16, sequences up to 257             153 / 107 / 84 us
+//   2 x 1024 x 64 (fill 2.2)                          451 / 347 / 358 us
+//   4 x 1024 x 64 (fill 4.3)                          592 / 584 / 647 us
+//   32 x 256 x 32 (fill 6.9)                          250 / 255 / 312 us
+//   2 x 4096 x 64 (fill 7.4)                          2.76 / 2.86 / 3.66 ms
+//   2 x 8192 x 64 (fill 14)                           9.48 / 10.4 / 13.7 ms
 // Value rows of more than 16 components (two sign tables) never take four: their column windows and
 // four sets of diagonals leave no registers to overlap anything (packed 32768 x 16, 32 components:
-// 14.0 / 8.1 / 10.2 ms).
+// 14.0 / 8.2 / 10.2 ms).
 template <int NG>
 int launch_s1_tiled(const VjpArgs& a, unsigned grid, cudaStream_t stream) {
   const float fill = vjp_fill(a);
