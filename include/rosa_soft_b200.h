@@ -117,9 +117,8 @@ ROSA_B200_API int rosa_b200_hard_forward_packed(
  * `stream` by each call, and calls that overlap on the same GPU race -- order them.
  * An inconsistent `cu_seqlens` makes the call a no-op with zero outputs, like the workspace
  * variant; rosa_b200_read_status(NULL, stream, &status) reports it.  The variant always uses
- * the run-length matcher (one symbol compare per causal pair): it has no room for the
- * occurrence bitmaps of the bit-parallel matchers, so on symbols of up to 8 bits it is several
- * times slower than rosa_b200_hard_forward; results are identical. */
+ * the run-length matcher (one symbol compare per causal pair): it has no room for the chains of
+ * rosa_b200_hard_forward and is many times slower; results are identical. */
 ROSA_B200_API int rosa_b200_hard_forward_static(
     const void* query, const void* key, const void* value, int dtype, int64_t N, int H, int D,
     int Hv, int Dv, const int32_t* cu_seqlens, int64_t num_seq, int64_t uniform_len,

@@ -1,5 +1,5 @@
-// Bit-parallel latest-longest suffix matcher for symbols of at most 8 bits, shared by the
-// training forward (hard_forward.cu) and the streaming runtime (stream_runtime.cu).
+// Bit-parallel latest-longest suffix matcher for symbols of at most 8 bits, of the streaming update
+// whose state is bitmaps (stream_runtime.cu).
 //
 // The key stream of a head is kept as one occurrence bitmap per symbol: bit g of E[s] is set
 // iff the key symbol at position g is s.  For a query row i the positions whose last L symbols
